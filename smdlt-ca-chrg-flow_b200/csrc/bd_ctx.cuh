@@ -193,9 +193,10 @@ struct bd_ctx {
   int pme_plan_f, pme_plan_b;
   int pme_mplan_k[4], pme_mplan_f[4];  // packed-pair transforms for k right-hand sides
   int rl_cap, rl_ncell_cap;  // real-space pair rows
-  int *rl_cnt, *rl_rows, *rl_cell_of, *rl_beads, *rl_cell_count, *rl_cell_start, *rl_cursor;
+  int *rl_cnt, *rl_rows, *rl_cell_of, *rl_cell_count, *rl_cell_start, *rl_cursor;
   int *rl_need;      // longest pair row of the last build that overflowed the cap (0: none)
   void *rl_pos;      // lab-frame positions of the last preparation (double4)
+  void *rl_spos;     // the same in real-space cell order, bead index in w
   float *pme_vpk;    // FP32 block products: per packed pair and bead the pair's
                      // 6 input values (+2 padding), written by the spread
   void *rl_tt;       // per pair t1 and t2 / r^2 of the real-space tensor (FP64 or FP32)

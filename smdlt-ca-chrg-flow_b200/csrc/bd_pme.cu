@@ -38,6 +38,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "bd_ctx.cuh"
@@ -356,50 +357,45 @@ __global__ void k_pme_apply_influence(const R* __restrict__ infl, Cx* spec, size
 }
 
 // Real-space Beenakker kernel t1 I + t2 r r^T/r^2 (shear/src/main26.c:
-// 1727-1741) at split parameter alpha; with far the r > 2 form at any r.
-__device__ __forceinline__ void real_kernel(double alpha, double rr, bool far, double& t1,
-                                            double& t2) {
-  double r = sqrt(rr), a = alpha, a2 = a * a, a3 = a2 * a, a5 = a3 * a2, a7 = a5 * a2;
+// 1727-1741) at split parameter alpha; with FAR the r > 2 form at any r.  irr
+// = 1/rr and ir = 1/r are formed once by the caller: a double division costs
+// as much as ten multiplications, and the terms hold eight of them.
+template <bool FAR>
+__device__ __forceinline__ void real_kernel(double alpha, double rr, double r, double ir,
+                                            double irr, double& t1, double& t2) {
+  double a = alpha, a2 = a * a, a3 = a2 * a, a5 = a3 * a2, a7 = a5 * a2;
   double C1, C2, C3, C4;
-  if (far || r > 2.0) {
-    C1 = 0.75 / r + 0.5 / (r * rr);
-    C2 = 4.0 * a7 * rr * rr + 3.0 * a3 * rr - 20.0 * a5 * rr - 4.5 * a + 14.0 * a3 + a / rr;
-    C3 = 0.75 / r - 1.5 / (r * rr);
-    C4 = -4.0 * a7 * rr * rr - 3.0 * a3 * rr + 16.0 * a5 * rr + 1.5 * a - 2.0 * a3 - 3.0 * a / rr;
+  if (FAR || r > 2.0) {
+    C1 = ir * (0.75 + 0.5 * irr);
+    C2 = 4.0 * a7 * rr * rr + 3.0 * a3 * rr - 20.0 * a5 * rr - 4.5 * a + 14.0 * a3 + a * irr;
+    C3 = ir * (0.75 - 1.5 * irr);
+    C4 = -4.0 * a7 * rr * rr - 3.0 * a3 * rr + 16.0 * a5 * rr + 1.5 * a - 2.0 * a3 -
+         3.0 * a * irr;
   } else {
     C1 = 1.0 - 0.28125 * r;
     C2 = 64.0 * a7 + 12.0 * a3 - 80.0 * a5 - 4.5 * a + 14.0 * a3 + 0.25 * a;
     C3 = 0.09375 * r;
     C4 = -64.0 * a7 - 12.0 * a3 + 64.0 * a5 + 1.5 * a - 2.0 * a3 - 0.75 * a;
   }
-  double ec = erfc(a * r), ex = exp(-a2 * rr) / sqrt(M_PI);
+  const double irtpi = 0.56418958354775628695;  // 1/sqrt(pi)
+  double ec = erfc(a * r), ex = exp(-a2 * rr) * irtpi;
   t1 = C1 * ec + C2 * ex;
   t2 = C3 * ec + C4 * ex;
 }
 
-// The overlap branch (bonded and touching beads), kept out of line.
-__device__ __noinline__ void overlap_terms(double alpha, double alpha_ref, double rr,
-                                           double* t) {
-  double f1, f2, o1, o2, g1, g2;
-  real_kernel(alpha, rr, true, f1, f2);
-  real_kernel(alpha_ref, rr, false, o1, o2);
-  real_kernel(alpha_ref, rr, true, g1, g2);
-  t[0] = f1 + (o1 - g1);
-  t[1] = f2 + (o2 - g2);
-}
-
 // t1, t2 of the real-space pair tensor at split alpha, with calcHI's overlap
-// convention for r < 2 (the far form at alpha plus the overlap correction at
-// its own split parameter alpha_ref).
-__device__ __forceinline__ void pair_terms(double alpha, double alpha_ref, double rr, double& t1,
-                                           double& t2) {
-  if (rr < 4.0) {
-    double t[2];
-    overlap_terms(alpha, alpha_ref, rr, t);
-    t1 = t[0];
-    t2 = t[1];
-  } else {
-    real_kernel(alpha, rr, false, t1, t2);
+// convention for r < 2 (OVERLAP: the far form at alpha plus the overlap
+// correction at its own split parameter alpha_ref).
+template <bool OVERLAP>
+__device__ __forceinline__ void pair_terms(double alpha, double alpha_ref, double rr, double r,
+                                           double ir, double irr, double& t1, double& t2) {
+  real_kernel<OVERLAP>(alpha, rr, r, ir, irr, t1, t2);
+  if constexpr (OVERLAP) {
+    double o1, o2, g1, g2;
+    real_kernel<false>(alpha_ref, rr, r, ir, irr, o1, o2);
+    real_kernel<true>(alpha_ref, rr, r, ir, irr, g1, g2);
+    t1 += o1 - g1;
+    t2 += o2 - g2;
   }
 }
 
@@ -702,78 +698,164 @@ __global__ void k_rl_scan(int ncell, int* cell_count, int* cell_start, int* curs
   if (t == nt - 1) cell_start[ncell] = part[t];
 }
 
+// Positions in cell order, the bead index in the fourth component: the row
+// build streams a cell's beads with one contiguous load each.
 __global__ void k_rl_fill(const int* __restrict__ cell_of, const int* __restrict__ cell_start,
-                          int* cursor, int* beads, int N) {
+                          int* cursor, const double4* __restrict__ pos, double4* spos, int N) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   int c = cell_of[i];
-  beads[cell_start[c] + atomicAdd(&cursor[c], 1)] = i;
+  double4 p = pos[i];
+  p.w = __longlong_as_double((long long)i);
+  spos[cell_start[c] + atomicAdd(&cursor[c], 1)] = p;
 }
 
 // Pairs within rc (lattice minimum image): rows of bead indices and, per
-// pair, t1 and t2 / r^2 of the real-space tensor.
+// pair, the stored tensor: (t1, w) where the products read it (rw, FP32 block
+// contexts), else t1 and t2 / r^2.
+// One warp per bead.  The at most 27 neighbour cells form one candidate list
+// (lane l takes cell l's range, a warp scan places candidate m); the lanes
+// test 32 candidates at a time and queue the hits in shared memory, and the
+// pair terms (erfc, exp: most of the FP64 work, needed by about one candidate
+// in eight) are formed 32 queued pairs at a time, so no lane idles in them
+// and the row's stores are contiguous.  Overlapping pairs, whose terms cost
+// three times as much, have a queue of their own.  Bound by the FP64 pipe:
+// 193 M tests and 24 M pair terms at 50 000 beads, cutoff 14.5.  A thread per
+// bead, with its stores a row apart, took 6.01 ms there; this takes 1.33 ms.
 template <typename R>
-__global__ void k_rl_rows(Cell cell, RGeom g, const double4* __restrict__ pos, int N,
-                          const int* __restrict__ cell_start, const int* __restrict__ beads,
-                          double rc2, double alpha, double alpha_ref, int rcap, int* cnt,
-                          int* rows, R* tt, float4* rw, int* need, int* err) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256, 3)
+    k_rl_rows(Cell cell, RGeom g, const double4* __restrict__ pos, int N,
+              const int* __restrict__ cell_start, const double4* __restrict__ spos, double rc2,
+              double alpha, double alpha_ref, int rcap, int* cnt, int* rows, R* tt, float4* rw,
+              int* need, int* err) {
+  __shared__ int c_start[8][32], c_excl[8][32], c_incl[8][32], c_queue[8][2][64];
+  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * 8 + wl;
   if (i >= N) return;
-  double4 p = pos[i];
-  int cd[3];
+  const double4 p = pos[i];
+  int cd[3], lo[3], nd[3];
   rcell(cell, g, p.x, p.y, p.z, cd);
-  int lo[3], hi[3];
+#pragma unroll
   for (int d = 0; d < 3; d++) {
     lo[d] = g.n[d] >= 3 ? -1 : 0;
-    hi[d] = g.n[d] >= 3 ? 1 : g.n[d] - 1;
+    nd[d] = g.n[d] >= 3 ? 3 : g.n[d];
   }
-  int n = 0, nall = 0;
-  bool over = false;
-  for (int a = lo[0]; a <= hi[0]; a++)
-    for (int b = lo[1]; b <= hi[1]; b++)
-      for (int c = lo[2]; c <= hi[2]; c++) {
-        int e0 = g.n[0] >= 3 ? (cd[0] + a + g.n[0]) % g.n[0] : a;
-        int e1 = g.n[1] >= 3 ? (cd[1] + b + g.n[1]) % g.n[1] : b;
-        int e2 = g.n[2] >= 3 ? (cd[2] + c + g.n[2]) % g.n[2] : c;
-        int cc = (e0 * g.n[1] + e1) * g.n[2] + e2;
-        for (int q = cell_start[cc]; q < cell_start[cc + 1]; q++) {
-          int j = beads[q];
-          if (j == i) continue;
-          double4 pj = pos[j];
-          double dx = pj.x - p.x, dy = pj.y - p.y, dz = pj.z - p.z, s[3];
-          frac_of(cell, dx, dy, dz, s);
-          for (int d = 0; d < 3; d++) s[d] -= rint(s[d]);
-          dx = cell.H[0] * s[0] + cell.H[1] * s[1] + cell.H[2] * s[2];
-          dy = cell.H[3] * s[0] + cell.H[4] * s[1] + cell.H[5] * s[2];
-          dz = cell.H[6] * s[0] + cell.H[7] * s[1] + cell.H[8] * s[2];
-          double rr = dx * dx + dy * dy + dz * dz;
-          if (rr >= rc2) continue;
-          if (n >= rcap) {
-            over = true;
-            nall++;
-            continue;
-          }
-          double t1, t2;
-          pair_terms(alpha, alpha_ref, rr, t1, t2);
-          rows[(size_t)i * rcap + n] = j;
-          tt[2 * ((size_t)i * rcap + n)] = (R)t1;
-          tt[2 * ((size_t)i * rcap + n) + 1] = (R)(t2 / rr);
-          if (rw) {
-            double sw = sqrt(fabs(t2 / rr));
-            unsigned b = (__float_as_uint((float)t1) & ~1u) | (t2 < 0.0 ? 1u : 0u);
-            rw[(size_t)i * rcap + n] =
-                make_float4(__uint_as_float(b), (float)(sw * dx), (float)(sw * dy), (float)(sw * dz));
-          }
-          n++;
-          nall++;
-        }
-      }
-  cnt[i] = n;
-  if (over) {
-    if (need)
-      atomicMax(need, nall);  // the host grows the rows and builds them again
-    else
-      atomicOr(err, ERRB_NBR_OVERFLOW);
+  int my_s = 0, my_n = 0;
+  if (lane < nd[0] * nd[1] * nd[2]) {
+    int a = lo[0] + lane / (nd[1] * nd[2]), b = lo[1] + (lane / nd[2]) % nd[1],
+        c = lo[2] + lane % nd[2];
+    int e0 = g.n[0] >= 3 ? (cd[0] + a + g.n[0]) % g.n[0] : a;
+    int e1 = g.n[1] >= 3 ? (cd[1] + b + g.n[1]) % g.n[1] : b;
+    int e2 = g.n[2] >= 3 ? (cd[2] + c + g.n[2]) % g.n[2] : c;
+    int cc = (e0 * g.n[1] + e1) * g.n[2] + e2;
+    my_s = cell_start[cc];
+    my_n = cell_start[cc + 1] - my_s;
+  }
+  int incl = my_n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  c_start[wl][lane] = my_s;
+  c_excl[wl][lane] = incl - my_n;
+  c_incl[wl][lane] = incl;
+  __syncwarp();
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  // displacement to a bead, minimum image; the cell is (b1, b2) in the xy
+  // plane and L e_z, and the nearest integer of |s| < 2^51 comes from adding
+  // and subtracting 1.5 2^52 (two additions for one slow conversion)
+  const double h00 = cell.H[0], h01 = cell.H[1], h10 = cell.H[3], h11 = cell.H[4];
+  const double g00 = cell.Hi[0], g01 = cell.Hi[1], g10 = cell.Hi[3], g11 = cell.Hi[4];
+  const double Lz = cell.H[8], iLz = cell.Hi[8];
+  auto nearest = [](double s) {
+    return __dsub_rn(__dadd_rn(s, 6755399441055744.0), 6755399441055744.0);
+  };
+  auto image = [&](const double4& pj, double& dx, double& dy, double& dz) {
+    dx = pj.x - p.x, dy = pj.y - p.y, dz = pj.z - p.z;
+    double n0 = nearest(g00 * dx + g01 * dy), n1 = nearest(g10 * dx + g11 * dy),
+           n2 = nearest(iLz * dz);
+    dx -= h00 * n0 + h01 * n1;
+    dy -= h10 * n0 + h11 * n1;
+    dz -= Lz * n2;
+    return dx * dx + dy * dy + dz * dz;
+  };
+  // pair terms of the first nq pairs of a queue into the row from entry n on
+  auto emit = [&](auto overlap, int n, int nq) {
+    constexpr bool OV = decltype(overlap)::value;
+    if (lane >= nq || n + lane >= rcap) return;
+    double4 pj = spos[c_queue[wl][OV][lane]];
+    int j = (int)__double_as_longlong(pj.w);
+    double dx, dy, dz, t1, t2, rr = image(pj, dx, dy, dz);
+    double r = sqrt(rr), ir = 1.0 / r, irr = ir * ir;
+    pair_terms<OV>(alpha, alpha_ref, rr, r, ir, irr, t1, t2);
+    size_t e = (size_t)i * rcap + n + lane;
+    rows[e] = j;
+    if (rw) {
+      double sw = sqrt(fabs(t2)) * ir;
+      unsigned b = (__float_as_uint((float)t1) & ~1u) | (t2 < 0.0 ? 1u : 0u);
+      rw[e] = make_float4(__uint_as_float(b), (float)(sw * dx), (float)(sw * dy),
+                          (float)(sw * dz));
+    } else {
+      tt[2 * e] = (R)t1;
+      tt[2 * e + 1] = (R)(t2 * irr);
+    }
+  };
+  int n = 0, nq0 = 0, nq1 = 0, cl = 0;
+  // appends the hits of one kind to their queue; a full batch goes to the row
+  auto push = [&](auto overlap, bool in, int j, int& nq) {
+    constexpr bool OV = decltype(overlap)::value;
+    unsigned hit = __ballot_sync(0xffffffffu, in);
+    if (hit == 0) return;
+    int* queue = c_queue[wl][OV];
+    if (in) queue[nq + __popc(hit & ((1u << lane) - 1u))] = j;
+    nq += __popc(hit);
+    __syncwarp();
+    if (nq >= 32) {
+      emit(overlap, n, 32);
+      n += 32;
+      nq -= 32;
+      __syncwarp();
+      int rest = lane < nq ? queue[32 + lane] : 0;
+      __syncwarp();
+      if (lane < nq) queue[lane] = rest;
+      __syncwarp();
+    }
+  };
+  // the next candidate's load is in flight while this one is tested
+  int at = -1, next_at = -1;
+  double4 pj = p, next = p;
+  auto fetch = [&](int m) {
+    next_at = -1;
+    if (m < total) {
+      while (m >= c_incl[wl][cl]) cl++;  // ends at the last cell: m < total
+      next_at = c_start[wl][cl] + (m - c_excl[wl][cl]);
+      next = spos[next_at];
+    }
+  };
+  fetch(lane);
+  for (int m0 = 0; m0 < total; m0 += 32) {
+    at = next_at;
+    pj = next;
+    fetch(m0 + 32 + lane);
+    double dx, dy, dz, rr = image(pj, dx, dy, dz);
+    bool in = at >= 0 && !(rr >= rc2) && (int)__double_as_longlong(pj.w) != i;
+    bool near = rr < 4.0;
+    push(std::integral_constant<bool, false>(), in && !near, at, nq0);
+    push(std::integral_constant<bool, true>(), in && near, at, nq1);
+  }
+  emit(std::integral_constant<bool, false>(), n, nq0);
+  n += nq0;
+  emit(std::integral_constant<bool, true>(), n, nq1);
+  n += nq1;
+  if (lane == 0) {
+    cnt[i] = min(n, rcap);
+    if (n > rcap) {
+      if (need)
+        atomicMax(need, n);  // the host grows the rows and builds them again
+      else
+        atomicOr(err, ERRB_NBR_OVERFLOW);
+    }
   }
 }
 
@@ -816,18 +898,20 @@ int pme_alloc(bd_ctx* c) {
     CU(cudaMalloc(&c->pme_rsum, 48 * (size_t)N * ((nr + 1) / 2)));
     CU(cudaMalloc(&c->rl_w, 16 * (size_t)N * c->rl_cap));
     c->bytes += 80 * (size_t)N * ((nr + 1) / 2) + 16 * (size_t)N * c->rl_cap;
+  } else {  // the products of contexts with rl_w read the pair tensors there
+    CU(cudaMalloc(&c->rl_tt, 2 * es * (size_t)N * c->rl_cap));
+    c->bytes += 2 * es * (size_t)N * c->rl_cap;
   }
-  CU(cudaMalloc(&c->rl_tt, 2 * es * (size_t)N * c->rl_cap));
   c->rl_ncell_cap = 4096;
   CU(cudaMalloc(&c->rl_cell_of, 4 * (size_t)N));
-  CU(cudaMalloc(&c->rl_beads, 4 * (size_t)N));
+  CU(cudaMalloc(&c->rl_spos, 32 * (size_t)N));
   CU(cudaMalloc(&c->rl_cell_count, 4 * (size_t)c->rl_ncell_cap));
   CU(cudaMalloc(&c->rl_cell_start, 4 * (size_t)(c->rl_ncell_cap + 1)));
   CU(cudaMalloc(&c->rl_cursor, 4 * (size_t)c->rl_ncell_cap));
   CU(cudaMemsetAsync(c->rl_cell_count, 0, 4 * (size_t)c->rl_ncell_cap, c->stream));
   c->bytes += es * (3 * K3 * nr + 6 * Ks) + spec_bytes + 24 * (size_t)K + 12 * (size_t)N +
-              24 * (size_t)N * kMaxOrder + 4 * (size_t)N + (size_t)N * c->rl_cap * (4 + 2 * es) + 32 * (size_t)N +
-              8 * (size_t)N + 12 * (size_t)c->rl_ncell_cap;
+              24 * (size_t)N * kMaxOrder + 4 * (size_t)N + (size_t)N * c->rl_cap * 4 + 32 * (size_t)N +
+              36 * (size_t)N + 12 * (size_t)c->rl_ncell_cap;
   int n[3] = {K, K, K};
   cufftHandle f, b;
   CF(cufftPlanMany(&f, 3, n, nullptr, 1, (int)K3, nullptr, 1, (int)Ks,
@@ -887,7 +971,7 @@ void pme_free(bd_ctx* c) {
       c->pme_mplan_k[q] = 0;
     }
   void* ptrs[] = {c->pme_vpk, c->pme_rsum, c->rl_w, c->rl_need, c->pme_grid, c->pme_spec, c->pme_infl, c->pme_bsq, c->pme_soff, c->pme_base, c->pme_w,
-                  c->rl_cnt, c->rl_rows, c->rl_pos, c->rl_tt, c->rl_cell_of, c->rl_beads, c->rl_cell_count,
+                  c->rl_cnt, c->rl_rows, c->rl_pos, c->rl_tt, c->rl_cell_of, c->rl_spos, c->rl_cell_count,
                   c->rl_cell_start, c->rl_cursor};
   for (void* q : ptrs)
     if (q) cudaFree(q);
@@ -903,12 +987,15 @@ static int rl_grow(bd_ctx* c, int cap) {
   size_t N = c->N, es = c->pme_f32 ? 4 : 8, old = (size_t)c->rl_cap;
   CU(cudaStreamSynchronize(c->stream));
   cudaFree(c->rl_rows);
-  cudaFree(c->rl_tt);
   c->rl_rows = nullptr;
-  c->rl_tt = nullptr;
   CU(cudaMalloc(&c->rl_rows, 4 * N * cap));
-  CU(cudaMalloc(&c->rl_tt, 2 * es * N * cap));
-  c->bytes += (4 + 2 * es) * N * (cap - old);
+  c->bytes += 4 * N * (cap - old);
+  if (c->rl_tt) {
+    cudaFree(c->rl_tt);
+    c->rl_tt = nullptr;
+    CU(cudaMalloc(&c->rl_tt, 2 * es * N * cap));
+    c->bytes += 2 * es * N * (cap - old);
+  }
   if (c->rl_w) {
     cudaFree(c->rl_w);
     c->rl_w = nullptr;
@@ -974,19 +1061,22 @@ int pme_prepare(bd_ctx* c, const Lat& l) {
                                                   c->rl_cell_of, c->rl_cell_count);
   k_rl_scan<<<1, 1024, 0, c->stream>>>(ncell, c->rl_cell_count, c->rl_cell_start, c->rl_cursor);
   k_rl_fill<<<nblk(N, 256), 256, 0, c->stream>>>(c->rl_cell_of, c->rl_cell_start, c->rl_cursor,
-                                                 c->rl_beads, N);
+                                                 (const double4*)c->rl_pos,
+                                                 (double4*)c->rl_spos, N);
   if ((s = launch_ok(c)) != BD_OK) return s;
   // the pair rows; with the default cap (no pme_max_pairs), rows that
   // overflow it are grown to 1.25 times the longest row and built again
   int* need = c->p.pme_max_pairs > 0 ? nullptr : c->rl_need;
   for (int pass = 0; pass < 2; pass++) {
     if (c->pme_f32)
-      k_rl_rows<float><<<nblk(N, 128), 128, 0, c->stream>>>(
-          cell, g, (const double4*)c->rl_pos, N, c->rl_cell_start, c->rl_beads, rc * rc, alpha,
+      k_rl_rows<float><<<nblk(N, 8), 256, 0, c->stream>>>(
+          cell, g, (const double4*)c->rl_pos, N, c->rl_cell_start, (const double4*)c->rl_spos,
+          rc * rc, alpha,
           alpha_ref, c->rl_cap, c->rl_cnt, c->rl_rows, (float*)c->rl_tt, c->rl_w, need, c->err);
     else
-      k_rl_rows<double><<<nblk(N, 128), 128, 0, c->stream>>>(
-          cell, g, (const double4*)c->rl_pos, N, c->rl_cell_start, c->rl_beads, rc * rc, alpha,
+      k_rl_rows<double><<<nblk(N, 8), 256, 0, c->stream>>>(
+          cell, g, (const double4*)c->rl_pos, N, c->rl_cell_start, (const double4*)c->rl_spos,
+          rc * rc, alpha,
           alpha_ref, c->rl_cap, c->rl_cnt, c->rl_rows, (double*)c->rl_tt, nullptr, need, c->err);
     if (!need) break;
     int longest = 0;
