@@ -64,6 +64,71 @@ __device__ __forceinline__ void bspline_t(double f, double* w) {
   for (int k = 0; k < P; k++) w[k] = a[k];
 }
 
+// The at most 27 neighbour cells of one cell as a single candidate list for a
+// warp: lane l < ncell takes cell l's range, a warp scan of the counts places
+// candidate m in the cell whose range holds it, so the lanes walk all cells
+// at once (no chain of dependent loads per cell).  The arrays are the warp's
+// own shared memory.
+struct CandList {
+  int start[32], excl[32], incl[32];
+
+  // n cells per direction, cd the cell, cell_start the ranges; returns the
+  // number of candidates (every lane)
+  __device__ __forceinline__ int open(const int* n, const int* cd,
+                                      const int* __restrict__ cell_start) {
+    int lane = threadIdx.x & 31, lo[3], nd[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      lo[d] = n[d] >= 3 ? -1 : 0;
+      nd[d] = n[d] >= 3 ? 3 : n[d];
+    }
+    int my_s = 0, my_n = 0;
+    if (lane < nd[0] * nd[1] * nd[2]) {
+      int a = lo[0] + lane / (nd[1] * nd[2]), b = lo[1] + (lane / nd[2]) % nd[1],
+          c = lo[2] + lane % nd[2];
+      int e0 = n[0] >= 3 ? (cd[0] + a + n[0]) % n[0] : a;
+      int e1 = n[1] >= 3 ? (cd[1] + b + n[1]) % n[1] : b;
+      int e2 = n[2] >= 3 ? (cd[2] + c + n[2]) % n[2] : c;
+      int cc = (e0 * n[1] + e1) * n[2] + e2;
+      my_s = cell_start[cc];
+      my_n = cell_start[cc + 1] - my_s;
+    }
+    int in = my_n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      int t = __shfl_up_sync(0xffffffffu, in, o);
+      if (lane >= o) in += t;
+    }
+    __syncwarp();  // the previous list has been read
+    start[lane] = my_s;
+    excl[lane] = in - my_n;
+    incl[lane] = in;
+    __syncwarp();
+    return __shfl_sync(0xffffffffu, in, 31);
+  }
+
+  // place of candidate m < total; cl is the lane's cursor, 0 before its first
+  // candidate, candidates in increasing order
+  __device__ __forceinline__ int at(int m, int& cl) const {
+    while (m >= incl[cl]) cl++;  // ends at the last cell: m < total
+    return start[cl] + (m - excl[cl]);
+  }
+};
+
+// Cell of a lab-frame position (0 for non-finite input).
+__device__ __forceinline__ int cell_of_pos(const Cell& cell, const int* n, double x, double y,
+                                           double z, int* cd) {
+  double s[3];
+  frac_of(cell, x, y, z, s);
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    double sd = s[d] - floor(s[d]);
+    int c = (sd >= 0.0 && sd <= 1.0) ? (int)(sd * n[d]) : 0;
+    cd[d] = c >= n[d] ? n[d] - 1 : c;
+  }
+  return (cd[0] * n[1] + cd[1]) * n[2] + cd[2];
+}
+
 static inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 
 // Lab-frame cell of the current lattice: columns b1, b2, L e_z with (b1, b2)

@@ -813,6 +813,7 @@ int bd_destroy(bd_ctx* c) {
     if (q) cudaFree(q);
   pme_free(c);
   coulomb_free(c);
+  if (c->hop_work) cudaFree(c->hop_work);
   if (c->hop_cells) cudaFree(c->hop_cells);
   if (c->hop_de) cudaFree(c->hop_de);
   if (c->cb_part) cudaFree(c->cb_part);

@@ -244,12 +244,19 @@ __global__ void k_cc_scan(int ncell, int* count, int* start, int* cursor) {
   if (t == nt - 1) start[ncell] = part[t];
 }
 
+// The charges in cell order: index, and lab-frame position with the charge.
 __global__ void k_cc_fill(const int* __restrict__ cell_of, const int* __restrict__ start,
-                          int* cursor, int* idx, int nch) {
+                          int* cursor, const double4* __restrict__ cq, double cr, double sr,
+                          int* idx, double4* sorted, int nch) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nch) return;
   int c = cell_of[k];
-  idx[start[c] + atomicAdd(&cursor[c], 1)] = k;
+  int at = start[c] + atomicAdd(&cursor[c], 1);
+  double4 q = cq[k];
+  double x, y;
+  lab_of(q.x, q.y, cr, sr, x, y);
+  idx[at] = k;
+  sorted[at] = make_double4(x, y, q.z, q.w);
 }
 
 // Forces on each charge: reciprocal part from the potential grid and the
@@ -409,13 +416,14 @@ static int coul_alloc(bd_ctx* c) {
   CU(cudaMalloc(&c->cw_w, 2 * 8 * 3 * (size_t)n * kMaxOrder));
   CU(cudaMalloc(&c->cw_cell_of, 4 * (size_t)n));
   CU(cudaMalloc(&c->cw_idx, 4 * (size_t)n));
+  CU(cudaMalloc(&c->cw_sorted, 32 * (size_t)n));
   CU(cudaMalloc(&c->cw_count, 4 * (size_t)kCellCap));
   CU(cudaMalloc(&c->cw_start, 4 * (size_t)(kCellCap + 1)));
   CU(cudaMalloc(&c->cw_cursor, 4 * (size_t)kCellCap));
   CU(cudaMemsetAsync(c->cw_count, 0, 4 * (size_t)kCellCap, c->stream));
   CU(cudaMemsetAsync(c->cw_energy, 0, 32, c->stream));
   c->bytes += 8 * K3 + 16 * Ks + 24 * (size_t)K + 8 * (size_t)std::max(6 * c->cw_nblk, n) + 32 +
-              (size_t)n * (12 + 48 * kMaxOrder + 8) + 12 * (size_t)kCellCap;
+              (size_t)n * (12 + 48 * kMaxOrder + 40) + 12 * (size_t)kCellCap;
   int dims[3] = {K, K, K};
   cufftHandle f, b;
   CF(cufftPlanMany(&f, 3, dims, nullptr, 1, (int)K3, nullptr, 1, (int)Ks, CUFFT_D2Z, 1));
@@ -437,7 +445,7 @@ void coulomb_free(bd_ctx* c) {
   if (c->cw_plan_f) cufftDestroy((cufftHandle)c->cw_plan_f);
   if (c->cw_plan_b) cufftDestroy((cufftHandle)c->cw_plan_b);
   void* ptrs[] = {c->cw_grid, c->cw_spec, c->cw_bsq, c->cw_epart, c->cw_energy, c->cw_base,
-                  c->cw_w, c->cw_cell_of, c->cw_idx, c->cw_count, c->cw_start, c->cw_cursor};
+                  c->cw_w, c->cw_cell_of, c->cw_idx, c->cw_sorted, c->cw_count, c->cw_start, c->cw_cursor};
   for (void* q : ptrs)
     if (q) cudaFree(q);
 }
@@ -496,6 +504,52 @@ int coulomb_quadform(bd_ctx* c, const Lat& l, double* Q6) {
   return launch_ok(c);
 }
 
+// Cell list of the charges gathered in cq, cells at least coulomb_rc wide: n
+// cells per direction, their ranges in cw_start, the charges in cell order in
+// cw_idx (index) and cw_sorted (lab-frame position, charge).  Any cutoff is
+// served (fewer than three cells in a direction: all are neighbours); *width
+// gets the narrowest cell width of the lattice.
+int coulomb_cells(bd_ctx* c, const Lat& l, const double4* cq, int* n, double* width) {
+  int s, nch = c->nch;
+  if ((s = coul_alloc(c)) != BD_OK) return s;
+  Cell cell = make_cell(l);
+  double cr = 1.0, sr = 0.0;
+  if (l.flow == BD_FLOW_EXT) {
+    cr = l.cth;
+    sr = l.sth;
+  }
+  // widths V / |a_j x a_k| >= rc
+  double wdt[3];
+  for (int j = 0; j < 3; j++) {
+    double a[3][3];
+    for (int q = 0; q < 3; q++)
+      for (int d = 0; d < 3; d++) a[q][d] = cell.H[d * 3 + q];
+    const double* u = a[(j + 1) % 3];
+    const double* v = a[(j + 2) % 3];
+    double cx = u[1] * v[2] - u[2] * v[1], cy = u[2] * v[0] - u[0] * v[2],
+           cz = u[0] * v[1] - u[1] * v[0];
+    wdt[j] = cell.V / sqrt(cx * cx + cy * cy + cz * cz);
+  }
+  double rc = c->cw_rc;
+  if (width) *width = std::min(wdt[0], std::min(wdt[1], wdt[2]));
+  CGeom g;
+  for (int d = 0; d < 3; d++) g.n[d] = std::max(1, (int)floor(wdt[d] / rc));
+  while ((long)g.n[0] * g.n[1] * g.n[2] > kCellCap) {
+    int d = g.n[0] >= g.n[1] && g.n[0] >= g.n[2] ? 0 : (g.n[1] >= g.n[2] ? 1 : 2);
+    g.n[d]--;
+  }
+  for (int d = 0; d < 3; d++) n[d] = g.n[d];
+  int ncell = n[0] * n[1] * n[2];
+  c->launches += 3;
+  k_cc_count<<<nblk(nch, 256), 256, 0, c->stream>>>(cell, g, cq, nch, cr, sr, c->cw_cell_of,
+                                                    c->cw_count);
+  k_cc_scan<<<1, 1024, 0, c->stream>>>(ncell, c->cw_count, c->cw_start, c->cw_cursor);
+  k_cc_fill<<<nblk(nch, 256), 256, 0, c->stream>>>(c->cw_cell_of, c->cw_start, c->cw_cursor, cq,
+                                                   cr, sr, c->cw_idx, (double4*)c->cw_sorted,
+                                                   nch);
+  return launch_ok(c);
+}
+
 // Ewald Coulomb forces for the charges gathered in cq (positions in the frame
 // the force routines receive them: stored frame, rotated to the lab frame by
 // the lattice angle in extension), added to fx, fy, fz; energies into
@@ -510,31 +564,14 @@ int coulomb_ewald(bd_ctx* c, const Lat& l, const double4* cq) {
     cr = l.cth;
     sr = l.sth;
   }
-  // cell list: widths V / |a_j x a_k| >= rc
-  double wdt[3];
-  for (int j = 0; j < 3; j++) {
-    double a[3][3];
-    for (int q = 0; q < 3; q++)
-      for (int d = 0; d < 3; d++) a[q][d] = cell.H[d * 3 + q];
-    const double* u = a[(j + 1) % 3];
-    const double* v = a[(j + 2) % 3];
-    double cx = u[1] * v[2] - u[2] * v[1], cy = u[2] * v[0] - u[0] * v[2],
-           cz = u[0] * v[1] - u[1] * v[0];
-    wdt[j] = cell.V / sqrt(cx * cx + cy * cy + cz * cz);
-  }
-  double rc = c->cw_rc;
-  if (2 * rc > std::min(wdt[0], std::min(wdt[1], wdt[2]))) return BD_ERR_ARG;
   CGeom g;
-  for (int d = 0; d < 3; d++) g.n[d] = std::max(1, (int)floor(wdt[d] / rc));
-  while ((long)g.n[0] * g.n[1] * g.n[2] > kCellCap) {
-    int d = g.n[0] >= g.n[1] && g.n[0] >= g.n[2] ? 0 : (g.n[1] >= g.n[2] ? 1 : 2);
-    g.n[d]--;
-  }
-  int ncell = g.n[0] * g.n[1] * g.n[2];
+  double rc = c->cw_rc, width;
+  if ((s = coulomb_cells(c, l, cq, g.n, &width)) != BD_OK) return s;
+  if (2 * rc > width) return BD_ERR_ARG;
   size_t K3 = (size_t)K * K * K;
   double* w = c->cw_w;
   double* dw = c->cw_w + 3 * (size_t)nch * kMaxOrder;
-  c->launches += 9;
+  c->launches += 6;
 #define CW_WEIGHTS(P_)                                                                      \
   k_cw_weights<P_><<<nblk(3 * (long long)nch, 128), 128, 0, c->stream>>>(cell, cq, nch, cr, sr, K, \
                                                                         c->cw_base, w, dw, c->err)
@@ -552,11 +589,6 @@ int coulomb_ewald(bd_ctx* c, const Lat& l, const double4* cq) {
                                                     c->cw_epart);
   k_sum_into<<<1, 32, 0, c->stream>>>(c->cw_epart, c->cw_nblk, c->cw_energy + 1);
   CF(cufftExecZ2D((cufftHandle)c->cw_plan_b, (cufftDoubleComplex*)c->cw_spec, c->cw_grid));
-  k_cc_count<<<nblk(nch, 256), 256, 0, c->stream>>>(cell, g, cq, nch, cr, sr, c->cw_cell_of,
-                                                    c->cw_count);
-  k_cc_scan<<<1, 1024, 0, c->stream>>>(ncell, c->cw_count, c->cw_start, c->cw_cursor);
-  k_cc_fill<<<nblk(nch, 256), 256, 0, c->stream>>>(c->cw_cell_of, c->cw_start, c->cw_cursor,
-                                                   c->cw_idx, nch);
 #define CW_FORCES(P_)                                                                        \
   k_cw_forces<P_><<<nblk(nch, 8), 256, 0, c->stream>>>(                                       \
       cell, g, cq, c->track, nch, cr, sr, K, c->cw_base, w, dw, c->cw_grid, c->cw_cell_of,    \

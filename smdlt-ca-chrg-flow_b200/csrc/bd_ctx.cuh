@@ -153,6 +153,7 @@ struct bd_ctx {
   // parallel charge-hop sweep
   double hop_R;
   int *hop_cells;
+  double *hop_work;  // scratch of the parallel sweep, 16 N + 8
   double *hop_de;  // energy change of each charge's last parallel-sweep trial
   unsigned long long hop_sweeps;
 
@@ -160,6 +161,7 @@ struct bd_ctx {
   double cw_beta, cw_rc, cw_q2, cw_Q, cw_cell_V;
   double *cw_grid, *cw_bsq, *cw_epart, *cw_energy, *cw_w;
   void *cw_spec;
+  void *cw_sorted;  // charges in cell order: lab-frame position and charge (double4)
   int *cw_base, *cw_cell_of, *cw_idx, *cw_count, *cw_start, *cw_cursor;
   int cw_nblk, cw_plan_f, cw_plan_b;
 
@@ -264,6 +266,7 @@ int ewald_bin(bd_ctx* c, double* eps, std::vector<double>& rowsum);
 // Ewald Coulomb
 int coulomb_ewald(bd_ctx* c, const Lat& l, const double4* cq);
 int coulomb_mesh_potential(bd_ctx* c, const Lat& l, const double4* cq);
+int coulomb_cells(bd_ctx* c, const Lat& l, const double4* cq, int* n, double* width);
 int coulomb_quadform(bd_ctx* c, const Lat& l, double* Q6);
 void coulomb_free(bd_ctx* c);
 

@@ -651,18 +651,6 @@ struct RGeom {
   int n[3];
 };
 
-__device__ __forceinline__ int rcell(const Cell& cell, const RGeom& g, double x, double y, double z,
-                                     int* cd) {
-  double s[3];
-  frac_of(cell, x, y, z, s);
-  for (int d = 0; d < 3; d++) {
-    double sd = s[d] - floor(s[d]);
-    int c = (sd >= 0.0 && sd <= 1.0) ? (int)(sd * g.n[d]) : 0;  // 0 for non-finite input
-    cd[d] = c >= g.n[d] ? g.n[d] - 1 : c;
-  }
-  return (cd[0] * g.n[1] + cd[1]) * g.n[2] + cd[2];
-}
-
 __global__ void k_rl_count(Cell cell, RGeom g, const double* __restrict__ rx,
                            const double* __restrict__ ry, const double* __restrict__ rz,
                            double cr, double sr, int N, int* cell_of, int* cell_count) {
@@ -670,7 +658,7 @@ __global__ void k_rl_count(Cell cell, RGeom g, const double* __restrict__ rx,
   if (i >= N) return;
   int cd[3];
   double x = rx[i] * cr - ry[i] * sr, y = rx[i] * sr + ry[i] * cr;
-  int c = rcell(cell, g, x, y, rz[i], cd);
+  int c = cell_of_pos(cell, g.n, x, y, rz[i], cd);
   cell_of[i] = c;
   atomicAdd(&cell_count[c], 1);
 }
@@ -728,40 +716,15 @@ __global__ void __launch_bounds__(256, 3)
               const int* __restrict__ cell_start, const double4* __restrict__ spos, double rc2,
               double alpha, double alpha_ref, int rcap, int* cnt, int* rows, R* tt, float4* rw,
               int* need, int* err) {
-  __shared__ int c_start[8][32], c_excl[8][32], c_incl[8][32], c_queue[8][2][64];
+  __shared__ CandList c_list[8];
+  __shared__ int c_queue[8][2][64];
   const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = blockIdx.x * 8 + wl;
   if (i >= N) return;
   const double4 p = pos[i];
-  int cd[3], lo[3], nd[3];
-  rcell(cell, g, p.x, p.y, p.z, cd);
-#pragma unroll
-  for (int d = 0; d < 3; d++) {
-    lo[d] = g.n[d] >= 3 ? -1 : 0;
-    nd[d] = g.n[d] >= 3 ? 3 : g.n[d];
-  }
-  int my_s = 0, my_n = 0;
-  if (lane < nd[0] * nd[1] * nd[2]) {
-    int a = lo[0] + lane / (nd[1] * nd[2]), b = lo[1] + (lane / nd[2]) % nd[1],
-        c = lo[2] + lane % nd[2];
-    int e0 = g.n[0] >= 3 ? (cd[0] + a + g.n[0]) % g.n[0] : a;
-    int e1 = g.n[1] >= 3 ? (cd[1] + b + g.n[1]) % g.n[1] : b;
-    int e2 = g.n[2] >= 3 ? (cd[2] + c + g.n[2]) % g.n[2] : c;
-    int cc = (e0 * g.n[1] + e1) * g.n[2] + e2;
-    my_s = cell_start[cc];
-    my_n = cell_start[cc + 1] - my_s;
-  }
-  int incl = my_n;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    int t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
-  c_start[wl][lane] = my_s;
-  c_excl[wl][lane] = incl - my_n;
-  c_incl[wl][lane] = incl;
-  __syncwarp();
-  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  int cd[3];
+  cell_of_pos(cell, g.n, p.x, p.y, p.z, cd);
+  const int total = c_list[wl].open(g.n, cd, cell_start);
   // displacement to a bead, minimum image; the cell is (b1, b2) in the xy
   // plane and L e_z, and the nearest integer of |s| < 2^51 comes from adding
   // and subtracting 1.5 2^52 (two additions for one slow conversion)
@@ -828,8 +791,7 @@ __global__ void __launch_bounds__(256, 3)
   auto fetch = [&](int m) {
     next_at = -1;
     if (m < total) {
-      while (m >= c_incl[wl][cl]) cl++;  // ends at the last cell: m < total
-      next_at = c_start[wl][cl] + (m - c_excl[wl][cl]);
+      next_at = c_list[wl].at(m, cl);
       next = spos[next_at];
     }
   };
