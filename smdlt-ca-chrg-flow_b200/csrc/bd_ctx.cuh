@@ -184,16 +184,16 @@ struct bd_ctx {
   double pme_rc, pme_alpha, pme_self;
   bool pme_ready;
   bool pme_f32;      // grids, spectra, influence and pair tensors in FP32
-  void *pme_grid;    // 3 x K^3 real grids
-  void *pme_spec;    // 3 x K*K*(K/2+1) complex spectra
+  void *pme_grid;    // packed pairs' complex grids, 3 components per point, K^3 points each
+  void *pme_tw;      // exp(-2 pi i m / K), m < K
   void *pme_infl;    // 6 x half spectrum influence tensor
   double *pme_bsq;   // |b_d(m)|^2, 3 x K
   double *pme_soff;  // self-block off-diagonal (xy, xz, yz), then per-block partials
   int pme_nblk;      // blocks of the influence kernel
   int *pme_base;     // per bead base grid index, 3 x N
-  double *pme_w;     // per bead spline weights, 3 x N x 8
-  int pme_plan_f, pme_plan_b;
-  int pme_mplan_k[4], pme_mplan_f[4];  // packed-pair transforms for k right-hand sides
+  void *pme_w;       // per bead spline weights, 3 x N x 8 (FP64 or FP32, as the grids)
+  int pme_plan;      // 1 + cuFFT plan of one pair's grid, for sizes bd_fft.cuh does not
+                     // cover (0: none)
   int rl_cap, rl_ncell_cap;  // real-space pair rows
   int *rl_cnt, *rl_rows, *rl_cell_of, *rl_cell_count, *rl_cell_start, *rl_cursor;
   int *rl_need;      // longest pair row of the last build that overflowed the cap (0: none)
@@ -202,9 +202,13 @@ struct bd_ctx {
   float *pme_vpk;    // FP32 block products: per packed pair and bead the pair's
                      // 6 input values (+2 padding), written by the spread
   void *rl_tt;       // per pair t1 and t2 / r^2 of the real-space tensor (FP64 or FP32)
-  double *pme_rsum;  // FP32 block products: real-space sums of every packed pair (6 per bead)
   float4 *rl_w;      // FP32 block products: per pair (t1, w), w = sqrt(|t2| / r^2) d, the sign
                      // of t2 in the lowest mantissa bit of t1
+  // spreading by grid columns and interpolation (bd_mesh.cu): up to two column
+  // layouts (packed pairs per warp), beads per column and base index, starts
+  int mesh_ng[2];
+  int *mesh_ent[2], *mesh_bin[2], *mesh_sums, *mesh_cursor;
+  double *mesh_val;  // interpolated values, 6 per bead and pair
   double pme_cellbuf[19];  // its cell: H, H^-1, volume
   double pme_alpha_ref;    // calcHI's split parameter at that step
 
@@ -257,7 +261,6 @@ int pme_prepare(bd_ctx* c, const Lat& l);
 int pme_apply(bd_ctx* c, const VecIn& v, double* o0, double* o1, double* o2, int ostride);
 // Y_r = M X_r for k vectors in Lanczos layout (3 x NTp), RHS strides xs, ys
 int pme_apply_multi(bd_ctx* c, int k, const double* X, size_t xs, double* Y, size_t ys);
-int pme_multi_plan(bd_ctx* c, int k);  // creates the batched transforms for k
 void pme_free(bd_ctx* c);
 
 // CA-TEA sampling

@@ -1494,7 +1494,6 @@ static int lanczos_sqrt_block(bd_ctx* c, int k) {
   if ((s = alloc_lanczos(c)) != BD_OK) return s;
   if ((s = alloc_blocks(c)) != BD_OK) return s;
   if (k < 1 || k > c->nbk) return BD_ERR_ARG;
-  if (k > 1 && (s = pme_multi_plan(c, k)) != BD_OK) return s;
   size_t n = 3 * (size_t)c->NT * 32;
   bool pre = c->pre_kind != BD_PRECOND_NONE && c->pre_ready;
   std::vector<int> mr;
@@ -1609,7 +1608,6 @@ int bd_mobility_apply_block(bd_ctx* c, int k, const double* v, double* out) {
     return BD_OK;
   }
   int s;
-  if ((s = pme_multi_plan(c, k)) != BD_OK) return s;
   int N = c->N, NTp = c->NT * 32;
   size_t n = 3 * (size_t)NTp;
   std::vector<double> soa(n * k, 0.0), res(n * k);

@@ -1,0 +1,661 @@
+// Spreading and interpolation of the particle-mesh mobility without atomics.
+//
+// No counterpart in the reference (see bd_pme.cu).  Grids hold, per packed
+// pair of right-hand sides, K^3 points of three complex components, the
+// component fastest.
+//
+// Spreading: the grid is cut into columns of CY x CZ points in (y, z), running
+// along x.  A warp owns a column (or a segment of it) for NG packed pairs, a
+// lane per (y, z) and pair: it walks the beads whose stencil meets the column
+// in order of their base index along x, holding the P grid levels that the
+// current base reaches in registers.  A bead's P x-weights times the lane's y
+// and z weights and the bead's values are added to those levels; a level is
+// written when the walk has passed it (every point is written exactly once, so
+// the grid needs no clearing), and the window shifts.
+// An order-8 stencil covers 8 x 8 of the (y, z) plane and meets (7 + CY)(7 +
+// CZ)/(CY CZ) columns, so small columns waste fewer lanes (the share of them
+// inside the stencil is 39 % at 4 x 8, 71 % at 2 x 3) as long as the warp's
+// other lanes serve other pairs: 5 pairs by 2 x 3, 4 by 2 x 4, 3 by 2 x 5, 2 by
+// 4 x 4, 1 by 4 x 8.
+// Bound by the FP32 (FP64) pipe and the issue of its instructions: 48 (P = 8)
+// multiply-adds per lane and bead, two at a time (fma.rn.f32x2) in FP32, next
+// to about 20 others.
+// Five pairs, order 8: 169 us at 50 000 beads on 100^3 (one complex L2 atomic
+// per stencil point, component and pair took about 400), 47 us at 8000 beads on
+// 64^3 (74); FP64 70 us there (385).
+//
+// Interpolation: a warp per bead and pair reads the stencil's 64 rows of 24
+// complex values (192 contiguous bytes, FP32), a lane the same third of a row
+// position throughout, so its y and z weights and addresses stay in registers.
+// Bound by L1 throughput.
+// Five pairs, order 8: 238 us at 50 000 beads on 100^3 (separate component
+// grids, 64 bytes a row, FP64 sums per lane: about 300), 40 us at 8000 beads on
+// 64^3 (54); FP64 72 us there.
+//
+// The columns' lists are built once per mobility build (the positions are
+// frozen until the next): per column and base index the beads in increasing
+// index, so the sums are formed in a fixed order and a product is
+// reproducible bit by bit.
+#include <algorithm>
+#include <type_traits>
+
+#include "bd_ctx.cuh"
+#include "bd_cell.cuh"
+#include "bd_mesh.cuh"
+
+using namespace bd;
+
+#define CU(call) BD_CU(call)
+
+namespace {
+
+constexpr int kMaxTouched = 8;  // columns that a stencil can meet along y or z
+
+// The distinct column indices of size-w cells that the rows b, b - 1, ..,
+// b - P + 1 (modulo K) lie in.
+__device__ __forceinline__ int touched(int b, int P, int K, int w, int* out) {
+  int n = 0, last = -1;
+  for (int d = 0; d < P; d++) {
+    int y = b - d;
+    y += y < 0 ? K : 0;
+    int c = y / w;
+    if (c == last) continue;
+    last = c;
+    bool seen = false;
+    for (int q = 0; q < n; q++) seen |= out[q] == c;
+    if (!seen) out[n++] = c;
+  }
+  return n;
+}
+
+// Beads per (column, base index); with ent also their entries from bin[] on.
+__global__ void k_mesh_list(const int* __restrict__ base, int N, int K, int P, int CY, int CZ,
+                            int npz, int* count, const int* __restrict__ bin, int* ent) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  int cy[kMaxTouched], cz[kMaxTouched];
+  int ny = touched(base[3 * i + 1], P, K, CY, cy);
+  int nz = touched(base[3 * i + 2], P, K, CZ, cz);
+  for (int a = 0; a < ny; a++)
+    for (int b = 0; b < nz; b++) {
+      size_t q = (size_t)(cy[a] * npz + cz[b]) * K + base[3 * i];
+      int at = atomicAdd(count + q, 1);
+      if (ent) ent[bin[q] + at] = i;
+    }
+}
+
+// Each bin in increasing bead index (bins hold a few beads).
+__global__ void k_mesh_sort(const int* __restrict__ bin, size_t nbin, int* ent) {
+  size_t b = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= nbin) return;
+  int lo = bin[b], hi = bin[b + 1];
+  for (int a = lo + 1; a < hi; a++) {
+    int v = ent[a], q = a - 1;
+    for (; q >= lo && ent[q] > v; q--) ent[q + 1] = ent[q];
+    ent[q + 1] = v;
+  }
+}
+
+// Exclusive scan of a[0 .. n) in place, the total at a[n]: 2048 entries per
+// block, the block totals scanned by one block in between.
+constexpr int kScanBlock = 2048;
+
+__device__ __forceinline__ int block_scan_excl(int v, int* sh, int& total) {
+  int t = threadIdx.x, lane = t & 31, w = t >> 5, in = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    int x = __shfl_up_sync(0xffffffffu, in, o);
+    if (lane >= o) in += x;
+  }
+  if (lane == 31) sh[w] = in;
+  __syncthreads();
+  int before = 0;
+  total = 0;
+  for (int q = 0; q < (int)(blockDim.x >> 5); q++) {
+    if (q < w) before += sh[q];
+    total += sh[q];
+  }
+  __syncthreads();
+  return before + in - v;
+}
+
+__global__ void __launch_bounds__(256) k_scan_sums(const int* __restrict__ a, size_t n, int* sums) {
+  __shared__ int sh[8];
+  size_t lo = (size_t)blockIdx.x * kScanBlock;
+  int s = 0, total;
+  for (int q = threadIdx.x; q < kScanBlock; q += 256)
+    if (lo + q < n) s += a[lo + q];
+  block_scan_excl(s, sh, total);
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(1024) k_scan_blocks(int* sums, int nb, int* total_out) {
+  __shared__ int sh[32];
+  int run = 0;
+  for (int b0 = 0; b0 < nb; b0 += 1024) {
+    int b = b0 + threadIdx.x, v = b < nb ? sums[b] : 0, total;
+    int e = block_scan_excl(v, sh, total);
+    if (b < nb) sums[b] = run + e;
+    run += total;
+  }
+  if (threadIdx.x == 0) *total_out = run;
+}
+
+__global__ void __launch_bounds__(256) k_scan_place(int* a, size_t n, const int* __restrict__ sums) {
+  __shared__ int sh[8];
+  size_t lo = (size_t)blockIdx.x * kScanBlock + threadIdx.x * 8;
+  int v[8], s = 0, total;
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    v[q] = lo + q < n ? a[lo + q] : 0;
+    s += v[q];
+  }
+  int run = sums[blockIdx.x] + block_scan_excl(s, sh, total);
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    if (lo + q < n) a[lo + q] = run;
+    run += v[q];
+  }
+}
+
+// FP32 values of a pair of right-hand sides, per bead six (re xyz, im xyz)
+// and two zeros: one 32-byte record for the spreading and the pair sums.
+__global__ void k_mesh_pack(VecIn v, size_t vr, int k, int N, float* vpk) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x, p = blockIdx.y;
+  if (i >= N) return;
+  size_t oa = (size_t)(2 * p) * vr + (size_t)i * v.stride;
+  float4 x = make_float4((float)v.p[0][oa], (float)v.p[1][oa], (float)v.p[2][oa], 0.f);
+  float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (2 * p + 1 < k) {
+    size_t ob = oa + vr;
+    x.w = (float)v.p[0][ob];
+    y.x = (float)v.p[1][ob];
+    y.y = (float)v.p[2][ob];
+  }
+  float4* o = (float4*)(vpk + ((size_t)p * N + i) * 8);
+  o[0] = x;
+  o[1] = y;
+}
+
+// ---------------------------------------------------------------------------
+
+template <typename R>
+struct GridVal;
+template <>
+struct GridVal<float> {
+  using T = float2;
+  using W = float2;  // a weight in both halves, as fma.rn.f32x2 wants it
+};
+template <>
+struct GridVal<double> {
+  using T = double2;
+  using W = double;
+};
+
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long d, x = *reinterpret_cast<unsigned long long*>(&a),
+                        y = *reinterpret_cast<unsigned long long*>(&b),
+                        z = *reinterpret_cast<unsigned long long*>(&c);
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(x), "l"(y), "l"(z));
+  return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ void madd(float2 w, float2 x, float2& a) { a = fma2(w, x, a); }
+__device__ __forceinline__ void madd(double w, double2 x, double2& a) {
+  a.x = fma(w, x.x, a.x);
+  a.y = fma(w, x.y, a.y);
+}
+__device__ __forceinline__ void madd(float w, float x, float& a) { a = fmaf(w, x, a); }
+__device__ __forceinline__ void madd(double w, double x, double& a) { a = fma(w, x, a); }
+__device__ __forceinline__ float2 weight(float x) { return make_float2(x, x); }
+__device__ __forceinline__ double weight(double x) { return x; }
+__device__ __forceinline__ void put(float2& w, float x) { w = make_float2(x, x); }
+__device__ __forceinline__ void put(float& w, float x) { w = x; }
+__device__ __forceinline__ void put(double& w, double x) { w = x; }
+// Accumulated values: a complex pair, or a real number where a single
+// right-hand side leaves the imaginary parts zero.
+__device__ __forceinline__ void zero(float& a) { a = 0.f; }
+__device__ __forceinline__ void zero(double& a) { a = 0.0; }
+__device__ __forceinline__ void zero(float2& a) { a = make_float2(0.f, 0.f); }
+__device__ __forceinline__ void zero(double2& a) { a = make_double2(0.0, 0.0); }
+__device__ __forceinline__ float2 as_pair(float a) { return make_float2(a, 0.f); }
+__device__ __forceinline__ double2 as_pair(double a) { return make_double2(a, 0.0); }
+__device__ __forceinline__ float2 as_pair(float2 a) { return a; }
+__device__ __forceinline__ double2 as_pair(double2 a) { return a; }
+__device__ __forceinline__ float scaled(float w, float a) { return w * a; }
+__device__ __forceinline__ double scaled(double w, double a) { return w * a; }
+__device__ __forceinline__ float2 scaled(float w, float2 a) { return make_float2(w * a.x, w * a.y); }
+__device__ __forceinline__ double2 scaled(double w, double2 a) {
+  return make_double2(w * a.x, w * a.y);
+}
+__device__ __forceinline__ void set_pair(float2& f, float x, float y) { f = make_float2(x, y); }
+__device__ __forceinline__ void set_pair(double2& f, double x, double y) { f = make_double2(x, y); }
+__device__ __forceinline__ void set_pair(float& f, float x, float) { f = x; }
+__device__ __forceinline__ void set_pair(double& f, double x, double) { f = x; }
+
+// One bead of a column's walk in shared memory: x-weights from the lowest
+// level up, the weights of the column's rows and points, the pairs' values,
+// the base index along x.  Padded to an odd number of 16-byte words, so that
+// the lanes of a warp store their records without bank conflicts.
+template <int P, typename R, int NG, int CY, int CZ, bool ONE>
+struct RecData {
+  std::conditional_t<ONE, R, typename GridVal<R>::W> wx[P];
+  std::conditional_t<ONE, R, typename GridVal<R>::T> f[NG][3];
+  R wy[CY], wz[CZ];
+  int at;
+};
+template <typename S>
+struct alignas(16) Rec : S {
+  static constexpr int words = (int)((sizeof(S) + 15) / 16);
+  char fill[16 * (words + (words % 2 == 0 ? 1 : 0)) - sizeof(S)];
+};
+
+struct SpreadArgs {
+  const int* base;
+  const void* w;  // 8 weights per bead and direction, R
+  const int* ent;
+  const int* bin;
+  int K, npz, npatch, nseg, nset, np, N;
+  VecIn v;
+  size_t vr;
+  int k;
+  const float* vpk;  // packed values, or null: read from v
+};
+
+template <int P, typename R, int NG, int CY, int CZ, bool ONE>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2) k_mesh_spread(SpreadArgs m, R* grid) {
+  using T = typename GridVal<R>::T;
+  using V = std::conditional_t<ONE, R, T>;
+  using S = Rec<RecData<P, R, NG, CY, CZ, ONE>>;
+  static_assert(NG * CY * CZ <= 32, "a lane per point and pair");
+  __shared__ S s_rec[4][32];
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const int job = blockIdx.x * 4 + wl;
+  if (job >= m.npatch * m.nseg * m.nset) return;
+  // columns fastest: the neighbours along z of a block complete its sectors
+  const int patch = job % m.npatch, seg = job / m.npatch % m.nseg,
+            set = job / (m.npatch * m.nseg);
+  const int K = m.K, xs = (int)((long long)seg * K / m.nseg),
+            xe = (int)((long long)(seg + 1) * K / m.nseg);
+  const int y0 = patch / m.npz * CY, z0 = patch % m.npz * CZ;
+  const int g = lane / (CY * CZ) < NG ? lane / (CY * CZ) : 0;
+  const int ly = lane % (CY * CZ) / CZ, lz = lane % CZ;
+  const int pr = set * NG + g;
+  const bool own = lane < NG * CY * CZ && pr < m.np && y0 + ly < K && z0 + lz < K;
+  const size_t K2 = (size_t)K * K;
+  T* out = (T*)grid + 3 * ((size_t)(own ? pr : 0) * K2 * K + (size_t)(y0 + ly) * K + (z0 + lz));
+  // bases xs .. xe + P - 2, wrapped: entries [e0, e0 + n0), then [f0, f0 + n1)
+  const int* bin = m.bin + (size_t)patch * K;
+  const int top = xe + P - 1;
+  const int e0 = bin[xs], n0 = bin[min(K, top)] - e0;
+  const int f0 = bin[0], n1 = top > K ? bin[top - K] - f0 : 0;
+  const int n = n0 + n1;
+  V acc[P][3];
+#pragma unroll
+  for (int a = 0; a < P; a++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) zero(acc[a][c]);
+  int lo = xs - (P - 1);  // grid level of acc[0]
+  auto advance = [&]() {
+    if (lo >= xs && own) {
+      T* o = out + 3 * K2 * (size_t)lo;
+      o[0] = as_pair(acc[0][0]);
+      o[1] = as_pair(acc[0][1]);
+      o[2] = as_pair(acc[0][2]);
+    }
+#pragma unroll
+    for (int a = 0; a + 1 < P; a++)
+#pragma unroll
+      for (int c = 0; c < 3; c++) acc[a][c] = acc[a + 1][c];
+#pragma unroll
+    for (int c = 0; c < 3; c++) zero(acc[P - 1][c]);
+    lo++;
+  };
+  // records straight into shared memory; only the next batch's bead indices are
+  // read ahead (the other warps of the SM cover the records' latency, and the
+  // registers go to the window)
+  auto entry = [&](int t) { return t >= n ? 0 : t < n0 ? m.ent[e0 + t] : m.ent[f0 + t - n0]; };
+  auto stage = [&](int t, int i) {
+    if (t >= n) return;
+    S& r = s_rec[wl][lane];
+    const R* w = (const R*)m.w + (size_t)i * 3 * kMaxOrder;
+    const int b1 = m.base[3 * i + 1], b2 = m.base[3 * i + 2];
+    r.at = m.base[3 * i] + (t < n0 ? 0 : K);
+#pragma unroll
+    for (int a = 0; a < P; a++) put(r.wx[a], w[P - 1 - a]);
+#pragma unroll
+    for (int q = 0; q < CY; q++) {
+      int d = b1 - (y0 + q);
+      d += d < 0 ? K : 0;
+      r.wy[q] = d < P && y0 + q < K ? w[kMaxOrder + d] : (R)0;
+    }
+#pragma unroll
+    for (int q = 0; q < CZ; q++) {
+      int d = b2 - (z0 + q);
+      d += d < 0 ? K : 0;
+      r.wz[q] = d < P && z0 + q < K ? w[2 * kMaxOrder + d] : (R)0;
+    }
+#pragma unroll
+    for (int u = 0; u < NG; u++) {
+      const int p = min(set * NG + u, m.np - 1);
+      if (sizeof(R) == 4 && m.vpk) {
+        const float4* q = (const float4*)(m.vpk + ((size_t)p * m.N + i) * 8);
+        float4 a = q[0];
+        float2 b = *(const float2*)(q + 1);
+        set_pair(r.f[u][0], a.x, a.w);
+        set_pair(r.f[u][1], a.y, b.x);
+        set_pair(r.f[u][2], a.z, b.y);
+      } else {
+        const size_t oa = (size_t)(2 * p) * m.vr + (size_t)i * m.v.stride;
+        const bool two = 2 * p + 1 < m.k;
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+          set_pair(r.f[u][c], (R)m.v.p[c][oa], two ? (R)m.v.p[c][oa + m.vr] : (R)0);
+      }
+    }
+  };
+  int bead = entry(lane);
+  for (int t0 = 0; t0 < n; t0 += 32) {
+    __syncwarp();
+    stage(t0 + lane, bead);
+    bead = entry(t0 + 32 + lane);
+    __syncwarp();
+    const int nb = min(32, n - t0);
+#pragma unroll 1
+    for (int u = 0; u < nb; u++) {
+      const S& q = s_rec[wl][u];
+      const R wyz = q.wy[ly] * q.wz[lz];
+      V t[3];
+#pragma unroll
+      for (int c = 0; c < 3; c++) t[c] = scaled(wyz, q.f[g][c]);
+      const int want = q.at - (P - 1);
+#pragma unroll 1
+      while (lo < want) advance();
+#pragma unroll
+      for (int a = 0; a < P; a++) {
+        const auto wx = q.wx[a];
+#pragma unroll
+        for (int c = 0; c < 3; c++) madd(wx, t[c], acc[a][c]);
+      }
+    }
+  }
+#pragma unroll 1
+  while (lo < xe) advance();
+}
+
+// val[(pr N + i) 6 + 3 h + c] = sum_g W_i(g) grid (h: real, imaginary part):
+// a warp per bead and pair.  The stencil's 3 P^3 complex values are taken 32 at
+// a time in memory order (rows of P points along z, three components each);
+// 96 values are a whole number of points, so load t of a lane always holds
+// component (2 t + lane) mod 3: one sum for each t mod 3, put in component
+// order at the end.  FP32 sums per lane (order 8: 16 terms each) and over four
+// lanes, FP64 beyond.
+template <int P, typename R>
+__global__ void __launch_bounds__(256)
+    k_mesh_gather(const int* __restrict__ base, const R* __restrict__ w,
+                  const R* __restrict__ grid, int N, int K, double* __restrict__ val) {
+  using T = typename GridVal<R>::T;
+  const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, pr = blockIdx.y;
+  if (i >= N) return;
+  const R* w0 = w + (size_t)i * 3 * kMaxOrder;
+  const R* w1 = w0 + kMaxOrder;
+  const R* w2 = w1 + kMaxOrder;
+  const int b0 = base[3 * i], b1 = base[3 * i + 1], b2 = base[3 * i + 2];
+  const size_t K2 = (size_t)K * K;
+  const T* gp = (const T*)grid + (size_t)pr * 3 * K2 * K;
+  T s[3];
+#pragma unroll
+  for (int j = 0; j < 3; j++) s[j].x = s[j].y = 0;
+  if constexpr (P == 8) {
+    // four rows in three loads; rows 4 q + (0..3) of x level q / 2: the lane's
+    // point and its offset within (y, z) depend on q only by its parity
+    int off[3][2];
+    R wyz[3][2];
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      const int f = 32 * j + lane, ro = f / 24, z = f % 24 / 3;
+      int gz = b2 - (P - 1) + z;
+      gz += gz < 0 ? K : 0;
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        int gy = b1 - (4 * h + ro);
+        gy += gy < 0 ? K : 0;
+        off[j][h] = (gy * K + gz) * 3 + f % 3;
+        wyz[j][h] = w1[4 * h + ro] * w2[P - 1 - z];
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < P; a++) {
+      int gx = b0 - a;
+      gx += gx < 0 ? K : 0;
+      const T* gl = gp + 3 * K2 * (size_t)gx;
+      const R wx = w0[a];
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) madd(weight(wx * wyz[j][h]), gl[off[j][h]], s[j]);
+    }
+  } else {
+#pragma unroll 1
+    for (int t0 = 0; 32 * t0 < 3 * P * P * P; t0 += 3) {
+#pragma unroll
+      for (int j = 0; j < 3; j++) {
+        const int f = 32 * (t0 + j) + lane;
+        if (f >= 3 * P * P * P) break;
+        const int z = f / 3 % P, row = f / (3 * P), b = row % P, a = row / P;
+        int gx = b0 - a, gy = b1 - b, gz = b2 - (P - 1) + z;
+        gx += gx < 0 ? K : 0;
+        gy += gy < 0 ? K : 0;
+        gz += gz < 0 ? K : 0;
+        madd(weight(w0[a] * w1[b] * w2[P - 1 - z]),
+             gp[3 * ((size_t)gx * K2 + (size_t)gy * K + gz) + f % 3], s[j]);
+      }
+    }
+  }
+  // component c is in sum 2 (c - lane) mod 3
+  const int r = lane % 3;
+  T c0 = r == 0 ? s[0] : r == 1 ? s[1] : s[2];
+  T c1 = r == 0 ? s[2] : r == 1 ? s[0] : s[1];
+  T c2 = r == 0 ? s[1] : r == 1 ? s[2] : s[0];
+  // real parts to the lower, imaginary parts to the upper half of the warp
+  const bool up = lane & 16;
+  R x[3] = {up ? c0.y : c0.x, up ? c1.y : c1.x, up ? c2.y : c2.x};
+  R y[3] = {up ? c0.x : c0.y, up ? c1.x : c1.y, up ? c2.x : c2.y};
+  double d[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    x[c] += __shfl_xor_sync(0xffffffffu, y[c], 16);
+    x[c] += __shfl_xor_sync(0xffffffffu, x[c], 8);
+    d[c] = (double)x[c];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) d[c] += __shfl_xor_sync(0xffffffffu, d[c], o);
+  }
+  const int e = lane & 15;
+  if (e < 3) val[((size_t)pr * N + i) * 6 + (up ? 3 : 0) + e] = e == 0 ? d[0] : e == 1 ? d[1] : d[2];
+}
+
+// ---------------------------------------------------------------------------
+
+// Columns of the layouts, by the number of pairs a warp serves.
+constexpr int kCols[6][2] = {{0, 0}, {4, 8}, {4, 4}, {2, 5}, {2, 4}, {2, 3}};
+
+// Work of a spreading of np pairs in layout ng: bead visits times warps.
+double layout_cost(int np, int ng, int P) {
+  double cy = kCols[ng][0], cz = kCols[ng][1];
+  return (P - 1 + cy) * (P - 1 + cz) / (cy * cz) * ((np + ng - 1) / ng);
+}
+
+// Segments of a column: enough warps for about 16 on every SM, none shorter
+// than half a stencil (a segment repeats P - 1 levels of its beads).
+int segments(int K, int njob) {
+  int want = (148 * 16 + njob - 1) / njob;
+  return std::max(1, std::min(want, K / 4));
+}
+
+size_t patches(int K, int ng) {
+  return (size_t)((K + kCols[ng][0] - 1) / kCols[ng][0]) *
+         ((K + kCols[ng][1] - 1) / kCols[ng][1]);
+}
+
+// Columns that a stencil can meet: P rows over cells of w, one more where the
+// last cell is short.
+int most_touched(int K, int P, int w) {
+  return std::min((P + w - 2) / w + 1 + (K % w ? 1 : 0), (K + w - 1) / w);
+}
+
+template <int P, typename R>
+void launch_spread(bd_ctx* c, int ng, int nb, const SpreadArgs& m, R* grid) {
+#define SPREAD(...) k_mesh_spread<P, R, __VA_ARGS__><<<nb, 128, 0, c->stream>>>(m, grid)
+  switch (ng) {
+    case 1:
+      if (m.k == 1)
+        SPREAD(1, 4, 8, true);
+      else
+        SPREAD(1, 4, 8, false);
+      break;
+    case 2: SPREAD(2, 4, 4, false); break;
+    case 3: SPREAD(3, 2, 5, false); break;
+    case 4: SPREAD(4, 2, 4, false); break;
+    default: SPREAD(5, 2, 3, false);
+  }
+#undef SPREAD
+}
+
+template <typename R>
+int spread_t(bd_ctx* c, int k, const VecIn& v, size_t vr, R* grid) {
+  const int np = (k + 1) / 2, K = c->pmeK, P = c->pme_p;
+  // of the context's layouts the one with the least work for np pairs
+  int l = 0;
+  if (c->mesh_ng[1] && layout_cost(np, c->mesh_ng[1], P) < layout_cost(np, c->mesh_ng[0], P)) l = 1;
+  const int ng = c->mesh_ng[l];
+  SpreadArgs m;
+  m.base = c->pme_base;
+  m.w = c->pme_w;
+  m.ent = c->mesh_ent[l];
+  m.bin = c->mesh_bin[l];
+  m.K = K;
+  m.npz = (K + kCols[ng][1] - 1) / kCols[ng][1];
+  m.npatch = (int)patches(K, ng);
+  m.nset = (np + ng - 1) / ng;
+  m.nseg = segments(K, m.npatch * m.nset);
+  m.np = np;
+  m.N = c->N;
+  m.v = v;
+  m.vr = vr;
+  m.k = k;
+  m.vpk = c->pme_vpk;
+  if (c->pme_vpk) {
+    c->launches++;
+    k_mesh_pack<<<dim3(nblk(c->N, 256), np), 256, 0, c->stream>>>(v, vr, k, c->N, c->pme_vpk);
+  }
+  const int nb = nblk((long long)m.npatch * m.nseg * m.nset, 4);
+  c->launches++;
+  switch (P) {
+    case 4: launch_spread<4, R>(c, ng, nb, m, grid); break;
+    case 6: launch_spread<6, R>(c, ng, nb, m, grid); break;
+    default: launch_spread<8, R>(c, ng, nb, m, grid);
+  }
+  return BD_OK;
+}
+
+template <typename R>
+int gather_t(bd_ctx* c, int k, const R* grid) {
+  const dim3 g(nblk(c->N, 8), (k + 1) / 2);
+  const R* w = (const R*)c->pme_w;
+  c->launches++;
+  switch (c->pme_p) {
+    case 4:
+      k_mesh_gather<4, R><<<g, 256, 0, c->stream>>>(c->pme_base, w, grid, c->N, c->pmeK, c->mesh_val);
+      break;
+    case 6:
+      k_mesh_gather<6, R><<<g, 256, 0, c->stream>>>(c->pme_base, w, grid, c->N, c->pmeK, c->mesh_val);
+      break;
+    default:
+      k_mesh_gather<8, R><<<g, 256, 0, c->stream>>>(c->pme_base, w, grid, c->N, c->pmeK, c->mesh_val);
+  }
+  return BD_OK;
+}
+
+}  // namespace
+
+namespace bd {
+
+int mesh_alloc(bd_ctx* c) {
+  if (c->mesh_val) return BD_OK;
+  const int K = c->pmeK, N = c->N, P = c->pme_p, np = std::max(1, (c->nbk + 1) / 2);
+  // a layout for single products and, where another does less work, one for
+  // full blocks
+  int best = 1;
+  for (int ng = 2; ng <= 5; ng++)
+    if (layout_cost(np, ng, P) < layout_cost(np, best, P)) best = ng;
+  c->mesh_ng[0] = 1;
+  c->mesh_ng[1] = best > 1 ? best : 0;
+  size_t nbin_max = 0;
+  for (int l = 0; l < 2 && c->mesh_ng[l]; l++) {
+    int ng = c->mesh_ng[l];
+    size_t nbin = patches(K, ng) * K;
+    size_t nent = (size_t)N * most_touched(K, P, kCols[ng][0]) * most_touched(K, P, kCols[ng][1]);
+    CU(cudaMalloc(&c->mesh_ent[l], 4 * nent));
+    CU(cudaMalloc(&c->mesh_bin[l], 4 * (nbin + 1)));
+    c->bytes += 4 * (nent + nbin + 1);
+    nbin_max = std::max(nbin_max, nbin);
+  }
+  size_t nscan = nbin_max / kScanBlock + 1;
+  CU(cudaMalloc(&c->mesh_sums, 4 * nscan));
+  CU(cudaMalloc(&c->mesh_cursor, 4 * nbin_max));
+  CU(cudaMalloc(&c->mesh_val, 48 * (size_t)N * np));
+  c->bytes += 4 * (nscan + nbin_max) + 48 * (size_t)N * np;
+  return BD_OK;
+}
+
+void mesh_free(bd_ctx* c) {
+  for (void* q : {(void*)c->mesh_ent[0], (void*)c->mesh_ent[1], (void*)c->mesh_bin[0],
+                  (void*)c->mesh_bin[1], (void*)c->mesh_sums, (void*)c->mesh_cursor,
+                  (void*)c->mesh_val})
+    if (q) cudaFree(q);
+}
+
+static void scan_excl(bd_ctx* c, int* a, size_t n) {
+  int nb = (int)((n + kScanBlock - 1) / kScanBlock);
+  c->launches += 3;
+  k_scan_sums<<<nb, 256, 0, c->stream>>>(a, n, c->mesh_sums);
+  k_scan_blocks<<<1, 1024, 0, c->stream>>>(c->mesh_sums, nb, a + n);
+  k_scan_place<<<nb, 256, 0, c->stream>>>(a, n, c->mesh_sums);
+}
+
+// The columns' bead lists for the base indices of the last k_pme_weights.
+int mesh_prepare(bd_ctx* c) {
+  int s;
+  if ((s = mesh_alloc(c)) != BD_OK) return s;
+  const int N = c->N, P = c->pme_p, K = c->pmeK;
+  for (int l = 0; l < 2 && c->mesh_ng[l]; l++) {
+    const int CY = kCols[c->mesh_ng[l]][0], CZ = kCols[c->mesh_ng[l]][1], npz = (K + CZ - 1) / CZ;
+    const size_t nbin = patches(K, c->mesh_ng[l]) * K;
+    CU(cudaMemsetAsync(c->mesh_bin[l], 0, 4 * nbin, c->stream));
+    CU(cudaMemsetAsync(c->mesh_cursor, 0, 4 * nbin, c->stream));
+    c->launches += 3;
+    k_mesh_list<<<nblk(N, 128), 128, 0, c->stream>>>(c->pme_base, N, K, P, CY, CZ, npz,
+                                                     c->mesh_bin[l], nullptr, nullptr);
+    scan_excl(c, c->mesh_bin[l], nbin);
+    k_mesh_list<<<nblk(N, 128), 128, 0, c->stream>>>(c->pme_base, N, K, P, CY, CZ, npz,
+                                                     c->mesh_cursor, c->mesh_bin[l],
+                                                     c->mesh_ent[l]);
+    k_mesh_sort<<<nblk((long long)nbin, 128), 128, 0, c->stream>>>(c->mesh_bin[l], nbin,
+                                                                   c->mesh_ent[l]);
+  }
+  return launch_ok(c);
+}
+
+// grid = the spread of k right-hand sides v (component pointers, vr apart), as
+// packed pairs.
+int mesh_spread(bd_ctx* c, int k, const VecIn& v, size_t vr, void* grid) {
+  return c->pme_f32 ? spread_t<float>(c, k, v, vr, (float*)grid)
+                    : spread_t<double>(c, k, v, vr, (double*)grid);
+}
+
+// The pairs' interpolated values into mesh_val.
+int mesh_gather(bd_ctx* c, int k, const void* grid) {
+  return c->pme_f32 ? gather_t<float>(c, k, (const float*)grid)
+                    : gather_t<double>(c, k, (const double*)grid);
+}
+
+}  // namespace bd

@@ -29,10 +29,10 @@
 //  * calcHI stores only the diagonal entries of the self blocks
 //    (shear/src/main26.c:1663-1700); the off-diagonal entries of the k-space
 //    self sum, which a sheared or stretched cell makes non-zero, are removed.
-// cuFFT is used for the transforms only.  Spreading uses atomics in the grid
-// precision; several right-hand sides share each launch (blockIdx.y).  The
-// spline weights and pair tensors are computed once per step because the
-// positions do not change during a Krylov solve.
+// Spreading and interpolation are in bd_mesh.cu, the transforms in bd_fft.cuh
+// (cuFFT for grid sizes it does not cover).  The spline weights, the columns' lists and the pair tensors are
+// computed once per mobility build because its positions do not change during
+// the Krylov solves.
 #include <cufft.h>
 #include <math.h>
 #include <string.h>
@@ -43,6 +43,8 @@
 
 #include "bd_ctx.cuh"
 #include "bd_cell.cuh"
+#include "bd_fft.cuh"
+#include "bd_mesh.cuh"
 
 using namespace bd;
 
@@ -54,9 +56,10 @@ using namespace bd;
 // frame are taken to the lab frame with (cr, sr) = (cos, sin) of the lattice
 // angle, x = x' cr - y' sr, y = x' sr + y' cr (inverseCoords,
 // extensional/src/main14.c:1525-1535); lab-frame positions pass (1, 0).
+template <typename R>
 __global__ void k_pme_weights(Cell cell, const double* __restrict__ rx,
                               const double* __restrict__ ry, const double* __restrict__ rz,
-                              double cr, double sr, int N, int K, int p, int* base, double* w,
+                              double cr, double sr, int N, int K, int p, int* base, R* w,
                               double4* pos, int* err) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -75,169 +78,28 @@ __global__ void k_pme_weights(Cell cell, const double* __restrict__ rx,
     double f = u - fl;
     if (fl >= K) fl -= K;
     base[3 * i + d] = fl;
-    bspline(f, p, w + ((size_t)3 * i + d) * kMaxOrder);
+    double wd[kMaxOrder];
+    bspline(f, p, wd);
+    for (int k = 0; k < p; k++) w[((size_t)3 * i + d) * kMaxOrder + k] = (R)wd[k];
   }
 }
 
-// FP32 grids: the spread skips stencil points whose weight W_i(g) is below
-// 1e-9 (for order 8, 35 % of the 512 points, carrying at most 2.7e-8 of the
-// stencil's unit weight, mean 1.4e-8: below FP32 rounding, 6e-8, and two
-// orders below the particle-mesh error), saving their atomics; the
-// interpolation keeps every point (skipping there only added divergence), so
-// the product is symmetric to ~3e-8, inside the rounding of its FP32 grids.
-// (1e-8 would skip 42 % but drop up to 3e-7 of the weight, the size of the
-// FP32 storage error itself.)  The FP64 path keeps every point.
-constexpr double kSkipWeight = 1e-9;
+// Right-hand sides are packed in pairs: 2p and 2p + 1 are the real and
+// imaginary parts of one complex grid of three components (the component
+// fastest, pair p from 3 p K^3 on).  The influence tensor is real and even in
+// k, so one complex transform, the multiplication and the inverse transform
+// give both products, with no unpacking.  An odd last right-hand side, or a
+// single one, has a zero imaginary part.
 
-// Q_r[c][g] += v_r,c(i) W_i(g) for the right-hand sides r0 .. r0 + kc - 1
-// of chunk blockIdx.y (r0 = KS blockIdx.y; KS = 1 for single products): one
-// warp per bead, the P^3 stencil points spread over the lanes with the
-// fastest index along the contiguous grid direction, so each atomic
-// instruction of a warp covers runs of P adjacent grid values; the weights
-// and the bead's values are loaded once for the chunk.  Right-hand side r
-// reads its vector vr entries further on and owns the grids 3 K^3 entries
-// further on.
-
-template <int P, typename R, int KS>
-__global__ void __launch_bounds__(256) k_pme_spread(const int* __restrict__ base,
-                                                    const double* __restrict__ w, int N, int K,
-                                                    VecIn v, size_t vr, int k, R* grid) {
-  int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (i >= N) return;
-  int r0 = KS * blockIdx.y, kc = min(KS, k - r0);
-  size_t K3 = (size_t)K * K * K;
-  R f[3 * KS];
-#pragma unroll
-  for (int r = 0; r < KS; r++) {
-    size_t o = (size_t)(r0 + (r < kc ? r : 0)) * vr + (size_t)i * v.stride;
-    f[3 * r] = (R)v.p[0][o];
-    f[3 * r + 1] = (R)v.p[1][o];
-    f[3 * r + 2] = (R)v.p[2][o];
-  }
-  R* g0p = grid + (size_t)r0 * 3 * K3;
-  const double* w0 = w + ((size_t)3 * i + 0) * kMaxOrder;
-  const double* w1 = w + ((size_t)3 * i + 1) * kMaxOrder;
-  const double* w2 = w + ((size_t)3 * i + 2) * kMaxOrder;
-  int b0 = base[3 * i], b1 = base[3 * i + 1], b2 = base[3 * i + 2];
-  // fully unrolled: the stencil index of each lane is a compile-time
-  // function of the iteration, so the weights stay in registers
-#pragma unroll
-  for (int it = 0; it < (P * P * P + 31) / 32; it++) {
-    int q = lane + 32 * it;
-    if (q >= P * P * P) break;
-    int c = q % P, b = (q / P) % P, a = q / (P * P);
-    int g0 = b0 - a, g1 = b1 - b, g2 = b2 - c;
-    g0 += g0 < 0 ? K : 0;
-    g1 += g1 < 0 ? K : 0;
-    g2 += g2 < 0 ? K : 0;
-    double wt = w0[a] * w1[b] * w2[c];
-    if (sizeof(R) == 4 && wt < kSkipWeight) continue;  // FP32: negligible corner
-    R wr = (R)wt;
-    size_t g = ((size_t)g0 * K + g1) * K + g2;
-#pragma unroll
-    for (int r = 0; r < KS; r++) {
-      if (r >= kc) break;
-      R* gr = g0p + (size_t)r * 3 * K3 + g;
-      if constexpr (sizeof(R) == 8) {
-        atomicAdd(gr, wt * f[3 * r]);
-        atomicAdd(gr + K3, wt * f[3 * r + 1]);
-        atomicAdd(gr + 2 * K3, wt * f[3 * r + 2]);
-      } else {
-        atomicAdd(gr, wr * f[3 * r]);
-        atomicAdd(gr + K3, wr * f[3 * r + 1]);
-        atomicAdd(gr + 2 * K3, wr * f[3 * r + 2]);
-      }
-    }
-  }
-}
-
-// Products of k >= 2 right-hand sides pack them in pairs: right-hand sides
-// 2p and 2p + 1 are the real and imaginary parts of one complex grid per
-// component (pair p, component c at (3 p + c) K^3).  The influence tensor is
-// real and even in k, so one complex transform, the multiplication and the
-// inverse transform give both products, with no unpacking: spreading takes
-// one float2 atomic per pair and grid point, interpolation one float2 load,
-// and the transforms are contiguous C2C batches.
-template <typename R>
-struct Pair;
-template <>
-struct Pair<float> {
-  using T = float2;
-};
-template <>
-struct Pair<double> {
-  using T = double2;
-};
-
-// With vpk (FP32), lanes 0..7 of a bead's warp also store the pair's six
-// input values (plus two zeros) at vpk[(p N + i) 8], for the real-space sums
-// to read as a float4 and a float2.
-template <int P, typename R>
-__global__ void __launch_bounds__(256) k_pme_spread_pairs(const int* __restrict__ base,
-                                                          const double* __restrict__ w, int N,
-                                                          int K, VecIn v, size_t vr, int k,
-                                                          typename Pair<R>::T* cgrid,
-                                                          float* vpk) {
-  using C2 = typename Pair<R>::T;
-  int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (i >= N) return;
-  int pr = blockIdx.y, ra = 2 * pr, rb = 2 * pr + 1;
-  size_t K3 = (size_t)K * K * K;
-  size_t oa = (size_t)ra * vr + (size_t)i * v.stride;
-  size_t ob = (size_t)(rb < k ? rb : ra) * vr + (size_t)i * v.stride;
-  R fb_on = rb < k ? (R)1 : (R)0;
-  R fa0 = (R)v.p[0][oa], fa1 = (R)v.p[1][oa], fa2 = (R)v.p[2][oa];
-  R fb0 = fb_on * (R)v.p[0][ob], fb1 = fb_on * (R)v.p[1][ob], fb2 = fb_on * (R)v.p[2][ob];
-  if (vpk && lane < 8) {
-    R x = lane == 0 ? fa0 : lane == 1 ? fa1 : lane == 2 ? fa2
-        : lane == 3 ? fb0 : lane == 4 ? fb1 : lane == 5 ? fb2 : (R)0;
-    vpk[((size_t)pr * N + i) * 8 + lane] = (float)x;
-  }
-  C2* gp = cgrid + (size_t)pr * 3 * K3;
-  const double* w0 = w + ((size_t)3 * i + 0) * kMaxOrder;
-  const double* w1 = w + ((size_t)3 * i + 1) * kMaxOrder;
-  const double* w2 = w + ((size_t)3 * i + 2) * kMaxOrder;
-  int b0 = base[3 * i], b1 = base[3 * i + 1], b2 = base[3 * i + 2];
-#pragma unroll
-  for (int it = 0; it < (P * P * P + 31) / 32; it++) {
-    int q = lane + 32 * it;
-    if (q >= P * P * P) break;
-    int c = q % P, b = (q / P) % P, a = q / (P * P);
-    int g0 = b0 - a, g1 = b1 - b, g2 = b2 - c;
-    g0 += g0 < 0 ? K : 0;
-    g1 += g1 < 0 ? K : 0;
-    g2 += g2 < 0 ? K : 0;
-    double wt = w0[a] * w1[b] * w2[c];
-    if (sizeof(R) == 4 && wt < kSkipWeight) continue;  // FP32: negligible corner
-    size_t g = ((size_t)g0 * K + g1) * K + g2;
-    if constexpr (sizeof(R) == 4) {
-      float wr = (float)wt;
-      atomicAdd(gp + g, make_float2(wr * fa0, wr * fb0));
-      atomicAdd(gp + K3 + g, make_float2(wr * fa1, wr * fb1));
-      atomicAdd(gp + 2 * K3 + g, make_float2(wr * fa2, wr * fb2));
-    } else {
-      atomicAdd(&gp[g].x, wt * fa0);
-      atomicAdd(&gp[g].y, wt * fb0);
-      atomicAdd(&gp[K3 + g].x, wt * fa1);
-      atomicAdd(&gp[K3 + g].y, wt * fb1);
-      atomicAdd(&gp[2 * K3 + g].x, wt * fa2);
-      atomicAdd(&gp[2 * K3 + g].y, wt * fb2);
-    }
-  }
-}
-
-// The influence tensor on the full spectrum of the packed pairs (thread per
-// point and pair): points with m2 > K/2 take the tensor of their mirror -m,
-// stored in the half spectrum (the tensor is even in k; on the Nyquist planes
-// of an even K the stored pairs differ in the sign of off-diagonal entries,
-// where the influence is below 1e-14 of its peak).
+// The influence tensor on the full spectrum of the packed pairs, for grid sizes
+// that go through cuFFT (thread per point and pair): points with m2 > K/2 take
+// the tensor of their mirror -m, stored in the half spectrum.
 template <typename R, typename Cx>
-__global__ void k_pme_apply_influence_full(const R* __restrict__ infl, Cx* cgrid, int K,
-                                           size_t np3) {
+__global__ void k_pme_apply_influence(const R* __restrict__ infl, Cx* cgrid, int K, size_t np) {
   size_t K3 = (size_t)K * K * K;
   size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= K3 * np3) return;
-  size_t m = e % K3, pc = e / K3;  // pair index (components 3 apart)
+  if (e >= K3 * np) return;
+  size_t m = e % K3;
   int Kh = K / 2 + 1;
   int m0 = (int)(m / ((size_t)K * K)), m1 = (int)((m / K) % K), m2 = (int)(m % K);
   if (m2 > K / 2) {
@@ -246,8 +108,8 @@ __global__ void k_pme_apply_influence_full(const R* __restrict__ infl, Cx* cgrid
     m2 = K - m2;
   }
   const R* t = infl + 6 * (((size_t)m0 * K + m1) * Kh + m2);
-  Cx* b = cgrid + pc * 3 * K3 + m;
-  Cx x = b[0], y = b[K3], z = b[2 * K3];
+  Cx* b = cgrid + 3 * e;
+  Cx x = b[0], y = b[1], z = b[2];
   Cx u, v, ww;
   u.x = t[0] * x.x + t[1] * y.x + t[2] * z.x;
   u.y = t[0] * x.y + t[1] * y.y + t[2] * z.y;
@@ -256,8 +118,8 @@ __global__ void k_pme_apply_influence_full(const R* __restrict__ infl, Cx* cgrid
   ww.x = t[2] * x.x + t[4] * y.x + t[5] * z.x;
   ww.y = t[2] * x.y + t[4] * y.y + t[5] * z.y;
   b[0] = u;
-  b[K3] = v;
-  b[2 * K3] = ww;
+  b[1] = v;
+  b[2] = ww;
 }
 
 // Influence tensor on the half spectrum: (phi(k)/V)(I - k k^T/k^2) |b|^2,
@@ -280,23 +142,32 @@ __global__ void __launch_bounds__(256) k_pme_influence(Cell cell, int K, double 
     if (m0 == 0 && m1 == 0 && m2 == 0) {
       for (int a = 0; a < 6; a++) o[a] = (R)0;
     } else {
-      int s0 = m0 < (K + 1) / 2 ? m0 : m0 - K, s1 = m1 < (K + 1) / 2 ? m1 : m1 - K, s2 = m2;
-      // k = 2 pi (s0 b0 + s1 b1 + s2 b2), b_d = row d of H^-1
-      double k[3];
-      for (int a = 0; a < 3; a++)
-        k[a] = 2.0 * M_PI *
-               (s0 * cell.Hi[0 * 3 + a] + s1 * cell.Hi[1 * 3 + a] + s2 * cell.Hi[2 * 3 + a]);
-      double kk = k[0] * k[0] + k[1] * k[1] + k[2] * k[2];
-      double a2 = alpha * alpha;
-      double phi = (1.0 - kk / 3.0) * (1.0 + kk / (4.0 * a2) + kk * kk / (8.0 * a2 * a2)) * 6.0 *
-                   M_PI / kk * exp(-kk / (4.0 * a2)) / cell.V;
-      double f = phi * bsq[m0] * bsq[K + m1] * bsq[2 * K + m2];
-      o[0] = (R)(f * (1.0 - k[0] * k[0] / kk));
-      o[1] = (R)(f * (-k[0] * k[1] / kk));
-      o[2] = (R)(f * (-k[0] * k[2] / kk));
-      o[3] = (R)(f * (1.0 - k[1] * k[1] / kk));
-      o[4] = (R)(f * (-k[1] * k[2] / kk));
-      o[5] = (R)(f * (1.0 - k[2] * k[2] / kk));
+      const double a2 = alpha * alpha;
+      double t[6] = {0, 0, 0, 0, 0, 0}, k[3], kk = 0, phi = 0;
+      auto add = [&](int n0, int n1, double share) {
+        int s0 = n0 < (K + 1) / 2 ? n0 : n0 - K, s1 = n1 < (K + 1) / 2 ? n1 : n1 - K, s2 = m2;
+        // k = 2 pi (s0 b0 + s1 b1 + s2 b2), b_d = row d of H^-1
+        for (int a = 0; a < 3; a++)
+          k[a] = 2.0 * M_PI *
+                 (s0 * cell.Hi[0 * 3 + a] + s1 * cell.Hi[1 * 3 + a] + s2 * cell.Hi[2 * 3 + a]);
+        kk = k[0] * k[0] + k[1] * k[1] + k[2] * k[2];
+        phi = (1.0 - kk / 3.0) * (1.0 + kk / (4.0 * a2) + kk * kk / (8.0 * a2 * a2)) * 6.0 *
+              M_PI / kk * exp(-kk / (4.0 * a2)) / cell.V;
+        double f = share * phi * bsq[n0] * bsq[K + n1] * bsq[2 * K + m2];
+        t[0] += f * (1.0 - k[0] * k[0] / kk);
+        t[1] += f * (-k[0] * k[1] / kk);
+        t[2] += f * (-k[0] * k[2] / kk);
+        t[3] += f * (1.0 - k[1] * k[1] / kk);
+        t[4] += f * (-k[1] * k[2] / kk);
+        t[5] += f * (1.0 - k[2] * k[2] / kk);
+      };
+      // on the planes m2 = 0 and K/2 a point and its mirror are both stored:
+      // their mean is even in k for the Nyquist indices of an even K too, so
+      // the two right-hand sides of a pair do not mix
+      bool both = m2 == 0 || 2 * m2 == K;
+      if (both) add((K - m0) % K, (K - m1) % K, 0.5);
+      add(m0, m1, both ? 0.5 : 1.0);
+      for (int a = 0; a < 6; a++) o[a] = (R)t[a];
       double mult = (m2 == 0 || (K % 2 == 0 && m2 == K / 2)) ? 1.0 : 2.0;
       sxy = -mult * phi * k[0] * k[1] / kk;
       sxz = -mult * phi * k[0] * k[2] / kk;
@@ -334,26 +205,6 @@ __global__ void k_pme_soff_fin(const double* __restrict__ part, int nb, double* 
     __syncthreads();
   }
   if (threadIdx.x < 3) soff[threadIdx.x] = red[threadIdx.x][0];
-}
-
-// Right-hand side blockIdx.y owns the spectra 3 n entries further on.
-template <typename R, typename Cx>
-__global__ void k_pme_apply_influence(const R* __restrict__ infl, Cx* spec, size_t n) {
-  size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  spec += (size_t)blockIdx.y * 3 * n;
-  const R* t = infl + 6 * e;
-  Cx x = spec[e], y = spec[n + e], z = spec[2 * n + e];
-  Cx u, v, w;
-  u.x = t[0] * x.x + t[1] * y.x + t[2] * z.x;
-  u.y = t[0] * x.y + t[1] * y.y + t[2] * z.y;
-  v.x = t[1] * x.x + t[3] * y.x + t[4] * z.x;
-  v.y = t[1] * x.y + t[3] * y.y + t[4] * z.y;
-  w.x = t[2] * x.x + t[4] * y.x + t[5] * z.x;
-  w.y = t[2] * x.y + t[4] * y.y + t[5] * z.y;
-  spec[e] = u;
-  spec[n + e] = v;
-  spec[2 * n + e] = w;
 }
 
 // Real-space Beenakker kernel t1 I + t2 r r^T/r^2 (shear/src/main26.c:
@@ -399,73 +250,60 @@ __device__ __forceinline__ void pair_terms(double alpha, double alpha_ref, doubl
   }
 }
 
-// out_r,c(i) = sum_g W_i(g) grid_r,c(g) + self v_r,c(i) - (S_off v_r(i))_c
-//              + sum_j (T_ij v_r,j)_c (row list)
-// for the right-hand sides r0 .. r0 + kc - 1 of chunk blockIdx.y (r0 =
-// KG blockIdx.y; KG = 1 for single products).  One warp per bead: the lanes
-// share the stencil points (weights computed once for the chunk) and the pair
-// row (pair terms, positions and minimum image once for the chunk), then a
-// butterfly reduction; lane e < 3 kc writes component e % 3 of right-hand
-// side r0 + e / 3.
-template <int P, typename R, int KG, bool PK, bool RS = false>
-__global__ void __launch_bounds__(256) k_pme_gather(
-    const int* __restrict__ base, const double* __restrict__ w, int N, int K,
-    const R* __restrict__ grid, int k, double self, const double* __restrict__ soff, VecIn v,
-    size_t vr, const int* __restrict__ rcnt, const int* __restrict__ rrows,
-    const double4* __restrict__ pos, Cell cell, const R* __restrict__ tt, int rcap,
-    double* o0, double* o1, double* o2, int ostride, size_t orr,
-    const double* __restrict__ rsum) {
-  constexpr int NA = 3 * KG;
+// Self part and the interpolated value of component c, right-hand side r, bead
+// i: mesh + self v - (S_off v)_c.
+__device__ __forceinline__ double with_self(double mesh, int c, double self,
+                                            const double* __restrict__ soff, const VecIn& v,
+                                            size_t o) {
+  double v0 = v.p[0][o], v1 = v.p[1][o], v2 = v.p[2][o];
+  double sxy = soff[0], sxz = soff[1], syz = soff[2];
+  if (c == 0) return mesh + self * v0 - sxy * v1 - sxz * v2;
+  if (c == 1) return mesh + self * v1 - sxy * v0 - syz * v2;
+  return mesh + self * v2 - sxz * v0 - syz * v1;
+}
+
+// What the last kernel of a product adds to its real-space sums and where it
+// writes them.
+struct Finish {
+  const double* val;  // the interpolated values, 6 per bead and pair
+  int N;
+  double self;
+  const double* soff;
+  VecIn v;
+  size_t vr;
+  double* o[3];
+  int ostride;
+  size_t orr;
+  int k;
+
+  // value e = 3 h + c of packed pair pr, real-space sum x
+  __device__ __forceinline__ void write(double x, int pr, int e, int i) const {
+    int r = 2 * pr + e / 3, c = e % 3;
+    if (r >= k) return;
+    double mesh = x + val[((size_t)pr * N + i) * 6 + e];
+    double* dst = c == 0 ? o[0] : c == 1 ? o[1] : o[2];
+    dst[(size_t)r * orr + (size_t)i * ostride] =
+        with_self(mesh, c, self, soff, v, (size_t)r * vr + (size_t)i * v.stride);
+  }
+};
+
+// The real-space sums from (t1, t2 / r^2) per pair, the minimum image formed
+// here, FP64 sums (FP64 contexts, and FP32 ones without the stored (t1, w)),
+// and the rest of the product, for packed pair blockIdx.y.  One warp per bead, lanes over the pair row,
+// a butterfly, lane e < 6 writes value e.
+template <typename R>
+__global__ void __launch_bounds__(256)
+    k_pme_real_rows(int N, const int* __restrict__ rcnt, const int* __restrict__ rrows,
+                    const double4* __restrict__ pos, Cell cell, const R* __restrict__ tt, int rcap,
+                    Finish fin) {
+  constexpr int KG = 2, NA = 3 * KG;
   int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= N) return;
-  int r0 = KG * blockIdx.y, kc = min(KG, k - r0), nj = 3 * kc;
-  size_t K3 = (size_t)K * K * K;
-  const R* gbase = grid + (size_t)r0 * 3 * K3;
-  const double* w0 = w + ((size_t)3 * i + 0) * kMaxOrder;
-  const double* w1 = w + ((size_t)3 * i + 1) * kMaxOrder;
-  const double* w2 = w + ((size_t)3 * i + 2) * kMaxOrder;
-  int b0 = base[3 * i], b1 = base[3 * i + 1], b2 = base[3 * i + 2];
+  const VecIn& v = fin.v;
+  int r0 = KG * blockIdx.y, kc = min(KG, fin.k - r0);
   double u[NA];
 #pragma unroll
   for (int e = 0; e < NA; e++) u[e] = 0.0;
-#pragma unroll
-  for (int it = 0; it < (P * P * P + 31) / 32; it++) {
-    int q = lane + 32 * it;
-    if (q >= P * P * P) break;
-    int c = q % P, b = (q / P) % P, a = q / (P * P);
-    int g0 = b0 - a, g1 = b1 - b, g2 = b2 - c;
-    g0 += g0 < 0 ? K : 0;
-    g1 += g1 < 0 ? K : 0;
-    g2 += g2 < 0 ? K : 0;
-    double wt = w0[a] * w1[b] * w2[c];
-    const R* gp = gbase + ((size_t)g0 * K + g1) * K + g2;
-    if constexpr (PK) {
-      // packed pair blockIdx.y: right-hand sides r0, r0 + 1 as real and
-      // imaginary parts (the grid argument is the pairs' complex grid)
-      using C2 = typename Pair<R>::T;
-      const C2* gq = (const C2*)grid + (size_t)blockIdx.y * 3 * K3 +
-                     (((size_t)g0 * K + g1) * K + g2);
-      C2 x0 = gq[0], x1 = gq[K3], x2 = gq[2 * K3];
-      u[0] += wt * (double)x0.x;
-      u[1] += wt * (double)x1.x;
-      u[2] += wt * (double)x2.x;
-      u[3] += wt * (double)x0.y;
-      u[4] += wt * (double)x1.y;
-      u[5] += wt * (double)x2.y;
-    } else {
-#pragma unroll
-      for (int r = 0; r < KG; r++) {
-        if (r >= kc) break;
-        const R* gr = gp + (size_t)r * 3 * K3;
-        u[3 * r] += wt * (double)gr[0];
-        u[3 * r + 1] += wt * (double)gr[K3];
-        u[3 * r + 2] += wt * (double)gr[2 * K3];
-      }
-    }
-  }
-  // real-space pairs: the tensor t1 I + t2 d d^T/r^2 of the minimum-image
-  // displacement d; t1 and t2/r^2 are stored per pair (8 or 16 bytes), d is
-  // recomputed from the frozen lab-frame positions (L2-resident)
   int n = rcnt[i];
   const int* prow = rrows + (size_t)i * rcap;
   // the cell is (b1, b2) in the xy plane and L e_z: a 2 x 2 block and L
@@ -473,72 +311,48 @@ __global__ void __launch_bounds__(256) k_pme_gather(
   const double h00 = cell.H[0], h01 = cell.H[1], h10 = cell.H[3], h11 = cell.H[4];
   const double g00 = cell.Hi[0], g01 = cell.Hi[1], g10 = cell.Hi[3], g11 = cell.Hi[4];
   const double Lz = cell.H[8], iLz = cell.Hi[8];
-  if constexpr (RS) {
-    // the real-space sums of this packed pair, formed for all pairs at once
-    // by k_pme_real_pairs (added below)
-  } else {
-    for (int kk = lane; kk < n; kk += 32) {
-      int j = prow[kk];
-      double4 pj = pos[j];
-      double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-      double s0 = g00 * dx + g01 * dy, s1 = g10 * dx + g11 * dy, s2 = iLz * dz;
-      s0 -= rint(s0);
-      s1 -= rint(s1);
-      s2 -= rint(s2);
-      dx = h00 * s0 + h01 * s1;
-      dy = h10 * s0 + h11 * s1;
-      dz = Lz * s2;
-      const R* tk = tt + 2 * ((size_t)i * rcap + kk);
-      double t1 = tk[0], t2r = tk[1];  // t1 and t2 / r^2 of the pair
+  for (int kk = lane; kk < n; kk += 32) {
+    int j = prow[kk];
+    double4 pj = pos[j];
+    double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+    double s0 = g00 * dx + g01 * dy, s1 = g10 * dx + g11 * dy, s2 = iLz * dz;
+    s0 -= rint(s0);
+    s1 -= rint(s1);
+    s2 -= rint(s2);
+    dx = h00 * s0 + h01 * s1;
+    dy = h10 * s0 + h11 * s1;
+    dz = Lz * s2;
+    const R* tk = tt + 2 * ((size_t)i * rcap + kk);
+    double t1 = tk[0], t2r = tk[1];  // t1 and t2 / r^2 of the pair
 #pragma unroll
-      for (int r = 0; r < KG; r++) {
-        if (r >= kc) break;
-        size_t o = (size_t)(r0 + r) * vr + (size_t)j * v.stride;
-        double x0 = v.p[0][o], x1 = v.p[1][o], x2 = v.p[2][o];
-        double qq = t2r * (dx * x0 + dy * x1 + dz * x2);
-        u[3 * r] += t1 * x0 + qq * dx;
-        u[3 * r + 1] += t1 * x1 + qq * dy;
-        u[3 * r + 2] += t1 * x2 + qq * dz;
-      }
+    for (int r = 0; r < KG; r++) {
+      if (r >= kc) break;
+      size_t o = (size_t)(r0 + r) * fin.vr + (size_t)j * v.stride;
+      double x0 = v.p[0][o], x1 = v.p[1][o], x2 = v.p[2][o];
+      double qq = t2r * (dx * x0 + dy * x1 + dz * x2);
+      u[3 * r] += t1 * x0 + qq * dx;
+      u[3 * r + 1] += t1 * x1 + qq * dy;
+      u[3 * r + 2] += t1 * x2 + qq * dz;
     }
   }
-
 #pragma unroll
-  for (int e = 0; e < NA; e++) {
-    if (e >= nj) break;
+  for (int e = 0; e < NA; e++)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) u[e] += __shfl_xor_sync(0xffffffffu, u[e], o);
-  }
   double mine = 0.0;
 #pragma unroll
   for (int e = 0; e < NA; e++)
     if (e == lane) mine = u[e];
-  if constexpr (RS)
-    if (lane < nj) mine += rsum[((size_t)blockIdx.y * N + i) * 6 + lane];
-  if (lane < nj) {
-    int r = lane / 3, c = lane % 3;
-    size_t o = (size_t)(r0 + r) * vr + (size_t)i * v.stride;
-    double vi0 = v.p[0][o], vi1 = v.p[1][o], vi2 = v.p[2][o];
-    double sxy = soff[0], sxz = soff[1], syz = soff[2];
-    double out;
-    if (c == 0)
-      out = mine + self * vi0 - sxy * vi1 - sxz * vi2;
-    else if (c == 1)
-      out = mine + self * vi1 - sxy * vi0 - syz * vi2;
-    else
-      out = mine + self * vi2 - sxz * vi0 - syz * vi1;
-    double* dst = c == 0 ? o0 : (c == 1 ? o1 : o2);
-    dst[(size_t)(r0 + r) * orr + (size_t)i * ostride] = out;
-  }
+  if (lane < NA) fin.write(mine, blockIdx.y, lane, i);
 }
 
-// The real-space part of a block product (FP32 block products): for every
-// packed pair p and bead i, rsum[(p N + i) 6 + 3h + c] = sum_j (T_ij v_j)_c of
-// the pair's vector h (0: real part, 1: imaginary part), for NP pairs (at
-// most five) in one pass over the pair rows.  One warp per bead; a lane takes
+// The real-space part of a block product and the rest of it (FP32 block
+// products): for every packed pair p0 + p and bead i, sum_j (T_ij v_j)_c of the
+// pair's vector h (0: real part, 1: imaginary part), for NP pairs (at most
+// five) in one pass over the pair rows.  One warp per bead; a lane takes
 // row entries, each an index and the preparation's float4 (t1, w): T_ij =
 // t1 I + s w w^T, the sign s of t2 kept in the lowest mantissa bit of t1;
-// then it reads the neighbour's six inputs of every pair (the spread's
+// then it reads the neighbour's six inputs of every pair (the packed record
 // vpk[(p N + j) 8], a float4 and a float2) and adds T_ij v into 6 NP FP32
 // partial sums (a lane sums about a 32nd of the row).  The
 // partials are summed over the warp by a transposing butterfly (31 exchanges
@@ -547,7 +361,7 @@ __global__ void __launch_bounds__(256) k_pme_gather(
 template <int NP>
 __global__ void __launch_bounds__(256, 3) k_pme_real_pairs(
     const int* __restrict__ rcnt, const int* __restrict__ rrows, const float4* __restrict__ rw,
-    int rcap, const float* __restrict__ vpk, int N, double* __restrict__ rsum) {
+    int rcap, const float* __restrict__ vpk, int N, int p0, Finish fin) {
   constexpr int NV = 6 * NP;
   int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= N) return;
@@ -563,7 +377,7 @@ __global__ void __launch_bounds__(256, 3) k_pme_real_pairs(
     float s = (__float_as_uint(q.x) & 1u) ? -1.f : 1.f;
 #pragma unroll
     for (int p = 0; p < NP; p++) {
-      const float4* vj = (const float4*)(vpk + ((size_t)p * N + j) * 8);
+      const float4* vj = (const float4*)(vpk + ((size_t)(p0 + p) * N + j) * 8);
       float4 a = __ldg(vj);
       float2 b = __ldg((const float2*)(vj + 1));
       float qa = s * (q.y * a.x + q.z * a.y + q.w * a.z);
@@ -603,47 +417,8 @@ __global__ void __launch_bounds__(256, 3) k_pme_real_pairs(
       d[e] = keep + __shfl_xor_sync(0xffffffffu, send, off);
     }
   }
-  // value e = 6 p + 3 h + c
-  if (lane < NV) rsum[((size_t)(lane / 6) * N + i) * 6 + lane % 6] = d[0];
-}
-
-// The real-space part of a single product (FP32 contexts that hold the
-// mobility build's pair data): one warp per bead; per row entry the index
-// and (t1, w) as for the block products, the neighbour's three input values
-// taken to FP32, FP32 partial sums per lane, summed over the warp in FP64;
-// rsum[6 i + c] for c < 3, which the interpolation adds.
-__global__ void __launch_bounds__(256) k_pme_real_single(
-    const int* __restrict__ rcnt, const int* __restrict__ rrows, const float4* __restrict__ rw,
-    int rcap, VecIn v, int N, double* __restrict__ rsum) {
-  int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (i >= N) return;
-  float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-  int n = rcnt[i];
-  const int* prow = rrows + (size_t)i * rcap;
-  const float4* prw = rw + (size_t)i * rcap;
-  for (int kk = lane; kk < n; kk += 32) {
-    int j = __ldg(prow + kk);
-    float4 q = __ldg(prw + kk);
-    size_t o = (size_t)j * v.stride;
-    float x0 = (float)v.p[0][o], x1 = (float)v.p[1][o], x2 = (float)v.p[2][o];
-    float d = q.y * x0 + q.z * x1 + q.w * x2;
-    d = (__float_as_uint(q.x) & 1u) ? -d : d;
-    a0 += q.x * x0 + d * q.y;
-    a1 += q.x * x1 + d * q.z;
-    a2 += q.x * x2 + d * q.w;
-  }
-  double d0 = a0, d1 = a1, d2 = a2;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    d0 += __shfl_xor_sync(0xffffffffu, d0, o);
-    d1 += __shfl_xor_sync(0xffffffffu, d1, o);
-    d2 += __shfl_xor_sync(0xffffffffu, d2, o);
-  }
-  if (lane == 0) {
-    rsum[6 * (size_t)i] = d0;
-    rsum[6 * (size_t)i + 1] = d1;
-    rsum[6 * (size_t)i + 2] = d2;
-  }
+  // value 6 p + 3 h + c
+  if (lane < NV) fin.write(d[0], p0 + lane / 6, lane % 6, i);
 }
 
 // Cells of the real-space list (fractional, width >= rc).
@@ -829,19 +604,17 @@ int pme_alloc(bd_ctx* c) {
   size_t K3 = (size_t)K * K * K, Ks = (size_t)K * K * (K / 2 + 1);
   c->pme_f32 = c->p.precision == BD_PREC_FP32;
   size_t es = c->pme_f32 ? 4 : 8;  // grid, spectrum, influence and pair tensors
-  // grids and spectra for the largest number of right-hand sides of a product
+  // the packed pairs' grids for the largest number of right-hand sides
   size_t nr = (size_t)std::max(1, c->nbk);
-  CU(cudaMalloc(&c->pme_grid, es * 3 * K3 * nr));
-  // the spectra; for products of several right-hand sides the same buffer
-  // holds the packed pairs' complex grids (3 ceil(k/2) K^3 complex values)
-  size_t spec_bytes = std::max(2 * es * 3 * Ks * nr, nr > 1 ? 2 * es * 3 * K3 * ((nr + 1) / 2) : 0);
-  CU(cudaMalloc(&c->pme_spec, spec_bytes));
+  size_t grid_bytes = 2 * es * 3 * K3 * ((nr + 1) / 2);
+  CU(cudaMalloc(&c->pme_grid, grid_bytes));
+  CU(cudaMalloc(&c->pme_tw, 2 * es * K));
   CU(cudaMalloc(&c->pme_infl, es * 6 * Ks));
   CU(cudaMalloc(&c->pme_bsq, 8 * 3 * (size_t)K));
   c->pme_nblk = (int)((Ks + 255) / 256);
   CU(cudaMalloc(&c->pme_soff, 8 * (3 * (size_t)c->pme_nblk + 3)));
   CU(cudaMalloc(&c->pme_base, 4 * 3 * (size_t)N));
-  CU(cudaMalloc(&c->pme_w, 8 * 3 * (size_t)N * kMaxOrder));
+  CU(cudaMalloc(&c->pme_w, es * 3 * (size_t)N * kMaxOrder));
   // default row cap: 2.5 times the mean number of beads within the cutoff at
   // the system's density, at least 512, a multiple of 32
   if (c->p.pme_max_pairs > 0) {
@@ -857,9 +630,8 @@ int pme_alloc(bd_ctx* c) {
   CU(cudaMalloc(&c->rl_pos, 32 * (size_t)N));
   if (c->pme_f32 && nr > 1) {
     CU(cudaMalloc(&c->pme_vpk, 32 * (size_t)N * ((nr + 1) / 2)));
-    CU(cudaMalloc(&c->pme_rsum, 48 * (size_t)N * ((nr + 1) / 2)));
     CU(cudaMalloc(&c->rl_w, 16 * (size_t)N * c->rl_cap));
-    c->bytes += 80 * (size_t)N * ((nr + 1) / 2) + 16 * (size_t)N * c->rl_cap;
+    c->bytes += 32 * (size_t)N * ((nr + 1) / 2) + 16 * (size_t)N * c->rl_cap;
   } else {  // the products of contexts with rl_w read the pair tensors there
     CU(cudaMalloc(&c->rl_tt, 2 * es * (size_t)N * c->rl_cap));
     c->bytes += 2 * es * (size_t)N * c->rl_cap;
@@ -871,19 +643,27 @@ int pme_alloc(bd_ctx* c) {
   CU(cudaMalloc(&c->rl_cell_start, 4 * (size_t)(c->rl_ncell_cap + 1)));
   CU(cudaMalloc(&c->rl_cursor, 4 * (size_t)c->rl_ncell_cap));
   CU(cudaMemsetAsync(c->rl_cell_count, 0, 4 * (size_t)c->rl_ncell_cap, c->stream));
-  c->bytes += es * (3 * K3 * nr + 6 * Ks) + spec_bytes + 24 * (size_t)K + 12 * (size_t)N +
-              24 * (size_t)N * kMaxOrder + 4 * (size_t)N + (size_t)N * c->rl_cap * 4 + 32 * (size_t)N +
+  c->bytes += grid_bytes + es * 6 * Ks + (24 + 2 * es) * (size_t)K + 12 * (size_t)N +
+              3 * es * (size_t)N * kMaxOrder + 4 * (size_t)N + (size_t)N * c->rl_cap * 4 + 32 * (size_t)N +
               36 * (size_t)N + 12 * (size_t)c->rl_ncell_cap;
-  int n[3] = {K, K, K};
-  cufftHandle f, b;
-  CF(cufftPlanMany(&f, 3, n, nullptr, 1, (int)K3, nullptr, 1, (int)Ks,
-                   c->pme_f32 ? CUFFT_R2C : CUFFT_D2Z, 3));
-  CF(cufftPlanMany(&b, 3, n, nullptr, 1, (int)Ks, nullptr, 1, (int)K3,
-                   c->pme_f32 ? CUFFT_C2R : CUFFT_Z2D, 3));
-  CF(cufftSetStream(f, c->stream));
-  CF(cufftSetStream(b, c->stream));
-  c->pme_plan_f = (int)f;
-  c->pme_plan_b = (int)b;
+  if (!fft_has_size(K)) {
+    // one pair's three interleaved components, in place
+    int n[3] = {K, K, K};
+    cufftHandle f;
+    CF(cufftPlanMany(&f, 3, n, n, 3, 1, n, 3, 1, c->pme_f32 ? CUFFT_C2C : CUFFT_Z2Z, 3));
+    CF(cufftSetStream(f, c->stream));
+    c->pme_plan = (int)f + 1;
+  }
+  std::vector<double> tw(2 * (size_t)K);
+  std::vector<float> tw32(2 * (size_t)K);
+  for (int m = 0; m < K; m++) {
+    tw[2 * m] = cos(2.0 * M_PI * m / K);
+    tw[2 * m + 1] = -sin(2.0 * M_PI * m / K);
+    tw32[2 * m] = (float)tw[2 * m];
+    tw32[2 * m + 1] = (float)tw[2 * m + 1];
+  }
+  CU(cudaMemcpyAsync(c->pme_tw, c->pme_f32 ? (const void*)tw32.data() : (const void*)tw.data(),
+                     2 * es * K, cudaMemcpyHostToDevice, c->stream));
   std::vector<double> bs(3 * (size_t)K);
   bspline_moduli(K, c->pme_p, bs.data());
   for (int d = 1; d < 3; d++)
@@ -893,46 +673,10 @@ int pme_alloc(bd_ctx* c) {
   return BD_OK;
 }
 
-// In-place complex transforms of the 3 ceil(k/2) packed-pair grids of a
-// k-right-hand-side product (one plan, used forward and inverse), created
-// outside any stream capture and kept for up to four values of k (replacing
-// one drops the captured iterations that use it).
-int pme_multi_plan(bd_ctx* c, int k) {
-  int slot = -1;
-  for (int q = 0; q < 4; q++)
-    if (c->pme_mplan_k[q] == k) return BD_OK;
-  for (int q = 0; q < 4 && slot < 0; q++)
-    if (c->pme_mplan_k[q] == 0) slot = q;
-  if (slot < 0) {
-    slot = 3;
-    lanczos_graphs_reset(c);
-    cufftDestroy((cufftHandle)c->pme_mplan_f[slot]);
-    c->pme_mplan_k[slot] = 0;
-  }
-  int K = c->pmeK;
-  size_t K3 = (size_t)K * K * K;
-  int n[3] = {K, K, K};
-  cufftHandle f;
-  CF(cufftPlanMany(&f, 3, n, nullptr, 1, (int)K3, nullptr, 1, (int)K3,
-                   c->pme_f32 ? CUFFT_C2C : CUFFT_Z2Z, 3 * ((k + 1) / 2)));
-  if (cufftSetStream(f, c->stream) != CUFFT_SUCCESS) {
-    cufftDestroy(f);
-    return BD_ERR_CUDA;
-  }
-  c->pme_mplan_f[slot] = (int)f;
-  c->pme_mplan_k[slot] = k;
-  return BD_OK;
-}
-
 void pme_free(bd_ctx* c) {
-  if (c->pme_plan_f) cufftDestroy((cufftHandle)c->pme_plan_f);
-  if (c->pme_plan_b) cufftDestroy((cufftHandle)c->pme_plan_b);
-  for (int q = 0; q < 4; q++)
-    if (c->pme_mplan_k[q]) {
-      cufftDestroy((cufftHandle)c->pme_mplan_f[q]);
-      c->pme_mplan_k[q] = 0;
-    }
-  void* ptrs[] = {c->pme_vpk, c->pme_rsum, c->rl_w, c->rl_need, c->pme_grid, c->pme_spec, c->pme_infl, c->pme_bsq, c->pme_soff, c->pme_base, c->pme_w,
+  if (c->pme_plan) cufftDestroy((cufftHandle)(c->pme_plan - 1));
+  mesh_free(c);
+  void* ptrs[] = {c->pme_vpk, c->rl_w, c->rl_need, c->pme_grid, c->pme_tw, c->pme_infl, c->pme_bsq, c->pme_soff, c->pme_base, c->pme_w,
                   c->rl_cnt, c->rl_rows, c->rl_pos, c->rl_tt, c->rl_cell_of, c->rl_spos, c->rl_cell_count,
                   c->rl_cell_start, c->rl_cursor};
   for (void* q : ptrs)
@@ -984,9 +728,15 @@ int pme_prepare(bd_ctx* c, const Lat& l) {
   double rce = l.treal <= c->tp / 2 ? l.L2yp : 2.0 * l.L2yp;
   double alpha_ref = 4.0 / rce;
   c->launches += 3;
-  k_pme_weights<<<nblk(N, 256), 256, 0, c->stream>>>(cell, c->rx, c->ry, c->rz, cr, sr, N, K,
-                                                     c->pme_p, c->pme_base, c->pme_w,
-                                                     (double4*)c->rl_pos, c->err);
+  if (c->pme_f32)
+    k_pme_weights<float><<<nblk(N, 128), 128, 0, c->stream>>>(
+        cell, c->rx, c->ry, c->rz, cr, sr, N, K, c->pme_p, c->pme_base, (float*)c->pme_w,
+        (double4*)c->rl_pos, c->err);
+  else
+    k_pme_weights<double><<<nblk(N, 128), 128, 0, c->stream>>>(
+        cell, c->rx, c->ry, c->rz, cr, sr, N, K, c->pme_p, c->pme_base, (double*)c->pme_w,
+        (double4*)c->rl_pos, c->err);
+  if ((s = mesh_prepare(c)) != BD_OK) return s;
   if (c->pme_f32)
     k_pme_influence<float><<<c->pme_nblk, 256, 0, c->stream>>>(
         cell, K, alpha, c->pme_bsq, (float*)c->pme_infl, c->pme_soff + 3);
@@ -1062,117 +812,60 @@ int pme_prepare(bd_ctx* c, const Lat& l) {
 }
 
 // out_r = M v_r by PME for k right-hand sides given by component pointers
-// (VecIn) and RHS strides vr (input) and orr (output); k = 1 is the
-// single-vector product with the context's own transforms.
+// (VecIn) and RHS strides vr (input) and orr (output).
 template <typename R, typename Cx>
 static int pme_apply_t(bd_ctx* c, int k, const VecIn& v, size_t vr, double* o0, double* o1,
                        double* o2, int ostride, size_t orr) {
-  int K = c->pmeK, N = c->N, p = c->pme_p;
-  size_t K3 = (size_t)K * K * K, Ks = (size_t)K * K * (K / 2 + 1);
+  int K = c->pmeK, N = c->N, s;
+  size_t K3 = (size_t)K * K * K;
   if (k < 1 || k > std::max(1, c->nbk)) return BD_ERR_ARG;
-  int nb8 = nblk(N, 8);
-  Cell cell;
-  memcpy(cell.H, c->pme_cellbuf, sizeof(cell.H));
-  memcpy(cell.Hi, c->pme_cellbuf + 9, sizeof(cell.Hi));
-  cell.V = c->pme_cellbuf[18];
-  c->launches += 3;  // spread, influence, gather (the transforms are cuFFT's)
-  if (k == 1) {
-    // one right-hand side: three real grids, R2C / C2R
-    R* grid = (R*)c->pme_grid;
-    Cx* spec = (Cx*)c->pme_spec;
-    CU(cudaMemsetAsync(grid, 0, sizeof(R) * 3 * K3, c->stream));
-#define PME_SPREAD(P_) \
-  k_pme_spread<P_, R, 1><<<nb8, 256, 0, c->stream>>>(c->pme_base, c->pme_w, N, K, v, vr, 1, grid)
-    switch (p) {
-      case 4: PME_SPREAD(4); break;
-      case 6: PME_SPREAD(6); break;
-      default: PME_SPREAD(8);
-    }
-#undef PME_SPREAD
-    if constexpr (sizeof(R) == 4)
-      CF(cufftExecR2C((cufftHandle)c->pme_plan_f, (cufftReal*)grid, (cufftComplex*)spec));
-    else
-      CF(cufftExecD2Z((cufftHandle)c->pme_plan_f, (cufftDoubleReal*)grid,
-                      (cufftDoubleComplex*)spec));
-    k_pme_apply_influence<R, Cx><<<nblk((long long)Ks, 256), 256, 0, c->stream>>>(
-        (const R*)c->pme_infl, spec, Ks);
-    if constexpr (sizeof(R) == 4)
-      CF(cufftExecC2R((cufftHandle)c->pme_plan_b, (cufftComplex*)spec, (cufftReal*)grid));
-    else
-      CF(cufftExecZ2D((cufftHandle)c->pme_plan_b, (cufftDoubleComplex*)spec,
-                      (cufftDoubleReal*)grid));
-    // FP32 with the stored pair data: the real-space sums in their own pass
-    // (as for the block products), the interpolation then only reads the grid
-    bool rs = sizeof(R) == 4 && c->rl_w && c->pme_rsum;
-    if (rs) {
-      c->launches++;
-      k_pme_real_single<<<nb8, 256, 0, c->stream>>>(c->rl_cnt, c->rl_rows, c->rl_w, c->rl_cap, v,
-                                                     N, c->pme_rsum);
-    }
-#define PME_GATHER(P_, RS_)                                                                   \
-  k_pme_gather<P_, R, 1, false, RS_><<<nb8, 256, 0, c->stream>>>(                             \
-      c->pme_base, c->pme_w, N, K, grid, 1, c->pme_self, c->pme_soff, v, vr, c->rl_cnt,       \
-      c->rl_rows, (const double4*)c->rl_pos, cell, (const R*)c->rl_tt, c->rl_cap, o0, o1, o2, \
-      ostride, orr, RS_ ? c->pme_rsum : nullptr)
-    if (rs) {
-      switch (p) {
-        case 4: PME_GATHER(4, true); break;
-        case 6: PME_GATHER(6, true); break;
-        default: PME_GATHER(8, true);
+  int nb8 = nblk(N, 8), np = (k + 1) / 2;
+  Cx* g = (Cx*)c->pme_grid;
+  if ((s = mesh_spread(c, k, v, vr, g)) != BD_OK) return s;
+  if (!c->pme_plan) {
+    s = sizeof(R) == 4 ? fft_influence_f32(c, K, g, np, c->pme_infl, c->pme_tw)
+                       : fft_influence_f64(c, K, g, np, c->pme_infl, c->pme_tw);
+    if (s != BD_OK) return s;
+  } else {
+    for (int dir : {CUFFT_FORWARD, CUFFT_INVERSE}) {
+      for (int p = 0; p < np; p++) {
+        Cx* gp = g + 3 * K3 * p;
+        if constexpr (sizeof(R) == 4)
+          CF(cufftExecC2C((cufftHandle)(c->pme_plan - 1), (cufftComplex*)gp, (cufftComplex*)gp, dir));
+        else
+          CF(cufftExecZ2Z((cufftHandle)(c->pme_plan - 1), (cufftDoubleComplex*)gp,
+                          (cufftDoubleComplex*)gp, dir));
       }
-    } else {
-      switch (p) {
-        case 4: PME_GATHER(4, false); break;
-        case 6: PME_GATHER(6, false); break;
-        default: PME_GATHER(8, false);
+      if (dir == CUFFT_FORWARD) {
+        c->launches++;
+        k_pme_apply_influence<R, Cx><<<nblk((long long)K3 * np, 256), 256, 0, c->stream>>>(
+            (const R*)c->pme_infl, g, K, (size_t)np);
       }
     }
-#undef PME_GATHER
-    return BD_OK;
   }
-  // k >= 2: packed pairs in the spectrum buffer, in-place complex transforms
-  int q = 0;
-  while (q < 4 && c->pme_mplan_k[q] != k) q++;
-  if (q == 4) return BD_ERR_STATE;  // pme_multi_plan(c, k) first
-  cufftHandle plan = (cufftHandle)c->pme_mplan_f[q];
-  int np = (k + 1) / 2;
-  using C2 = typename Pair<R>::T;
-  C2* cg = (C2*)c->pme_spec;
-  CU(cudaMemsetAsync(cg, 0, sizeof(C2) * 3 * K3 * np, c->stream));
-  dim3 gp(nb8, np);
-  float* vpk = sizeof(R) == 4 ? c->pme_vpk : nullptr;
-#define PME_SPREAD(P_)                                                                       \
-  k_pme_spread_pairs<P_, R><<<gp, 256, 0, c->stream>>>(c->pme_base, c->pme_w, N, K, v, vr, k, cg, \
-                                                       vpk)
-  switch (p) {
-    case 4: PME_SPREAD(4); break;
-    case 6: PME_SPREAD(6); break;
-    default: PME_SPREAD(8);
-  }
-#undef PME_SPREAD
-  if constexpr (sizeof(R) == 4)
-    CF(cufftExecC2C(plan, (cufftComplex*)cg, (cufftComplex*)cg, CUFFT_FORWARD));
-  else
-    CF(cufftExecZ2Z(plan, (cufftDoubleComplex*)cg, (cufftDoubleComplex*)cg, CUFFT_FORWARD));
-  k_pme_apply_influence_full<R, C2><<<nblk((long long)K3 * np, 256), 256, 0, c->stream>>>(
-      (const R*)c->pme_infl, cg, K, (size_t)np);
-  if constexpr (sizeof(R) == 4)
-    CF(cufftExecC2C(plan, (cufftComplex*)cg, (cufftComplex*)cg, CUFFT_INVERSE));
-  else
-    CF(cufftExecZ2Z(plan, (cufftDoubleComplex*)cg, (cufftDoubleComplex*)cg, CUFFT_INVERSE));
-  // FP32: the real-space sums of the packed pairs, in passes over the rows of
-  // up to five pairs (30 FP32 partial sums per lane at 80 registers)
-  double* rsum = nullptr;
+  if ((s = mesh_gather(c, k, g)) != BD_OK) return s;
+  Finish fin;
+  fin.val = c->mesh_val;
+  fin.N = N;
+  fin.self = c->pme_self;
+  fin.soff = c->pme_soff;
+  fin.v = v;
+  fin.vr = vr;
+  fin.o[0] = o0;
+  fin.o[1] = o1;
+  fin.o[2] = o2;
+  fin.ostride = ostride;
+  fin.orr = orr;
+  fin.k = k;
   if constexpr (sizeof(R) == 4) {
-    if (vpk && c->pme_rsum && c->rl_w) {
-      rsum = c->pme_rsum;
+    // FP32 contexts with the stored (t1, w): passes over the rows of up to five
+    // pairs (30 FP32 partial sums per lane at 80 registers)
+    if (c->rl_w) {
       for (int p0 = 0; p0 < np; p0 += 5) {
-        const float* vp = vpk + (size_t)p0 * N * 8;
-        double* rs = rsum + (size_t)p0 * N * 6;
         c->launches++;
 #define PME_REAL(NP_)                                                                        \
   k_pme_real_pairs<NP_><<<nb8, 256, 0, c->stream>>>(c->rl_cnt, c->rl_rows, c->rl_w, c->rl_cap, \
-                                                    vp, N, rs)
+                                                    c->pme_vpk, N, p0, fin)
         switch (std::min(5, np - p0)) {
           case 1: PME_REAL(1); break;
           case 2: PME_REAL(2); break;
@@ -1182,27 +875,17 @@ static int pme_apply_t(bd_ctx* c, int k, const VecIn& v, size_t vr, double* o0, 
         }
 #undef PME_REAL
       }
+      return BD_OK;
     }
   }
-#define PME_GATHER(P_, RS_)                                                                   \
-  k_pme_gather<P_, R, 2, true, RS_><<<gp, 256, 0, c->stream>>>(                               \
-      c->pme_base, c->pme_w, N, K, (const R*)cg, k, c->pme_self, c->pme_soff, v, vr,          \
-      c->rl_cnt, c->rl_rows, (const double4*)c->rl_pos, cell, (const R*)c->rl_tt, c->rl_cap,  \
-      o0, o1, o2, ostride, orr, rsum)
-  if (rsum) {
-    switch (p) {
-      case 4: PME_GATHER(4, true); break;
-      case 6: PME_GATHER(6, true); break;
-      default: PME_GATHER(8, true);
-    }
-  } else {
-    switch (p) {
-      case 4: PME_GATHER(4, false); break;
-      case 6: PME_GATHER(6, false); break;
-      default: PME_GATHER(8, false);
-    }
-  }
-#undef PME_GATHER
+  Cell cell;
+  memcpy(cell.H, c->pme_cellbuf, sizeof(cell.H));
+  memcpy(cell.Hi, c->pme_cellbuf + 9, sizeof(cell.Hi));
+  cell.V = c->pme_cellbuf[18];
+  c->launches++;
+  k_pme_real_rows<R><<<dim3(nb8, np), 256, 0, c->stream>>>(
+      N, c->rl_cnt, c->rl_rows, (const double4*)c->rl_pos, cell, (const R*)c->rl_tt, c->rl_cap,
+      fin);
   return BD_OK;
 }
 
