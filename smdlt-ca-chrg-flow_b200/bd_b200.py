@@ -24,7 +24,7 @@ ROOT = os.path.dirname(PKG)
 LIB = os.path.join(PKG, "libbd_b200.so")
 INCLUDE = os.path.join(ROOT, "include")
 SOURCES = ["bd_core.cu", "bd_neighbors.cu", "bd_mobility.cu", "bd_mc.cu", "bd_lanczos.cu",
-           "bd_noalloc.cu", "bd_pme.cu", "bd_mesh.cu", "bd_fft32.cu", "bd_fft64.cu", "bd_precond.cu", "bd_mpnn.cu", "bd_coulomb.cu",
+           "bd_noalloc.cu", "bd_pme.cu", "bd_mesh.cu", "bd_real.cu", "bd_fft32.cu", "bd_fft64.cu", "bd_precond.cu", "bd_mpnn.cu", "bd_coulomb.cu",
            "bd_batch.cu", "bd_catea.cu", "bd_msd.cu", "bd_output.cu"]
 CUDA_LIB = "/usr/local/cuda/lib64"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

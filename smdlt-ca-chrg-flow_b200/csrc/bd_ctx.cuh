@@ -194,23 +194,19 @@ struct bd_ctx {
   void *pme_w;       // per bead spline weights, 3 x N x 8 (FP64 or FP32, as the grids)
   int pme_plan;      // 1 + cuFFT plan of one pair's grid, for sizes bd_fft.cuh does not
                      // cover (0: none)
-  int rl_cap, rl_ncell_cap;  // real-space pair rows
+  // real-space rows of groups of four beads (bd_real.cu)
+  int rl_cap, rl_ncell_cap;
   int *rl_cnt, *rl_rows, *rl_cell_of, *rl_cell_count, *rl_cell_start, *rl_cursor;
   int *rl_need;      // longest pair row of the last build that overflowed the cap (0: none)
   void *rl_pos;      // lab-frame positions of the last preparation (double4)
   void *rl_spos;     // the same in real-space cell order, bead index in w
-  float *pme_vpk;    // FP32 block products: per packed pair and bead the pair's
-                     // 6 input values (+2 padding), written by the spread
-  void *rl_tt;       // per pair t1 and t2 / r^2 of the real-space tensor (FP64 or FP32)
-  float4 *rl_w;      // FP32 block products: per pair (t1, w), w = sqrt(|t2| / r^2) d, the sign
-                     // of t2 in the lowest mantissa bit of t1
+  void *pme_vpk;     // a product's input values, packed pairs side by side per bead and component
+  void *rl_w;        // per entry the four tensors (t1, w), FP64 or FP32
   // spreading by grid columns and interpolation (bd_mesh.cu): up to two column
   // layouts (packed pairs per warp), beads per column and base index, starts
   int mesh_ng[2];
   int *mesh_ent[2], *mesh_bin[2], *mesh_sums, *mesh_cursor;
   double *mesh_val;  // interpolated values, 6 per bead and pair
-  double pme_cellbuf[19];  // its cell: H, H^-1, volume
-  double pme_alpha_ref;    // calcHI's split parameter at that step
 
   size_t bytes;
 

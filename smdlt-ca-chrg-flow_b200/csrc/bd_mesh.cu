@@ -158,23 +158,23 @@ __global__ void __launch_bounds__(256) k_scan_place(int* a, size_t n, const int*
   }
 }
 
-// FP32 values of a pair of right-hand sides, per bead six (re xyz, im xyz)
-// and two zeros: one 32-byte record for the spreading and the pair sums.
-__global__ void k_mesh_pack(VecIn v, size_t vr, int k, int N, float* vpk) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, p = blockIdx.y;
+// The values of the packed pairs for the spreading and the real-space sums:
+// component c of pair p (both right-hand sides) at vpk[(c N + i) np + p], a
+// bead's pairs side by side.
+template <typename T>
+__global__ void k_mesh_pack(VecIn v, size_t vr, int k, int np, int N, T* vpk) {
+  using R = decltype(vpk->x);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, p = blockIdx.y;
   if (i >= N) return;
-  size_t oa = (size_t)(2 * p) * vr + (size_t)i * v.stride;
-  float4 x = make_float4((float)v.p[0][oa], (float)v.p[1][oa], (float)v.p[2][oa], 0.f);
-  float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (2 * p + 1 < k) {
-    size_t ob = oa + vr;
-    x.w = (float)v.p[0][ob];
-    y.x = (float)v.p[1][ob];
-    y.y = (float)v.p[2][ob];
+  const size_t oa = (size_t)(2 * p) * vr + (size_t)i * v.stride;
+  const bool two = 2 * p + 1 < k;
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    T x;
+    x.x = (R)v.p[c][oa];
+    x.y = two ? (R)v.p[c][oa + vr] : (R)0;
+    vpk[((size_t)c * N + i) * np + p] = x;
   }
-  float4* o = (float4*)(vpk + ((size_t)p * N + i) * 8);
-  o[0] = x;
-  o[1] = y;
 }
 
 // ---------------------------------------------------------------------------
@@ -255,10 +255,7 @@ struct SpreadArgs {
   const int* ent;
   const int* bin;
   int K, npz, npatch, nseg, nset, np, N;
-  VecIn v;
-  size_t vr;
-  int k;
-  const float* vpk;  // packed values, or null: read from v
+  const void* vpk;  // packed values
 };
 
 template <int P, typename R, int NG, int CY, int CZ, bool ONE>
@@ -337,19 +334,10 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2) k_mesh_spread(Spr
 #pragma unroll
     for (int u = 0; u < NG; u++) {
       const int p = min(set * NG + u, m.np - 1);
-      if (sizeof(R) == 4 && m.vpk) {
-        const float4* q = (const float4*)(m.vpk + ((size_t)p * m.N + i) * 8);
-        float4 a = q[0];
-        float2 b = *(const float2*)(q + 1);
-        set_pair(r.f[u][0], a.x, a.w);
-        set_pair(r.f[u][1], a.y, b.x);
-        set_pair(r.f[u][2], a.z, b.y);
-      } else {
-        const size_t oa = (size_t)(2 * p) * m.vr + (size_t)i * m.v.stride;
-        const bool two = 2 * p + 1 < m.k;
 #pragma unroll
-        for (int c = 0; c < 3; c++)
-          set_pair(r.f[u][c], (R)m.v.p[c][oa], two ? (R)m.v.p[c][oa + m.vr] : (R)0);
+      for (int c = 0; c < 3; c++) {
+        const T a = ((const T*)m.vpk)[((size_t)c * m.N + i) * m.np + p];
+        set_pair(r.f[u][c], a.x, a.y);
       }
     }
   };
@@ -503,11 +491,11 @@ int most_touched(int K, int P, int w) {
 }
 
 template <int P, typename R>
-void launch_spread(bd_ctx* c, int ng, int nb, const SpreadArgs& m, R* grid) {
+void launch_spread(bd_ctx* c, int k, int ng, int nb, const SpreadArgs& m, R* grid) {
 #define SPREAD(...) k_mesh_spread<P, R, __VA_ARGS__><<<nb, 128, 0, c->stream>>>(m, grid)
   switch (ng) {
     case 1:
-      if (m.k == 1)
+      if (k == 1)
         SPREAD(1, 4, 8, true);
       else
         SPREAD(1, 4, 8, false);
@@ -539,20 +527,16 @@ int spread_t(bd_ctx* c, int k, const VecIn& v, size_t vr, R* grid) {
   m.nseg = segments(K, m.npatch * m.nset);
   m.np = np;
   m.N = c->N;
-  m.v = v;
-  m.vr = vr;
-  m.k = k;
   m.vpk = c->pme_vpk;
-  if (c->pme_vpk) {
-    c->launches++;
-    k_mesh_pack<<<dim3(nblk(c->N, 256), np), 256, 0, c->stream>>>(v, vr, k, c->N, c->pme_vpk);
-  }
+  c->launches++;
+  k_mesh_pack<<<dim3(nblk(c->N, 128), np), 128, 0, c->stream>>>(
+      v, vr, k, np, c->N, (typename GridVal<R>::T*)c->pme_vpk);
   const int nb = nblk((long long)m.npatch * m.nseg * m.nset, 4);
   c->launches++;
   switch (P) {
-    case 4: launch_spread<4, R>(c, ng, nb, m, grid); break;
-    case 6: launch_spread<6, R>(c, ng, nb, m, grid); break;
-    default: launch_spread<8, R>(c, ng, nb, m, grid);
+    case 4: launch_spread<4, R>(c, k, ng, nb, m, grid); break;
+    case 6: launch_spread<6, R>(c, k, ng, nb, m, grid); break;
+    default: launch_spread<8, R>(c, k, ng, nb, m, grid);
   }
   return BD_OK;
 }

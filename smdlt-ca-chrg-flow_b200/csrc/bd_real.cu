@@ -1,0 +1,705 @@
+// Real-space part of the particle-mesh mobility: pair lists, tensors, products.
+//
+// No counterpart in the reference (see bd_pme.cu).  The beads are taken four
+// at a time (consecutive indices: neighbours along a chain, whose cutoff
+// spheres nearly coincide).  A group's row lists every bead within the cutoff
+// of one of its four, and per entry the four pair tensors T = t1 I + s w w^T,
+// w = sqrt(|t2| / r^2) d, the sign s of t2 in the lowest mantissa bit of t1
+// (zero where a pair is beyond the cutoff).  The product then reads a
+// neighbour's input values once for four pairs, and positions and minimum
+// images not at all.  Rows are sorted by index: a chain that passes through the
+// cutoff sphere gives a run of consecutive neighbours, whose input values lie
+// side by side.
+#include <math.h>
+
+#include <algorithm>
+#include <type_traits>
+
+#include "bd_real.cuh"
+
+using namespace bd;
+
+#define CU(call) BD_CU(call)
+
+namespace {
+
+constexpr int kGroup = 4;  // beads per row
+
+template <typename R>
+struct Vec4;
+template <>
+struct Vec4<float> {
+  using T = float4;
+};
+template <>
+struct Vec4<double> {
+  using T = double4;
+};
+
+// Real-space Beenakker kernel t1 I + t2 r r^T/r^2 (shear/src/main26.c:
+// 1727-1741) at split parameter alpha; with FAR the r > 2 form at any r.  irr
+// = 1/rr and ir = 1/r are formed once by the caller: a double division costs
+// as much as ten multiplications, and the terms hold eight of them.
+template <bool FAR>
+__device__ __forceinline__ void real_kernel(double alpha, double rr, double r, double ir,
+                                            double irr, double& t1, double& t2) {
+  double a = alpha, a2 = a * a, a3 = a2 * a, a5 = a3 * a2, a7 = a5 * a2;
+  double C1, C2, C3, C4;
+  if (FAR || r > 2.0) {
+    C1 = ir * (0.75 + 0.5 * irr);
+    C2 = 4.0 * a7 * rr * rr + 3.0 * a3 * rr - 20.0 * a5 * rr - 4.5 * a + 14.0 * a3 + a * irr;
+    C3 = ir * (0.75 - 1.5 * irr);
+    C4 = -4.0 * a7 * rr * rr - 3.0 * a3 * rr + 16.0 * a5 * rr + 1.5 * a - 2.0 * a3 -
+         3.0 * a * irr;
+  } else {
+    C1 = 1.0 - 0.28125 * r;
+    C2 = 64.0 * a7 + 12.0 * a3 - 80.0 * a5 - 4.5 * a + 14.0 * a3 + 0.25 * a;
+    C3 = 0.09375 * r;
+    C4 = -64.0 * a7 - 12.0 * a3 + 64.0 * a5 + 1.5 * a - 2.0 * a3 - 0.75 * a;
+  }
+  const double irtpi = 0.56418958354775628695;  // 1/sqrt(pi)
+  double ec = erfc(a * r), ex = exp(-a2 * rr) * irtpi;
+  t1 = C1 * ec + C2 * ex;
+  t2 = C3 * ec + C4 * ex;
+}
+
+// t1, t2 of the real-space pair tensor at split alpha, with calcHI's overlap
+// convention for r < 2 (OVERLAP: the far form at alpha plus the overlap
+// correction at its own split parameter alpha_ref).
+template <bool OVERLAP>
+__device__ __forceinline__ void pair_terms(double alpha, double alpha_ref, double rr, double r,
+                                           double ir, double irr, double& t1, double& t2) {
+  real_kernel<OVERLAP>(alpha, rr, r, ir, irr, t1, t2);
+  if constexpr (OVERLAP) {
+    double o1, o2, g1, g2;
+    real_kernel<false>(alpha_ref, rr, r, ir, irr, o1, o2);
+    real_kernel<true>(alpha_ref, rr, r, ir, irr, g1, g2);
+    t1 += o1 - g1;
+    t2 += o2 - g2;
+  }
+}
+
+// Cells of the real-space list (fractional, width >= rc).
+struct RGeom {
+  int n[3];
+};
+
+__global__ void k_rl_count(Cell cell, RGeom g, const double* __restrict__ rx,
+                           const double* __restrict__ ry, const double* __restrict__ rz,
+                           double cr, double sr, int N, int* cell_of, int* cell_count) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  int cd[3];
+  double x = rx[i] * cr - ry[i] * sr, y = rx[i] * sr + ry[i] * cr;
+  int c = cell_of_pos(cell, g.n, x, y, rz[i], cd);
+  cell_of[i] = c;
+  atomicAdd(&cell_count[c], 1);
+}
+
+__global__ void k_rl_scan(int ncell, int* cell_count, int* cell_start, int* cursor) {
+  __shared__ int part[1024];
+  int t = threadIdx.x, nt = blockDim.x;
+  int per = (ncell + nt - 1) / nt, lo = t * per, hi = min(ncell, lo + per), s = 0;
+  for (int c = lo; c < hi; c++) s += cell_count[c];
+  part[t] = s;
+  __syncthreads();
+  for (int o = 1; o < nt; o <<= 1) {
+    int v = t >= o ? part[t - o] : 0;
+    __syncthreads();
+    part[t] += v;
+    __syncthreads();
+  }
+  int b = part[t] - s;
+  for (int c = lo; c < hi; c++) {
+    cell_start[c] = b;
+    cursor[c] = 0;
+    b += cell_count[c];
+    cell_count[c] = 0;
+  }
+  if (t == nt - 1) cell_start[ncell] = part[t];
+}
+
+// Positions in cell order, the bead index in the fourth component: the row
+// build streams a cell's beads with one contiguous load each.
+__global__ void k_rl_fill(const int* __restrict__ cell_of, const int* __restrict__ cell_start,
+                          int* cursor, const double4* __restrict__ pos, double4* spos, int N) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  int c = cell_of[i];
+  double4 p = pos[i];
+  p.w = __longlong_as_double((long long)i);
+  spos[cell_start[c] + atomicAdd(&cursor[c], 1)] = p;
+}
+
+// (t1, w) of a pair as stored; d = d(alpha, r) its displacement.
+__device__ __forceinline__ float4 stored(float, double t1, double t2, double sw, double dx,
+                                         double dy, double dz) {
+  unsigned b = (__float_as_uint((float)t1) & ~1u) | (t2 < 0.0 ? 1u : 0u);
+  return make_float4(__uint_as_float(b), (float)(sw * dx), (float)(sw * dy), (float)(sw * dz));
+}
+__device__ __forceinline__ double4 stored(double, double t1, double t2, double sw, double dx,
+                                          double dy, double dz) {
+  long long b = (__double_as_longlong(t1) & ~1ll) | (t2 < 0.0 ? 1ll : 0ll);
+  return make_double4(__longlong_as_double(b), sw * dx, sw * dy, sw * dz);
+}
+
+// Minimum-image displacement; the cell is (b1, b2) in the xy plane and L e_z, and
+// the nearest integer of |s| < 2^51 comes from adding and subtracting 1.5 2^52
+// (two additions for one slow conversion).
+struct Image {
+  double h00, h01, h10, h11, g00, g01, g10, g11, Lz, iLz;
+  __device__ __forceinline__ explicit Image(const Cell& c)
+      : h00(c.H[0]), h01(c.H[1]), h10(c.H[3]), h11(c.H[4]), g00(c.Hi[0]), g01(c.Hi[1]),
+        g10(c.Hi[3]), g11(c.Hi[4]), Lz(c.H[8]), iLz(c.Hi[8]) {}
+  static __device__ __forceinline__ double nearest(double s) {
+    return __dsub_rn(__dadd_rn(s, 6755399441055744.0), 6755399441055744.0);
+  }
+  __device__ __forceinline__ double operator()(const double4& pj, const double4& pi, double& dx,
+                                               double& dy, double& dz) const {
+    dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
+    double n0 = nearest(g00 * dx + g01 * dy), n1 = nearest(g10 * dx + g11 * dy),
+           n2 = nearest(iLz * dz);
+    dx -= h00 * n0 + h01 * n1;
+    dy -= h10 * n0 + h11 * n1;
+    dz -= Lz * n2;
+    return dx * dx + dy * dy + dz * dz;
+  }
+};
+
+// Neighbour indices of the groups' rows, cap entries a row, in no order.  One
+// warp per group.  For each of its beads the at most 27 neighbour cells form
+// one candidate list; the lanes test 32 candidates at a time and queue the
+// hits in shared memory.  Batches of hits are then tested against the group's
+// earlier beads: a neighbour is listed by the first bead that has it within
+// the cutoff.  Bound by the FP64 pipe: 193 M candidates at 50 000 beads, cutoff
+// 14.5.
+__global__ void __launch_bounds__(128, 4)
+    k_rl_find(Cell cell, RGeom g, const double4* __restrict__ pos, int N, int ngroup,
+              const int* __restrict__ cell_start, const double4* __restrict__ spos, double rc2,
+              int cap, int* cnt, int* rows, int* need, int* err) {
+  __shared__ CandList c_list[4];
+  __shared__ int c_queue[4][64];
+  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = blockIdx.x * 4 + wl;
+  if (grp >= ngroup) return;
+  const int i0 = kGroup * grp, nb = min(kGroup, N - i0);
+  const Image image(cell);
+  int* row = rows + (size_t)grp * cap;
+  int* queue = c_queue[wl];
+  int n = 0, nq = 0;
+  // the first m hits of bead b: those that no earlier bead lists
+  auto list = [&](int b, int m) {
+    bool keep = lane < m;
+    int j = 0;
+    if (keep) {
+      const double4 pj = spos[queue[lane]];
+      j = (int)__double_as_longlong(pj.w);
+      for (int q = 0; q < b; q++) {
+        double dx, dy, dz;
+        if (j != i0 + q && !(image(pj, pos[i0 + q], dx, dy, dz) >= rc2)) keep = false;
+      }
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, keep);
+    const int at = n + __popc(hit & ((1u << lane) - 1u));
+    if (keep && at < cap) row[at] = j;
+    n += __popc(hit);
+    nq -= m;
+    const int rest = lane < nq ? queue[m + lane] : 0;
+    __syncwarp();
+    if (lane < nq) queue[lane] = rest;
+    __syncwarp();
+  };
+#pragma unroll 1
+  for (int b = 0; b < nb; b++) {
+    const double4 pb = pos[i0 + b];
+    int cd[3], cl = 0, next_at = -1;
+    cell_of_pos(cell, g.n, pb.x, pb.y, pb.z, cd);
+    const int total = c_list[wl].open(g.n, cd, cell_start);
+    // the next candidate's load is in flight while this one is tested
+    double4 next = pb;
+    auto fetch = [&](int m) {
+      next_at = -1;
+      if (m < total) {
+        next_at = c_list[wl].at(m, cl);
+        next = spos[next_at];
+      }
+    };
+    fetch(lane);
+#pragma unroll 1
+    for (int m0 = 0; m0 < total; m0 += 32) {
+      const int at = next_at;
+      const double4 pj = next;
+      fetch(m0 + 32 + lane);
+      double dx, dy, dz;
+      const double rr = image(pj, pb, dx, dy, dz);
+      const bool in = at >= 0 && !(rr >= rc2) && (int)__double_as_longlong(pj.w) != i0 + b;
+      const unsigned hit = __ballot_sync(0xffffffffu, in);
+      if (in) queue[nq + __popc(hit & ((1u << lane) - 1u))] = at;
+      nq += __popc(hit);
+      __syncwarp();
+      if (nq >= 32) list(b, 32);
+    }
+    if (nq > 0) list(b, nq);
+  }
+  if (lane == 0) {
+    cnt[grp] = min(n, cap);
+    if (n > cap) {
+      if (need)
+        atomicMax(need, n);  // the host grows the rows and builds them again
+      else
+        atomicOr(err, ERRB_NBR_OVERFLOW);
+    }
+  }
+}
+
+// Rows in increasing index (bitonic, a block per row); rows longer than the
+// shared memory stay as they are.
+constexpr int kSortMax = 4096;
+__global__ void __launch_bounds__(128) k_rl_sort(const int* __restrict__ cnt, int cap, int* rows) {
+  __shared__ int s[kSortMax];
+  const int n = cnt[blockIdx.x];
+  if (n > kSortMax) return;
+  int* row = rows + (size_t)blockIdx.x * cap;
+  int m = 32;
+  while (m < n) m <<= 1;
+  for (int i = threadIdx.x; i < m; i += blockDim.x) s[i] = i < n ? row[i] : 0x7fffffff;
+  for (int k = 2; k <= m; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      __syncthreads();
+      for (int t = threadIdx.x; t < m / 2; t += blockDim.x) {
+        const int a = 2 * t - (t & (j - 1)), b = a + j;
+        const int x = s[a], y = s[b];
+        if ((x > y) == ((a & k) == 0)) {
+          s[a] = y;
+          s[b] = x;
+        }
+      }
+    }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) row[i] = s[i];
+}
+
+// The four tensors of every entry, a warp per group, and each bead's number of
+// pairs against an explicit cap.  Tensor b of entry k at rw[4 (group cap + k) +
+// b].  Overlapping pairs (r < 2), whose terms cost three times as much, are
+// queued and formed 32 at a time.  Bound by the FP64 pipe (erfc, exp).
+template <typename R>
+__global__ void __launch_bounds__(128, 4)
+    k_rl_tensors(Cell cell, const double4* __restrict__ pos, int N, int ngroup,
+                 const int* __restrict__ cnt, const int* __restrict__ rows, int cap, double rc2,
+                 double alpha, double alpha_ref, int bead_cap, typename Vec4<R>::T* rw, int* err) {
+  __shared__ int c_queue[4][64];  // 4 k + b of overlapping pairs
+  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = blockIdx.x * 4 + wl;
+  if (grp >= ngroup) return;
+  const int i0 = kGroup * grp, nb = min(kGroup, N - i0), n = cnt[grp];
+  const Image image(cell);
+  const int* row = rows + (size_t)grp * cap;
+  typename Vec4<R>::T* out = rw + (size_t)kGroup * grp * cap;
+  int* queue = c_queue[wl];
+  int nq = 0;
+  auto store = [&](auto overlap, int k, int b, double rr, double dx, double dy, double dz) {
+    constexpr bool OV = decltype(overlap)::value;
+    const double r = sqrt(rr), ir = 1.0 / r, irr = ir * ir;
+    double t1, t2;
+    pair_terms<OV>(alpha, alpha_ref, rr, r, ir, irr, t1, t2);
+    out[(size_t)kGroup * k + b] = stored((R)0, t1, t2, sqrt(fabs(t2)) * ir, dx, dy, dz);
+  };
+  auto flush = [&](int m) {
+    if (lane < m) {
+      const int k = queue[lane] >> 2, b = queue[lane] & 3;
+      double dx, dy, dz;
+      const double rr = image(pos[row[k]], pos[i0 + b], dx, dy, dz);
+      store(std::integral_constant<bool, true>(), k, b, rr, dx, dy, dz);
+    }
+    nq -= m;
+    const int rest = lane < nq ? queue[m + lane] : 0;
+    __syncwarp();
+    if (lane < nq) queue[lane] = rest;
+    __syncwarp();
+  };
+  int longest = 0;
+#pragma unroll 1
+  for (int b = 0; b < kGroup; b++) {
+    const double4 pb = pos[min(i0 + b, N - 1)];
+    int count = 0;
+#pragma unroll 1
+    for (int k0 = 0; k0 < n; k0 += 32) {
+      const int k = k0 + lane;
+      bool near = false;
+      if (k < n) {
+        const int j = row[k];
+        double dx, dy, dz;
+        const double rr = image(pos[j], pb, dx, dy, dz);
+        if (b < nb && j != i0 + b && !(rr >= rc2)) {
+          count++;
+          near = rr < 4.0;
+          if (!near) store(std::integral_constant<bool, false>(), k, b, rr, dx, dy, dz);
+        } else {
+          out[(size_t)kGroup * k + b] = stored((R)0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0);
+        }
+      }
+      const unsigned hit = __ballot_sync(0xffffffffu, near);
+      if (near) queue[nq + __popc(hit & ((1u << lane) - 1u))] = 4 * k + b;
+      nq += __popc(hit);
+      __syncwarp();
+      if (nq >= 32) flush(32);
+    }
+    for (int o = 16; o > 0; o >>= 1) count += __shfl_xor_sync(0xffffffffu, count, o);
+    longest = max(longest, count);
+  }
+  if (nq > 0) flush(nq);
+  if (lane == 0 && bead_cap > 0 && longest > bead_cap) atomicOr(err, ERRB_NBR_OVERFLOW);
+}
+
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ float2 pack2(float x) { return make_float2(x, x); }
+__device__ __forceinline__ double pack2(double x) { return x; }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long d, x = *reinterpret_cast<unsigned long long*>(&a),
+                        y = *reinterpret_cast<unsigned long long*>(&b);
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+  return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long d, x = *reinterpret_cast<unsigned long long*>(&a),
+                        y = *reinterpret_cast<unsigned long long*>(&b),
+                        z = *reinterpret_cast<unsigned long long*>(&c);
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(x), "l"(y), "l"(z));
+  return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ double2 mul2(double a, double2 b) {
+  return make_double2(a * b.x, a * b.y);
+}
+__device__ __forceinline__ double2 fma2(double a, double2 b, double2 c) {
+  return make_double2(fma(a, b.x, c.x), fma(a, b.y, c.y));
+}
+__device__ __forceinline__ double2 fma2(double2 a, double b, double2 c) {
+  return make_double2(fma(b, a.x, c.x), fma(b, a.y, c.y));
+}
+// -a where t1 carries the sign of t2
+__device__ __forceinline__ float2 signed_by(float t1, float2 a) {
+  unsigned s = __float_as_uint(t1) << 31;
+  return make_float2(__uint_as_float(__float_as_uint(a.x) ^ s),
+                     __uint_as_float(__float_as_uint(a.y) ^ s));
+}
+__device__ __forceinline__ double2 signed_by(double t1, double2 a) {
+  return __double_as_longlong(t1) & 1 ? make_double2(-a.x, -a.y) : a;
+}
+template <typename R>
+struct Real2;
+template <>
+struct Real2<float> {
+  using T = float2;
+};
+template <>
+struct Real2<double> {
+  using T = double2;
+};
+
+__device__ __forceinline__ void copy_async(void* to, const void* from, int bytes16) {
+  unsigned d = (unsigned)__cvta_generic_to_shared(to);
+  if (bytes16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(from) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(from) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+}
+
+// The real-space sums of NP packed pairs (p0 on) and the rest of the product.
+// One warp per group of four beads: a lane serves one pair and every S-th
+// entry of the row (S = 32 / NP), so NP lanes read a neighbour's packed values
+// (component c of pair p at vpk[(c N + j) np + p]) side by side and use them
+// for the four beads.  The row (68 bytes an entry, read once) streams through
+// shared memory, about 30 entries at a time with two more such pieces under
+// way: with loads to registers, an entry ahead, too few bytes were in flight
+// to cover the latency of L2 and HBM (430 us at 50 000 beads, cutoff 14.5,
+// five pairs).  FP32: two right-hand sides per instruction, partial sums of
+// about 16 entries folded into a second set; lanes added in FP64.  REAL_FIGURES
+// SPLIT warps share a group's row where there are too few groups to fill the
+// chip with a warp each.
+template <int NP, typename R>
+struct Stage {
+  static constexpr int S = 32 / NP, ITS = 32 / S, CH = S * ITS;  // entries a piece
+  typename Vec4<R>::T w[CH * kGroup];
+  int j[(CH + 3) / 4 * 4];
+};
+
+template <int NP, int SPLIT, typename R>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2)
+    k_real_apply(const int* __restrict__ cnt, const int* __restrict__ rows,
+                 const typename Vec4<R>::T* __restrict__ rw, int cap,
+                 const typename Real2<R>::T* __restrict__ vpk, int np, int p0, int N, int ngroup,
+                 Finish fin) {
+  using V = typename Real2<R>::T;
+  using Q = typename Vec4<R>::T;
+  using P = Stage<NP, R>;
+  constexpr int S = P::S, ITS = P::ITS, CH = P::CH, DEEP = sizeof(R) == 4 ? 3 : 2, W = 25;
+  constexpr int FOLD = 16 / ITS, PER = kGroup * (int)sizeof(Q) / 16;  // 16-byte words an entry
+  union Shared {
+    P stage[4][DEEP];
+    R sum[4][32 * W];
+  };
+  __shared__ __align__(16) unsigned char raw[sizeof(Shared)];
+  Shared& sh = *reinterpret_cast<Shared*>(raw);
+  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = blockIdx.x * (4 / SPLIT) + wl / SPLIT, piece0 = wl % SPLIT;
+  const int slot = lane / NP, pr = lane % NP;  // slot S and up: idle lanes
+  V sum[kGroup][3], part[kGroup][3];
+#pragma unroll
+  for (int b = 0; b < kGroup; b++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) sum[b][c].x = sum[b][c].y = part[b][c].x = part[b][c].y = 0;
+  if (grp < ngroup) {
+    const int n = cnt[grp];
+    const int* row = rows + (size_t)grp * cap;
+    const Q* rq = rw + (size_t)grp * cap * kGroup;
+    const V* vp = vpk + p0 + pr;
+    const size_t plane = (size_t)N * np;
+    P* st = sh.stage[wl];
+    auto issue = [&](int piece, int buf) {
+      const int k0 = piece * CH, m = min(CH, n - k0);
+      const char* from = (const char*)(rq + (size_t)k0 * kGroup);
+      for (int e = lane; e < m * PER; e += 32)
+        copy_async((char*)st[buf].w + 16 * e, from + 16 * e, 1);
+      if (lane < m) copy_async(st[buf].j + lane, row + k0 + lane, 0);
+      copy_commit();
+    };
+#pragma unroll
+    for (int d = 0; d < DEEP - 1; d++) issue(piece0 + d * SPLIT, d);
+    int buf = 0, folded = 0;
+#pragma unroll 1
+    for (int piece = piece0; piece * CH < n; piece += SPLIT) {
+      copy_wait<DEEP - 2>();
+      __syncwarp();
+      const int m = min(CH, n - piece * CH);
+      const P& p = st[buf];
+      V x[ITS][3];
+#pragma unroll
+      for (int t = 0; t < ITS; t++) {
+        const int k = t * S + slot;
+        const V* vj = vp + (size_t)(slot < S && k < m ? p.j[k] : 0) * np;
+#pragma unroll
+        for (int c = 0; c < 3; c++) x[t][c] = __ldg(vj + c * plane);
+      }
+      // the buffer used last is free: every lane is past the barrier above
+      issue(piece + (DEEP - 1) * SPLIT, buf == 0 ? DEEP - 1 : buf - 1);
+#pragma unroll
+      for (int t = 0; t < ITS; t++) {
+        const int k = t * S + slot;
+        if (slot < S && k < m) {
+#pragma unroll
+          for (int b = 0; b < kGroup; b++) {
+            const Q q = p.w[kGroup * k + b];
+            const auto t1 = pack2(q.x), w0 = pack2(q.y), w1 = pack2(q.z), w2 = pack2(q.w);
+            const V d = signed_by(q.x, fma2(w2, x[t][2], fma2(w1, x[t][1], mul2(w0, x[t][0]))));
+            part[b][0] = fma2(d, w0, fma2(t1, x[t][0], part[b][0]));
+            part[b][1] = fma2(d, w1, fma2(t1, x[t][1], part[b][1]));
+            part[b][2] = fma2(d, w2, fma2(t1, x[t][2], part[b][2]));
+          }
+        }
+      }
+      buf = buf + 1 == DEEP ? 0 : buf + 1;
+      if (++folded == FOLD) {
+        folded = 0;
+#pragma unroll
+        for (int b = 0; b < kGroup; b++)
+#pragma unroll
+          for (int c = 0; c < 3; c++) {
+            sum[b][c].x += part[b][c].x;
+            sum[b][c].y += part[b][c].y;
+            part[b][c].x = part[b][c].y = 0;
+          }
+      }
+    }
+    copy_wait<0>();
+  }
+  __syncthreads();  // the stages' memory holds the sums from here on
+  R* o = sh.sum[wl] + lane * W;
+#pragma unroll
+  for (int b = 0; b < kGroup; b++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      o[6 * b + c] = sum[b][c].x + part[b][c].x;
+      o[6 * b + 3 + c] = sum[b][c].y + part[b][c].y;
+    }
+  __syncthreads();
+  if (grp >= ngroup) return;
+  const int w0 = wl / SPLIT * SPLIT;
+  for (int e = lane + 32 * piece0; e < 6 * kGroup * NP; e += 32 * SPLIT) {
+    const int b = e / (6 * NP), p = e / 6 % NP, i = kGroup * grp + b;
+    if (i >= N) break;
+    double s = 0;
+    for (int w = w0; w < w0 + SPLIT; w++)
+      for (int u = 0; u < S; u++) s += (double)sh.sum[w][(u * NP + p) * W + 6 * b + e % 6];
+    fin.write(s, p0 + p, e % 6, i);
+  }
+}
+
+template <int NP, typename R>
+void launch_apply(bd_ctx* c, int np, int p0, const Finish& fin) {
+  const int ng = (c->N + kGroup - 1) / kGroup;
+#define REAL(SPLIT_)                                                                      \
+  k_real_apply<NP, SPLIT_, R><<<nblk(ng, 4 / SPLIT_), 128, 0, c->stream>>>(               \
+      c->rl_cnt, c->rl_rows, (const typename Vec4<R>::T*)c->rl_w, c->rl_cap,              \
+      (const typename Real2<R>::T*)c->pme_vpk, np, p0, c->N, ng, fin)
+  // about 16 warps an SM
+  if (ng >= 148 * 12)
+    REAL(1);
+  else if (ng >= 148 * 6)
+    REAL(2);
+  else
+    REAL(4);
+#undef REAL
+}
+
+template <typename R>
+int apply_t(bd_ctx* c, int np, const Finish& fin) {
+  for (int p0 = 0; p0 < np; p0 += 5) {
+    c->launches++;
+    switch (std::min(5, np - p0)) {
+      case 1: launch_apply<1, R>(c, np, p0, fin); break;
+      case 2: launch_apply<2, R>(c, np, p0, fin); break;
+      case 3: launch_apply<3, R>(c, np, p0, fin); break;
+      case 4: launch_apply<4, R>(c, np, p0, fin); break;
+      default: launch_apply<5, R>(c, np, p0, fin);
+    }
+  }
+  return launch_ok(c);
+}
+
+}  // namespace
+
+namespace bd {
+
+// Rows of cap entries for every group.
+static int rows_alloc(bd_ctx* c, int cap) {
+  size_t ng = ((size_t)c->N + kGroup - 1) / kGroup, es = c->pme_f32 ? 4 : 8;
+  size_t old = (size_t)c->rl_cap, each = 4 + 4 * es * kGroup;
+  if (c->rl_rows) {
+    CU(cudaStreamSynchronize(c->stream));
+    cudaFree(c->rl_rows);
+    cudaFree(c->rl_w);
+    c->rl_rows = nullptr;
+    c->rl_w = nullptr;
+    c->bytes -= each * ng * old;
+  }
+  c->rl_cap = cap;
+  CU(cudaMalloc(&c->rl_rows, 4 * ng * cap));
+  CU(cudaMalloc(&c->rl_w, 4 * es * kGroup * ng * cap));
+  c->bytes += each * ng * cap;
+  return BD_OK;
+}
+
+int real_alloc(bd_ctx* c) {
+  int N = c->N, s;
+  // row cap: an explicit cap per bead bounds a group's row by four times that;
+  // the default is 1.6 times the mean number of beads within the cutoff at the
+  // system's density, at least 512 (rows that overflow it are grown); no row
+  // is longer than N
+  long cap;
+  if (c->p.pme_max_pairs > 0) {
+    cap = (long)kGroup * c->p.pme_max_pairs;
+  } else {
+    double mean = 4.0 / 3.0 * M_PI * c->pme_rc * c->pme_rc * c->pme_rc * N / c->boxvol;
+    cap = std::max(512, ((int)ceil(1.6 * mean) + 31) / 32 * 32);
+  }
+  if ((s = rows_alloc(c, (int)std::min(cap, (long)std::max(N, 1)))) != BD_OK) return s;
+  CU(cudaMalloc(&c->rl_cnt, 4 * (size_t)N));
+  CU(cudaMalloc(&c->rl_need, 4));
+  CU(cudaMemsetAsync(c->rl_need, 0, 4, c->stream));
+  c->rl_ncell_cap = 4096;
+  CU(cudaMalloc(&c->rl_cell_of, 4 * (size_t)N));
+  CU(cudaMalloc(&c->rl_spos, 32 * (size_t)N));
+  CU(cudaMalloc(&c->rl_cell_count, 4 * (size_t)c->rl_ncell_cap));
+  CU(cudaMalloc(&c->rl_cell_start, 4 * (size_t)(c->rl_ncell_cap + 1)));
+  CU(cudaMalloc(&c->rl_cursor, 4 * (size_t)c->rl_ncell_cap));
+  CU(cudaMemsetAsync(c->rl_cell_count, 0, 4 * (size_t)c->rl_ncell_cap, c->stream));
+  c->bytes += 40 * (size_t)N + 12 * (size_t)c->rl_ncell_cap;
+  return BD_OK;
+}
+
+void real_free(bd_ctx* c) {
+  void* ptrs[] = {c->rl_rows, c->rl_w, c->rl_cnt, c->rl_need, c->rl_cell_of, c->rl_spos,
+                  c->rl_cell_count, c->rl_cell_start, c->rl_cursor};
+  for (void* q : ptrs)
+    if (q) cudaFree(q);
+}
+
+// The groups' rows for the positions in rl_pos (lab frame; rx, ry, rz and the
+// rotation (cr, sr) give the same); alpha_ref is calcHI's split parameter.
+int real_prepare(bd_ctx* c, const Cell& cell, double cr, double sr, double alpha_ref) {
+  int s, N = c->N;
+  double rc = c->pme_rc, alpha = c->pme_alpha;
+  // real-space cells: perpendicular widths V/|a_j x a_k|
+  double w[3];
+  {
+    const double* H = cell.H;
+    double a[3][3];
+    for (int j = 0; j < 3; j++)
+      for (int d = 0; d < 3; d++) a[j][d] = H[d * 3 + j];
+    for (int j = 0; j < 3; j++) {
+      const double* u = a[(j + 1) % 3];
+      const double* v = a[(j + 2) % 3];
+      double cx = u[1] * v[2] - u[2] * v[1], cy = u[2] * v[0] - u[0] * v[2],
+             cz = u[0] * v[1] - u[1] * v[0];
+      w[j] = cell.V / sqrt(cx * cx + cy * cy + cz * cz);
+    }
+  }
+  if (2 * rc > std::min(w[0], std::min(w[1], w[2]))) return BD_ERR_ARG;  // rc beyond half a width
+  RGeom g;
+  for (int d = 0; d < 3; d++) g.n[d] = std::max(1, (int)floor(w[d] / rc));
+  while ((long)g.n[0] * g.n[1] * g.n[2] > c->rl_ncell_cap) {
+    int d = g.n[0] >= g.n[1] && g.n[0] >= g.n[2] ? 0 : (g.n[1] >= g.n[2] ? 1 : 2);
+    g.n[d]--;
+  }
+  int ncell = g.n[0] * g.n[1] * g.n[2];
+  c->launches += 4;
+  k_rl_count<<<nblk(N, 256), 256, 0, c->stream>>>(cell, g, c->rx, c->ry, c->rz, cr, sr, N,
+                                                  c->rl_cell_of, c->rl_cell_count);
+  k_rl_scan<<<1, 1024, 0, c->stream>>>(ncell, c->rl_cell_count, c->rl_cell_start, c->rl_cursor);
+  k_rl_fill<<<nblk(N, 256), 256, 0, c->stream>>>(c->rl_cell_of, c->rl_cell_start, c->rl_cursor,
+                                                 (const double4*)c->rl_pos,
+                                                 (double4*)c->rl_spos, N);
+  if ((s = launch_ok(c)) != BD_OK) return s;
+  // the rows; with the default cap (no pme_max_pairs), rows that
+  // overflow it are grown to 1.25 times the longest row and built again
+  int* need = c->p.pme_max_pairs > 0 ? nullptr : c->rl_need;
+  const int ng = (N + kGroup - 1) / kGroup;
+  for (int pass = 0; pass < 2; pass++) {
+    c->launches++;
+    k_rl_find<<<nblk(ng, 4), 128, 0, c->stream>>>(
+        cell, g, (const double4*)c->rl_pos, N, ng, c->rl_cell_start, (const double4*)c->rl_spos,
+        rc * rc, c->rl_cap, c->rl_cnt, c->rl_rows, need, c->err);
+    if (!need) break;
+    int longest = 0;
+    CU(cudaMemcpyAsync(&longest, need, 4, cudaMemcpyDeviceToHost, c->stream));
+    if ((s = check(c)) != BD_OK) return s;
+    if (longest <= c->rl_cap) break;
+    if ((s = rows_alloc(c, std::min(N, ((int)ceil(1.25 * longest) + 31) / 32 * 32))) != BD_OK)
+      return s;
+    CU(cudaMemsetAsync(c->rl_need, 0, 4, c->stream));
+  }
+  c->launches += 2;
+  k_rl_sort<<<ng, 128, 0, c->stream>>>(c->rl_cnt, c->rl_cap, c->rl_rows);
+  if (c->pme_f32)
+    k_rl_tensors<float><<<nblk(ng, 4), 128, 0, c->stream>>>(
+        cell, (const double4*)c->rl_pos, N, ng, c->rl_cnt, c->rl_rows, c->rl_cap, rc * rc, alpha,
+        alpha_ref, c->p.pme_max_pairs, (float4*)c->rl_w, c->err);
+  else
+    k_rl_tensors<double><<<nblk(ng, 4), 128, 0, c->stream>>>(
+        cell, (const double4*)c->rl_pos, N, ng, c->rl_cnt, c->rl_rows, c->rl_cap, rc * rc, alpha,
+        alpha_ref, c->p.pme_max_pairs, (double4*)c->rl_w, c->err);
+  return launch_ok(c);
+}
+
+int real_apply(bd_ctx* c, int np, const Finish& fin) {
+  return c->pme_f32 ? apply_t<float>(c, np, fin) : apply_t<double>(c, np, fin);
+}
+
+}  // namespace bd
