@@ -20,9 +20,9 @@
 // Bound by the FP32 (FP64) pipe and the issue of its instructions: 48 (P = 8)
 // multiply-adds per lane and bead, two at a time (fma.rn.f32x2) in FP32, next
 // to about 20 others.
-// Five pairs, order 8: 169 us at 50 000 beads on 100^3 (one complex L2 atomic
-// per stencil point, component and pair took about 400), 47 us at 8000 beads on
-// 64^3 (74); FP64 70 us there (385).
+// Five pairs, order 8: 150 us at 50 000 beads on 100^3 (one complex L2 atomic
+// per stencil point, component and pair took about 400), 42 us at 8000 beads on
+// 64^3 (74); FP64 66 us there (385).
 //
 // Interpolation: a warp per bead and pair reads the stencil's 64 rows of 24
 // complex values (192 contiguous bytes, FP32), a lane the same third of a row
@@ -259,15 +259,16 @@ struct SpreadArgs {
 };
 
 template <int P, typename R, int NG, int CY, int CZ, bool ONE>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2) k_mesh_spread(SpreadArgs m, R* grid) {
+__global__ void __launch_bounds__(32, sizeof(R) == 4 ? 16 : 8)
+    k_mesh_spread(SpreadArgs m, R* grid) {
   using T = typename GridVal<R>::T;
   using V = std::conditional_t<ONE, R, T>;
   using S = Rec<RecData<P, R, NG, CY, CZ, ONE>>;
   static_assert(NG * CY * CZ <= 32, "a lane per point and pair");
-  __shared__ S s_rec[4][32];
-  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  const int job = blockIdx.x * 4 + wl;
-  if (job >= m.npatch * m.nseg * m.nset) return;
+  // a warp per block: columns differ in their beads by a factor of two and
+  // more, and single warps leave the fewest idle slots behind
+  __shared__ S s_rec[32];
+  const int lane = threadIdx.x, job = blockIdx.x;
   // columns fastest: the neighbours along z of a block complete its sectors
   const int patch = job % m.npatch, seg = job / m.npatch % m.nseg,
             set = job / (m.npatch * m.nseg);
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2) k_mesh_spread(Spr
   auto entry = [&](int t) { return t >= n ? 0 : t < n0 ? m.ent[e0 + t] : m.ent[f0 + t - n0]; };
   auto stage = [&](int t, int i) {
     if (t >= n) return;
-    S& r = s_rec[wl][lane];
+    S& r = s_rec[lane];
     const R* w = (const R*)m.w + (size_t)i * 3 * kMaxOrder;
     const int b1 = m.base[3 * i + 1], b2 = m.base[3 * i + 2];
     r.at = m.base[3 * i] + (t < n0 ? 0 : K);
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2) k_mesh_spread(Spr
     const int nb = min(32, n - t0);
 #pragma unroll 1
     for (int u = 0; u < nb; u++) {
-      const S& q = s_rec[wl][u];
+      const S& q = s_rec[u];
       const R wyz = q.wy[ly] * q.wz[lz];
       V t[3];
 #pragma unroll
@@ -472,10 +473,12 @@ double layout_cost(int np, int ng, int P) {
   return (P - 1 + cy) * (P - 1 + cz) / (cy * cz) * ((np + ng - 1) / ng);
 }
 
-// Segments of a column: enough warps for about 16 on every SM, none shorter
-// than half a stencil (a segment repeats P - 1 levels of its beads).
+// Segments of a column: about 14 warps on every SM (16 fit), none shorter than
+// half a stencil (a segment repeats P - 1 levels of its beads).  Segments
+// measured, us: 1700 columns of 100 levels 1: 154, 2: 159, 3: 155, 6: 163; 704
+// columns of 64 levels 1: 56, 2: 45, 3: 42, 4: 43, 6: 46.
 int segments(int K, int njob) {
-  int want = (148 * 16 + njob - 1) / njob;
+  int want = (148 * 14 + njob / 2) / njob;
   return std::max(1, std::min(want, K / 4));
 }
 
@@ -492,7 +495,8 @@ int most_touched(int K, int P, int w) {
 
 template <int P, typename R>
 void launch_spread(bd_ctx* c, int k, int ng, int nb, const SpreadArgs& m, R* grid) {
-#define SPREAD(...) k_mesh_spread<P, R, __VA_ARGS__><<<nb, 128, 0, c->stream>>>(m, grid)
+#define SPREAD(...) \
+  k_mesh_spread<P, R, __VA_ARGS__><<<nb, 32, 0, c->stream>>>(m, grid)
   switch (ng) {
     case 1:
       if (k == 1)
@@ -531,7 +535,7 @@ int spread_t(bd_ctx* c, int k, const VecIn& v, size_t vr, R* grid) {
   c->launches++;
   k_mesh_pack<<<dim3(nblk(c->N, 128), np), 128, 0, c->stream>>>(
       v, vr, k, np, c->N, (typename GridVal<R>::T*)c->pme_vpk);
-  const int nb = nblk((long long)m.npatch * m.nseg * m.nset, 4);
+  const int nb = m.npatch * m.nseg * m.nset;
   c->launches++;
   switch (P) {
     case 4: launch_spread<4, R>(c, k, ng, nb, m, grid); break;

@@ -25,17 +25,6 @@ namespace {
 
 constexpr int kGroup = 4;  // beads per row
 
-template <typename R>
-struct Vec4;
-template <>
-struct Vec4<float> {
-  using T = float4;
-};
-template <>
-struct Vec4<double> {
-  using T = double4;
-};
-
 // Real-space Beenakker kernel t1 I + t2 r r^T/r^2 (shear/src/main26.c:
 // 1727-1741) at split parameter alpha; with FAR the r > 2 form at any r.  irr
 // = 1/rr and ir = 1/r are formed once by the caller: a double division costs
@@ -131,16 +120,25 @@ __global__ void k_rl_fill(const int* __restrict__ cell_of, const int* __restrict
   spos[cell_start[c] + atomicAdd(&cursor[c], 1)] = p;
 }
 
-// (t1, w) of a pair as stored; d = d(alpha, r) its displacement.
-__device__ __forceinline__ float4 stored(float, double t1, double t2, double sw, double dx,
-                                         double dy, double dz) {
-  unsigned b = (__float_as_uint((float)t1) & ~1u) | (t2 < 0.0 ? 1u : 0u);
-  return make_float4(__uint_as_float(b), (float)(sw * dx), (float)(sw * dy), (float)(sw * dz));
+// t1 with the sign of t2 in its lowest mantissa bit.
+__device__ __forceinline__ float with_sign(float, double t1, double t2) {
+  return __uint_as_float((__float_as_uint((float)t1) & ~1u) | (t2 < 0.0 ? 1u : 0u));
 }
-__device__ __forceinline__ double4 stored(double, double t1, double t2, double sw, double dx,
-                                          double dy, double dz) {
-  long long b = (__double_as_longlong(t1) & ~1ll) | (t2 < 0.0 ? 1ll : 0ll);
-  return make_double4(__longlong_as_double(b), sw * dx, sw * dy, sw * dz);
+__device__ __forceinline__ double with_sign(double, double t1, double t2) {
+  return __longlong_as_double((__double_as_longlong(t1) & ~1ll) | (t2 < 0.0 ? 1ll : 0ll));
+}
+
+// The four tensors of an entry: 16 numbers, for beads (0, 1) and (2, 3) the
+// pairs of t1, w_x, w_y, w_z, so that the product takes two beads per
+// instruction.
+template <typename R>
+__device__ __forceinline__ void store_tensor(R* entry, int b, double t1, double t2, double sw,
+                                             double dx, double dy, double dz) {
+  R* o = entry + 8 * (b >> 1) + (b & 1);
+  o[0] = with_sign((R)0, t1, t2);
+  o[2] = (R)(sw * dx);
+  o[4] = (R)(sw * dy);
+  o[6] = (R)(sw * dz);
 }
 
 // Minimum-image displacement; the cell is (b1, b2) in the xy plane and L e_z, and
@@ -280,14 +278,13 @@ __global__ void __launch_bounds__(128) k_rl_sort(const int* __restrict__ cnt, in
 }
 
 // The four tensors of every entry, a warp per group, and each bead's number of
-// pairs against an explicit cap.  Tensor b of entry k at rw[4 (group cap + k) +
-// b].  Overlapping pairs (r < 2), whose terms cost three times as much, are
+// pairs against an explicit cap.  Entry k at rw[16 (group cap + k)].  Overlapping pairs (r < 2), whose terms cost three times as much, are
 // queued and formed 32 at a time.  Bound by the FP64 pipe (erfc, exp).
 template <typename R>
 __global__ void __launch_bounds__(128, 4)
     k_rl_tensors(Cell cell, const double4* __restrict__ pos, int N, int ngroup,
                  const int* __restrict__ cnt, const int* __restrict__ rows, int cap, double rc2,
-                 double alpha, double alpha_ref, int bead_cap, typename Vec4<R>::T* rw, int* err) {
+                 double alpha, double alpha_ref, int bead_cap, R* rw, int* err) {
   __shared__ int c_queue[4][64];  // 4 k + b of overlapping pairs
   const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = blockIdx.x * 4 + wl;
@@ -295,7 +292,7 @@ __global__ void __launch_bounds__(128, 4)
   const int i0 = kGroup * grp, nb = min(kGroup, N - i0), n = cnt[grp];
   const Image image(cell);
   const int* row = rows + (size_t)grp * cap;
-  typename Vec4<R>::T* out = rw + (size_t)kGroup * grp * cap;
+  R* out = rw + 16 * (size_t)grp * cap;
   int* queue = c_queue[wl];
   int nq = 0;
   auto store = [&](auto overlap, int k, int b, double rr, double dx, double dy, double dz) {
@@ -303,7 +300,7 @@ __global__ void __launch_bounds__(128, 4)
     const double r = sqrt(rr), ir = 1.0 / r, irr = ir * ir;
     double t1, t2;
     pair_terms<OV>(alpha, alpha_ref, rr, r, ir, irr, t1, t2);
-    out[(size_t)kGroup * k + b] = stored((R)0, t1, t2, sqrt(fabs(t2)) * ir, dx, dy, dz);
+    store_tensor(out + 16 * (size_t)k, b, t1, t2, sqrt(fabs(t2)) * ir, dx, dy, dz);
   };
   auto flush = [&](int m) {
     if (lane < m) {
@@ -336,7 +333,7 @@ __global__ void __launch_bounds__(128, 4)
           near = rr < 4.0;
           if (!near) store(std::integral_constant<bool, false>(), k, b, rr, dx, dy, dz);
         } else {
-          out[(size_t)kGroup * k + b] = stored((R)0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0);
+          store_tensor(out + 16 * (size_t)k, b, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0);
         }
       }
       const unsigned hit = __ballot_sync(0xffffffffu, near);
@@ -354,8 +351,9 @@ __global__ void __launch_bounds__(128, 4)
 
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ float2 pack2(float x) { return make_float2(x, x); }
-__device__ __forceinline__ double pack2(double x) { return x; }
+// Two beads at a time: the beads' numbers in the halves, one input value for both.
+__device__ __forceinline__ float2 twice(float x) { return make_float2(x, x); }
+__device__ __forceinline__ double twice(double x) { return x; }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   unsigned long long d, x = *reinterpret_cast<unsigned long long*>(&a),
                         y = *reinterpret_cast<unsigned long long*>(&b);
@@ -369,24 +367,25 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(x), "l"(y), "l"(z));
   return *reinterpret_cast<float2*>(&d);
 }
-__device__ __forceinline__ double2 mul2(double a, double2 b) {
-  return make_double2(a * b.x, a * b.y);
-}
-__device__ __forceinline__ double2 fma2(double a, double2 b, double2 c) {
-  return make_double2(fma(a, b.x, c.x), fma(a, b.y, c.y));
+__device__ __forceinline__ double2 mul2(double2 a, double b) {
+  return make_double2(a.x * b, a.y * b);
 }
 __device__ __forceinline__ double2 fma2(double2 a, double b, double2 c) {
-  return make_double2(fma(b, a.x, c.x), fma(b, a.y, c.y));
+  return make_double2(fma(a.x, b, c.x), fma(a.y, b, c.y));
 }
-// -a where t1 carries the sign of t2
-__device__ __forceinline__ float2 signed_by(float t1, float2 a) {
-  unsigned s = __float_as_uint(t1) << 31;
-  return make_float2(__uint_as_float(__float_as_uint(a.x) ^ s),
-                     __uint_as_float(__float_as_uint(a.y) ^ s));
+__device__ __forceinline__ double2 fma2(double2 a, double2 b, double2 c) {
+  return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
 }
-__device__ __forceinline__ double2 signed_by(double t1, double2 a) {
-  return __double_as_longlong(t1) & 1 ? make_double2(-a.x, -a.y) : a;
+// negative where the bead's t1 carries a negative sign
+__device__ __forceinline__ float2 signed_by(float2 t1, float2 a) {
+  return make_float2(__uint_as_float(__float_as_uint(a.x) ^ (__float_as_uint(t1.x) << 31)),
+                     __uint_as_float(__float_as_uint(a.y) ^ (__float_as_uint(t1.y) << 31)));
 }
+__device__ __forceinline__ double2 signed_by(double2 t1, double2 a) {
+  return make_double2(__double_as_longlong(t1.x) & 1 ? -a.x : a.x,
+                      __double_as_longlong(t1.y) & 1 ? -a.y : a.y);
+}
+
 template <typename R>
 struct Real2;
 template <>
@@ -415,32 +414,33 @@ __device__ __forceinline__ void copy_wait() {
 // One warp per group of four beads: a lane serves one pair and every S-th
 // entry of the row (S = 32 / NP), so NP lanes read a neighbour's packed values
 // (component c of pair p at vpk[(c N + j) np + p]) side by side and use them
-// for the four beads.  The row (68 bytes an entry, read once) streams through
+// for the four beads, two at a time.  The row (68 bytes an entry, read once) streams through
 // shared memory, about 30 entries at a time with two more such pieces under
 // way: with loads to registers, an entry ahead, too few bytes were in flight
 // to cover the latency of L2 and HBM (430 us at 50 000 beads, cutoff 14.5,
-// five pairs).  FP32: two right-hand sides per instruction, partial sums of
-// about 16 entries folded into a second set; lanes added in FP64.  REAL_FIGURES
+// five pairs).  FP32: partial sums of about 16 entries folded into a second
+// set; lanes added in FP64.  Five pairs: 257 us at 50 000 beads, cutoff 14.5,
+// 38 us at 8000 beads, cutoff 12.1 (a warp per bead, every neighbour's values read
+// once per bead: 435 and 50).
 // SPLIT warps share a group's row where there are too few groups to fill the
 // chip with a warp each.
 template <int NP, typename R>
 struct Stage {
   static constexpr int S = 32 / NP, ITS = 32 / S, CH = S * ITS;  // entries a piece
-  typename Vec4<R>::T w[CH * kGroup];
+  alignas(16) R w[16 * CH];
   int j[(CH + 3) / 4 * 4];
 };
 
 template <int NP, int SPLIT, typename R>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2)
     k_real_apply(const int* __restrict__ cnt, const int* __restrict__ rows,
-                 const typename Vec4<R>::T* __restrict__ rw, int cap,
+                 const R* __restrict__ rw, int cap,
                  const typename Real2<R>::T* __restrict__ vpk, int np, int p0, int N, int ngroup,
                  Finish fin) {
   using V = typename Real2<R>::T;
-  using Q = typename Vec4<R>::T;
   using P = Stage<NP, R>;
   constexpr int S = P::S, ITS = P::ITS, CH = P::CH, DEEP = sizeof(R) == 4 ? 3 : 2, W = 25;
-  constexpr int FOLD = 16 / ITS, PER = kGroup * (int)sizeof(Q) / 16;  // 16-byte words an entry
+  constexpr int FOLD = 16 / ITS, PER = (int)sizeof(R);  // 16-byte words an entry
   union Shared {
     P stage[4][DEEP];
     R sum[4][32 * W];
@@ -450,21 +450,21 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2)
   const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = blockIdx.x * (4 / SPLIT) + wl / SPLIT, piece0 = wl % SPLIT;
   const int slot = lane / NP, pr = lane % NP;  // slot S and up: idle lanes
-  V sum[kGroup][3], part[kGroup][3];
+  V sum[2][6], part[2][6];  // beads (0, 1), (2, 3); values 3 h + c
 #pragma unroll
-  for (int b = 0; b < kGroup; b++)
+  for (int b = 0; b < 2; b++)
 #pragma unroll
-    for (int c = 0; c < 3; c++) sum[b][c].x = sum[b][c].y = part[b][c].x = part[b][c].y = 0;
+    for (int e = 0; e < 6; e++) sum[b][e].x = sum[b][e].y = part[b][e].x = part[b][e].y = 0;
   if (grp < ngroup) {
     const int n = cnt[grp];
     const int* row = rows + (size_t)grp * cap;
-    const Q* rq = rw + (size_t)grp * cap * kGroup;
+    const R* rq = rw + 16 * (size_t)grp * cap;
     const V* vp = vpk + p0 + pr;
     const size_t plane = (size_t)N * np;
     P* st = sh.stage[wl];
     auto issue = [&](int piece, int buf) {
       const int k0 = piece * CH, m = min(CH, n - k0);
-      const char* from = (const char*)(rq + (size_t)k0 * kGroup);
+      const char* from = (const char*)(rq + 16 * (size_t)k0);
       for (int e = lane; e < m * PER; e += 32)
         copy_async((char*)st[buf].w + 16 * e, from + 16 * e, 1);
       if (lane < m) copy_async(st[buf].j + lane, row + k0 + lane, 0);
@@ -494,13 +494,28 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2)
         const int k = t * S + slot;
         if (slot < S && k < m) {
 #pragma unroll
-          for (int b = 0; b < kGroup; b++) {
-            const Q q = p.w[kGroup * k + b];
-            const auto t1 = pack2(q.x), w0 = pack2(q.y), w1 = pack2(q.z), w2 = pack2(q.w);
-            const V d = signed_by(q.x, fma2(w2, x[t][2], fma2(w1, x[t][1], mul2(w0, x[t][0]))));
-            part[b][0] = fma2(d, w0, fma2(t1, x[t][0], part[b][0]));
-            part[b][1] = fma2(d, w1, fma2(t1, x[t][1], part[b][1]));
-            part[b][2] = fma2(d, w2, fma2(t1, x[t][2], part[b][2]));
+          for (int b = 0; b < 2; b++) {
+            V t1, w0, w1, w2;
+            if constexpr (sizeof(R) == 4) {
+              const float4 u = *(const float4*)(p.w + 16 * k + 8 * b),
+                           v = *(const float4*)(p.w + 16 * k + 8 * b + 4);
+              t1 = make_float2(u.x, u.y), w0 = make_float2(u.z, u.w);
+              w1 = make_float2(v.x, v.y), w2 = make_float2(v.z, v.w);
+            } else {
+              const V* q = (const V*)(p.w + 16 * k + 8 * b);
+              t1 = q[0], w0 = q[1], w1 = q[2], w2 = q[3];
+            }
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              const auto y0 = twice(h ? x[t][0].y : x[t][0].x),
+                         y1 = twice(h ? x[t][1].y : x[t][1].x),
+                         y2 = twice(h ? x[t][2].y : x[t][2].x);
+              const V d = signed_by(t1, fma2(w2, y2, fma2(w1, y1, mul2(w0, y0))));
+              V* o = part[b] + 3 * h;
+              o[0] = fma2(w0, d, fma2(t1, y0, o[0]));
+              o[1] = fma2(w1, d, fma2(t1, y1, o[1]));
+              o[2] = fma2(w2, d, fma2(t1, y2, o[2]));
+            }
           }
         }
       }
@@ -508,12 +523,12 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2)
       if (++folded == FOLD) {
         folded = 0;
 #pragma unroll
-        for (int b = 0; b < kGroup; b++)
+        for (int b = 0; b < 2; b++)
 #pragma unroll
-          for (int c = 0; c < 3; c++) {
-            sum[b][c].x += part[b][c].x;
-            sum[b][c].y += part[b][c].y;
-            part[b][c].x = part[b][c].y = 0;
+          for (int e = 0; e < 6; e++) {
+            sum[b][e].x += part[b][e].x;
+            sum[b][e].y += part[b][e].y;
+            part[b][e].x = part[b][e].y = 0;
           }
       }
     }
@@ -522,11 +537,11 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2)
   __syncthreads();  // the stages' memory holds the sums from here on
   R* o = sh.sum[wl] + lane * W;
 #pragma unroll
-  for (int b = 0; b < kGroup; b++)
+  for (int b = 0; b < 2; b++)
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      o[6 * b + c] = sum[b][c].x + part[b][c].x;
-      o[6 * b + 3 + c] = sum[b][c].y + part[b][c].y;
+    for (int e = 0; e < 6; e++) {
+      o[12 * b + e] = sum[b][e].x + part[b][e].x;
+      o[12 * b + 6 + e] = sum[b][e].y + part[b][e].y;
     }
   __syncthreads();
   if (grp >= ngroup) return;
@@ -546,7 +561,7 @@ void launch_apply(bd_ctx* c, int np, int p0, const Finish& fin) {
   const int ng = (c->N + kGroup - 1) / kGroup;
 #define REAL(SPLIT_)                                                                      \
   k_real_apply<NP, SPLIT_, R><<<nblk(ng, 4 / SPLIT_), 128, 0, c->stream>>>(               \
-      c->rl_cnt, c->rl_rows, (const typename Vec4<R>::T*)c->rl_w, c->rl_cap,              \
+      c->rl_cnt, c->rl_rows, (const R*)c->rl_w, c->rl_cap,                                \
       (const typename Real2<R>::T*)c->pme_vpk, np, p0, c->N, ng, fin)
   // about 16 warps an SM
   if (ng >= 148 * 12)
@@ -690,11 +705,11 @@ int real_prepare(bd_ctx* c, const Cell& cell, double cr, double sr, double alpha
   if (c->pme_f32)
     k_rl_tensors<float><<<nblk(ng, 4), 128, 0, c->stream>>>(
         cell, (const double4*)c->rl_pos, N, ng, c->rl_cnt, c->rl_rows, c->rl_cap, rc * rc, alpha,
-        alpha_ref, c->p.pme_max_pairs, (float4*)c->rl_w, c->err);
+        alpha_ref, c->p.pme_max_pairs, (float*)c->rl_w, c->err);
   else
     k_rl_tensors<double><<<nblk(ng, 4), 128, 0, c->stream>>>(
         cell, (const double4*)c->rl_pos, N, ng, c->rl_cnt, c->rl_rows, c->rl_cap, rc * rc, alpha,
-        alpha_ref, c->p.pme_max_pairs, (double4*)c->rl_w, c->err);
+        alpha_ref, c->p.pme_max_pairs, (double*)c->rl_w, c->err);
   return launch_ok(c);
 }
 
