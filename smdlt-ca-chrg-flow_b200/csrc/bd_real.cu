@@ -7,9 +7,8 @@
 // w = sqrt(|t2| / r^2) d, the sign s of t2 in the lowest mantissa bit of t1
 // (zero where a pair is beyond the cutoff).  The product then reads a
 // neighbour's input values once for four pairs, and positions and minimum
-// images not at all.  Rows are sorted by index: a chain that passes through the
-// cutoff sphere gives a run of consecutive neighbours, whose input values lie
-// side by side.
+// images not at all.  The beads of a cell are in increasing index, so a row's
+// order, and with it a product's rounding, is the same in every build.
 #include <math.h>
 
 #include <algorithm>
@@ -108,16 +107,40 @@ __global__ void k_rl_scan(int ncell, int* cell_count, int* cell_start, int* curs
   if (t == nt - 1) cell_start[ncell] = part[t];
 }
 
-// Positions in cell order, the bead index in the fourth component: the row
-// build streams a cell's beads with one contiguous load each.
 __global__ void k_rl_fill(const int* __restrict__ cell_of, const int* __restrict__ cell_start,
-                          int* cursor, const double4* __restrict__ pos, double4* spos, int N) {
+                          int* cursor, int* beads, int N) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   int c = cell_of[i];
-  double4 p = pos[i];
-  p.w = __longlong_as_double((long long)i);
-  spos[cell_start[c] + atomicAdd(&cursor[c], 1)] = p;
+  beads[cell_start[c] + atomicAdd(&cursor[c], 1)] = i;
+}
+
+// Positions in cell order, a cell's beads in increasing index, the index in the
+// fourth component: the row build streams a cell's beads with one contiguous
+// load each.  One block per cell, each bead placed by its rank.
+__global__ void __launch_bounds__(256) k_rl_order(const int* __restrict__ cell_start,
+                                                  const int* __restrict__ beads,
+                                                  const double4* __restrict__ pos,
+                                                  double4* spos) {
+  __shared__ int s[1024];
+  const int lo = cell_start[blockIdx.x], n = cell_start[blockIdx.x + 1] - lo;
+  for (int e0 = 0; e0 < n; e0 += blockDim.x) {
+    const int e = e0 + threadIdx.x, v = e < n ? beads[lo + e] : 0;
+    int rank = 0;
+    for (int t0 = 0; t0 < n; t0 += 1024) {
+      const int m = min(1024, n - t0);
+      __syncthreads();
+      for (int q = threadIdx.x; q < m; q += blockDim.x) s[q] = beads[lo + t0 + q];
+      __syncthreads();
+      if (e < n)
+        for (int q = 0; q < m; q++) rank += s[q] < v;
+    }
+    if (e < n) {
+      double4 p = pos[v];
+      p.w = __longlong_as_double((long long)v);
+      spos[lo + rank] = p;
+    }
+  }
 }
 
 // t1 with the sign of t2 in its lowest mantissa bit.
@@ -250,42 +273,19 @@ __global__ void __launch_bounds__(128, 4)
   }
 }
 
-// Rows in increasing index (bitonic, a block per row); rows longer than the
-// shared memory stay as they are.
-constexpr int kSortMax = 4096;
-__global__ void __launch_bounds__(128) k_rl_sort(const int* __restrict__ cnt, int cap, int* rows) {
-  __shared__ int s[kSortMax];
-  const int n = cnt[blockIdx.x];
-  if (n > kSortMax) return;
-  int* row = rows + (size_t)blockIdx.x * cap;
-  int m = 32;
-  while (m < n) m <<= 1;
-  for (int i = threadIdx.x; i < m; i += blockDim.x) s[i] = i < n ? row[i] : 0x7fffffff;
-  for (int k = 2; k <= m; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      __syncthreads();
-      for (int t = threadIdx.x; t < m / 2; t += blockDim.x) {
-        const int a = 2 * t - (t & (j - 1)), b = a + j;
-        const int x = s[a], y = s[b];
-        if ((x > y) == ((a & k) == 0)) {
-          s[a] = y;
-          s[b] = x;
-        }
-      }
-    }
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) row[i] = s[i];
-}
-
 // The four tensors of every entry, a warp per group, and each bead's number of
-// pairs against an explicit cap.  Entry k at rw[16 (group cap + k)].  Overlapping pairs (r < 2), whose terms cost three times as much, are
-// queued and formed 32 at a time.  Bound by the FP64 pipe (erfc, exp).
+// pairs against an explicit cap.  Entry k at rw[16 (group cap + k)].  32 entries
+// at a time are formed in shared memory and written side by side (from the
+// lanes, 64 bytes apart, every sector would be written eight times).
+// Overlapping pairs (r < 2), whose terms cost three times as much, are queued
+// and formed 32 at a time.  Bound by the FP64 pipe (erfc, exp).
 template <typename R>
 __global__ void __launch_bounds__(128, 4)
     k_rl_tensors(Cell cell, const double4* __restrict__ pos, int N, int ngroup,
                  const int* __restrict__ cnt, const int* __restrict__ rows, int cap, double rc2,
                  double alpha, double alpha_ref, int bead_cap, R* rw, int* err) {
-  __shared__ int c_queue[4][64];  // 4 k + b of overlapping pairs
+  __shared__ int c_queue[4][160];  // 4 k + b of overlapping pairs
+  __shared__ alignas(16) R s_entry[4][32 * 20];  // entries 20 apart: fewer bank conflicts
   const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = blockIdx.x * 4 + wl;
   if (grp >= ngroup) return;
@@ -294,58 +294,61 @@ __global__ void __launch_bounds__(128, 4)
   const int* row = rows + (size_t)grp * cap;
   R* out = rw + 16 * (size_t)grp * cap;
   int* queue = c_queue[wl];
-  int nq = 0;
-  auto store = [&](auto overlap, int k, int b, double rr, double dx, double dy, double dz) {
+  int nq = 0, count[kGroup] = {0, 0, 0, 0};
+  auto form = [&](auto overlap, R* entry, int b, double rr, double dx, double dy, double dz) {
     constexpr bool OV = decltype(overlap)::value;
     const double r = sqrt(rr), ir = 1.0 / r, irr = ir * ir;
     double t1, t2;
     pair_terms<OV>(alpha, alpha_ref, rr, r, ir, irr, t1, t2);
-    store_tensor(out + 16 * (size_t)k, b, t1, t2, sqrt(fabs(t2)) * ir, dx, dy, dz);
+    store_tensor(entry, b, t1, t2, sqrt(fabs(t2)) * ir, dx, dy, dz);
   };
   auto flush = [&](int m) {
     if (lane < m) {
-      const int k = queue[lane] >> 2, b = queue[lane] & 3;
+      const int k = queue[nq - m + lane] >> 2, b = queue[nq - m + lane] & 3;
       double dx, dy, dz;
       const double rr = image(pos[row[k]], pos[i0 + b], dx, dy, dz);
-      store(std::integral_constant<bool, true>(), k, b, rr, dx, dy, dz);
+      form(std::integral_constant<bool, true>(), out + 16 * (size_t)k, b, rr, dx, dy, dz);
     }
     nq -= m;
-    const int rest = lane < nq ? queue[m + lane] : 0;
-    __syncwarp();
-    if (lane < nq) queue[lane] = rest;
     __syncwarp();
   };
-  int longest = 0;
 #pragma unroll 1
-  for (int b = 0; b < kGroup; b++) {
-    const double4 pb = pos[min(i0 + b, N - 1)];
-    int count = 0;
+  for (int k0 = 0; k0 < n; k0 += 32) {
+    const int k = k0 + lane, m = min(32, n - k0);
+    R* entry = s_entry[wl] + 20 * lane;
+    const int j = k < n ? row[k] : 0;
+    const double4 pj = pos[j];
 #pragma unroll 1
-    for (int k0 = 0; k0 < n; k0 += 32) {
-      const int k = k0 + lane;
+    for (int b = 0; b < kGroup; b++) {
       bool near = false;
-      if (k < n) {
-        const int j = row[k];
-        double dx, dy, dz;
-        const double rr = image(pos[j], pb, dx, dy, dz);
-        if (b < nb && j != i0 + b && !(rr >= rc2)) {
-          count++;
-          near = rr < 4.0;
-          if (!near) store(std::integral_constant<bool, false>(), k, b, rr, dx, dy, dz);
-        } else {
-          store_tensor(out + 16 * (size_t)k, b, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0);
-        }
+      double dx, dy, dz;
+      const double rr = image(pj, pos[min(i0 + b, N - 1)], dx, dy, dz);
+      if (k < n && b < nb && j != i0 + b && !(rr >= rc2)) {
+        count[0] += b == 0, count[1] += b == 1, count[2] += b == 2, count[3] += b == 3;
+        near = rr < 4.0;
+        if (!near) form(std::integral_constant<bool, false>(), entry, b, rr, dx, dy, dz);
+      } else {
+        store_tensor(entry, b, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0);
       }
       const unsigned hit = __ballot_sync(0xffffffffu, near);
       if (near) queue[nq + __popc(hit & ((1u << lane) - 1u))] = 4 * k + b;
       nq += __popc(hit);
-      __syncwarp();
-      if (nq >= 32) flush(32);
     }
-    for (int o = 16; o > 0; o >>= 1) count += __shfl_xor_sync(0xffffffffu, count, o);
-    longest = max(longest, count);
+    __syncwarp();
+    constexpr int WORDS = (int)sizeof(R);  // 16-byte words an entry
+    float4* to = (float4*)(out + 16 * (size_t)k0);
+    for (int e = lane; e < m * WORDS; e += 32)
+      to[e] = ((const float4*)(s_entry[wl] + 20 * (e / WORDS)))[e % WORDS];
+    __syncwarp();
+    while (nq >= 32) flush(32);
   }
   if (nq > 0) flush(nq);
+  int longest = 0;
+#pragma unroll
+  for (int b = 0; b < kGroup; b++) {
+    for (int o = 16; o > 0; o >>= 1) count[b] += __shfl_xor_sync(0xffffffffu, count[b], o);
+    longest = max(longest, count[b]);
+  }
   if (lane == 0 && bead_cap > 0 && longest > bead_cap) atomicOr(err, ERRB_NBR_OVERFLOW);
 }
 
@@ -614,7 +617,7 @@ static int rows_alloc(bd_ctx* c, int cap) {
 int real_alloc(bd_ctx* c) {
   int N = c->N, s;
   // row cap: an explicit cap per bead bounds a group's row by four times that;
-  // the default is 1.6 times the mean number of beads within the cutoff at the
+  // the default is 2.5 times the mean number of beads within the cutoff at the
   // system's density, at least 512 (rows that overflow it are grown); no row
   // is longer than N
   long cap;
@@ -622,7 +625,7 @@ int real_alloc(bd_ctx* c) {
     cap = (long)kGroup * c->p.pme_max_pairs;
   } else {
     double mean = 4.0 / 3.0 * M_PI * c->pme_rc * c->pme_rc * c->pme_rc * N / c->boxvol;
-    cap = std::max(512, ((int)ceil(1.6 * mean) + 31) / 32 * 32);
+    cap = std::max(512, ((int)ceil(2.5 * mean) + 31) / 32 * 32);
   }
   if ((s = rows_alloc(c, (int)std::min(cap, (long)std::max(N, 1)))) != BD_OK) return s;
   CU(cudaMalloc(&c->rl_cnt, 4 * (size_t)N));
@@ -631,16 +634,17 @@ int real_alloc(bd_ctx* c) {
   c->rl_ncell_cap = 4096;
   CU(cudaMalloc(&c->rl_cell_of, 4 * (size_t)N));
   CU(cudaMalloc(&c->rl_spos, 32 * (size_t)N));
+  CU(cudaMalloc(&c->rl_beads, 4 * (size_t)N));
   CU(cudaMalloc(&c->rl_cell_count, 4 * (size_t)c->rl_ncell_cap));
   CU(cudaMalloc(&c->rl_cell_start, 4 * (size_t)(c->rl_ncell_cap + 1)));
   CU(cudaMalloc(&c->rl_cursor, 4 * (size_t)c->rl_ncell_cap));
   CU(cudaMemsetAsync(c->rl_cell_count, 0, 4 * (size_t)c->rl_ncell_cap, c->stream));
-  c->bytes += 40 * (size_t)N + 12 * (size_t)c->rl_ncell_cap;
+  c->bytes += 44 * (size_t)N + 12 * (size_t)c->rl_ncell_cap;
   return BD_OK;
 }
 
 void real_free(bd_ctx* c) {
-  void* ptrs[] = {c->rl_rows, c->rl_w, c->rl_cnt, c->rl_need, c->rl_cell_of, c->rl_spos,
+  void* ptrs[] = {c->rl_rows, c->rl_w, c->rl_cnt, c->rl_need, c->rl_cell_of, c->rl_spos, c->rl_beads,
                   c->rl_cell_count, c->rl_cell_start, c->rl_cursor};
   for (void* q : ptrs)
     if (q) cudaFree(q);
@@ -679,8 +683,10 @@ int real_prepare(bd_ctx* c, const Cell& cell, double cr, double sr, double alpha
                                                   c->rl_cell_of, c->rl_cell_count);
   k_rl_scan<<<1, 1024, 0, c->stream>>>(ncell, c->rl_cell_count, c->rl_cell_start, c->rl_cursor);
   k_rl_fill<<<nblk(N, 256), 256, 0, c->stream>>>(c->rl_cell_of, c->rl_cell_start, c->rl_cursor,
-                                                 (const double4*)c->rl_pos,
-                                                 (double4*)c->rl_spos, N);
+                                                 c->rl_beads, N);
+  c->launches++;
+  k_rl_order<<<ncell, 256, 0, c->stream>>>(c->rl_cell_start, c->rl_beads,
+                                           (const double4*)c->rl_pos, (double4*)c->rl_spos);
   if ((s = launch_ok(c)) != BD_OK) return s;
   // the rows; with the default cap (no pme_max_pairs), rows that
   // overflow it are grown to 1.25 times the longest row and built again
@@ -700,8 +706,7 @@ int real_prepare(bd_ctx* c, const Cell& cell, double cr, double sr, double alpha
       return s;
     CU(cudaMemsetAsync(c->rl_need, 0, 4, c->stream));
   }
-  c->launches += 2;
-  k_rl_sort<<<ng, 128, 0, c->stream>>>(c->rl_cnt, c->rl_cap, c->rl_rows);
+  c->launches++;
   if (c->pme_f32)
     k_rl_tensors<float><<<nblk(ng, 4), 128, 0, c->stream>>>(
         cell, (const double4*)c->rl_pos, N, ng, c->rl_cnt, c->rl_rows, c->rl_cap, rc * rc, alpha,
