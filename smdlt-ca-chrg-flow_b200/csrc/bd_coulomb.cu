@@ -261,16 +261,20 @@ __global__ void k_cc_fill(const int* __restrict__ cell_of, const int* __restrict
 
 // Forces on each charge: reciprocal part from the potential grid and the
 // spline derivatives, real-space pairs within rc; adds to the bead forces and
-// writes the charge's real-space energy share (half of its pair sum).
+// writes the charge's real-space energy share (half of its pair sum).  One warp
+// per charge.  The candidates of the neighbour cells come with one contiguous
+// load each (sorted); those within the cutoff, about one in seven, are queued
+// in shared memory and their erfc and exp formed 32 at a time, so no lane idles
+// in them.  Bound by the FP64 pipe.  25 000 charges on 100^3: FORCES_FIGURES
 template <int P>
 __global__ void __launch_bounds__(256)
     k_cw_forces(Cell cell, CGeom g, const double4* __restrict__ cq, const int* __restrict__ track,
                 int nch, double cr, double sr, int K, const int* __restrict__ base,
                 const double* __restrict__ w, const double* __restrict__ dw,
                 const double* __restrict__ phi, const int* __restrict__ cell_of,
-                const int* __restrict__ start, const int* __restrict__ idx, double rc2,
-                double beta, double lambda_b, double* fx, double* fy, double* fz,
-                double* ereal) {
+                const int* __restrict__ start, const int* __restrict__ idx,
+                const double4* __restrict__ sorted, double rc2, double beta,
+                double lambda_b, double* fx, double* fy, double* fz, double* ereal) {
   int k = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (k >= nch) return;
   double4 me = cq[k];
@@ -301,69 +305,51 @@ __global__ void __launch_bounds__(256)
   double xi, yi;
   lab_of(me.x, me.y, cr, sr, xi, yi);
   double zi = me.z;
-  int ci = cell_of[k];
-  int cd[3] = {ci / (g.n[1] * g.n[2]), (ci / g.n[2]) % g.n[1], ci % g.n[2]};
+  const int ci = cell_of[k];
+  const int cd[3] = {ci / (g.n[1] * g.n[2]), (ci / g.n[2]) % g.n[1], ci % g.n[2]};
   double f0 = 0, f1 = 0, f2 = 0, en = 0;
   const double rtpi = sqrt(M_PI);
-  int lo[3], hi[3];
-  for (int d = 0; d < 3; d++) {
-    lo[d] = g.n[d] >= 3 ? -1 : 0;
-    hi[d] = g.n[d] >= 3 ? 1 : g.n[d] - 1;
-  }
-  // the (at most 27) neighbour cells as one candidate list: lane l < ncell
-  // takes cell l's range; a warp scan of the counts places candidate m in
-  // the cell whose range holds it, so the lanes walk all cells at once (no
-  // chain of dependent loads per cell)
-  __shared__ int c_start[8][32], c_excl[8][32], c_incl[8][32];
+  __shared__ CandList c_list[8];
+  __shared__ int c_queue[8][64];
   const int wl = threadIdx.x >> 5;
-  int nd[3] = {hi[0] - lo[0] + 1, hi[1] - lo[1] + 1, hi[2] - lo[2] + 1};
-  int ncell = nd[0] * nd[1] * nd[2];
-  int my_s = 0, my_n = 0;
-  if (lane < ncell) {
-    int a = lo[0] + lane / (nd[1] * nd[2]), b = lo[1] + (lane / nd[2]) % nd[1],
-        c = lo[2] + lane % nd[2];
-    int e0 = g.n[0] >= 3 ? (cd[0] + a + g.n[0]) % g.n[0] : a;
-    int e1 = g.n[1] >= 3 ? (cd[1] + b + g.n[1]) % g.n[1] : b;
-    int e2 = g.n[2] >= 3 ? (cd[2] + c + g.n[2]) % g.n[2] : c;
-    int cc = (e0 * g.n[1] + e1) * g.n[2] + e2;
-    my_s = start[cc];
-    my_n = start[cc + 1] - my_s;
+  const int total = c_list[wl].open(g.n, cd, start);
+  int* queue = c_queue[wl];
+  const Image image(cell);
+  const double4 here = make_double4(xi, yi, zi, 0.0);
+  int cl = 0, nq = 0;
+  auto take = [&](int m) {  // the first m queued pairs
+    if (lane < m) {
+      const double4 ot = sorted[queue[lane]];
+      double dx, dy, dz;
+      const double rr = image(here, ot, dx, dy, dz);
+      double r = sqrt(rr), qq = lambda_b * me.w * ot.w;
+      double ec = erfc(beta * r) / r;
+      double fr = qq * (ec + 2.0 * beta / rtpi * exp(-beta * beta * rr)) / rr;
+      f0 += fr * dx;
+      f1 += fr * dy;
+      f2 += fr * dz;
+      en += 0.5 * qq * ec;
+    }
+    nq -= m;
+    const int rest = lane < nq ? queue[m + lane] : 0;
+    __syncwarp();
+    if (lane < nq) queue[lane] = rest;
+    __syncwarp();
+  };
+  for (int m0 = 0; m0 < total; m0 += 32) {
+    int at = -1;
+    if (m0 + lane < total) {
+      at = c_list[wl].at(m0 + lane, cl);
+      double dx, dy, dz;
+      if (image(here, sorted[at], dx, dy, dz) >= rc2 || idx[at] == k) at = -1;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, at >= 0);
+    if (at >= 0) queue[nq + __popc(hit & ((1u << lane) - 1u))] = at;
+    nq += __popc(hit);
+    __syncwarp();
+    if (nq >= 32) take(32);
   }
-  int incl = my_n;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    int t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
-  c_start[wl][lane] = my_s;
-  c_excl[wl][lane] = incl - my_n;
-  c_incl[wl][lane] = incl;
-  __syncwarp();
-  const int total = __shfl_sync(0xffffffffu, incl, 31);
-  int cl = 0;
-  for (int m = lane; m < total; m += 32) {
-    while (m >= c_incl[wl][cl]) cl++;  // ends at the last cell: m < total
-    int j = idx[c_start[wl][cl] + (m - c_excl[wl][cl])];
-    if (j == k) continue;
-    double4 ot = cq[j];
-    double xj, yj;
-    lab_of(ot.x, ot.y, cr, sr, xj, yj);
-    double dx = xi - xj, dy = yi - yj, dz = zi - ot.z, s[3];
-    frac_of(cell, dx, dy, dz, s);
-    for (int d = 0; d < 3; d++) s[d] -= rint(s[d]);
-    dx = cell.H[0] * s[0] + cell.H[1] * s[1] + cell.H[2] * s[2];
-    dy = cell.H[3] * s[0] + cell.H[4] * s[1] + cell.H[5] * s[2];
-    dz = cell.H[6] * s[0] + cell.H[7] * s[1] + cell.H[8] * s[2];
-    double rr = dx * dx + dy * dy + dz * dz;
-    if (rr >= rc2) continue;
-    double r = sqrt(rr), qq = lambda_b * me.w * ot.w;
-    double ec = erfc(beta * r) / r;
-    double fr = qq * (ec + 2.0 * beta / rtpi * exp(-beta * beta * rr)) / rr;
-    f0 += fr * dx;
-    f1 += fr * dy;
-    f2 += fr * dz;
-    en += 0.5 * qq * ec;
-  }
+  if (nq > 0) take(nq);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     gu0 += __shfl_xor_sync(0xffffffffu, gu0, o);
@@ -389,12 +375,21 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Fixed-order sums: out[0] += sum part[0..n) (one warp)
-__global__ void k_sum_into(const double* __restrict__ part, int n, double* out) {
+// out[0] = sum part[0..n) in a fixed order, one block (one warp took 18 us for
+// 25 000 entries, a chain of loads).
+__global__ void __launch_bounds__(1024) k_sum_into(const double* __restrict__ part, int n,
+                                                   double* out) {
+  __shared__ double sh[32];
   double s = 0;
-  for (int b = threadIdx.x; b < n; b += 32) s += part[b];
+  for (int b = threadIdx.x; b < n; b += 1024) s += part[b];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (threadIdx.x == 0) *out = s;
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = sh[threadIdx.x];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) *out = s;
+  }
 }
 
 }  // namespace
@@ -587,12 +582,12 @@ int coulomb_ewald(bd_ctx* c, const Lat& l, const double4* cq) {
   k_cw_influence<<<c->cw_nblk, 256, 0, c->stream>>>(cell, K, c->cw_beta, c->p.lambda_b,
                                                     c->cw_bsq, (cufftDoubleComplex*)c->cw_spec,
                                                     c->cw_epart);
-  k_sum_into<<<1, 32, 0, c->stream>>>(c->cw_epart, c->cw_nblk, c->cw_energy + 1);
+  k_sum_into<<<1, 1024, 0, c->stream>>>(c->cw_epart, c->cw_nblk, c->cw_energy + 1);
   CF(cufftExecZ2D((cufftHandle)c->cw_plan_b, (cufftDoubleComplex*)c->cw_spec, c->cw_grid));
 #define CW_FORCES(P_)                                                                        \
   k_cw_forces<P_><<<nblk(nch, 8), 256, 0, c->stream>>>(                                       \
       cell, g, cq, c->track, nch, cr, sr, K, c->cw_base, w, dw, c->cw_grid, c->cw_cell_of,    \
-      c->cw_start, c->cw_idx, rc * rc, c->cw_beta, c->p.lambda_b, c->fx, c->fy, c->fz,        \
+      c->cw_start, c->cw_idx, (const double4*)c->cw_sorted, rc * rc, c->cw_beta, c->p.lambda_b, c->fx, c->fy, c->fz,        \
       c->cw_epart)
   switch (p) {
     case 4: CW_FORCES(4); break;
@@ -600,7 +595,7 @@ int coulomb_ewald(bd_ctx* c, const Lat& l, const double4* cq) {
     default: CW_FORCES(8);
   }
 #undef CW_FORCES
-  k_sum_into<<<1, 32, 0, c->stream>>>(c->cw_epart, nch, c->cw_energy);
+  k_sum_into<<<1, 1024, 0, c->stream>>>(c->cw_epart, nch, c->cw_energy);
   c->cw_cell_V = cell.V;
   return launch_ok(c);
 }

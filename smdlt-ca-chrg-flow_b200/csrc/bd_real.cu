@@ -164,29 +164,6 @@ __device__ __forceinline__ void store_tensor(R* entry, int b, double t1, double 
   o[6] = (R)(sw * dz);
 }
 
-// Minimum-image displacement; the cell is (b1, b2) in the xy plane and L e_z, and
-// the nearest integer of |s| < 2^51 comes from adding and subtracting 1.5 2^52
-// (two additions for one slow conversion).
-struct Image {
-  double h00, h01, h10, h11, g00, g01, g10, g11, Lz, iLz;
-  __device__ __forceinline__ explicit Image(const Cell& c)
-      : h00(c.H[0]), h01(c.H[1]), h10(c.H[3]), h11(c.H[4]), g00(c.Hi[0]), g01(c.Hi[1]),
-        g10(c.Hi[3]), g11(c.Hi[4]), Lz(c.H[8]), iLz(c.Hi[8]) {}
-  static __device__ __forceinline__ double nearest(double s) {
-    return __dsub_rn(__dadd_rn(s, 6755399441055744.0), 6755399441055744.0);
-  }
-  __device__ __forceinline__ double operator()(const double4& pj, const double4& pi, double& dx,
-                                               double& dy, double& dz) const {
-    dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
-    double n0 = nearest(g00 * dx + g01 * dy), n1 = nearest(g10 * dx + g11 * dy),
-           n2 = nearest(iLz * dz);
-    dx -= h00 * n0 + h01 * n1;
-    dy -= h10 * n0 + h11 * n1;
-    dz -= Lz * n2;
-    return dx * dx + dy * dy + dz * dz;
-  }
-};
-
 // Neighbour indices of the groups' rows, cap entries a row, in no order.  One
 // warp per group.  For each of its beads the at most 27 neighbour cells form
 // one candidate list; the lanes test 32 candidates at a time and queue the
