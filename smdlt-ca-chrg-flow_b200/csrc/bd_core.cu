@@ -57,14 +57,74 @@ int launch_ok_at(bd_ctx* c, const char* file, int line) {
 }
 
 int check(bd_ctx* c) {
-  int bits = 0;
-  CU(cudaMemcpyAsync(&bits, c->err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  // the error word through the pinned staging's last entry
+  int* word = (int*)(c->stage + 2 * kStages * (size_t)c->N);
+  CU(cudaMemcpyAsync(word, c->err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CU(cudaStreamSynchronize(c->stream));
+  const int bits = *word;
   if (bits) {
     CU(cudaMemsetAsync(c->err, 0, sizeof(int), c->stream));
     CU(cudaStreamSynchronize(c->stream));
   }
   return set_error_from_bits(bits);
+}
+
+// Host arrays pass through pinned memory, kStages pieces of 2 N numbers used in
+// turn: a copy from or to pageable memory is staged by the driver piece by
+// piece, each with a round trip (three force arrays of 50 000 beads took 390
+// us), and blocks the caller.
+static int stage_next(bd_ctx* c, int* k) {
+  *k = c->stage_at;
+  c->stage_at = (c->stage_at + 1) % kStages;
+  if (c->stage_busy[*k]) CU(cudaEventSynchronize(c->stage_ev[*k]));
+  c->stage_busy[*k] = false;
+  return BD_OK;
+}
+
+// dev[0 .. n) = host[0 .. n), in stream order; the host array is free at return.
+int stage_up(bd_ctx* c, double* dev, const double* host, size_t n) {
+  int s, k;
+  const size_t piece = 2 * (size_t)c->N;
+  for (size_t o = 0; o < n; o += piece) {
+    const size_t m = std::min(piece, n - o);
+    if ((s = stage_next(c, &k)) != BD_OK) return s;
+    double* p = c->stage + k * piece;
+    memcpy(p, host + o, 8 * m);
+    CU(cudaMemcpyAsync(dev + o, p, 8 * m, cudaMemcpyHostToDevice, c->stream));
+    CU(cudaEventRecord(c->stage_ev[k], c->stream));
+    c->stage_busy[k] = true;
+  }
+  return BD_OK;
+}
+
+// host[r][0 .. n) = dev[r][0 .. n) for r < count; synchronises and returns the
+// status of the device work before it, as check does.
+int stage_down(bd_ctx* c, int count, const double* const* dev, double* const* host, size_t n) {
+  int s;
+  const size_t piece = 2 * (size_t)c->N, each = (n + piece - 1) / piece, all = each * count;
+  int slot[kStages];
+  for (size_t q = 0; q < all + kStages; q++) {
+    if (q >= (size_t)kStages) {  // the piece sent kStages ago
+      const size_t r = (q - kStages) / each, o = (q - kStages) % each * piece;
+      if (r < (size_t)count) {
+        const int k = slot[q % kStages];
+        CU(cudaEventSynchronize(c->stage_ev[k]));
+        c->stage_busy[k] = false;
+        memcpy(host[r] + o, c->stage + k * piece, 8 * std::min(piece, n - o));
+      }
+    }
+    if (q < all) {
+      const size_t r = q / each, o = q % each * piece;
+      int k;
+      if ((s = stage_next(c, &k)) != BD_OK) return s;
+      slot[q % kStages] = k;
+      CU(cudaMemcpyAsync(c->stage + k * piece, dev[r] + o, 8 * std::min(piece, n - o),
+                         cudaMemcpyDeviceToHost, c->stream));
+      CU(cudaEventRecord(c->stage_ev[k], c->stream));
+      c->stage_busy[k] = true;
+    }
+  }
+  return check(c);
 }
 
 static const double kEP = 0.9624;  // strain period constant (shear/src/Parameters.h:37)
@@ -888,6 +948,17 @@ int bd_create(const bd_params* p, bd_ctx** out) {
       return BD_ERR_OOM;
     }
   }
+  // the transfers' pinned staging (bd_ctx.cuh), here for the same reason
+  if (cudaMallocHost(&c->stage, 8 * (2 * kStages * (size_t)N + 8)) != cudaSuccess) {
+    c->stage = nullptr;
+    bd_destroy(c);
+    return BD_ERR_OOM;
+  }
+  for (int k = 0; k < kStages; k++)
+    if (cudaEventCreateWithFlags(&c->stage_ev[k], cudaEventDisableTiming) != cudaSuccess) {
+      bd_destroy(c);
+      return BD_ERR_CUDA;
+    }
   c->use_graphs = true;
   c->device_krylov = true;
   c->t = 0;
@@ -914,6 +985,11 @@ int bd_destroy(bd_ctx* c) {
     if (q) cudaFree(q);
   pme_free(c);
   coulomb_free(c);
+  if (c->stage) cudaFreeHost(c->stage);
+  for (int k = 0; k < kStages; k++)
+    if (c->stage_ev[k]) cudaEventDestroy(c->stage_ev[k]);
+  for (double* q : {c->io, c->io_x, c->io_y})
+    if (q) cudaFree(q);
   if (c->hop_work) cudaFree(c->hop_work);
   if (c->hop_cells) cudaFree(c->hop_cells);
   if (c->hop_de) cudaFree(c->hop_de);
@@ -992,22 +1068,20 @@ size_t bd_device_bytes(const bd_ctx* c) { return c ? c->bytes : 0; }
 static int up3(bd_ctx* c, double* a, double* b, double* d, const double* x, const double* y,
                const double* z) {
   if (!c || !x || !y || !z) return BD_ERR_ARG;
-  size_t n = 8 * (size_t)c->N;
-  CU(cudaMemcpyAsync(a, x, n, cudaMemcpyHostToDevice, c->stream));
-  CU(cudaMemcpyAsync(b, y, n, cudaMemcpyHostToDevice, c->stream));
-  CU(cudaMemcpyAsync(d, z, n, cudaMemcpyHostToDevice, c->stream));
-  CU(cudaStreamSynchronize(c->stream));
+  int s;
+  double* dev[3] = {a, b, d};
+  const double* host[3] = {x, y, z};
+  for (int k = 0; k < 3; k++)
+    if ((s = stage_up(c, dev[k], host[k], c->N)) != BD_OK) return s;
   return BD_OK;
 }
 
 static int down3(bd_ctx* c, const double* a, const double* b, const double* d, double* x,
                  double* y, double* z) {
   if (!c || !x || !y || !z) return BD_ERR_ARG;
-  size_t n = 8 * (size_t)c->N;
-  CU(cudaMemcpyAsync(x, a, n, cudaMemcpyDeviceToHost, c->stream));
-  CU(cudaMemcpyAsync(y, b, n, cudaMemcpyDeviceToHost, c->stream));
-  CU(cudaMemcpyAsync(z, d, n, cudaMemcpyDeviceToHost, c->stream));
-  return check(c);
+  const double* dev[3] = {a, b, d};
+  double* host[3] = {x, y, z};
+  return stage_down(c, 3, dev, host, c->N);
 }
 
 int bd_upload_positions(bd_ctx* c, const double* x, const double* y, const double* z) {
@@ -1043,15 +1117,13 @@ int bd_reset_stress(bd_ctx* c) {
 
 int bd_upload_noise(bd_ctx* c, const double* R) {
   if (!c || !R) return BD_ERR_ARG;
-  CU(cudaMemcpyAsync(c->R, R, 24 * (size_t)c->N, cudaMemcpyHostToDevice, c->stream));
-  CU(cudaStreamSynchronize(c->stream));
-  return BD_OK;
+  return stage_up(c, c->R, R, 3 * (size_t)c->N);
 }
 
 int bd_download_noise(bd_ctx* c, double* R) {
   if (!c || !R) return BD_ERR_ARG;
-  CU(cudaMemcpyAsync(R, c->R, 24 * (size_t)c->N, cudaMemcpyDeviceToHost, c->stream));
-  return check(c);
+  const double* dev = c->R;
+  return stage_down(c, 1, &dev, &R, 3 * (size_t)c->N);
 }
 
 int bd_set_charges(bd_ctx* c, const int* track, int nch) {

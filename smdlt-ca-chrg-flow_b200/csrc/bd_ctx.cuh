@@ -20,6 +20,8 @@
 
 // Largest Krylov dimension of the Lanczos square root.
 constexpr int kMaxKrylov = 400;
+// Pieces of the transfers' pinned staging.
+constexpr int kStages = 3;
 // Largest block of the segment preconditioner, in beads.
 constexpr int kMaxSegment = BD_PRECOND_MAX_SEGMENT;
 
@@ -28,6 +30,16 @@ struct bd_ctx {
   int N, Nb, Nc;
   cudaStream_t stream;
   int device;
+
+  // host transfers: kStages pinned pieces of 2 N numbers and the error word; the
+  // copies that use them, in turn
+  double *stage;
+  cudaEvent_t stage_ev[kStages];
+  bool stage_busy[kStages];
+  int stage_at;
+  // device side of the vector calls: interleaved vectors, and inputs and outputs
+  // in the Lanczos layout (as many as a noise block has)
+  double *io, *io_x, *io_y;
 
   // derived constants
   double rv, r2cut, rnew, qmax2, kappa_d, boxvol, kappas_eff;
@@ -225,6 +237,8 @@ void prof_clear(bd_ctx* c);
 
 int set_error_from_bits(int bits);
 int check(bd_ctx* c);                 // synchronise and fold device error bits
+int stage_up(bd_ctx* c, double* dev, const double* host, size_t n);
+int stage_down(bd_ctx* c, int count, const double* const* dev, double* const* host, size_t n);
 // report a launch error (or an earlier asynchronous one), recording the call
 // site for bd_last_error_detail
 int launch_ok_at(bd_ctx* c, const char* file, int line);

@@ -55,18 +55,28 @@ __global__ void k_norm_fin(const double* __restrict__ part, int nblk, double* sc
   }
 }
 
-// v (SoA, padded) = z (bead-interleaved) / |z|; padding entries are zero.
-// Right-hand side blockIdx.y: z zs, v vs entries further on, scalars 2.
+// v (SoA, padded) = z (bead-interleaved) / |z| (sc null: z itself); padding
+// entries are zero.  Right-hand side blockIdx.y: z zs, v vs entries further on,
+// scalars 2.
 __global__ void k_interleaved_to_soa(const double* __restrict__ z, size_t zs,
                                      const double* __restrict__ sc, double* v, size_t vs, int N,
                                      int NTp) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= NTp) return;
   z += (size_t)blockIdx.y * zs;
-  sc += 2 * blockIdx.y;
   v += (size_t)blockIdx.y * vs;
-  double f = sc[1];
+  double f = sc ? sc[2 * blockIdx.y + 1] : 1.0;
   for (int a = 0; a < 3; a++) v[(size_t)a * NTp + i] = i < N ? z[3 * i + a] * f : 0.0;
+}
+
+// z (bead-interleaved) = v (SoA); right-hand side blockIdx.y.
+__global__ void k_soa_to_interleaved(const double* __restrict__ v, size_t vs, double* z, size_t zs,
+                                     int N, int NTp) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  v += (size_t)blockIdx.y * vs;
+  z += (size_t)blockIdx.y * zs;
+  for (int a = 0; a < 3; a++) z[3 * (size_t)i + a] = v[(size_t)a * NTp + i];
 }
 
 // y_r = |z_r| sum_k c_r[k] V_r,k for the right-hand sides of a block
@@ -1576,25 +1586,66 @@ int lanczos_inv_sqrt(bd_ctx* c, const double* z, double* out, int* iters, bool* 
 
 }  // namespace bd
 
+// Device buffers of the vector calls for k vectors, made at the first call.
+static int io_alloc(bd_ctx* c) {
+  if (c->io) return BD_OK;
+  const size_t k = (size_t)std::max(1, c->nbk), n = 3 * (size_t)c->NT * 32;
+  if (cudaMalloc(&c->io, 24 * (size_t)c->N * k) != cudaSuccess ||
+      cudaMalloc(&c->io_x, 8 * n * k) != cudaSuccess ||
+      cudaMalloc(&c->io_y, 8 * n * k) != cudaSuccess) {
+    cudaGetLastError();  // not a sticky error: the next launch check must not see it
+    for (double** q : {&c->io, &c->io_x, &c->io_y}) {
+      cudaFree(*q);
+      *q = nullptr;
+    }
+    return BD_ERR_OOM;
+  }
+  c->bytes += (24 * (size_t)c->N + 16 * n) * k;
+  return BD_OK;
+}
+
+// k vectors (Lanczos layout, n apart) to the host, bead-interleaved.
+static int io_out(bd_ctx* c, int k, const double* v, double* out) {
+  const int N = c->N, NTp = c->NT * 32;
+  const size_t n3 = 3 * (size_t)N;
+  c->launches++;
+  k_soa_to_interleaved<<<dim3((N + 255) / 256, k), 256, 0, c->stream>>>(v, 3 * (size_t)NTp, c->io,
+                                                                       n3, N, NTp);
+  int s = launch_ok(c);
+  if (s != BD_OK) return s;
+  std::vector<const double*> dev(k);
+  std::vector<double*> host(k);
+  for (int r = 0; r < k; r++) {
+    dev[r] = c->io + n3 * r;
+    host[r] = out + n3 * r;
+  }
+  return stage_down(c, k, dev.data(), host.data(), n3);
+}
+
+// k host vectors, bead-interleaved, into c->io_x (Lanczos layout, n apart).
+static int io_in(bd_ctx* c, int k, const double* v) {
+  const int N = c->N, NTp = c->NT * 32;
+  const size_t n3 = 3 * (size_t)N;
+  int s = stage_up(c, c->io, v, n3 * k);
+  if (s != BD_OK) return s;
+  c->launches++;
+  k_interleaved_to_soa<<<dim3((NTp + 255) / 256, k), 256, 0, c->stream>>>(
+      c->io, n3, nullptr, c->io_x, 3 * (size_t)NTp, N, NTp);
+  return launch_ok(c);
+}
+
 extern "C" {
 
 int bd_mobility_apply(bd_ctx* c, const double* v, double* out) {
   if (!c || !v || !out) return BD_ERR_ARG;
   if (!c->hi_built) return BD_ERR_STATE;
   int s;
-  if ((s = alloc_lanczos(c)) != BD_OK) return s;
-  int N = c->N, NTp = c->NT * 32;
-  std::vector<double> soa(3 * (size_t)NTp, 0.0), res(3 * (size_t)NTp);
-  for (int i = 0; i < N; i++)
-    for (int a = 0; a < 3; a++) soa[(size_t)a * NTp + i] = v[3 * i + a];
-  CU(cudaMemcpyAsync(c->Lw, soa.data(), 8 * soa.size(), cudaMemcpyHostToDevice, c->stream));
-  VecIn vi = {{c->Lw, c->Lw + NTp, c->Lw + 2 * NTp}, 1};
+  if ((s = alloc_lanczos(c)) != BD_OK || (s = io_alloc(c)) != BD_OK) return s;
+  int NTp = c->NT * 32;
+  if ((s = io_in(c, 1, v)) != BD_OK) return s;
+  VecIn vi = {{c->io_x, c->io_x + NTp, c->io_x + 2 * NTp}, 1};
   if ((s = sym_matvec(c, 1, vi, vi, c->Yz, c->Yz, true)) != BD_OK) return s;
-  CU(cudaMemcpyAsync(res.data(), c->Yz, 8 * res.size(), cudaMemcpyDeviceToHost, c->stream));
-  if ((s = check(c)) != BD_OK) return s;
-  for (int i = 0; i < N; i++)
-    for (int a = 0; a < 3; a++) out[3 * i + a] = res[(size_t)a * NTp + i];
-  return BD_OK;
+  return io_out(c, 1, c->Yz, out);
 }
 
 int bd_mobility_apply_block(bd_ctx* c, int k, const double* v, double* out) {
@@ -1608,53 +1659,22 @@ int bd_mobility_apply_block(bd_ctx* c, int k, const double* v, double* out) {
     return BD_OK;
   }
   int s;
-  int N = c->N, NTp = c->NT * 32;
-  size_t n = 3 * (size_t)NTp;
-  std::vector<double> soa(n * k, 0.0), res(n * k);
-  for (int r = 0; r < k; r++)
-    for (int i = 0; i < N; i++)
-      for (int a = 0; a < 3; a++) soa[r * n + (size_t)a * NTp + i] = v[(size_t)r * 3 * N + 3 * i + a];
-  double *X = nullptr, *Y = nullptr;
-  if (cudaMalloc(&X, 8 * n * k) != cudaSuccess || cudaMalloc(&Y, 8 * n * k) != cudaSuccess) {
-    cudaGetLastError();  // not a sticky error: the next launch check must not see it
-    cudaFree(X);
-    return BD_ERR_OOM;
-  }
-  cudaError_t e = cudaMemcpyAsync(X, soa.data(), 8 * n * k, cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) {
-    prof_begin(c, BD_PROF_BLOCK);  // the product alone, for timing (autotuner)
-    s = pme_apply_multi(c, k, X, n, Y, n);
-    prof_end(c, BD_PROF_BLOCK);
-  } else {
-    s = bd::cuda_fail((int)e, cudaGetErrorString(e), __FILE__, __LINE__);
-  }
-  if (s == BD_OK) {
-    e = cudaMemcpyAsync(res.data(), Y, 8 * n * k, cudaMemcpyDeviceToHost, c->stream);
-    s = e == cudaSuccess ? check(c)
-                         : bd::cuda_fail((int)e, cudaGetErrorString(e), __FILE__, __LINE__);
-  }
-  cudaStreamSynchronize(c->stream);
-  cudaFree(X);
-  cudaFree(Y);
+  if ((s = io_alloc(c)) != BD_OK || (s = io_in(c, k, v)) != BD_OK) return s;
+  const size_t n = 3 * (size_t)c->NT * 32;
+  prof_begin(c, BD_PROF_BLOCK);  // the product alone, for timing (autotuner)
+  s = pme_apply_multi(c, k, c->io_x, n, c->io_y, n);
+  prof_end(c, BD_PROF_BLOCK);
   if (s != BD_OK) return s;
-  for (int r = 0; r < k; r++)
-    for (int i = 0; i < N; i++)
-      for (int a = 0; a < 3; a++) out[(size_t)r * 3 * N + 3 * i + a] = res[r * n + (size_t)a * NTp + i];
-  return BD_OK;
+  return io_out(c, k, c->io_y, out);
 }
 
 int bd_lanczos_sqrt(bd_ctx* c, const double* z, double* out, int* iters) {
   if (!c || !z || !out) return BD_ERR_ARG;
   int s;
-  CU(cudaMemcpyAsync(c->R, z, 24 * (size_t)c->N, cudaMemcpyHostToDevice, c->stream));
+  if ((s = stage_up(c, c->R, z, 3 * (size_t)c->N)) != BD_OK) return s;
   if ((s = lanczos_sqrt(c, c->R, false, iters)) != BD_OK) return s;
-  int N = c->N, NTp = c->NT * 32;
-  std::vector<double> res(3 * (size_t)NTp);
-  CU(cudaMemcpyAsync(res.data(), c->Yz, 8 * res.size(), cudaMemcpyDeviceToHost, c->stream));
-  if ((s = check(c)) != BD_OK) return s;
-  for (int i = 0; i < N; i++)
-    for (int a = 0; a < 3; a++) out[3 * i + a] = res[(size_t)a * NTp + i];
-  return BD_OK;
+  if ((s = io_alloc(c)) != BD_OK) return s;
+  return io_out(c, 1, c->Yz, out);
 }
 
 int bd_lanczos_inv_sqrt(bd_ctx* c, const double* z, double* out, int* iters) {
@@ -1663,15 +1683,10 @@ int bd_lanczos_inv_sqrt(bd_ctx* c, const double* z, double* out, int* iters) {
   bool conv = false;
   if (!c->hi_built) return BD_ERR_STATE;
   // the work vectors exist only after the first allocation; Lt2 is read below
-  if ((s = alloc_lanczos(c)) != BD_OK) return s;
-  CU(cudaMemcpyAsync(c->R, z, 24 * (size_t)c->N, cudaMemcpyHostToDevice, c->stream));
+  if ((s = alloc_lanczos(c)) != BD_OK || (s = io_alloc(c)) != BD_OK) return s;
+  if ((s = stage_up(c, c->R, z, 3 * (size_t)c->N)) != BD_OK) return s;
   if ((s = lanczos_inv_sqrt(c, c->R, c->Lt2, iters, &conv)) != BD_OK) return s;
-  int N = c->N, NTp = c->NT * 32;
-  std::vector<double> res(3 * (size_t)NTp);
-  CU(cudaMemcpyAsync(res.data(), c->Lt2, 8 * res.size(), cudaMemcpyDeviceToHost, c->stream));
-  if ((s = check(c)) != BD_OK) return s;
-  for (int i = 0; i < N; i++)
-    for (int a = 0; a < 3; a++) out[3 * i + a] = res[(size_t)a * NTp + i];
+  if ((s = io_out(c, 1, c->Lt2, out)) != BD_OK) return s;
   return conv ? BD_OK : BD_ERR_LANCZOS;
 }
 
