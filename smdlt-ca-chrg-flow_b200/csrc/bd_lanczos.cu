@@ -32,6 +32,15 @@ using namespace bd;
 
 static const int kDotBlocks = 148;  // one CTA per SM for the vector reductions
 
+// CTAs per vector of the orthogonalisation: at most `most`, none with fewer
+// than 256 entries down to 8 CTAs.  Every CTA sums all CTAs' partials, one set
+// per basis vector, so more of them only add reads: with 148 CTAs instead of 12
+// the square root of 1024 beads took 3.48 ms, not 3.43; from 38 000 entries on
+// the rule changes nothing.
+static int orth_chunks(size_t n, int most) {
+  return std::min(most, std::max(8, (int)(n / 256)));
+}
+
 // Fixed-order sum of n partials by one warp: lane-strided sums, then a
 // butterfly; every lane returns the same value.
 __device__ __forceinline__ double warp_sum_parts(const double* __restrict__ part, int n,
@@ -447,7 +456,8 @@ struct BlkCheck {
   const double* beta;
   int k, L1, lmax;
   double tol;
-  const int* jd;        // Krylov dimension reached
+  int* jd;              // iterations finished (this one not counted yet)
+  int* ticket;          // CTAs that have checked this iteration
   int* done;
   int* conv;
   int* neg;
@@ -501,10 +511,9 @@ __device__ void quad_sqrt_e1(const double* a, const double* b, int mm, double* c
 // check, with those of m-2 .. m-7), and the host path's stopping test (tail
 // d_m rho/(1-rho) <= tol, rho = (d_m/d_(m-6))^(1/6) capped at 0.99; or a
 // breakdown beta_(m-1) <= 1e-300; or the Krylov cap).
-__global__ void __launch_bounds__(kQuadNodes) k_block_check(BlkCheck q) {
+__device__ void block_check(const BlkCheck& q, int m) {
   extern __shared__ double sh[];
   int r = blockIdx.x, t = threadIdx.x, L1 = q.L1;
-  int m = *q.jd;
   if (q.done[r] || (m < *q.first && m < q.lmax)) return;  // uniform over the CTA
   double* a = sh;
   double* b = sh + L1;
@@ -574,14 +583,23 @@ __global__ void __launch_bounds__(kQuadNodes) k_block_check(BlkCheck q) {
   }
 }
 
-// The while node's condition: another iteration while a right-hand side is
-// open and the cap is not reached.
-__global__ void k_block_cond(const int* __restrict__ done, int k, const int* __restrict__ jd,
-                             int lmax, cudaGraphConditionalHandle h) {
+// Ends an iteration: the checks, one CTA per right-hand side; the last CTA to
+// finish counts the iteration and sets the while node's condition, another one
+// while a right-hand side is open and the cap is not reached.
+__global__ void __launch_bounds__(kQuadNodes) k_block_check(BlkCheck q,
+                                                            cudaGraphConditionalHandle h) {
+  const int m = *q.jd + 1;
+  block_check(q, m);
+  __syncthreads();  // every warp of this CTA has read jd before it can change
   if (threadIdx.x != 0) return;
+  __threadfence();
+  if (atomicAdd(q.ticket, 1) != q.k - 1) return;
+  __threadfence();
   int nd = 0;
-  for (int r = 0; r < k; r++) nd += done[r];
-  cudaGraphSetConditional(h, (nd < k && *jd < lmax) ? 1u : 0u);
+  for (int r = 0; r < q.k; r++) nd += *(volatile int*)(q.done + r);
+  *q.ticket = 0;
+  *q.jd = m;
+  cudaGraphSetConditional(h, (nd < q.k && m < q.lmax) ? 1u : 0u);
 }
 
 __global__ void k_set_int(int* p, int v) {
@@ -841,10 +859,11 @@ static int lanczos_iteration(bd_ctx* c, bool pre, bool force) {
   q.jd = c->Ljd;
   q.n = n;
   c->launches += 5;
-  k_orth0<<<blk, 256, 0, st>>>(q);
-  k_orth1<<<blk, 256, 0, st>>>(q);
-  k_orth2<false><<<blk, 256, 0, st>>>(q);  // single solves keep no FP32 copy
-  k_orth3<<<blk, 256, 0, st>>>(q);
+  const int g = orth_chunks(n, blk);
+  k_orth0<<<g, 256, 0, st>>>(q);
+  k_orth1<<<g, 256, 0, st>>>(q);
+  k_orth2<false><<<g, 256, 0, st>>>(q);  // single solves keep no FP32 copy
+  k_orth3<<<g, 256, 0, st>>>(q);
   k_next_j<<<1, 32, 0, st>>>(c->Ljd);
   return launch_ok(c);
 }
@@ -1069,7 +1088,9 @@ void noise_blocks_release(bd_ctx* c) {
 }
 
 // Chunks per right-hand side of the block orthogonalisation kernels.
-static int block_chunks(int k) { return std::min(kDotBlocks, std::max(8, 4 * kDotBlocks / k)); }
+static int block_chunks(size_t n, int k) {
+  return orth_chunks(n, std::min(kDotBlocks, std::max(8, 4 * kDotBlocks / k)));
+}
 
 // Layout of a block of k right-hand sides: basis vector j of r at
 // BV + (j k + r) n, alpha_j and beta_j at [j k + r].
@@ -1098,10 +1119,11 @@ static Kry block_kry(bd_ctx* c, int k) {
 
 // One iteration of the block, in two parts: the product W = A V_cur for the
 // k inputs (part 0), then the orthogonalisation of each against its own basis, beta, next
-// vectors, j += 1 (part 1).  The same launches every iteration (j is read on
-// the device), so each part can be captured as a graph; the product is timed
-// on its own (BD_PROF_BLOCK) between the two.
-static int block_part(bd_ctx* c, int k, bool pre, int part) {
+// vectors (part 1) and, with count, j += 1 (else k_block_check counts).  The
+// same launches every iteration (j is read on the device), so each part can be
+// captured as a graph; the product is timed on its own (BD_PROF_BLOCK) between
+// the two.
+static int block_part(bd_ctx* c, int k, bool pre, int part, bool count = true) {
   int s;
   size_t n = 3 * (size_t)c->NT * 32;
   cudaStream_t st = c->stream;
@@ -1119,8 +1141,8 @@ static int block_part(bd_ctx* c, int k, bool pre, int part) {
   // 4 x 148 CTAs in all: each right-hand side's vectors in 592 / k chunks
   // (at most 148), so every CTA re-sums only the chunk partials of its own
   // right-hand side while enough warps stay resident
-  dim3 g(block_chunks(k), k);
-  c->launches += 5;
+  dim3 g(block_chunks(n, k), k);
+  c->launches += count ? 5 : 4;
   k_orth0<<<g, 256, 0, st>>>(q);
   k_orth1<<<g, 256, 0, st>>>(q);
   if (q.Vs)
@@ -1128,7 +1150,7 @@ static int block_part(bd_ctx* c, int k, bool pre, int part) {
   else
     k_orth2<false><<<g, 256, 0, st>>>(q);
   k_orth3<<<g, 256, 0, st>>>(q);
-  k_next_j<<<1, 32, 0, st>>>(c->Bjd);
+  if (count) k_next_j<<<1, 32, 0, st>>>(c->Bjd);
   return launch_ok(c);
 }
 
@@ -1203,6 +1225,7 @@ static BlkCheck block_check_args(bd_ctx* c, int k, bool pre) {
   q.last = c->Bctl + 3 * k;
   q.nd = c->Bctl + 4 * k;
   q.first = c->Bctl + 5 * k;
+  q.ticket = c->Bctl + 5 * k + 1;
   q.mr = c->Bm;
   q.dh = c->Bdh;
   q.c = c->Bc;
@@ -1250,16 +1273,15 @@ static int block_while_graph(bd_ctx* c, int k, bool pre, cudaGraphExec_t* out) {
     if (e == cudaSuccess) {
       c->capturing = true;
       s = block_part(c, k, pre, 0);
-      if (s == BD_OK) s = block_part(c, k, pre, 1);
+      if (s == BD_OK) s = block_part(c, k, pre, 1, false);
       if (s == BD_OK) {
         BlkCheck q = block_check_args(c, k, pre);
         size_t smem = 8 * (3 * (size_t)q.L1 + 16);
         if (smem > 48 * 1024)
           cudaFuncSetAttribute(k_block_check, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)smem);
-        k_block_check<<<k, kQuadNodes, smem, st>>>(q);
-        k_block_cond<<<1, 32, 0, st>>>(c->Bctl, k, c->Bjd, c->lmax, h);
-        c->launches += 2;
+        k_block_check<<<k, kQuadNodes, smem, st>>>(q, h);
+        c->launches++;
       }
       cudaGraph_t cap = nullptr;
       cudaError_t e2 = cudaStreamEndCapture(st, &cap);
@@ -1311,7 +1333,7 @@ static int lanczos_run_multi_device(bd_ctx* c, int k, bool pre, double* out,
   CU(cudaMemsetAsync(c->Bjd, 0, sizeof(int), st));
   CU(cudaMemsetAsync(c->Bctl, 0, 4 * 3 * (size_t)k, st));             // done, conv, neg
   CU(cudaMemsetAsync(c->Bctl + 3 * k, 0xff, 4 * (size_t)k, st));      // last = -1
-  CU(cudaMemsetAsync(c->Bctl + 4 * k, 0, 4 * (size_t)k, st));         // nd
+  CU(cudaMemsetAsync(c->Bctl + 4 * k, 0, 4 * (size_t)(k + 2), st));   // nd, first, ticket
   k_set_int<<<1, 32, 0, st>>>(c->Bctl + 5 * k, std::max(kTailSpan + 2, c->blk_last - 2));
   if ((s = launch_ok(c)) != BD_OK) return s;
   CU(cudaGraphLaunch(ex, st));
