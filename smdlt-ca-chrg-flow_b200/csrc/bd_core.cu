@@ -561,20 +561,14 @@ __global__ void k_noise_philox(double* R, int n, unsigned long long seed, unsign
 }
 
 // getNoise with the reference's generator (shear/src/main26.c:708-713), one
-// warp.  The congruential sequence idum is known ahead (idum_{t+l} = 40014^l
-// idum_t mod 2147483563) and the deviates follow from pairs of uniforms, so
-// both are formed by the lanes side by side; only the shuffle table is a chain,
-// iy -> entry -> next iy, walked with the 32 entries in the lanes' registers: 64
-// uniforms, then their 32 pairs' acceptance and deviates.  The batch in which
-// the last deviate falls is walked again up to the uniforms it used, so the
-// generator ends where the one-by-one order leaves it.  Bound by the chain's
-// latency (a division by a constant, a shuffle, two adds a uniform): 1500
-// deviates in 86 us, 650 us by one thread.
-// A state with entries outside the generator's range, or not yet initialised,
-// is drawn from one by one.
+// warp: 64 uniforms (Ran1Warp), then their 32 pairs' acceptance and deviates
+// side by side.  The batch in which the last deviate falls is walked again up
+// to the uniforms it used, so the generator ends where the one-by-one order
+// leaves it.  Bound by the table's chain: 1500 deviates in
+// 51 us, 650 by one thread.
 __global__ void __launch_bounds__(32) k_gasdev_seq(Ran1* gs, double* R, int n) {
-  constexpr unsigned IM1 = 2147483563u, IA1 = 40014u, IMM1 = IM1 - 1, NDIV = 1 + IMM1 / 32;
-  __shared__ unsigned s_iy[64];
+  __shared__ uint4 s_next[64];
+  __shared__ unsigned s_y[64];
   const int lane = threadIdx.x;
   int at = 0;
   if (gs->idum <= 0) {  // the first call initialises the generator
@@ -586,10 +580,8 @@ __global__ void __launch_bounds__(32) k_gasdev_seq(Ran1* gs, double* R, int n) {
     at = min(n, 2);
     __syncwarp();
   }
-  const long long d0 = gs->idum, d2 = gs->idum2, y0 = gs->iy, v0 = gs->iv[lane];
-  const bool fine = d0 > 0 && d0 < IM1 && d2 >= 0 && d2 < IM1 && y0 >= 0 && y0 <= IMM1 &&
-                    v0 >= 0 && v0 < IM1;
-  if (!__all_sync(0xffffffffu, fine)) {
+  Ran1Warp r;
+  if (!r.load(gs)) {
     if (lane == 0) {
       Ran1 g = *gs;
       for (; at < n; at++) R[at] = (double)gasdev_dev(g);
@@ -597,8 +589,6 @@ __global__ void __launch_bounds__(32) k_gasdev_seq(Ran1* gs, double* R, int n) {
     }
     return;
   }
-  unsigned idum = (unsigned)d0, iy = (unsigned)y0, iv = (unsigned)v0;
-  const unsigned idum2 = (unsigned)d2;
   int iset = gs->iset;
   float gset = gs->gset;
   if (iset && at < n) {
@@ -606,37 +596,17 @@ __global__ void __launch_bounds__(32) k_gasdev_seq(Ran1* gs, double* R, int n) {
     at++;
     iset = 0;
   }
-  // 40014^(lane + 1) and 40014^32 mod IM1
-  unsigned long long p = 1, p32 = 1;
-  for (int l = 0; l < 32; l++) {
-    p32 = p32 * IA1 % IM1;
-    if (l == lane) p = p32;
-  }
-  // m uniforms (at most 64) from the sequence in a0, a1, their iy into s_iy
-  auto walk = [&](unsigned a0, unsigned a1, int m) {
-    for (int t = 0; t < m; t++) {
-      const unsigned next = __shfl_sync(0xffffffffu, t < 32 ? a0 : a1, t & 31);
-      const int j = (int)(iy / NDIV);
-      const int x = (int)__shfl_sync(0xffffffffu, iv, j) - (int)idum2;
-      if (lane == j) iv = next;
-      iy = (unsigned)(x < 1 ? x + (int)IMM1 : x);
-      if (lane == 0) s_iy[t] = iy;
-      idum = next;
-    }
-  };
-  auto uniform = [&](unsigned y) {
-    float temp = (float)((1.0 / (double)IM1) * (double)y);
-    return (double)temp > (1.0 - 1.2e-7) ? (float)(1.0 - 1.2e-7) : temp;
-  };
   while (at < n) {
-    const unsigned keep_iv = iv, keep_iy = iy;
-    const unsigned a0 = (unsigned)(p * idum % IM1), a1 = (unsigned)(p32 * a0 % IM1);
-    __syncwarp();
-    walk(a0, a1, 64);
+    const Ran1Warp keep = r;
+    unsigned y0 = 0, y1 = 0;
+    r.ahead(s_next);
+    r.walk(s_next, 64, y0, y1);
+    s_y[lane] = y0;
+    s_y[32 + lane] = y1;
     __syncwarp();
     // pair of this lane: polar Box-Muller as gasdev_dev
-    const float v1 = (float)(2.0 * (double)uniform(s_iy[2 * lane]) - 1.0);
-    const float v2 = (float)(2.0 * (double)uniform(s_iy[2 * lane + 1]) - 1.0);
+    const float v1 = (float)(2.0 * (double)Ran1Warp::uniform(s_y[2 * lane]) - 1.0);
+    const float v2 = (float)(2.0 * (double)Ran1Warp::uniform(s_y[2 * lane + 1]) - 1.0);
     const float rsq = __fadd_rn(__fmul_rn(v1, v1), __fmul_rn(v2, v2));
     const bool ok = !(rsq >= 1.0f || rsq == 0.0f);
     const unsigned hit = __ballot_sync(0xffffffffu, ok);
@@ -657,15 +627,11 @@ __global__ void __launch_bounds__(32) k_gasdev_seq(Ran1* gs, double* R, int n) {
     gset = __shfl_sync(0xffffffffu, gset, last);
     iset = (n - at) & 1;
     at = n;
-    iv = keep_iv;
-    iy = keep_iy;
-    __syncwarp();
-    walk(a0, a1, 2 * (last + 1));
+    r = keep;
+    r.walk(s_next, 2 * (last + 1), y0, y1);
   }
-  gs->iv[lane] = (long long)iv;
+  r.store(gs);
   if (lane == 0) {
-    gs->idum = (long long)idum;
-    gs->iy = (long long)iy;
     gs->iset = iset;
     gs->gset = gset;
   }
@@ -908,6 +874,7 @@ int bd_create(const bd_params* p, bd_ctx** out) {
   DALLOC(c->q, 8 * (size_t)N);
   DALLOC(c->dE, 64 * (size_t)std::max(N, 1));
   DALLOC(c->rng, sizeof(Ran1));
+  if (p->hop != BD_HOP_PARALLEL) DALLOC(c->hop_win, hop_win_bytes());
   cudaMemsetAsync(c->rx, 0, 8 * N, c->stream);
   cudaMemsetAsync(c->ry, 0, 8 * N, c->stream);
   cudaMemsetAsync(c->rz, 0, 8 * N, c->stream);
@@ -991,6 +958,7 @@ int bd_destroy(bd_ctx* c) {
   for (double* q : {c->io, c->io_x, c->io_y})
     if (q) cudaFree(q);
   if (c->hop_work) cudaFree(c->hop_work);
+  if (c->hop_win) cudaFree(c->hop_win);
   if (c->hop_cells) cudaFree(c->hop_cells);
   if (c->hop_de) cudaFree(c->hop_de);
   if (c->cb_part) cudaFree(c->cb_part);

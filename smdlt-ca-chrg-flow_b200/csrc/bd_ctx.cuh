@@ -162,6 +162,7 @@ struct bd_ctx {
   std::vector<double> cat_brun, cat_crun;
   std::vector<int> cat_gw;
 
+  void* hop_win;  // window scratch of the sequential charge-hop sweep
   // parallel charge-hop sweep
   double hop_R;
   int *hop_cells;
@@ -265,6 +266,7 @@ int sym_matvec(bd_ctx* c, int R, const VecIn& v0, const VecIn& v1, double* Y0, d
 
 // charge hopping
 int charge_hop(bd_ctx* c);
+size_t hop_win_bytes();  // window scratch of the sequential sweep
 
 // smooth-PME mobility
 int pme_prepare(bd_ctx* c, const Lat& l);

@@ -180,6 +180,92 @@ __device__ __forceinline__ float ran1_dev(Ran1& g) {
   return temp;
 }
 
+// ran1 by a warp.  The congruential sequence is known ahead (idum_{t+l} =
+// 40014^l idum_t mod 2147483563), so the lanes form 64 of its values side by
+// side (ahead); only the shuffle table is a chain, output -> entry -> next
+// output.  Lane l keeps entry l with the output it gives and the entry that
+// this output points at, so a uniform is one shuffle of that pointer, the
+// entry's replacement beside it: about 25 ns each, 43 with the entry's index
+// divided out of the output in turn, 340 by one thread.
+struct Ran1Warp {
+  static constexpr unsigned IM1 = 2147483563u, IA1 = 40014u, IMM1 = IM1 - 1;
+  static constexpr unsigned NDIV = 1 + IMM1 / 32;
+  unsigned iv, out, nxt;   // this lane's entry, its output and where that points
+  unsigned idum, iy, at;   // at: entry the next uniform comes from
+  unsigned idum2;
+  unsigned long long p, p32;  // 40014^(lane + 1), 40014^32 mod IM1
+
+  __device__ __forceinline__ unsigned output(unsigned v) const {
+    int x = (int)v - (int)idum2;
+    return (unsigned)(x < 1 ? x + (int)IMM1 : x);
+  }
+  // False (on every lane) for a state that is not initialised or has entries
+  // outside the generator's range: ran1_dev draws from those.
+  __device__ bool load(const Ran1* g) {
+    const int lane = threadIdx.x & 31;
+    const long long d0 = g->idum, d2 = g->idum2, y0 = g->iy, v0 = g->iv[lane];
+    const bool fine = d0 > 0 && d0 < IM1 && d2 >= 0 && d2 < IM1 && y0 >= 0 && y0 <= IMM1 &&
+                      v0 >= 0 && v0 < IM1;
+    if (!__all_sync(0xffffffffu, fine)) return false;
+    idum = (unsigned)d0;
+    idum2 = (unsigned)d2;
+    iy = (unsigned)y0;
+    at = iy / NDIV;
+    iv = (unsigned)v0;
+    out = output(iv);
+    nxt = out / NDIV;
+    unsigned long long sq = IA1;
+    p = 1;
+    for (int b = 0; b < 6; b++) {
+      if (((lane + 1) >> b) & 1) p = p * sq % IM1;
+      if (b == 5) p32 = sq;
+      sq = sq * sq % IM1;
+    }
+    return true;
+  }
+  // The next 64 values of the sequence, with their outputs and pointers.
+  __device__ __forceinline__ void ahead(uint4* s) const {
+    const int lane = threadIdx.x & 31;
+    const unsigned a0 = (unsigned)(p * idum % IM1), a1 = (unsigned)(p32 * a0 % IM1);
+    const unsigned o0 = output(a0), o1 = output(a1);
+    __syncwarp();
+    s[lane] = make_uint4(a0, o0, o0 / NDIV, 0u);
+    s[32 + lane] = make_uint4(a1, o1, o1 / NDIV, 0u);
+    __syncwarp();
+  }
+  // m <= 64 outputs from them, number t in lane t (y0) or t - 32 (y1).
+  __device__ __forceinline__ void walk(const uint4* s, int m, unsigned& y0, unsigned& y1) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 8
+    for (int t = 0; t < m; t++) {
+      const uint4 v = s[t];
+      const bool mine = lane == (int)at;
+      iy = __shfl_sync(0xffffffffu, out, at);
+      at = __shfl_sync(0xffffffffu, nxt, at);
+      if (mine) {
+        iv = v.x;
+        out = v.y;
+        nxt = v.z;
+      }
+      if (lane == t) y0 = iy;
+      if (lane + 32 == t) y1 = iy;
+      idum = v.x;
+    }
+  }
+  __device__ __forceinline__ void store(Ran1* g) const {
+    const int lane = threadIdx.x & 31;
+    g->iv[lane] = (long long)iv;
+    if (lane == 0) {
+      g->idum = (long long)idum;
+      g->iy = (long long)iy;
+    }
+  }
+  __device__ static __forceinline__ float uniform(unsigned y) {
+    float temp = (float)((1.0 / (double)IM1) * (double)y);
+    return (double)temp > (1.0 - 1.2e-7) ? (float)(1.0 - 1.2e-7) : temp;
+  }
+};
+
 }  // namespace bd
 
 // Checked CUDA runtime and cuFFT calls inside functions returning a status.

@@ -12,10 +12,16 @@
 // U(target, o) - U(source, o), which is the same quantity with a different
 // summation order.
 //
-// The sweep is inherently sequential, so it runs in one CTA of 1024 threads:
-// the neighbour scan, the occupancy test and the energy difference are
-// block-parallel with fixed-order reductions, and thread 0 owns the ran1
-// stream (the same draws, in the same order, as the reference).
+// Only the decisions are sequential.  A charge moves at most once in a sweep,
+// at its own turn, so its source, the first bead near it and with them its
+// three possible targets (c + 1, c - 1, that bead) are known beforehand.  The
+// charges are taken 32 at a time: k_hop_window forms, with one CTA per charge,
+// the energy change and the occupancy of each target for the sites at the
+// window's start, and what each possible move of an earlier charge of the
+// window adds to it; k_hop_decide then runs the window's trials in order with
+// one warp, lane k holding charge k's three targets, so that a trial is its
+// draws (the same, in the same order, as the reference), its Metropolis test
+// and, when accepted, three table rows added to the later lanes.
 #include <math.h>
 
 #include "bd_ctx.cuh"
@@ -23,7 +29,7 @@
 
 #define CU(call) BD_CU(call)
 
-static const int kHopThreads = 1024;
+static const int kHopWin = 32;  // charges per window: one per lane of the deciding warp
 
 __device__ __forceinline__ double dh_pair(const Lat& l, double xa, double ya, double za,
                                           double xb, double yb, double zb, double lambda_b,
@@ -66,131 +72,294 @@ __device__ double block_sum(double v, double* sh) {
   return sh[32];
 }
 
-__global__ void __launch_bounds__(1024) k_charge_hop(
-    Lat l, const double* __restrict__ rx, const double* __restrict__ ry,
-    const double* __restrict__ rz, int N, int Nb, int nch, int* track, int* old,
-    const double* __restrict__ qk_in, const double* __restrict__ rowsum, Ran1* rng,
-    double lambda_b, double kappa_d, double barrier, double barrier2, int* log, int* gidx,
-    double* gq) {
-  // charge sites and values in shared memory, or in global scratch (gidx,
-  // gq non-null) when they do not fit
-  extern __shared__ unsigned char smem[];
-  int* sidx = gidx ? gidx : (int*)smem;
-  double* sq = gq ? gq : (double*)(smem + (((size_t)nch * 4 + 15) & ~(size_t)15));
-  __shared__ double red[33];
-  __shared__ int s_first, s_c2, s_test, s_block, s_acc;
-  __shared__ double s_mm;
-  int t = threadIdx.x, nt = blockDim.x;
-  for (int k = t; k < nch; k += nt) {
-    sidx[k] = track[k];
-    sq[k] = qk_in[k];
+// First bead by index within |NID(c,j)|^2 < 4.41 of each charge, excluding
+// c-1, c, c+1 (N: none); a warp per charge, 32 beads at a time.
+__global__ void __launch_bounds__(256) k_hop_first(Lat l, const double* __restrict__ rx,
+                                                   const double* __restrict__ ry,
+                                                   const double* __restrict__ rz, int N, int nch,
+                                                   const int* __restrict__ track,
+                                                   int* __restrict__ first) {
+  int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (k >= nch) return;
+  int c = track[k], found = N;
+  double xc = rx[c], yc = ry[c], zc = rz[c];
+  for (int base = 0; base < N; base += 32) {
+    int j = base + lane;
+    bool hit = false;
+    if (j < N && j != c && j != c + 1 && j != c - 1) {
+      double vx, vy, vz;
+      min_image(l, subx(xc, rx[j]), subx(yc, ry[j]), subx(zc, rz[j]), vx, vy, vz);
+      hit = rr3(vx, vy, vz) < 4.41;
+    }
+    unsigned m = __ballot_sync(0xffffffffu, hit);
+    if (m) {
+      found = base + __ffs(m) - 1;
+      break;
+    }
   }
-  double e0 = 0;
-  for (int k = t; k < nch; k += nt) e0 += rowsum[k];
-  double E_init = (nch > 1) ? block_sum(e0, red) : 0.0;
-  double E_cur = E_init;
-  Ran1 g;
-  if (t == 0) g = *rng;
-  __syncthreads();
-  for (int k = 0; k < nch; k++) {
-    if (t == 0) {
-      s_mm = (double)ran1_dev(g);
-      s_first = 0x7fffffff;
-    }
-    __syncthreads();
-    int c = sidx[k];
-    double xc = rx[c], yc = ry[c], zc = rz[c];
-    // first bead by index within |NID(c,j)|^2 < 4.41, excluding c-1, c, c+1
-    for (int base = 0; base < N; base += nt) {
-      int j = base + t;
-      bool hit = false;
-      if (j < N && j != c && j != c + 1 && j != c - 1) {
-        double vx, vy, vz;
-        min_image(l, subx(xc, rx[j]), subx(yc, ry[j]), subx(zc, rz[j]), vx, vy, vz);
-        hit = rr3(vx, vy, vz) < 4.41;
-      }
-      if (hit) atomicMin(&s_first, j);
-      __syncthreads();
-      if (s_first != 0x7fffffff) break;
-    }
-    if (t == 0) {
-      double mm = s_mm;
-      int c2, test = 0, sblock;
-      if (s_first != 0x7fffffff) {
-        if (mm < .33) {
-          c2 = c + 1;
-          sblock = (c == N - 1 || c % Nb == Nb - 1 || c == Nb - 1);
-          test = 1;
-        } else if (mm > 0.66) {
-          c2 = c - 1;
-          sblock = (c2 < 0 || c == 0 || c % Nb == 0);
-          test = 1;
-        } else {
-          c2 = s_first;
-          sblock = 0;
-          test = 2;
-        }
-      } else if (mm > .5) {
-        c2 = c + 1;
-        sblock = (c == N - 1 || c % Nb == Nb - 1 || c == Nb - 1);
-      } else {
-        c2 = c - 1;
-        sblock = (c2 < 0 || c == 0 || c % Nb == 0);
-      }
-      s_c2 = c2;
-      s_test = test;
-      s_block = sblock;
-    }
-    __syncthreads();
-    int c2 = s_c2;
-    bool occ = false;
-    for (int o = t; o < nch; o += nt) occ |= (sidx[o] == c2);
-    int blocked = __syncthreads_or(occ ? 1 : 0) || s_block;
-    if (blocked) {
-      if (t == 0) {
-        log[3 * k] = 0;
-        log[3 * k + 1] = c2;
-        log[3 * k + 2] = 0;  // a blocked trial never sets the move kind
-      }
-      __syncthreads();
-      continue;
-    }
-    // energy change of moving charge k from c to c2 against all the others
-    double x2 = rx[c2], y2 = ry[c2], z2 = rz[c2], de = 0;
-    if (nch > 1) {
-      double qk = sq[k];
-      for (int o = t; o < nch; o += nt) {
-        if (o == k) continue;
-        int b = sidx[o];
-        double xb = rx[b], yb = ry[b], zb = rz[b];
-        de += qk * sq[o] *
-              (dh_pair(l, x2, y2, z2, xb, yb, zb, lambda_b, kappa_d) -
-               dh_pair(l, xc, yc, zc, xb, yb, zb, lambda_b, kappa_d));
-      }
-      de = block_sum(de, red);
-    }
-    double E_fin = (nch > 1) ? E_cur + de : 0.0;
-    if (t == 0) {
-      double bar = (s_test == 2) ? barrier2 : barrier;
-      double x = exp((-bar - 0.5 * (E_fin - E_init)));
-      int acc;
-      if (1 <= x)
-        acc = 1;
+  if (lane == 0) first[k] = found;
+}
+
+// A charge's source and its possible targets: the next and the previous bead
+// of its chain and the first bead near it; -1 where there is none (chain ends,
+// no bead near).
+struct HopSites {
+  int s[4];  // source, then the targets
+};
+__device__ __forceinline__ HopSites hop_sites(int c, int first, int N, int Nb) {
+  HopSites h;
+  h.s[0] = c;
+  h.s[1] = (c == N - 1 || c % Nb == Nb - 1 || c == Nb - 1) ? -1 : c + 1;
+  h.s[2] = (c - 1 < 0 || c == 0 || c % Nb == 0) ? -1 : c - 1;
+  h.s[3] = first < N ? first : -1;
+  return h;
+}
+
+// Scratch of a window: energy changes and occupancies of its charges' targets
+// at the window's start, the table of what accepted moves add, the sweep's
+// starting and current energy.
+struct HopWin {
+  double de[3 * kHopWin];                 // [target][charge]
+  int occ[3 * kHopWin];
+  double tab[kHopWin * 9 * kHopWin];      // [moved charge][its target][target][charge]
+  double e_init, e_cur;
+};
+
+struct HopArgs {
+  Lat l;
+  const double *rx, *ry, *rz;
+  int N, Nb, nch;
+  int* track;
+  const int* first;
+  const double* qk;
+  double lambda_b, kappa_d;
+  HopWin* win;
+};
+
+// One CTA per charge of the window.  The pair of a target with a charge that
+// sits on it is left out everywhere: the trial is blocked while it sits there.
+__global__ void __launch_bounds__(256) k_hop_window(HopArgs q, int k0) {
+  __shared__ double red[8][3];
+  __shared__ int redn[8][3];
+  __shared__ double su[kHopWin][16];
+  const int kk = blockIdx.x, k = k0 + kk, t = threadIdx.x;
+  const HopSites h = hop_sites(q.track[k], q.first[k], q.N, q.Nb);
+  double x[4], y[4], z[4];
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+    int b = max(h.s[a], 0);
+    x[a] = q.rx[b];
+    y[a] = q.ry[b];
+    z[a] = q.rz[b];
+  }
+  const double qk = q.qk[k];
+  double de[3] = {0, 0, 0};
+  int occ[3] = {0, 0, 0};
+  for (int o = t; o < q.nch; o += blockDim.x) {
+    if (o == k) continue;
+    int b = q.track[o];
+    double xb = q.rx[b], yb = q.ry[b], zb = q.rz[b], qq = qk * q.qk[o];
+    double uc = dh_pair(q.l, x[0], y[0], z[0], xb, yb, zb, q.lambda_b, q.kappa_d);
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      if (h.s[a + 1] < 0) continue;
+      double u = 0;
+      if (b == h.s[a + 1])
+        occ[a]++;
       else
-        acc = ((double)ran1_dev(g) <= x);
-      old[k] = c;
-      if (acc) sidx[k] = c2;
-      log[3 * k] = acc ? 1 : 2;
-      log[3 * k + 1] = c2;
-      log[3 * k + 2] = s_test;
-      s_acc = acc;
+        u = dh_pair(q.l, x[a + 1], y[a + 1], z[a + 1], xb, yb, zb, q.lambda_b, q.kappa_d);
+      de[a] += qq * (u - uc);
     }
-    __syncthreads();
-    if (s_acc) E_cur = E_fin;
+  }
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+    for (int off = 16; off > 0; off >>= 1) {
+      de[a] += __shfl_xor_sync(0xffffffffu, de[a], off);
+      occ[a] += __shfl_xor_sync(0xffffffffu, occ[a], off);
+    }
+  if ((t & 31) == 0)
+    for (int a = 0; a < 3; a++) {
+      red[t >> 5][a] = de[a];
+      redn[t >> 5][a] = occ[a];
+    }
+  // pairs with the sites of the window's earlier charges
+  for (int e = t; e < 16 * kk; e += blockDim.x) {
+    int m = e >> 4, a = (e >> 2) & 3, bb = e & 3;
+    HopSites g = hop_sites(q.track[k0 + m], q.first[k0 + m], q.N, q.Nb);
+    int sa = a == 0 ? h.s[0] : a == 1 ? h.s[1] : a == 2 ? h.s[2] : h.s[3];
+    int sb = bb == 0 ? g.s[0] : bb == 1 ? g.s[1] : bb == 2 ? g.s[2] : g.s[3];
+    double u = 0;
+    if (sa >= 0 && sb >= 0 && sa != sb)
+      u = dh_pair(q.l, q.rx[sa], q.ry[sa], q.rz[sa], q.rx[sb], q.ry[sb], q.rz[sb], q.lambda_b,
+                  q.kappa_d);
+    su[m][4 * a + bb] = u;
   }
   __syncthreads();
-  for (int k = t; k < nch; k += nt) track[k] = sidx[k];
-  if (t == 0) *rng = g;
+  if (t < 3) {
+    double s = 0;
+    int n = 0;
+    for (int w = 0; w < 8; w++) {
+      s += red[w][t];
+      n += redn[w][t];
+    }
+    q.win->de[t * kHopWin + kk] = s;
+    q.win->occ[t * kHopWin + kk] = n;
+  }
+  for (int e = t; e < 9 * kHopWin; e += blockDim.x) {
+    int m = e / 9, om = (e % 9) / 3, ok = e % 3;
+    double d = 0;
+    if (m < kk)
+      d = qk * q.qk[k0 + m] *
+          (su[m][4 * (ok + 1) + om + 1] - su[m][4 * (ok + 1)] - su[m][om + 1] + su[m][0]);
+    q.win->tab[e * kHopWin + kk] = d;
+  }
+}
+
+// Energy change of moving charge k from c to c2 for the sites as they are, by
+// one warp: for trials that the window's sums cannot give, a pair at distance
+// zero among them (infinite terms that would cancel).
+__device__ double hop_energy(const HopArgs& q, int k, int c, int c2) {
+  double de = 0, qk = q.qk[k];
+  for (int o = threadIdx.x & 31; o < q.nch; o += 32) {
+    if (o == k) continue;
+    int b = __ldcv(q.track + o);
+    de += qk * q.qk[o] *
+          (dh_pair(q.l, q.rx[c2], q.ry[c2], q.rz[c2], q.rx[b], q.ry[b], q.rz[b], q.lambda_b,
+                   q.kappa_d) -
+           dh_pair(q.l, q.rx[c], q.ry[c], q.rz[c], q.rx[b], q.ry[b], q.rz[b], q.lambda_b,
+                   q.kappa_d));
+  }
+  for (int off = 16; off > 0; off >>= 1) de += __shfl_xor_sync(0xffffffffu, de, off);
+  return de;
+}
+
+// The generator's next m <= 64 uniforms into u (unless null), by one warp; with
+// keep its state is left as it was, else advanced by m.
+__device__ void ran1_draws(Ran1* gs, uint4* next, int m, float* u, bool keep) {
+  const int lane = threadIdx.x & 31;
+  Ran1Warp r;
+  if (r.load(gs)) {
+    unsigned y0 = 0, y1 = 0;
+    r.ahead(next);
+    r.walk(next, m, y0, y1);
+    if (u) {
+      u[lane] = Ran1Warp::uniform(y0);
+      u[32 + lane] = Ran1Warp::uniform(y1);
+    }
+    if (!keep) r.store(gs);
+  } else if (lane == 0) {
+    Ran1 g = *gs;
+    for (int t = 0; t < m; t++) {
+      float x = ran1_dev(g);
+      if (u) u[t] = x;
+    }
+    if (!keep) *gs = g;
+  }
+  __syncwarp();
+}
+
+// The window's trials in order.  They use at most two uniforms each: 64 are
+// drawn before the trials, and the generator is advanced by those used after
+// them.  Bound by the trials' serial chain (test, exponential, table row):
+// 15.5 us a window, k_hop_window 8; a sweep over 250 charges among 500 beads
+// 0.2 ms, 0.73 ms with one block searching, testing and summing charge by
+// charge.
+__global__ void __launch_bounds__(256) k_hop_decide(HopArgs q, int k0,
+                                                    const double* __restrict__ rowsum,
+                                                    int* __restrict__ old, Ran1* rng,
+                                                    double barrier, double barrier2, int* log) {
+  extern __shared__ double tab[];
+  __shared__ double red[33];
+  __shared__ uint4 next[64];
+  __shared__ float u[64];
+  __shared__ double ud[65];  // one past the last: read, not used, when x >= 1
+  __shared__ int pick[64];   // target drawn with a bead near | without, 4 times
+  const int t = threadIdx.x, w = min(kHopWin, q.nch - k0);
+  double E_init, E_cur;
+  if (k0 == 0) {
+    double e0 = 0;
+    for (int k = t; k < q.nch; k += blockDim.x) e0 += rowsum[k];
+    E_init = q.nch > 1 ? block_sum(e0, red) : 0.0;
+    E_cur = E_init;
+  } else {
+    E_init = q.win->e_init;
+    E_cur = q.win->e_cur;
+  }
+  if (t < 32) {
+    ran1_draws(rng, next, 2 * kHopWin, u, true);
+    for (int e = t; e < 2 * kHopWin; e += 32) {
+      double mm = (double)u[e];
+      pick[e] = (mm < .33 ? 0 : mm > 0.66 ? 1 : 2) | (mm > .5 ? 0 : 4);
+      ud[e] = mm;
+    }
+  } else {
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(tab);
+    for (int e = t - 32; e < w * 9 * kHopWin / 2; e += blockDim.x - 32)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * e),
+                   "l"(q.win->tab + 2 * e));
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  }
+  __syncthreads();
+  if (t >= 32) return;
+  const int k = k0 + min(t, w - 1);
+  const int c = q.track[k];
+  const HopSites h = hop_sites(c, q.first[k], q.N, q.Nb);
+  const bool near = h.s[3] >= 0;
+  double de0 = q.win->de[t], de1 = q.win->de[kHopWin + t], de2 = q.win->de[2 * kHopWin + t];
+  int oc0 = h.s[1] < 0 ? 1 : q.win->occ[t], oc1 = h.s[2] < 0 ? 1 : q.win->occ[kHopWin + t];
+  int oc2 = q.win->occ[2 * kHopWin + t];
+  int used = 0, did = 0, to = c, kind = 0;  // this lane's trial: log, target, move kind
+  for (int kk = 0; kk < w; kk++) {
+    const int pk = pick[used], opt_l = near ? pk & 3 : pk >> 2;
+    const int tgt = opt_l == 0 ? c + 1 : opt_l == 1 ? c - 1 : h.s[3];
+    const int occ = opt_l == 0 ? oc0 : opt_l == 1 ? oc1 : oc2;
+    const double de_l = opt_l == 0 ? de0 : opt_l == 1 ? de1 : de2;
+    const int test_l = near ? (opt_l == 2 ? 2 : 1) : 0;
+    used++;
+    const int info = __shfl_sync(0xffffffffu, opt_l | (test_l << 2) | ((occ > 0) << 4), kk);
+    const int c2 = __shfl_sync(0xffffffffu, tgt, kk), c1 = __shfl_sync(0xffffffffu, c, kk);
+    double de = __shfl_sync(0xffffffffu, de_l, kk);
+    const int opt = info & 3, test = (info >> 2) & 3;
+    if (t == kk) to = c2;
+    if (info >> 4) continue;  // blocked: the log keeps no move kind
+    double E_fin = 0.0;
+    if (q.nch > 1) {
+      if (!isfinite(de)) {
+        if (t < kk && did == 1) q.track[k] = to;
+        __syncwarp();
+        de = hop_energy(q, k0 + kk, c1, c2);
+      }
+      E_fin = E_cur + de;
+    }
+    const double x = exp(-(test == 2 ? barrier2 : barrier) - 0.5 * (E_fin - E_init));
+    const bool sure = 1 <= x, acc = sure || ud[used] <= x;
+    used += !sure;
+    if (t == kk) {
+      did = acc ? 1 : 2;
+      kind = test;
+    }
+    if (!acc) continue;
+    E_cur = E_fin;
+    const double* row = tab + (size_t)(3 * kk + opt) * 3 * kHopWin + t;
+    de0 += row[0];
+    de1 += row[kHopWin];
+    de2 += row[2 * kHopWin];
+    oc0 += (h.s[1] == c2) - (h.s[1] == c1);
+    oc1 += (h.s[2] == c2) - (h.s[2] == c1);
+    oc2 += (h.s[3] == c2) - (h.s[3] == c1);
+  }
+  if (t < w) {
+    if (did) old[k] = c;
+    if (did == 1) q.track[k] = to;
+    log[3 * k] = did;
+    log[3 * k + 1] = to;
+    log[3 * k + 2] = kind;
+  }
+  ran1_draws(rng, next, used, nullptr, false);
+  if (t == 0) {
+    q.win->e_init = E_init;
+    q.win->e_cur = E_cur;
+  }
 }
 
 __global__ void k_charge_values(const double* __restrict__ q, const int* __restrict__ track,
@@ -228,6 +397,8 @@ __global__ void k_gather_charges_mc(const double* __restrict__ rx, const double*
 
 namespace bd {
 
+size_t hop_win_bytes() { return sizeof(HopWin); }
+
 int charge_hop_parallel(bd_ctx* c);
 
 int charge_hop(bd_ctx* c) {
@@ -235,20 +406,12 @@ int charge_hop(bd_ctx* c) {
   if (c->t % (unsigned long)c->p.MStep != 0) return BD_OK;
   if (c->p.hop == BD_HOP_PARALLEL) return charge_hop_parallel(c);
   int nch = c->nch, N = c->N;
-  size_t smem = (((size_t)nch * 4 + 15) & ~(size_t)15) + 8 * (size_t)nch;
   // scratch in dE (8 N doubles): [0, 4 nch) gathered (x,y,z,q); then row
-  // sums; then qk; then, for sweeps whose charges do not fit in shared
-  // memory, the working copies of the charge values and sites
+  // sums; then qk; then the first bead near each charge
   double4* cq = (double4*)c->dE;
   double* rowsum = c->dE + 4 * (size_t)nch;
   double* qk = rowsum + nch;
-  double* gq = nullptr;
-  int* gidx = nullptr;
-  if (smem > 200 * 1024) {
-    gq = qk + nch;
-    gidx = (int*)(gq + nch);
-    smem = 0;
-  }
+  int* first = (int*)(qk + nch);
   Lat l = c->lat;
   int treal = (int)(c->t % (unsigned long)c->tp);
   l.treal = treal;
@@ -261,13 +424,32 @@ int charge_hop(bd_ctx* c) {
   c->launches++;
   k_dh_energy_rows<<<(nch * 32 + 255) / 256, 256, 0, c->stream>>>(l, cq, nch, c->p.lambda_b,
                                                                    c->kappa_d, rowsum);
-  cudaFuncSetAttribute(k_charge_hop, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  HopArgs q;
+  q.l = l;
+  q.rx = c->rx;
+  q.ry = c->ry;
+  q.rz = c->rz;
+  q.N = N;
+  q.Nb = c->Nb;
+  q.nch = nch;
+  q.track = c->track;
+  q.first = first;
+  q.qk = qk;
+  q.lambda_b = c->p.lambda_b;
+  q.kappa_d = c->kappa_d;
+  q.win = (HopWin*)c->hop_win;
+  const int smem = 8 * 9 * kHopWin * kHopWin;
+  CU(cudaFuncSetAttribute(k_hop_decide, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   prof_begin(c, BD_PROF_HOP);
   c->launches++;
-  k_charge_hop<<<1, kHopThreads, smem, c->stream>>>(l, c->rx, c->ry, c->rz, N, c->Nb, nch,
-                                                    c->track, c->old, qk, rowsum, c->rng,
-                                                    c->p.lambda_b, c->kappa_d, c->p.barrier,
-                                                    c->p.barrier2, c->hoplog, gidx, gq);
+  k_hop_first<<<(nch * 32 + 255) / 256, 256, 0, c->stream>>>(l, c->rx, c->ry, c->rz, N, nch,
+                                                             c->track, first);
+  for (int k0 = 0; k0 < nch; k0 += kHopWin) {
+    c->launches += 2;
+    k_hop_window<<<std::min(kHopWin, nch - k0), 256, 0, c->stream>>>(q, k0);
+    k_hop_decide<<<1, 256, smem, c->stream>>>(q, k0, rowsum, c->old, c->rng, c->p.barrier,
+                                              c->p.barrier2, c->hoplog);
+  }
   prof_end(c, BD_PROF_HOP);
   c->launches++;
   k_clear_charges<<<(N + 255) / 256, 256, 0, c->stream>>>(c->cflags, c->q, N);
