@@ -40,7 +40,12 @@ constexpr float kCut = (float)BD_MPNN_CUTOFF;
 constexpr int oW1 = 0, ob1 = oW1 + WD * NR, oW2 = ob1 + WD, ob2 = oW2 + WD * WD;
 constexpr int oW34 = ob2 + WD, ob3 = oW34 + WD * 2 * WD, owa = ob3 + WD, oca = owa + WD;
 constexpr int owb = oca + 1, ocb = owb + WD, kParams = ocb + 1;
-constexpr int kGemmRows = 64;  // rows per CTA of the forward-type products
+// Rows per CTA of the forward-type products: 64, or 16 where 64 would leave
+// multiprocessors idle (2000 rows x 64 by 64 columns 3.6 us, not 9.7) and where
+// the weights, staged by every CTA, are small (K = 16: 24 000 rows 5.7 us, not
+// 8.2; 1.2 M rows 135, not 139).  With K = 64 and 128, 100 000 rows take 17.2 and
+// 27.8 us by 64, 18.0 and 31.5 by 16.
+constexpr int kGemmRows = 64, kGemmFew = 16, kSMs = 148;
 constexpr int kWgradCtas = 296;
 
 typedef __nv_bfloat16 bf16;
@@ -55,7 +60,7 @@ struct Mpnn {
   float *sa, *a, *te, *ce;
   float *zt;     // z (3N) then t (3N)
   float *dG, *du, *de, *dp3, *dX3, *dh, *do2, *dm, *dg1, *hg, *lossv;
-  float* part;   // kWgradCtas x 64 x 128 partial weight gradients
+  float* part;   // kWgradCtas x 64 x 129 partial weight and bias gradients
   double* G9;    // predicted blocks
   bool feat;
 };
@@ -79,30 +84,41 @@ __device__ __forceinline__ void mma16816(float* c, const uint32_t* a, const uint
 }
 
 // pre = A B^T + bias (A: M x K FP32 row-major, B: NOUT x K BF16 row-major),
-// post = silu(pre) when post is non-null.  64 rows per CTA, 16 per warp.
-template <int K, int NOUT>
+// post = silu(pre) when post is non-null.  ROWS rows per CTA, 16 per warp; with
+// 16 the four warps share the columns.  Bound by the latency of staging its
+// operands, read 16 bytes at a time: 2000 x 128 by 64 columns 4.3 us, 15.6 with
+// 64 rows per CTA and single loads.
+template <int K, int NOUT, int ROWS>
 __global__ void __launch_bounds__(128) k_gemm(const float* __restrict__ A, int M,
                                               const bf16* __restrict__ B,
                                               const float* __restrict__ bias, float* pre,
                                               float* post) {
-  constexpr int LD = K + 8;
-  __shared__ __align__(16) bf16 As[kGemmRows * LD];
+  constexpr int LD = K + 8, NT = ROWS == 64 ? NOUT / 8 : NOUT / 32;
+  static_assert(ROWS == 64 || ROWS == 16, "16 rows per warp or per CTA");
+  __shared__ __align__(16) bf16 As[ROWS * LD];
   __shared__ __align__(16) bf16 Bs[NOUT * LD];
-  int r0 = blockIdx.x * kGemmRows;
-  for (int e = threadIdx.x; e < kGemmRows * K; e += blockDim.x) {
-    int r = e / K, k = e % K;
-    float v = (r0 + r < M) ? A[(size_t)(r0 + r) * K + k] : 0.0f;
-    As[r * LD + k] = __float2bfloat16_rn(v);
+  const int r0 = blockIdx.x * ROWS;
+#pragma unroll 4
+  for (int e = threadIdx.x; e < ROWS * K / 4; e += 128) {
+    const int r = e / (K / 4), k = e % (K / 4) * 4;
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (r0 + r < M) v = *(const float4*)(A + (size_t)(r0 + r) * K + k);
+    *(uint2*)(As + r * LD + k) =
+        make_uint2(pack2(__float2bfloat16_rn(v.x), __float2bfloat16_rn(v.y)),
+                   pack2(__float2bfloat16_rn(v.z), __float2bfloat16_rn(v.w)));
   }
-  for (int e = threadIdx.x; e < NOUT * K; e += blockDim.x) Bs[(e / K) * LD + e % K] = B[e];
+#pragma unroll 4
+  for (int e = threadIdx.x; e < NOUT * K / 8; e += 128)
+    *(uint4*)(Bs + e / (K / 8) * LD + e % (K / 8) * 8) = *(const uint4*)(B + 8 * e);
   __syncthreads();
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  float acc[NOUT / 8][4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int w0 = ROWS == 64 ? warp * 16 : 0, n0 = ROWS == 64 ? 0 : warp * NT;
+  float acc[NT][4];
 #pragma unroll
-  for (int nt = 0; nt < NOUT / 8; nt++)
+  for (int nt = 0; nt < NT; nt++)
 #pragma unroll
     for (int q = 0; q < 4; q++) acc[nt][q] = 0.0f;
-  const bf16* Aw = As + warp * 16 * LD;
+  const bf16* Aw = As + w0 * LD;
 #pragma unroll
   for (int kk = 0; kk < K; kk += 16) {
     uint32_t a[4];
@@ -111,37 +127,40 @@ __global__ void __launch_bounds__(128) k_gemm(const float* __restrict__ A, int M
     a[2] = *(const uint32_t*)(Aw + g * LD + kk + 2 * t + 8);
     a[3] = *(const uint32_t*)(Aw + (g + 8) * LD + kk + 2 * t + 8);
 #pragma unroll
-    for (int nt = 0; nt < NOUT / 8; nt++) {
-      const bf16* Bn = Bs + (nt * 8 + g) * LD + kk + 2 * t;
+    for (int nt = 0; nt < NT; nt++) {
+      const bf16* Bn = Bs + ((n0 + nt) * 8 + g) * LD + kk + 2 * t;
       uint32_t b[2] = {*(const uint32_t*)Bn, *(const uint32_t*)(Bn + 8)};
       mma16816(acc[nt], a, b);
     }
   }
 #pragma unroll
-  for (int nt = 0; nt < NOUT / 8; nt++)
+  for (int nt = 0; nt < NT; nt++)
 #pragma unroll
     for (int hh = 0; hh < 2; hh++) {
-      int row = r0 + warp * 16 + g + 8 * hh;
+      int row = r0 + w0 + g + 8 * hh;
       if (row >= M) continue;
-#pragma unroll
-      for (int q = 0; q < 2; q++) {
-        int col = nt * 8 + 2 * t + q;
-        float v = acc[nt][2 * hh + q] + (bias ? bias[col] : 0.0f);
-        pre[(size_t)row * NOUT + col] = v;
-        if (post) post[(size_t)row * NOUT + col] = silu(v);
-      }
+      const int col = (n0 + nt) * 8 + 2 * t;
+      const float v0 = acc[nt][2 * hh] + (bias ? bias[col] : 0.0f);
+      const float v1 = acc[nt][2 * hh + 1] + (bias ? bias[col + 1] : 0.0f);
+      *(float2*)(pre + (size_t)row * NOUT + col) = make_float2(v0, v1);
+      if (post) *(float2*)(post + (size_t)row * NOUT + col) = make_float2(silu(v0), silu(v1));
     }
 }
 
 // part[cta] = dY^T X over this CTA's rows (dY: M x 64, X: M x K; result
 // 64 x K), BF16 operands, FP32 accumulation; the row dimension is the MMA's
-// reduction dimension.
+// reduction dimension; after it the column sums of dY (FP32, the bias
+// gradient).  Up to 64 rows are staged at a time, 16 bytes a load: bound by
+// that latency.  24 000 rows, K = 16: 7.9 us; 20.8 with 16 rows staged at a time and
+// single loads, and 5.8 for the column sums by a kernel of their own.
 template <int K>
 __global__ void __launch_bounds__(128) k_wgrad(const float* __restrict__ dY,
                                                const float* __restrict__ X, int M, int rpc,
                                                float* part) {
-  __shared__ __align__(16) bf16 Ys[16][WD + 8];
-  __shared__ __align__(16) bf16 Xs[16][K + 8];
+  constexpr int R = 64;
+  __shared__ __align__(16) bf16 Ys[R][WD + 8];
+  __shared__ __align__(16) bf16 Xs[R][K + 8];
+  __shared__ float4 cs[8][WD / 4];
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   int o0 = warp * 16;
   float acc[K / 8][4];
@@ -149,32 +168,50 @@ __global__ void __launch_bounds__(128) k_wgrad(const float* __restrict__ dY,
   for (int nt = 0; nt < K / 8; nt++)
 #pragma unroll
     for (int q = 0; q < 4; q++) acc[nt][q] = 0.0f;
+  float4 col = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // columns 4 (thread % 16) ..
   int rb = blockIdx.x * rpc, re = min(M, rb + rpc);
-  for (int r0 = rb; r0 < re; r0 += 16) {
+  for (int r0 = rb; r0 < re; r0 += R) {
+    const int rows = min(R, (re - r0 + 15) & ~15);
     __syncthreads();
-    for (int e = threadIdx.x; e < 16 * WD; e += blockDim.x) {
-      int r = e / WD, o = e % WD;
-      Ys[r][o] = __float2bfloat16_rn(r0 + r < re ? dY[(size_t)(r0 + r) * WD + o] : 0.0f);
+#pragma unroll 4
+    for (int e = threadIdx.x; e < rows * (WD / 4); e += 128) {
+      const int r = e / (WD / 4), o = e % (WD / 4) * 4;
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (r0 + r < re) v = *(const float4*)(dY + (size_t)(r0 + r) * WD + o);
+      col.x += v.x;
+      col.y += v.y;
+      col.z += v.z;
+      col.w += v.w;
+      *(uint2*)&Ys[r][o] =
+          make_uint2(pack2(__float2bfloat16_rn(v.x), __float2bfloat16_rn(v.y)),
+                     pack2(__float2bfloat16_rn(v.z), __float2bfloat16_rn(v.w)));
     }
-    for (int e = threadIdx.x; e < 16 * K; e += blockDim.x) {
-      int r = e / K, k = e % K;
-      Xs[r][k] = __float2bfloat16_rn(r0 + r < re ? X[(size_t)(r0 + r) * K + k] : 0.0f);
+#pragma unroll 4
+    for (int e = threadIdx.x; e < rows * (K / 4); e += 128) {
+      const int r = e / (K / 4), k = e % (K / 4) * 4;
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (r0 + r < re) v = *(const float4*)(X + (size_t)(r0 + r) * K + k);
+      *(uint2*)&Xs[r][k] =
+          make_uint2(pack2(__float2bfloat16_rn(v.x), __float2bfloat16_rn(v.y)),
+                     pack2(__float2bfloat16_rn(v.z), __float2bfloat16_rn(v.w)));
     }
     __syncthreads();
-    uint32_t a[4];
-    a[0] = pack2(Ys[2 * t][o0 + g], Ys[2 * t + 1][o0 + g]);
-    a[1] = pack2(Ys[2 * t][o0 + g + 8], Ys[2 * t + 1][o0 + g + 8]);
-    a[2] = pack2(Ys[2 * t + 8][o0 + g], Ys[2 * t + 9][o0 + g]);
-    a[3] = pack2(Ys[2 * t + 8][o0 + g + 8], Ys[2 * t + 9][o0 + g + 8]);
+    for (int s = 0; s < rows; s += 16) {
+      uint32_t a[4];
+      a[0] = pack2(Ys[s + 2 * t][o0 + g], Ys[s + 2 * t + 1][o0 + g]);
+      a[1] = pack2(Ys[s + 2 * t][o0 + g + 8], Ys[s + 2 * t + 1][o0 + g + 8]);
+      a[2] = pack2(Ys[s + 2 * t + 8][o0 + g], Ys[s + 2 * t + 9][o0 + g]);
+      a[3] = pack2(Ys[s + 2 * t + 8][o0 + g + 8], Ys[s + 2 * t + 9][o0 + g + 8]);
 #pragma unroll
-    for (int nt = 0; nt < K / 8; nt++) {
-      int n = nt * 8 + g;
-      uint32_t b[2] = {pack2(Xs[2 * t][n], Xs[2 * t + 1][n]),
-                       pack2(Xs[2 * t + 8][n], Xs[2 * t + 9][n])};
-      mma16816(acc[nt], a, b);
+      for (int nt = 0; nt < K / 8; nt++) {
+        int n = nt * 8 + g;
+        uint32_t b[2] = {pack2(Xs[s + 2 * t][n], Xs[s + 2 * t + 1][n]),
+                         pack2(Xs[s + 2 * t + 8][n], Xs[s + 2 * t + 9][n])};
+        mma16816(acc[nt], a, b);
+      }
     }
   }
-  float* P = part + (size_t)blockIdx.x * WD * K;
+  float* P = part + (size_t)blockIdx.x * (WD * K + WD);
 #pragma unroll
   for (int nt = 0; nt < K / 8; nt++)
 #pragma unroll
@@ -182,15 +219,32 @@ __global__ void __launch_bounds__(128) k_wgrad(const float* __restrict__ dY,
 #pragma unroll
       for (int q = 0; q < 2; q++)
         P[(size_t)(o0 + g + 8 * hh) * K + nt * 8 + 2 * t + q] = acc[nt][2 * hh + q];
+  cs[threadIdx.x / (WD / 4)][threadIdx.x % (WD / 4)] = col;
+  __syncthreads();
+  if (threadIdx.x < WD) {
+    float s = 0;
+    for (int q = 0; q < 8; q++) s += ((const float*)cs[q])[threadIdx.x];
+    P[WD * K + threadIdx.x] = s;
+  }
 }
 
-// out[e] = sum over CTAs of part[cta][e] (fixed order)
-__global__ void k_part_sum(const float* __restrict__ part, int nparts, int n, float* out) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
+// out[e] = sum over CTAs of part[cta][e]: 32 numbers per block, eight warps
+// each every eighth part, then their sums (fixed order).  8256 numbers of
+// 125 parts 5.1 us, 8.3 with a thread per number; 130 of 286 parts 4.5, not 12.3.
+__global__ void __launch_bounds__(256) k_part_sum(const float* __restrict__ part, int nparts,
+                                                  int n, float* out) {
+  __shared__ float sh[8][32];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, e = blockIdx.x * 32 + lane;
   float s = 0;
-  for (int b = 0; b < nparts; b++) s += part[(size_t)b * n + e];
-  out[e] = s;
+  if (e < n)
+#pragma unroll 8
+    for (int b = w; b < nparts; b += 8) s += part[(size_t)b * n + e];
+  sh[w][lane] = s;
+  __syncthreads();
+  if (w == 0 && e < n) {
+    for (int q = 1; q < 8; q++) s += sh[q][lane];
+    out[e] = s;
+  }
 }
 
 // part[cta][c] = column sums of Y (M x C) over this CTA's rows
@@ -479,9 +533,9 @@ int ensure(bd_ctx* c) {
     CU(cudaMalloc(&m->W2t, 2 * WD * WD));
     CU(cudaMalloc(&m->W34b, 2 * WD * 2 * WD));
     CU(cudaMalloc(&m->W34t, 2 * WD * 2 * WD));
-    CU(cudaMalloc(&m->part, 4 * (size_t)kWgradCtas * WD * 2 * WD));
+    CU(cudaMalloc(&m->part, 4 * (size_t)kWgradCtas * WD * (2 * WD + 1)));
     c->bytes += 16 * kParams + 2 * (WD * NR + 2 * WD * WD + 4 * WD * WD) +
-                4 * (size_t)kWgradCtas * WD * 2 * WD;
+                4 * (size_t)kWgradCtas * WD * (2 * WD + 1);
   }
   int N = c->N;
   if (m->cap < N) {
@@ -539,37 +593,39 @@ int features(bd_ctx* c, const Lat& l) {
   return BD_OK;
 }
 
+template <int K, int NOUT>
+void gemm(bd_ctx* c, const float* A, int M, const bf16* Bw, const float* bias, float* pre,
+          float* post) {
+  if (K == NR || nblk(M, kGemmRows) < kSMs)
+    k_gemm<K, NOUT, kGemmFew><<<nblk(M, kGemmFew), 128, 0, c->stream>>>(A, M, Bw, bias, pre, post);
+  else if constexpr (K != NR)
+    k_gemm<K, NOUT, kGemmRows><<<nblk(M, kGemmRows), 128, 0, c->stream>>>(A, M, Bw, bias, pre, post);
+}
+
 int forward(bd_ctx* c) {
   Mpnn* m = get(c);
   int N = c->N, E = N * KN;
   c->launches += 6;
-  k_gemm<NR, WD><<<nblk(E, kGemmRows), 128, 0, c->stream>>>(m->rbf, E, m->W1b, m->w + ob1,
-                                                            m->g1, m->e);
+  gemm<NR, WD>(c, m->rbf, E, m->W1b, m->w + ob1, m->g1, m->e);
   k_edge_mean<<<nblk(N, 4), 128, 0, c->stream>>>(m->e, m->nbr, N, m->mv);
-  k_gemm<WD, WD><<<nblk(N, kGemmRows), 128, 0, c->stream>>>(m->mv, N, m->W2b, m->w + ob2,
-                                                            m->o2, m->h);
+  gemm<WD, WD>(c, m->mv, N, m->W2b, m->w + ob2, m->o2, m->h);
   k_node_mean<<<nblk(N, 4), 128, 0, c->stream>>>(m->h, m->nbr, N, m->X3);
-  k_gemm<2 * WD, WD><<<nblk(N, kGemmRows), 128, 0, c->stream>>>(m->X3, N, m->W34b, m->w + ob3,
-                                                                m->p3, m->u);
+  gemm<2 * WD, WD>(c, m->X3, N, m->W34b, m->w + ob3, m->p3, m->u);
   k_heads<<<nblk(N, 4), 128, 0, c->stream>>>(m->w, m->u, m->e, m->nbr, m->nvec, N, m->sa, m->a,
                                              m->te, m->ce, m->G9);
   return BD_OK;
 }
 
-// weight gradient dY^T X (64 x K) into g + off, bias gradient colsum(dY)
+// weight gradient dY^T X (64 x K) into g + off, the bias gradient (column sums
+// of dY) behind it
 template <int K>
-void wgrad(bd_ctx* c, const float* dY, const float* X, int M, int off_w, int off_b) {
+void wgrad(bd_ctx* c, const float* dY, const float* X, int M, int off) {
   Mpnn* m = get(c);
   int rpc = ((M + kWgradCtas - 1) / kWgradCtas + 15) / 16 * 16;
-  int nct = nblk(M, rpc);
+  int nct = nblk(M, rpc), n = WD * K + WD;
   c->launches += 2;
   k_wgrad<K><<<nct, 128, 0, c->stream>>>(dY, X, M, rpc, m->part);
-  k_part_sum<<<nblk(WD * K, 256), 256, 0, c->stream>>>(m->part, nct, WD * K, m->g + off_w);
-  if (off_b >= 0) {
-    c->launches += 2;
-    k_colsum<<<nct, 64, 0, c->stream>>>(dY, M, WD, rpc, m->part);
-    k_part_sum<<<1, 64, 0, c->stream>>>(m->part, nct, WD, m->g + off_b);
-  }
+  k_part_sum<<<nblk(n, 32), 256, 0, c->stream>>>(m->part, nct, n, m->g + off);
 }
 
 int backward(bd_ctx* c, double* loss_out) {
@@ -585,26 +641,24 @@ int backward(bd_ctx* c, double* loss_out) {
   int nct = nblk(N, rpc);
   k_colsum<<<nct, 160, 0, c->stream>>>(m->hg, N, 2 * WD + 2, rpc, m->part);
   c->launches += 1;
-  k_part_sum<<<1, 160, 0, c->stream>>>(m->part, nct, 2 * WD + 2, m->g + owa);
+  k_part_sum<<<nblk(2 * WD + 2, 32), 256, 0, c->stream>>>(m->part, nct, 2 * WD + 2, m->g + owa);
   // layer 3
   c->launches += 1;
   k_silu_back<<<nblk((long long)nN, 256), 256, 0, c->stream>>>(m->du, m->p3, nN, m->dp3);
-  wgrad<2 * WD>(c, m->dp3, m->X3, N, oW34, ob3);
+  wgrad<2 * WD>(c, m->dp3, m->X3, N, oW34);
   c->launches += 3;
-  k_gemm<WD, 2 * WD><<<nblk(N, kGemmRows), 128, 0, c->stream>>>(m->dp3, N, m->W34t, nullptr,
-                                                                m->dX3, nullptr);
+  gemm<WD, 2 * WD>(c, m->dp3, N, m->W34t, nullptr, m->dX3, nullptr);
   CU(cudaMemsetAsync(m->dh, 0, 4 * nN, c->stream));
   k_dh<<<nblk(N, 4), 128, 0, c->stream>>>(m->dX3, m->nbr, N, m->dh);
   // layer 2
   k_silu_back<<<nblk((long long)nN, 256), 256, 0, c->stream>>>(m->dh, m->o2, nN, m->do2);
-  wgrad<WD>(c, m->do2, m->mv, N, oW2, ob2);
+  wgrad<WD>(c, m->do2, m->mv, N, oW2);
   c->launches += 3;
-  k_gemm<WD, WD><<<nblk(N, kGemmRows), 128, 0, c->stream>>>(m->do2, N, m->W2t, nullptr, m->dm,
-                                                            nullptr);
+  gemm<WD, WD>(c, m->do2, N, m->W2t, nullptr, m->dm, nullptr);
   // layer 1
   k_de_add<<<nblk((long long)nE, 256), 256, 0, c->stream>>>(m->dm, m->nbr, N, m->de);
   k_silu_back<<<nblk((long long)nE, 256), 256, 0, c->stream>>>(m->de, m->g1, nE, m->dg1);
-  wgrad<NR>(c, m->dg1, m->rbf, E, oW1, ob1);
+  wgrad<NR>(c, m->dg1, m->rbf, E, oW1);
   if (loss_out) {
     std::vector<float> lv(N);
     CU(cudaMemcpyAsync(lv.data(), m->lossv, 4 * (size_t)N, cudaMemcpyDeviceToHost, c->stream));
