@@ -17,6 +17,7 @@
 // iteration with Wilkinson shifts (Golub and Van Loan, Matrix Computations,
 // section 8.3).  Vectors live on the device in component-major SoA with the
 // tile padding (3 x NTp); every reduction is a fixed-order two-level sum.
+#include <cooperative_groups.h>
 #include <math.h>
 #include <string.h>
 
@@ -27,16 +28,23 @@
 #include "bd_hostpool.h"
 
 using namespace bd;
+namespace cg = cooperative_groups;
 
 #define CU(call) BD_CU(call)
 
 static const int kDotBlocks = 148;  // one CTA per SM for the vector reductions
 
+// Longest vectors orthogonalised by one cluster per right-hand side (2048 beads).
+// By it against the four kernels: 1000 beads one solve 3.41 and 3.53 ms, a
+// block of ten 2.90 and 2.98; 2000 beads 5.44 and 5.49, 3.83 and 3.88; 4000 beads
+// 9.43 and 8.65, 5.84 and 5.86.
+static const int kOrthShort = 6144;
+
 // CTAs per vector of the orthogonalisation: at most `most`, none with fewer
 // than 256 entries down to 8 CTAs.  Every CTA sums all CTAs' partials, one set
 // per basis vector, so more of them only add reads: with 148 CTAs instead of 12
-// the square root of 1024 beads took 3.48 ms, not 3.43; from 38 000 entries on
-// the rule changes nothing.
+// the square root of 1024 beads by these kernels took 3.48 ms, not 3.43; from
+// 38 000 entries on the rule changes nothing.
 static int orth_chunks(size_t n, int most) {
   return std::min(most, std::max(8, (int)(n / 256)));
 }
@@ -137,7 +145,7 @@ __device__ __forceinline__ void chunk_range(int n, int& lo, int& hi) {
 // chunk_dots over an FP32 basis, four rows per load (lo, hi multiples of 4)
 __device__ __forceinline__ void chunk_dots4(const float* __restrict__ V, size_t vs, int nv,
                                             const double* __restrict__ w, int lo, int hi,
-                                            double* part) {
+                                            double* part, int ps, int pb) {
   int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const double2* w2 = (const double2*)w;
   for (int k0 = 4 * wp; k0 < nv; k0 += 4 * nw) {
@@ -162,10 +170,10 @@ __device__ __forceinline__ void chunk_dots4(const float* __restrict__ V, size_t 
       s3 += __shfl_xor_sync(0xffffffffu, s3, o);
     }
     if (lane == 0) {
-      part[(size_t)k0 * gridDim.x + blockIdx.x] = s0;
-      if (k0 + 1 < nv) part[(size_t)(k0 + 1) * gridDim.x + blockIdx.x] = s1;
-      if (k0 + 2 < nv) part[(size_t)(k0 + 2) * gridDim.x + blockIdx.x] = s2;
-      if (k0 + 3 < nv) part[(size_t)(k0 + 3) * gridDim.x + blockIdx.x] = s3;
+      part[(size_t)k0 * ps + pb] = s0;
+      if (k0 + 1 < nv) part[(size_t)(k0 + 1) * ps + pb] = s1;
+      if (k0 + 2 < nv) part[(size_t)(k0 + 2) * ps + pb] = s2;
+      if (k0 + 3 < nv) part[(size_t)(k0 + 3) * ps + pb] = s3;
     }
   }
 }
@@ -222,7 +230,7 @@ __device__ __forceinline__ double combo_rows4(const float* __restrict__ V, size_
 template <typename T>
 __device__ __forceinline__ void chunk_dots(const T* __restrict__ V, size_t vs, int nv,
                                            const double* __restrict__ w, int lo, int hi,
-                                           double* part) {
+                                           double* part, int ps, int pb) {
   int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int k0 = 4 * wp; k0 < nv; k0 += 4 * nw) {
     const T* v0 = V + (size_t)k0 * vs;
@@ -245,10 +253,10 @@ __device__ __forceinline__ void chunk_dots(const T* __restrict__ V, size_t vs, i
       s3 += __shfl_xor_sync(0xffffffffu, s3, o);
     }
     if (lane == 0) {
-      part[(size_t)k0 * gridDim.x + blockIdx.x] = s0;
-      if (k0 + 1 < nv) part[(size_t)(k0 + 1) * gridDim.x + blockIdx.x] = s1;
-      if (k0 + 2 < nv) part[(size_t)(k0 + 2) * gridDim.x + blockIdx.x] = s2;
-      if (k0 + 3 < nv) part[(size_t)(k0 + 3) * gridDim.x + blockIdx.x] = s3;
+      part[(size_t)k0 * ps + pb] = s0;
+      if (k0 + 1 < nv) part[(size_t)(k0 + 1) * ps + pb] = s1;
+      if (k0 + 2 < nv) part[(size_t)(k0 + 2) * ps + pb] = s2;
+      if (k0 + 3 < nv) part[(size_t)(k0 + 3) * ps + pb] = s3;
     }
   }
 }
@@ -357,9 +365,11 @@ __global__ void __launch_bounds__(256, 4) k_orth1(Kry q) {
     w[i] = w[i] - alpha * vj[i] - bprev * vp[i];
   __syncthreads();
   if (q.Vs)
-    chunk_dots4(q.Vs + (size_t)r * q.n, q.bs, nv, w, lo, hi, q.part2 + r * q.pst);
+    chunk_dots4(q.Vs + (size_t)r * q.n, q.bs, nv, w, lo, hi, q.part2 + r * q.pst,
+                gridDim.x, blockIdx.x);
   else
-    chunk_dots(V, q.bs, nv, w, lo, hi, q.part2 + r * q.pst);
+    chunk_dots(V, q.bs, nv, w, lo, hi, q.part2 + r * q.pst,
+                gridDim.x, blockIdx.x);
 }
 
 template <bool SHADOW>  // the pass reads the FP32 copy of the basis (q.Vs)
@@ -422,14 +432,132 @@ __global__ void __launch_bounds__(256) k_orth3(Kry q) {
   }
 }
 
+__global__ void k_next_j(int* jd) {
+  if (threadIdx.x == 0 && blockIdx.x == 0) *jd += 1;
+}
+
+// The four steps in one launch for short vectors: a cluster of eight CTAs per
+// right-hand side, its chunk of w in shared memory, the partial sums exchanged
+// through the cluster's shared memory.  next (null for several right-hand
+// sides) advances j.  Bound by the cluster's barriers and the loads' latency:
+// 3072 entries and 48 vectors 12.8 us, 20.2 by the four kernels and k_next_j.
+constexpr int kOrthCluster = 8;
+
+template <bool SHADOW>
+__global__ void __cluster_dims__(kOrthCluster, 1, 1) __launch_bounds__(512)
+    k_orth_cluster(Kry q, int* next) {
+  extern __shared__ __align__(16) double chunk[];
+  __shared__ double part[kMaxKrylov + 1], h[kMaxKrylov + 1];
+  __shared__ double red[16], sums[2];
+  cg::cluster_group cl = cg::this_cluster();
+  const int t = threadIdx.x, lane = t & 31, r = blockIdx.y, j = *q.jd, nv = j + 1;
+  int lo, hi;
+  chunk_range(q.n, lo, hi);
+  const double* V = q.V + (size_t)r * q.n;
+  const double* vj = V + (size_t)j * q.bs;
+  const double* vp = V + (size_t)(j > 0 ? j - 1 : 0) * q.bs;
+  const double* wg = q.w + (size_t)r * q.n;
+  double* w = chunk - lo;
+  // sum over the CTA's threads into sums[e], then over the cluster's CTAs
+  auto sum = [&](double s, int e) {
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) red[t >> 5] = s;
+    __syncthreads();
+    if (t == 0) {
+      s = 0;
+      for (int p = 0; p < 16; p++) s += red[p];
+      sums[e] = s;
+    }
+    cl.sync();
+    s = cl.map_shared_rank(sums, lane % kOrthCluster)[e];
+    for (int o = kOrthCluster / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+  };
+  double s = 0;
+  for (int i = lo + t; i < hi; i += 512) {
+    double x = wg[i];
+    w[i] = x;
+    s += vj[i] * x;
+  }
+  const double alpha = sum(s, 0);
+  const double bprev = j > 0 ? q.beta[(size_t)(j - 1) * q.kst + r] : 0.0;
+  for (int i = lo + t; i < hi; i += 512) w[i] = w[i] - alpha * vj[i] - bprev * vp[i];
+  __syncthreads();
+  if constexpr (SHADOW)
+    chunk_dots4(q.Vs + (size_t)r * q.n, q.bs, nv, w, lo, hi, part, 1, 0);
+  else
+    chunk_dots(V, q.bs, nv, w, lo, hi, part, 1, 0);
+  cl.sync();
+  for (int k = t; k < nv; k += 512) {
+    double a = 0;
+#pragma unroll
+    for (int b = 0; b < kOrthCluster; b++) a += cl.map_shared_rank(part, b)[k];
+    h[k] = a;
+  }
+  __syncthreads();
+  s = 0;
+  if constexpr (SHADOW) {
+    const float* Vs = q.Vs + (size_t)r * q.n;
+    for (int i4 = (lo >> 2) + t; i4 < (hi >> 2); i4 += 512)
+      s += combo_rows4(Vs, q.bs, h, nv, i4, w);
+  } else {
+    for (int i = lo + t; i < hi; i += 512) {
+      double x = w[i] - combo_row(V, q.bs, h, nv, i);
+      w[i] = x;
+      s += x * x;
+    }
+  }
+  const double b = sqrt(sum(s, 1)), f = b > 0 ? 1.0 / b : 0.0;
+  if (t == 0 && blockIdx.x == 0) {
+    q.alpha[(size_t)j * q.kst + r] = alpha + h[j];
+    q.beta[(size_t)j * q.kst + r] = b;
+    if (next) *next = j + 1;
+  }
+  double* vnext = q.V + (size_t)(j + 1) * q.bs + (size_t)r * q.n;
+  double* vcur = q.vcur + (size_t)r * q.n;
+  for (int i = lo + t; i < hi; i += 512) {
+    double x = w[i] * f;
+    vnext[i] = x;
+    vcur[i] = x;
+    if constexpr (SHADOW) q.Vs[(size_t)(j + 1) * q.bs + (size_t)r * q.n + i] = (float)x;
+  }
+  cl.sync();  // the others have read this CTA's sums
+}
+
+// One orthogonalisation step of k right-hand sides, by a cluster each or in g
+// chunks each (kOrthShort); next (may be null): j, advanced here.
+static void orth_step(bd_ctx* c, const Kry& q, int g, int k, int* next) {
+  cudaStream_t st = c->stream;
+  if (q.n <= kOrthShort) {
+    const size_t smem = 8 * (size_t)(((q.n + kOrthCluster - 1) / kOrthCluster + 3) & ~3);
+    int* one = k == 1 ? next : nullptr;
+    if (q.Vs)
+      k_orth_cluster<true><<<dim3(kOrthCluster, k), 512, smem, st>>>(q, one);
+    else
+      k_orth_cluster<false><<<dim3(kOrthCluster, k), 512, smem, st>>>(q, one);
+    c->launches++;
+    if (one) return;
+  } else {
+    const dim3 grid(g, k);
+    c->launches += 4;
+    k_orth0<<<grid, 256, 0, st>>>(q);
+    k_orth1<<<grid, 256, 0, st>>>(q);
+    if (q.Vs)
+      k_orth2<true><<<grid, 256, 0, st>>>(q);
+    else
+      k_orth2<false><<<grid, 256, 0, st>>>(q);
+    k_orth3<<<grid, 256, 0, st>>>(q);
+  }
+  if (next) {
+    c->launches++;
+    k_next_j<<<1, 32, 0, st>>>(next);
+  }
+}
+
 __global__ void k_to_f32(const double* __restrict__ a, float* __restrict__ b, size_t n) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x)
     b[i] = (float)a[i];
-}
-
-__global__ void k_next_j(int* jd) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *jd += 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -858,13 +986,7 @@ static int lanczos_iteration(bd_ctx* c, bool pre, bool force) {
   q.kst = 1;
   q.jd = c->Ljd;
   q.n = n;
-  c->launches += 5;
-  const int g = orth_chunks(n, blk);
-  k_orth0<<<g, 256, 0, st>>>(q);
-  k_orth1<<<g, 256, 0, st>>>(q);
-  k_orth2<false><<<g, 256, 0, st>>>(q);  // single solves keep no FP32 copy
-  k_orth3<<<g, 256, 0, st>>>(q);
-  k_next_j<<<1, 32, 0, st>>>(c->Ljd);
+  orth_step(c, q, orth_chunks(n, blk), 1, c->Ljd);
   return launch_ok(c);
 }
 
@@ -1141,16 +1263,7 @@ static int block_part(bd_ctx* c, int k, bool pre, int part, bool count = true) {
   // 4 x 148 CTAs in all: each right-hand side's vectors in 592 / k chunks
   // (at most 148), so every CTA re-sums only the chunk partials of its own
   // right-hand side while enough warps stay resident
-  dim3 g(block_chunks(n, k), k);
-  c->launches += count ? 5 : 4;
-  k_orth0<<<g, 256, 0, st>>>(q);
-  k_orth1<<<g, 256, 0, st>>>(q);
-  if (q.Vs)
-    k_orth2<true><<<g, 256, 0, st>>>(q);
-  else
-    k_orth2<false><<<g, 256, 0, st>>>(q);
-  k_orth3<<<g, 256, 0, st>>>(q);
-  if (count) k_next_j<<<1, 32, 0, st>>>(c->Bjd);
+  orth_step(c, q, block_chunks(n, k), k, count ? c->Bjd : nullptr);
   return launch_ok(c);
 }
 
