@@ -49,7 +49,7 @@ typedef enum {
 
 typedef enum { BD_FLOW_SHEAR = 0, BD_FLOW_EXT = 1 } bd_flow;
 /* Brownian noise source for bd_get_noise: the reference's sequential
- * ran1/gasdev stream (bit-identical, one device thread) or counter-based
+ * ran1/gasdev stream (bit-identical, one warp) or counter-based
  * Philox4x32-10 Gaussians (parallel; the production source). */
 typedef enum { BD_NOISE_RAN1 = 0, BD_NOISE_PHILOX = 1 } bd_noise;
 /* Pair mobility: the reference's hybrid (Ewald sum below a minimum-image
@@ -130,9 +130,10 @@ typedef struct {
    * B-spline order (even, 4..8; 0 -> 8), real-space cutoff (0 -> the smaller
    * of 10 and 0.43 L; at most 0.43 L), split parameter (0 -> 4 / cutoff) and the cap on
    * real-space pairs per bead (0 -> 2.5 times the mean number of beads within
-   * the cutoff, at least 512, and rows that overflow it are grown to 1.25
-   * times the longest row at the mobility build; an explicit cap that
-   * overflows is BD_ERR_NBR_OVERFLOW). */
+   * the cutoff, at least 512; four consecutive beads in cell order share a row,
+   * and rows that overflow it are grown to 1.25 times the longest one at the
+   * mobility build; an explicit cap that a bead's pairs overflow is
+   * BD_ERR_NBR_OVERFLOW). */
   int pme_grid;
   int pme_order;
   double pme_rc;

@@ -30,7 +30,8 @@
 //    (shear/src/main26.c:1663-1700); the off-diagonal entries of the k-space
 //    self sum, which a sheared or stretched cell makes non-zero, are removed.
 // Spreading and interpolation are in bd_mesh.cu, the transforms in bd_fft.cuh
-// (cuFFT for grid sizes it does not cover).  The spline weights, the columns' lists and the pair tensors are
+// (cuFFT for grid sizes it does not cover).  The spline weights, the columns'
+// lists and the pair tensors are
 // computed once per mobility build because its positions do not change during
 // the Krylov solves.
 #include <cufft.h>

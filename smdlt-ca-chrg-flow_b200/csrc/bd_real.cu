@@ -170,7 +170,9 @@ __device__ __forceinline__ void store_tensor(R* entry, int b, double t1, double 
 // hits in shared memory.  Batches of hits are then tested against the group's
 // earlier beads: a neighbour is listed by the first bead that has it within
 // the cutoff.  Bound by the FP64 pipe: 193 M candidates at 50 000 beads, cutoff
-// 14.5.
+// 14.5, 0.86 ms (a thread per bead forming rows and tensors together took 6.0, a
+// warp per bead 1.3; this and k_rl_tensors 1.5, for rows the product reads 1.7 times
+// faster).
 __global__ void __launch_bounds__(128, 4)
     k_rl_find(Cell cell, RGeom g, const double4* __restrict__ pos, int N, int ngroup,
               const int* __restrict__ cell_start, const double4* __restrict__ spos, double rc2,
@@ -255,7 +257,8 @@ __global__ void __launch_bounds__(128, 4)
 // at a time are formed in shared memory and written side by side (from the
 // lanes, 64 bytes apart, every sector would be written eight times).
 // Overlapping pairs (r < 2), whose terms cost three times as much, are queued
-// and formed 32 at a time.  Bound by the FP64 pipe (erfc, exp).
+// and formed 32 at a time.  Bound by the FP64 pipe (erfc, exp): 0.62 ms at
+// 50 000 beads, cutoff 14.5; 0.76 with each lane writing its own entry.
 template <typename R>
 __global__ void __launch_bounds__(128, 4)
     k_rl_tensors(Cell cell, const double4* __restrict__ pos, int N, int ngroup,
@@ -394,8 +397,8 @@ __device__ __forceinline__ void copy_wait() {
 // One warp per group of four beads: a lane serves one pair and every S-th
 // entry of the row (S = 32 / NP), so NP lanes read a neighbour's packed values
 // (component c of pair p at vpk[(c N + j) np + p]) side by side and use them
-// for the four beads, two at a time.  The row (68 bytes an entry, read once) streams through
-// shared memory, about 30 entries at a time with two more such pieces under
+// for the four beads, two at a time.  The row (68 bytes an entry, read once)
+// streams through shared memory, about 30 entries at a time with two more such pieces under
 // way: with loads to registers, an entry ahead, too few bytes were in flight
 // to cover the latency of L2 and HBM (430 us at 50 000 beads, cutoff 14.5,
 // five pairs).  FP32: partial sums of about 16 entries folded into a second
