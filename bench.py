@@ -417,10 +417,9 @@ def build_context(w, seed, path="lanczos32", device_noise="philox", noise_seed=N
 
 
 # DRAM bytes (read + write, cold cache) of one block product, summed over its
-# kernels from ncu captures of the bench's own command
-# (profiles/launches_pme32-learned_c3.md); keyed by (beads, grid, cutoff,
-# right-hand sides per product)
-PRODUCT_TRAFFIC = {(50000, 100, 14.5, 10): 2.1933e9, (50000, 108, 13.6, 10): 2.6445e9}
+# kernels; keyed by (beads, grid, cutoff, right-hand sides per product).  None
+# measured for the kernels that run now
+PRODUCT_TRAFFIC = {}
 
 
 def ranks_max(values, dist):
@@ -844,7 +843,7 @@ def run_ours(args, rank, world, dist):
     value = world * N * K / (main["t_max_ms"] / 1e3)
     peak, kind = peaks()
     pme = PATHS[args.path]["mobility"] == "pme"
-    roof = {"kernel": ("particle-mesh product (spread, R2C, influence, C2R, gather)" if pme else
+    roof = {"kernel": ("particle-mesh product (spread, transforms with the influence tensor, interpolation, real-space rows)" if pme else
                        "k_sym_matvec<%s>" % ("float" if PATHS[args.path]["precision"] == "fp32"
                                              else "double")),
             "bound": "hbm", "achieved": main["achieved_gbs"], "peak": peak, "peak_kind": kind,
@@ -854,7 +853,7 @@ def run_ours(args, rank, world, dist):
     if main["block"]:
         b = main["block"]
         roof.update({"kernel": "particle-mesh product of a noise block (%.1f right-hand sides "
-                               "per launch: spread, R2C, influence, C2R, gather)"
+                               "per launch: spread, transforms with the influence tensor, interpolation, real-space rows)"
                                % b["rhs_per_iteration"],
                      "achieved": b["achieved_gbs"], "frac": b["achieved_gbs"] / peak,
                      "traffic": PRODUCT_TRAFFIC.get(
