@@ -402,11 +402,10 @@ __device__ __forceinline__ void copy_wait() {
 // way: with loads to registers, an entry ahead, too few bytes were in flight
 // to cover the latency of L2 and HBM (430 us at 50 000 beads, cutoff 14.5,
 // five pairs).  FP32: partial sums of about 16 entries folded into a second
-// set; lanes added in FP64.  Five pairs: 257 us at 50 000 beads, cutoff 14.5,
-// 38 us at 8000 beads, cutoff 12.1 (a warp per bead, every neighbour's values read
-// once per bead: 435 and 50).
-// SPLIT warps share a group's row where there are too few groups to fill the
-// chip with a warp each.
+// set; lanes added in FP64.  Five pairs: 257 us at 50 000 beads, cutoff 14.5
+// (a warp per bead, every neighbour's values read once per bead: 435); at 8000
+// beads, cutoff 12.1, 38 us by one warp a group against 50.
+// SPLIT warps share a group's row.
 template <int NP, typename R>
 struct Stage {
   static constexpr int S = 32 / NP, ITS = 32 / S, CH = S * ITS;  // entries a piece
@@ -546,13 +545,19 @@ void launch_apply(bd_ctx* c, int np, int p0, const Finish& fin) {
   k_real_apply<NP, SPLIT_, R><<<nblk(ng, 4 / SPLIT_), 128, 0, c->stream>>>(               \
       c->rl_cnt, c->rl_rows, (const R*)c->rl_w, c->rl_cap,                                \
       (const typename Real2<R>::T*)c->pme_vpk, np, p0, c->N, ng, fin)
-  // about 16 warps an SM
-  if (ng >= 148 * 12)
+  // More warps a group fill the chip sooner, fewer start fewer pieces.  By four,
+  // two and one, five pairs FP32: 500 beads 6.1, 8.0, 12.6 us, 8000 41.8, 46.5, 63.7,
+  // 16 000 70, 74, 79; FP64 8000 85, 90, 107, 16 000 151, 147, 160; one pair FP32
+  // 8000 24.0, 20.9, 24.4, 16 000 45.5, 35.2, 34.5.  At 50 000 beads of a run's
+  // chains five pairs took 268 by four and 257 by one, one pair 118 by two and 114
+  // by one.
+  const int four = NP < 5 ? 148 * 12 : sizeof(R) == 8 ? 148 * 20 : 148 * 40;
+  if (ng >= 148 * 40)
     REAL(1);
-  else if (ng >= 148 * 6)
-    REAL(2);
-  else
+  else if (ng < four)
     REAL(4);
+  else
+    REAL(2);
 #undef REAL
 }
 

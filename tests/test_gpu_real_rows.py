@@ -38,3 +38,23 @@ def test_rows_match_model(N, precision, tol):
     assert rel_err(got[0], ref[0]) < tol
     assert rel_err(got[2], ref[1]) < tol
     assert rel_err(c.mobility_apply(V[0].reshape(-1)), ref[0]) < tol
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-12), ("fp32", 2e-6)])
+@pytest.mark.parametrize("N", [7103, 11843, 23685])
+def test_blocks_of_nine_match_singles(N, precision, tol):
+    """Five packed pairs on the sides of their own rules, against one product per
+    vector (the bounds of the block product's other test)."""
+    L = (N / 0.05) ** (1 / 3)
+    r = np.random.default_rng(N)
+    c = B.Context(B.make_params(0, N, 1, L, 0.2, 5e-4, mobility="pme", noise="philox",
+                                precision=precision, pme_grid=40, pme_rc=6.0, pme_alpha=0.45,
+                                noise_block=10))
+    c.set_positions(*r.uniform(-L / 2, L / 2, (3, N)))
+    c.set_time(0, 0)
+    c.update_lattice(0)
+    c.apply_pbc()
+    c.calc_hi()
+    V = r.normal(size=(9, 3 * N))
+    got = c.mobility_apply_block(V)
+    assert max(rel_err(got[k], c.mobility_apply(V[k])) for k in range(9)) < tol
