@@ -23,6 +23,7 @@
 // draws (the same, in the same order, as the reference), its Metropolis test
 // and, when accepted, three table rows added to the later lanes.
 #include <math.h>
+#include <stddef.h>
 
 #include "bd_ctx.cuh"
 #include "bd_cell.cuh"
@@ -124,6 +125,7 @@ struct HopWin {
   double tab[kHopWin * 9 * kHopWin];      // [moved charge][its target][target][charge]
   double e_init, e_cur;
 };
+static_assert(offsetof(HopWin, tab) % 16 == 0, "the table is copied 16 bytes at a time");
 
 struct HopArgs {
   Lat l;
@@ -268,7 +270,7 @@ __global__ void __launch_bounds__(256) k_hop_decide(HopArgs q, int k0,
                                                     const double* __restrict__ rowsum,
                                                     int* __restrict__ old, Ran1* rng,
                                                     double barrier, double barrier2, int* log) {
-  extern __shared__ double tab[];
+  extern __shared__ __align__(16) double tab[];  // filled 16 bytes at a time
   __shared__ double red[33];
   __shared__ uint4 next[64];
   __shared__ float u[64];
