@@ -56,6 +56,36 @@ int launch_ok_at(bd_ctx* c, const char* file, int line) {
   return cuda_fail((int)e, cudaGetErrorString(e), file, line);
 }
 
+int alloc_all(bd_ctx* c, std::initializer_list<Buf> bufs) {
+  size_t sum = 0;
+  for (const Buf& b : bufs) {
+    const size_t n = std::max<size_t>(b.bytes, 16);
+    cudaError_t e = cudaMalloc((void**)b.at, n);
+    if (e != cudaSuccess) {
+      *(void**)b.at = nullptr;
+      for (const Buf& f : bufs) {
+        if (&f == &b) break;
+        free_all({f.at});
+      }
+      cudaGetLastError();  // not a sticky error: the next launch check must not see it
+      return e == cudaErrorMemoryAllocation
+                 ? BD_ERR_OOM
+                 : cuda_fail((int)e, cudaGetErrorString(e), __FILE__, __LINE__);
+    }
+    sum += n;
+  }
+  c->bytes += sum;
+  return BD_OK;
+}
+
+void free_all(std::initializer_list<void*> at) {
+  for (void* a : at) {
+    void** p = (void**)a;
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
+}
+
 int check(bd_ctx* c) {
   // the error word through the pinned staging's last entry
   int* word = (int*)(c->stage + 2 * kStages * (size_t)c->N);

@@ -397,37 +397,35 @@ __global__ void __launch_bounds__(1024) k_sum_into(const double* __restrict__ pa
 
 namespace bd {
 
-static int coul_alloc(bd_ctx* c) {
-  if (c->cw_grid) return BD_OK;
+static int coul_parts(bd_ctx* c) {
   // per-charge arrays sized for every bead charged (charges can be reset)
   int K = c->pmeK, n = std::max(c->N, 1);
   size_t K3 = (size_t)K * K * K, Ks = (size_t)K * K * (K / 2 + 1);
-  CU(cudaMalloc(&c->cw_grid, 8 * K3));
-  CU(cudaMalloc(&c->cw_spec, 16 * Ks));
-  CU(cudaMalloc(&c->cw_bsq, 24 * (size_t)K));
   c->cw_nblk = (int)((Ks + 255) / 256);
-  CU(cudaMalloc(&c->cw_epart, 8 * (size_t)std::max(6 * c->cw_nblk, n)));
-  CU(cudaMalloc(&c->cw_energy, 8 * 4));
-  CU(cudaMalloc(&c->cw_base, 12 * (size_t)n));
-  CU(cudaMalloc(&c->cw_w, 2 * 8 * 3 * (size_t)n * kMaxOrder));
-  CU(cudaMalloc(&c->cw_cell_of, 4 * (size_t)n));
-  CU(cudaMalloc(&c->cw_idx, 4 * (size_t)n));
-  CU(cudaMalloc(&c->cw_sorted, 32 * (size_t)n));
-  CU(cudaMalloc(&c->cw_count, 4 * (size_t)kCellCap));
-  CU(cudaMalloc(&c->cw_start, 4 * (size_t)(kCellCap + 1)));
-  CU(cudaMalloc(&c->cw_cursor, 4 * (size_t)kCellCap));
+  int s = alloc_all(c, {{&c->cw_grid, 8 * K3},
+                        {&c->cw_spec, 16 * Ks},
+                        {&c->cw_bsq, 24 * (size_t)K},
+                        {&c->cw_epart, 8 * (size_t)std::max(6 * c->cw_nblk, n)},
+                        {&c->cw_energy, 8 * 4},
+                        {&c->cw_base, 12 * (size_t)n},
+                        {&c->cw_w, 2 * 8 * 3 * (size_t)n * kMaxOrder},
+                        {&c->cw_cell_of, 4 * (size_t)n},
+                        {&c->cw_idx, 4 * (size_t)n},
+                        {&c->cw_sorted, 32 * (size_t)n},
+                        {&c->cw_count, 4 * (size_t)kCellCap},
+                        {&c->cw_start, 4 * (size_t)(kCellCap + 1)},
+                        {&c->cw_cursor, 4 * (size_t)kCellCap}});
+  if (s != BD_OK) return s;
   CU(cudaMemsetAsync(c->cw_count, 0, 4 * (size_t)kCellCap, c->stream));
   CU(cudaMemsetAsync(c->cw_energy, 0, 32, c->stream));
-  c->bytes += 8 * K3 + 16 * Ks + 24 * (size_t)K + 8 * (size_t)std::max(6 * c->cw_nblk, n) + 32 +
-              (size_t)n * (12 + 48 * kMaxOrder + 40) + 12 * (size_t)kCellCap;
   int dims[3] = {K, K, K};
   cufftHandle f, b;
   CF(cufftPlanMany(&f, 3, dims, nullptr, 1, (int)K3, nullptr, 1, (int)Ks, CUFFT_D2Z, 1));
+  c->cw_plan_f = (int)f + 1;
   CF(cufftPlanMany(&b, 3, dims, nullptr, 1, (int)Ks, nullptr, 1, (int)K3, CUFFT_Z2D, 1));
+  c->cw_plan_b = (int)b + 1;
   CF(cufftSetStream(f, c->stream));
   CF(cufftSetStream(b, c->stream));
-  c->cw_plan_f = (int)f;
-  c->cw_plan_b = (int)b;
   std::vector<double> bs(3 * (size_t)K);
   bspline_moduli(K, c->pme_p, bs.data());
   for (int d = 1; d < 3; d++)
@@ -438,12 +436,25 @@ static int coul_alloc(bd_ctx* c) {
 }
 
 void coulomb_free(bd_ctx* c) {
-  if (c->cw_plan_f) cufftDestroy((cufftHandle)c->cw_plan_f);
-  if (c->cw_plan_b) cufftDestroy((cufftHandle)c->cw_plan_b);
-  void* ptrs[] = {c->cw_grid, c->cw_spec, c->cw_bsq, c->cw_epart, c->cw_energy, c->cw_base,
-                  c->cw_w, c->cw_cell_of, c->cw_idx, c->cw_sorted, c->cw_count, c->cw_start, c->cw_cursor};
-  for (void* q : ptrs)
-    if (q) cudaFree(q);
+  for (int* plan : {&c->cw_plan_f, &c->cw_plan_b}) {
+    if (*plan) cufftDestroy((cufftHandle)(*plan - 1));
+    *plan = 0;
+  }
+  free_all({&c->cw_grid, &c->cw_spec, &c->cw_bsq, &c->cw_epart, &c->cw_energy, &c->cw_base,
+            &c->cw_w, &c->cw_cell_of, &c->cw_idx, &c->cw_sorted, &c->cw_count, &c->cw_start,
+            &c->cw_cursor});
+}
+
+// The Coulomb sum's buffers and plans, all or none (cw_grid tells).
+static int coul_alloc(bd_ctx* c) {
+  if (c->cw_grid) return BD_OK;
+  const size_t before = c->bytes;
+  const int s = coul_parts(c);
+  if (s != BD_OK) {
+    coulomb_free(c);
+    c->bytes = before;
+  }
+  return s;
 }
 
 // Reciprocal-space potential of the charges gathered in cq on the mesh:
@@ -477,11 +488,11 @@ int coulomb_mesh_potential(bd_ctx* c, const Lat& l, const double4* cq) {
 #undef CW_WEIGHTS
   CU(cudaMemsetAsync(c->cw_grid, 0, 8 * K3, c->stream));
   k_cw_spread<<<nblk(nch, 8), 256, 0, c->stream>>>(cq, c->cw_base, w, nch, K, p, c->cw_grid);
-  CF(cufftExecD2Z((cufftHandle)c->cw_plan_f, c->cw_grid, (cufftDoubleComplex*)c->cw_spec));
+  CF(cufftExecD2Z((cufftHandle)(c->cw_plan_f - 1), c->cw_grid, (cufftDoubleComplex*)c->cw_spec));
   k_cw_influence<<<c->cw_nblk, 256, 0, c->stream>>>(cell, K, c->cw_beta, c->p.lambda_b,
                                                     c->cw_bsq, (cufftDoubleComplex*)c->cw_spec,
                                                     c->cw_epart);
-  CF(cufftExecZ2D((cufftHandle)c->cw_plan_b, (cufftDoubleComplex*)c->cw_spec, c->cw_grid));
+  CF(cufftExecZ2D((cufftHandle)(c->cw_plan_b - 1), (cufftDoubleComplex*)c->cw_spec, c->cw_grid));
   return launch_ok(c);
 }
 
@@ -579,12 +590,12 @@ int coulomb_ewald(bd_ctx* c, const Lat& l, const double4* cq) {
 #undef CW_WEIGHTS
   CU(cudaMemsetAsync(c->cw_grid, 0, 8 * K3, c->stream));
   k_cw_spread<<<nblk(nch, 8), 256, 0, c->stream>>>(cq, c->cw_base, w, nch, K, p, c->cw_grid);
-  CF(cufftExecD2Z((cufftHandle)c->cw_plan_f, c->cw_grid, (cufftDoubleComplex*)c->cw_spec));
+  CF(cufftExecD2Z((cufftHandle)(c->cw_plan_f - 1), c->cw_grid, (cufftDoubleComplex*)c->cw_spec));
   k_cw_influence<<<c->cw_nblk, 256, 0, c->stream>>>(cell, K, c->cw_beta, c->p.lambda_b,
                                                     c->cw_bsq, (cufftDoubleComplex*)c->cw_spec,
                                                     c->cw_epart);
   k_sum_into<<<1, 1024, 0, c->stream>>>(c->cw_epart, c->cw_nblk, c->cw_energy + 1);
-  CF(cufftExecZ2D((cufftHandle)c->cw_plan_b, (cufftDoubleComplex*)c->cw_spec, c->cw_grid));
+  CF(cufftExecZ2D((cufftHandle)(c->cw_plan_b - 1), (cufftDoubleComplex*)c->cw_spec, c->cw_grid));
 #define CW_FORCES(P_)                                                                        \
   k_cw_forces<P_><<<nblk(nch, 8), 256, 0, c->stream>>>(                                       \
       cell, g, cq, c->track, nch, cr, sr, K, c->cw_base, w, dw, c->cw_grid, c->cw_cell_of,    \

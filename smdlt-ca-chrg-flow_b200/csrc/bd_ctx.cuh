@@ -14,6 +14,7 @@
 
 #include <cuda_runtime.h>
 
+#include <initializer_list>
 #include <vector>
 
 #include "bd_internal.cuh"
@@ -235,6 +236,16 @@ namespace bd {
 void prof_begin(bd_ctx* c, int slot);
 void prof_end(bd_ctx* c, int slot);
 void prof_clear(bd_ctx* c);
+
+// Device buffers of one use: all of them or, with BD_ERR_OOM, none (their
+// pointers null), so that a pointer which is set means that the others are.
+// `at` is the pointer's address.
+struct Buf {
+  void* at;
+  size_t bytes;
+};
+int alloc_all(bd_ctx* c, std::initializer_list<Buf> bufs);
+void free_all(std::initializer_list<void*> at);  // frees and clears the pointers
 
 int set_error_from_bits(int bits);
 int check(bd_ctx* c);                 // synchronise and fold device error bits

@@ -919,25 +919,25 @@ int alloc_lanczos(bd_ctx* c) {
   c->lmax = c->p.lanczos_max > 0 ? c->p.lanczos_max : 200;
   c->ltol = c->p.lanczos_tol > 0 ? c->p.lanczos_tol : 1e-6;
   size_t n = 3 * (size_t)c->NT * 32;
-  CU(cudaMalloc(&c->LV, 8 * n * (c->lmax + 1)));
-  CU(cudaMalloc(&c->Lw, 8 * n));
-  CU(cudaMalloc(&c->Lpart, 8 * (size_t)3 * (c->lmax + 1) * kDotBlocks));
-  CU(cudaMalloc(&c->Lh, 8 * (size_t)(c->lmax + 1)));
-  CU(cudaMalloc(&c->Lsc, 8 * (size_t)(c->lmax + 16)));
-  CU(cudaMalloc(&c->Lc, 8 * (size_t)(c->lmax + 1)));
-  CU(cudaMalloc(&c->MF, 8 * n));
-  CU(cudaMalloc(&c->Yz, 8 * n));
-  CU(cudaMalloc(&c->Lt1, 8 * n));
-  CU(cudaMalloc(&c->Lt2, 8 * n));
-  CU(cudaMalloc(&c->Lvcur, 8 * n));
-  CU(cudaMalloc(&c->Ljd, 16));
+  const size_t L1 = c->lmax + 1;
+  int s = alloc_all(c, {{&c->LV, 8 * n * L1},
+                        {&c->Lw, 8 * n},
+                        {&c->Lpart, 8 * 3 * L1 * kDotBlocks},
+                        {&c->Lh, 8 * L1},
+                        {&c->Lsc, 8 * (L1 + 15)},
+                        {&c->Lc, 8 * L1},
+                        {&c->MF, 8 * n},
+                        {&c->Yz, 8 * n},
+                        {&c->Lt1, 8 * n},
+                        {&c->Lt2, 8 * n},
+                        {&c->Lvcur, 8 * n},
+                        {&c->Ljd, 16}});
+  if (s != BD_OK) return s;
   // the padding entries (beads N..NTp-1) of the work vectors stay zero: the
   // orthogonalisation runs over all 3 NTp entries and the particle-mesh
   // product and the preconditioner write only the N beads
   for (double* q : {c->Lw, c->MF, c->Yz, c->Lt1, c->Lt2, c->Lvcur})
     CU(cudaMemsetAsync(q, 0, 8 * n, c->stream));
-  c->bytes += 8 * n * (c->lmax + 6) + 8 * (size_t)(c->lmax + 1) * (3 * kDotBlocks + 2) +
-              8 * (size_t)(c->lmax + 16);
   return BD_OK;
 }
 
@@ -1142,36 +1142,38 @@ void lanczos_graphs_reset(bd_ctx* c) {
 
 static int alloc_blocks(bd_ctx* c) {
   if (c->BV) return BD_OK;
-  int k = c->nbk, L1 = c->lmax + 1, blk = kDotBlocks;
-  size_t n = 3 * (size_t)c->NT * 32;
-  CU(cudaMalloc(&c->BV, 8 * n * k * L1));
-  if (c->p.precision == BD_PREC_FP32) {  // FP32 copy for the reorthogonalisation pass
-    CU(cudaMalloc(&c->BVs, 4 * n * k * L1));
-    c->bytes += 4 * n * k * L1;
-  }
-  for (double** q : {&c->Bw, &c->Bvcur, &c->Bt1, &c->Bt2, &c->BY}) {
-    CU(cudaMalloc(q, 8 * n * k));
-    CU(cudaMemsetAsync(*q, 0, 8 * n * k, c->stream));  // padding entries stay zero
-  }
-  CU(cudaMalloc(&c->BR, 8 * 3 * (size_t)c->N * k));
-  CU(cudaMalloc(&c->Bpart, 8 * (size_t)3 * k * L1 * blk));
-  CU(cudaMalloc(&c->Bh, 8 * (size_t)k * L1));
-  CU(cudaMalloc(&c->Bab, 8 * (size_t)2 * k * L1));
-  CU(cudaMalloc(&c->Bsc, 8 * (size_t)2 * k));
-  CU(cudaMalloc(&c->Bc, 8 * (size_t)k * L1));
-  CU(cudaMalloc(&c->Bm, 4 * (size_t)k));
-  CU(cudaMalloc(&c->Bjd, 16));
-  CU(cudaMalloc(&c->Bctl, 4 * (size_t)(5 * k + 4)));
-  CU(cudaMalloc(&c->Bdh, 8 * 8 * (size_t)k));
-  CU(cudaMalloc(&c->Bpsi, 8 * (size_t)k * L1 * kQuadNodes));
-  c->bytes += 4 * (size_t)(5 * k + 4) + 64 * (size_t)k + 8 * (size_t)k * L1 * kQuadNodes;
   if (!c->Bhost) return BD_ERR_STATE;  // pinned at bd_create (see there)
-  CU(cudaMalloc(&c->Brng, sizeof(Ran1) * (size_t)(k + 1)));
-  cudaEvent_t ev;
-  CU(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-  c->blk_ev = (void*)ev;
-  c->bytes += 8 * n * k * (L1 + 5) + 24 * (size_t)c->N * k + 8 * (size_t)k * L1 * (3 * blk + 4) +
-              24 * (size_t)k;
+  const size_t k = c->nbk, L1 = c->lmax + 1, blk = kDotBlocks, n = 3 * (size_t)c->NT * 32;
+  if (!c->blk_ev) {
+    cudaEvent_t ev;
+    CU(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    c->blk_ev = (void*)ev;
+  }
+  // FP32 contexts: an FP32 copy of the basis for the reorthogonalisation pass
+  const bool copy = c->p.precision == BD_PREC_FP32;
+  int s;
+  if (copy && !c->BVs && (s = alloc_all(c, {{&c->BVs, 4 * n * k * L1}})) != BD_OK) return s;
+  s = alloc_all(c, {{&c->BV, 8 * n * k * L1},
+                    {&c->Bw, 8 * n * k},
+                    {&c->Bvcur, 8 * n * k},
+                    {&c->Bt1, 8 * n * k},
+                    {&c->Bt2, 8 * n * k},
+                    {&c->BY, 8 * n * k},
+                    {&c->BR, 8 * 3 * (size_t)c->N * k},
+                    {&c->Bpart, 8 * 3 * k * L1 * blk},
+                    {&c->Bh, 8 * k * L1},
+                    {&c->Bab, 8 * 2 * k * L1},
+                    {&c->Bsc, 8 * 2 * k},
+                    {&c->Bc, 8 * k * L1},
+                    {&c->Bm, 4 * k},
+                    {&c->Bjd, 16},
+                    {&c->Bctl, 4 * (5 * k + 4)},
+                    {&c->Bdh, 8 * 8 * k},
+                    {&c->Bpsi, 8 * k * L1 * kQuadNodes},
+                    {&c->Brng, sizeof(Ran1) * (k + 1)}});
+  if (s != BD_OK) return s;
+  for (double* q : {c->Bw, c->Bvcur, c->Bt1, c->Bt2, c->BY})
+    CU(cudaMemsetAsync(q, 0, 8 * n * k, c->stream));  // padding entries stay zero
   return BD_OK;
 }
 
@@ -1725,18 +1727,7 @@ int lanczos_inv_sqrt(bd_ctx* c, const double* z, double* out, int* iters, bool* 
 static int io_alloc(bd_ctx* c) {
   if (c->io) return BD_OK;
   const size_t k = (size_t)std::max(1, c->nbk), n = 3 * (size_t)c->NT * 32;
-  if (cudaMalloc(&c->io, 24 * (size_t)c->N * k) != cudaSuccess ||
-      cudaMalloc(&c->io_x, 8 * n * k) != cudaSuccess ||
-      cudaMalloc(&c->io_y, 8 * n * k) != cudaSuccess) {
-    cudaGetLastError();  // not a sticky error: the next launch check must not see it
-    for (double** q : {&c->io, &c->io_x, &c->io_y}) {
-      cudaFree(*q);
-      *q = nullptr;
-    }
-    return BD_ERR_OOM;
-  }
-  c->bytes += (24 * (size_t)c->N + 16 * n) * k;
-  return BD_OK;
+  return alloc_all(c, {{&c->io, 24 * (size_t)c->N * k}, {&c->io_x, 8 * n * k}, {&c->io_y, 8 * n * k}});
 }
 
 // k vectors (Lanczos layout, n apart) to the host, bead-interleaved.

@@ -568,7 +568,6 @@ int gather_t(bd_ctx* c, int k, const R* grid) {
 namespace bd {
 
 int mesh_alloc(bd_ctx* c) {
-  if (c->mesh_val) return BD_OK;
   const int K = c->pmeK, N = c->N, P = c->pme_p, np = std::max(1, (c->nbk + 1) / 2);
   // a layout for single products and, where another does less work, one for
   // full blocks
@@ -578,28 +577,24 @@ int mesh_alloc(bd_ctx* c) {
   c->mesh_ng[0] = 1;
   c->mesh_ng[1] = best > 1 ? best : 0;
   size_t nbin_max = 0;
+  int s;
   for (int l = 0; l < 2 && c->mesh_ng[l]; l++) {
     int ng = c->mesh_ng[l];
     size_t nbin = patches(K, ng) * K;
     size_t nent = (size_t)N * most_touched(K, P, kCols[ng][0]) * most_touched(K, P, kCols[ng][1]);
-    CU(cudaMalloc(&c->mesh_ent[l], 4 * nent));
-    CU(cudaMalloc(&c->mesh_bin[l], 4 * (nbin + 1)));
-    c->bytes += 4 * (nent + nbin + 1);
+    s = alloc_all(c, {{&c->mesh_ent[l], 4 * nent}, {&c->mesh_bin[l], 4 * (nbin + 1)}});
+    if (s != BD_OK) return s;
     nbin_max = std::max(nbin_max, nbin);
   }
   size_t nscan = nbin_max / kScanBlock + 1;
-  CU(cudaMalloc(&c->mesh_sums, 4 * nscan));
-  CU(cudaMalloc(&c->mesh_cursor, 4 * nbin_max));
-  CU(cudaMalloc(&c->mesh_val, 48 * (size_t)N * np));
-  c->bytes += 4 * (nscan + nbin_max) + 48 * (size_t)N * np;
-  return BD_OK;
+  return alloc_all(c, {{&c->mesh_sums, 4 * nscan},
+                       {&c->mesh_cursor, 4 * nbin_max},
+                       {&c->mesh_val, 48 * (size_t)N * np}});
 }
 
 void mesh_free(bd_ctx* c) {
-  for (void* q : {(void*)c->mesh_ent[0], (void*)c->mesh_ent[1], (void*)c->mesh_bin[0],
-                  (void*)c->mesh_bin[1], (void*)c->mesh_sums, (void*)c->mesh_cursor,
-                  (void*)c->mesh_val})
-    if (q) cudaFree(q);
+  free_all({&c->mesh_ent[0], &c->mesh_ent[1], &c->mesh_bin[0], &c->mesh_bin[1], &c->mesh_sums,
+            &c->mesh_cursor, &c->mesh_val});
 }
 
 static void scan_excl(bd_ctx* c, int* a, size_t n) {
@@ -612,8 +607,6 @@ static void scan_excl(bd_ctx* c, int* a, size_t n) {
 
 // The columns' bead lists for the base indices of the last k_pme_weights.
 int mesh_prepare(bd_ctx* c) {
-  int s;
-  if ((s = mesh_alloc(c)) != BD_OK) return s;
   const int N = c->N, P = c->pme_p, K = c->pmeK;
   for (int l = 0; l < 2 && c->mesh_ng[l]; l++) {
     const int CY = kCols[c->mesh_ng[l]][0], CZ = kCols[c->mesh_ng[l]][1], npz = (K + CZ - 1) / CZ;

@@ -4,6 +4,7 @@
 #include "bd_ctx.cuh"
 
 namespace bd {
+int mesh_alloc(bd_ctx* c);
 int mesh_prepare(bd_ctx* c);
 int mesh_spread(bd_ctx* c, int k, const VecIn& v, size_t vr, void* grid);
 int mesh_gather(bd_ctx* c, int k, const void* grid);

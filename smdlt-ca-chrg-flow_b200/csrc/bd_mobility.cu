@@ -559,26 +559,37 @@ int alloc_mobility(bd_ctx* c) {
 // allocated on the first mobility build (they are O(N^2)).
 static int ensure_tiles(bd_ctx* c) {
   if (c->Mt) return BD_OK;
-  size_t nt = c->ntiles;
-  if (cudaMalloc(&c->Mt, 8 * nt * 6144) != cudaSuccess) return BD_ERR_OOM;
+  size_t nt = c->ntiles, vec = 8 * 3 * (size_t)c->NT * 32;
+  long long N = c->N;
+  c->near_cap = c->p.mobility == BD_MOB_EWALD ? 1 : std::min<long long>(N * (N - 1) / 2 + 1, 512 * N);
+  int s = alloc_all(c, {{&c->Mt, 8 * nt * 6144},
+                        {&c->tileI, 4 * nt},
+                        {&c->near_pairs, 8 * (size_t)c->near_cap},
+                        {&c->near_count, 16},
+                        {&c->rowpart, 8 * nt * 192},
+                        {&c->colpart, 8 * nt * 192 + 8 * (size_t)c->NT * kRedSplit * 192},
+                        {&c->U, vec},
+                        {&c->W, vec}});
+  if (s != BD_OK) return s;
   CU(cudaMemsetAsync(c->Mt, 0, 8 * nt * 6144, c->stream));
   std::vector<int> ti(nt);
   size_t k = 0;
   for (int I = 0; I < c->NT; I++)
     for (int J = I; J < c->NT; J++) ti[k++] = I;
-  CU(cudaMalloc(&c->tileI, 4 * nt));
   CU(cudaMemcpy(c->tileI, ti.data(), 4 * nt, cudaMemcpyHostToDevice));
-  long long N = c->N;
-  c->near_cap = c->p.mobility == BD_MOB_EWALD ? 1 : std::min<long long>(N * (N - 1) / 2 + 1, 512 * N);
-  CU(cudaMalloc(&c->near_pairs, 8 * c->near_cap));
-  CU(cudaMalloc(&c->near_count, 16));
-  CU(cudaMalloc(&c->rowpart, 8 * nt * 192));
-  CU(cudaMalloc(&c->colpart, 8 * nt * 192 + 8 * (size_t)c->NT * kRedSplit * 192));
-  CU(cudaMalloc(&c->U, 8 * 3 * (size_t)c->NT * 32));
-  CU(cudaMalloc(&c->W, 8 * 3 * (size_t)c->NT * 32));
-  c->bytes += 8 * nt * 6144 + 4 * nt + 8 * c->near_cap + 16 + 16 * nt * 192 +
-              8 * (size_t)c->NT * kRedSplit * 192 + 48 * (size_t)c->NT * 32;
   return BD_OK;
+}
+
+// Room for n k-vectors.
+static int kvec_alloc(bd_ctx* c, int n) {
+  if (n <= c->kvec_cap) return BD_OK;
+  CU(cudaStreamSynchronize(c->stream));
+  free_all({&c->kvec});
+  c->bytes -= 8 * 9 * (size_t)c->kvec_cap;
+  c->kvec_cap = 0;
+  const int s = alloc_all(c, {{&c->kvec, 8 * 9 * (size_t)(n + 64)}});
+  if (s == BD_OK) c->kvec_cap = n + 64;
+  return s;
 }
 
 // Ewald parameters, k-vector list with coefficients M2, and the self term Dtr
@@ -748,20 +759,17 @@ int calc_hi(bd_ctx* c) {
     s = pme_prepare(c, step_lat(c));
     if (s == BD_OK) s = precond_build(c, step_lat(c));
     prof_end(c, BD_PROF_HI_BUILD);
+    if (s != BD_OK) c->hi_built = false;
     return s;
   }
+  c->hi_built = false;  // until it is complete
   if ((s = ensure_tiles(c)) != BD_OK) return s;
   Lat l = step_lat(c);
   Ewald ew;
   std::vector<double> kv;
   bool ewald_all = c->p.mobility == BD_MOB_EWALD;
   hi_setup(c, l, &ew, &kv, c->Dtr, 4.0, 0, ewald_all);
-  if ((int)kv.size() / 9 > c->kvec_cap) {
-    CU(cudaStreamSynchronize(c->stream));
-    if (c->kvec) cudaFree(c->kvec);
-    c->kvec_cap = (int)kv.size() / 9 + 64;
-    CU(cudaMalloc(&c->kvec, 8 * 9 * (size_t)c->kvec_cap));
-  }
+  if ((s = kvec_alloc(c, (int)kv.size() / 9)) != BD_OK) return s;
   c->nk = ew.nk;
   if (!kv.empty())
     CU(cudaMemcpyAsync(c->kvec, kv.data(), 8 * kv.size(), cudaMemcpyHostToDevice, c->stream));
@@ -793,8 +801,7 @@ int calc_hi(bd_ctx* c) {
   if (c->p.precision == BD_PREC_FP32) {
     if (!c->Mt32) {
       CU(cudaStreamSynchronize(c->stream));
-      if (cudaMalloc(&c->Mt32, 4 * c->ntiles * 6144) != cudaSuccess) return BD_ERR_OOM;
-      c->bytes += 4 * c->ntiles * 6144;
+      if ((s = alloc_all(c, {{&c->Mt32, 4 * c->ntiles * 6144}})) != BD_OK) return s;
     }
     c->launches++;
     k_to_fp32<<<148 * 16, 256, 0, c->stream>>>(c->Mt, c->Mt32, c->ntiles * 6144);
@@ -944,12 +951,8 @@ extern "C" int bd_build_grid(bd_ctx* c, double grid_dt) {
     std::vector<double> kv;
     double unused[3];
     hi_setup(c, l, &ew, &kv, unused, 6.0, tp);
-    if ((int)kv.size() / 9 > c->kvec_cap) {
-      CU(cudaStreamSynchronize(c->stream));
-      if (c->kvec) cudaFree(c->kvec);
-      c->kvec_cap = (int)kv.size() / 9 + 64;
-      CU(cudaMalloc(&c->kvec, 8 * 9 * (size_t)c->kvec_cap));
-    }
+    int s = kvec_alloc(c, (int)kv.size() / 9);
+    if (s != BD_OK) return s;
     if (!kv.empty())
       CU(cudaMemcpyAsync(c->kvec, kv.data(), 8 * kv.size(), cudaMemcpyHostToDevice, c->stream));
     c->launches++;
@@ -1135,8 +1138,9 @@ int ewald_bin(bd_ctx* c, double* eps, std::vector<double>& rowsum) {
   int N = c->N, NT = (N + 31) / 32;
   long long ntl = (long long)NT * (NT + 1) / 2;
   if (!c->cb_part) {
-    CU(cudaMalloc(&c->cb_part, 8 * (size_t)ntl * 193 + 8 * (3 * (size_t)N + 1)));
-    CU(cudaMalloc(&c->cb_tileI, 4 * (size_t)ntl));
+    int s = alloc_all(c, {{&c->cb_part, 8 * (size_t)ntl * 193 + 8 * (3 * (size_t)N + 1)},
+                          {&c->cb_tileI, 4 * (size_t)ntl}});
+    if (s != BD_OK) return s;
     std::vector<int> ti(ntl);
     size_t k = 0;
     for (int I = 0; I < NT; I++)
@@ -1144,7 +1148,6 @@ int ewald_bin(bd_ctx* c, double* eps, std::vector<double>& rowsum) {
     CU(cudaMemcpyAsync(c->cb_tileI, ti.data(), 4 * (size_t)ntl, cudaMemcpyHostToDevice,
                        c->stream));
     CU(cudaStreamSynchronize(c->stream));
-    c->bytes += 8 * (size_t)ntl * 193 + 8 * (3 * (size_t)N + 1) + 4 * (size_t)ntl;
   }
   Lat l = step_lat(c);
   Ewald ew;

@@ -51,7 +51,6 @@ constexpr int kWgradCtas = 296;
 typedef __nv_bfloat16 bf16;
 
 struct Mpnn {
-  int cap;
   float *w, *g, *m1, *m2;
   bf16 *W1b, *W2b, *W34b, *W2t, *W34t;  // W (out x in) and W^T (in x out), BF16
   int* nbr;                             // N x K neighbour (or -1)
@@ -518,57 +517,37 @@ inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 Mpnn* get(bd_ctx* c) { return (Mpnn*)c->mpnn; }
 
 int ensure(bd_ctx* c) {
+  int s;
+  if (!c->mpnn) c->mpnn = new Mpnn();
   Mpnn* m = get(c);
-  if (!m) {
-    m = new Mpnn();
-    c->mpnn = m;
-    CU(cudaMalloc(&m->w, 4 * kParams));
-    CU(cudaMalloc(&m->g, 4 * kParams));
-    CU(cudaMalloc(&m->m1, 4 * kParams));
-    CU(cudaMalloc(&m->m2, 4 * kParams));
+  if (!m->w) {
+    s = alloc_all(c, {{&m->w, 4 * kParams},
+                      {&m->g, 4 * kParams},
+                      {&m->m1, 4 * kParams},
+                      {&m->m2, 4 * kParams},
+                      {&m->W1b, 2 * WD * NR},
+                      {&m->W2b, 2 * WD * WD},
+                      {&m->W2t, 2 * WD * WD},
+                      {&m->W34b, 2 * WD * 2 * WD},
+                      {&m->W34t, 2 * WD * 2 * WD},
+                      {&m->part, 4 * (size_t)kWgradCtas * WD * (2 * WD + 1)}});
+    if (s != BD_OK) return s;
     CU(cudaMemsetAsync(m->m1, 0, 4 * kParams, c->stream));
     CU(cudaMemsetAsync(m->m2, 0, 4 * kParams, c->stream));
-    CU(cudaMalloc(&m->W1b, 2 * WD * NR));
-    CU(cudaMalloc(&m->W2b, 2 * WD * WD));
-    CU(cudaMalloc(&m->W2t, 2 * WD * WD));
-    CU(cudaMalloc(&m->W34b, 2 * WD * 2 * WD));
-    CU(cudaMalloc(&m->W34t, 2 * WD * 2 * WD));
-    CU(cudaMalloc(&m->part, 4 * (size_t)kWgradCtas * WD * (2 * WD + 1)));
-    c->bytes += 16 * kParams + 2 * (WD * NR + 2 * WD * WD + 4 * WD * WD) +
-                4 * (size_t)kWgradCtas * WD * (2 * WD + 1);
   }
-  int N = c->N;
-  if (m->cap < N) {
-    void* old[] = {m->nbr, m->nvec, m->rbf, m->g1, m->e, m->mv, m->o2, m->h, m->X3, m->p3,
-                   m->u, m->sa, m->a, m->te, m->ce, m->zt, m->dG, m->du, m->de, m->dp3,
-                   m->dX3, m->dh, m->do2, m->dm, m->dg1, m->hg, m->lossv, m->G9};
-    for (void* q : old)
-      if (q) cudaFree(q);
-    size_t E = (size_t)N * KN;
-    CU(cudaMalloc(&m->nbr, 4 * E));
-    CU(cudaMalloc(&m->nvec, 12 * E));
-    CU(cudaMalloc(&m->rbf, 4 * E * NR));
-    CU(cudaMalloc(&m->g1, 4 * E * WD));
-    CU(cudaMalloc(&m->e, 4 * E * WD));
-    CU(cudaMalloc(&m->de, 4 * E * WD));
-    CU(cudaMalloc(&m->dg1, 4 * E * WD));
-    CU(cudaMalloc(&m->te, 4 * E));
-    CU(cudaMalloc(&m->ce, 4 * E));
-    float** nodes[] = {&m->mv, &m->o2, &m->h, &m->p3, &m->u, &m->du, &m->dp3, &m->dh, &m->do2,
-                       &m->dm};
-    for (float** q : nodes) CU(cudaMalloc(q, 4 * (size_t)N * WD));
-    CU(cudaMalloc(&m->X3, 8 * (size_t)N * WD));
-    CU(cudaMalloc(&m->dX3, 8 * (size_t)N * WD));
-    CU(cudaMalloc(&m->sa, 4 * (size_t)N));
-    CU(cudaMalloc(&m->a, 4 * (size_t)N));
-    CU(cudaMalloc(&m->lossv, 4 * (size_t)N));
-    CU(cudaMalloc(&m->zt, 24 * (size_t)N));
-    CU(cudaMalloc(&m->dG, 36 * (size_t)N));
-    CU(cudaMalloc(&m->hg, 4 * (size_t)N * (2 * WD + 2)));
-    CU(cudaMalloc(&m->G9, 72 * (size_t)N));
-    m->cap = N;
-    c->bytes += E * (4 + 12 + 4 * NR + 16 * WD + 8) + (size_t)N * (40 * WD + 16 * WD + 12 + 24 +
-                36 + 4 * (2 * WD + 2) + 72);
+  const size_t N = c->N, E = N * KN;
+  if (!m->nbr) {
+    s = alloc_all(c, {{&m->nbr, 4 * E},          {&m->nvec, 12 * E},     {&m->rbf, 4 * E * NR},
+                      {&m->g1, 4 * E * WD},      {&m->e, 4 * E * WD},    {&m->de, 4 * E * WD},
+                      {&m->dg1, 4 * E * WD},     {&m->te, 4 * E},        {&m->ce, 4 * E},
+                      {&m->mv, 4 * N * WD},      {&m->o2, 4 * N * WD},   {&m->h, 4 * N * WD},
+                      {&m->p3, 4 * N * WD},      {&m->u, 4 * N * WD},    {&m->du, 4 * N * WD},
+                      {&m->dp3, 4 * N * WD},     {&m->dh, 4 * N * WD},   {&m->do2, 4 * N * WD},
+                      {&m->dm, 4 * N * WD},      {&m->X3, 8 * N * WD},   {&m->dX3, 8 * N * WD},
+                      {&m->sa, 4 * N},           {&m->a, 4 * N},         {&m->lossv, 4 * N},
+                      {&m->zt, 24 * N},          {&m->dG, 36 * N},       {&m->hg, 4 * N * (2 * WD + 2)},
+                      {&m->G9, 72 * N}});
+    if (s != BD_OK) return s;
   }
   return BD_OK;
 }

@@ -210,30 +210,25 @@ __global__ void k_pme_soff_fin(const double* __restrict__ part, int nb, double* 
 
 namespace bd {
 
-int pme_alloc(bd_ctx* c) {
-  if (c->pme_grid) return BD_OK;
-  int K = c->pmeK, N = c->N;
+static int pme_parts(bd_ctx* c) {
+  int s, K = c->pmeK, N = c->N;
   size_t K3 = (size_t)K * K * K, Ks = (size_t)K * K * (K / 2 + 1);
   c->pme_f32 = c->p.precision == BD_PREC_FP32;
   size_t es = c->pme_f32 ? 4 : 8;  // grid, spectrum, influence and pair tensors
   // the packed pairs' grids for the largest number of right-hand sides
   size_t nr = (size_t)std::max(1, c->nbk);
   size_t grid_bytes = 2 * es * 3 * K3 * ((nr + 1) / 2);
-  CU(cudaMalloc(&c->pme_grid, grid_bytes));
-  CU(cudaMalloc(&c->pme_tw, 2 * es * K));
-  CU(cudaMalloc(&c->pme_infl, es * 6 * Ks));
-  CU(cudaMalloc(&c->pme_bsq, 8 * 3 * (size_t)K));
   c->pme_nblk = (int)((Ks + 255) / 256);
-  CU(cudaMalloc(&c->pme_soff, 8 * (3 * (size_t)c->pme_nblk + 3)));
-  CU(cudaMalloc(&c->pme_base, 4 * 3 * (size_t)N));
-  CU(cudaMalloc(&c->pme_w, es * 3 * (size_t)N * kMaxOrder));
-  CU(cudaMalloc(&c->pme_vpk, 6 * es * (size_t)N * ((nr + 1) / 2)));
-  CU(cudaMalloc(&c->rl_pos, 32 * (size_t)N));
-  int s;
-  if ((s = real_alloc(c)) != BD_OK) return s;
-  c->bytes += grid_bytes + es * 6 * Ks + (24 + 2 * es) * (size_t)K + 12 * (size_t)N +
-              3 * es * (size_t)N * kMaxOrder + 6 * es * (size_t)N * ((nr + 1) / 2) +
-              32 * (size_t)N;
+  s = alloc_all(c, {{&c->pme_grid, grid_bytes},
+                    {&c->pme_tw, 2 * es * K},
+                    {&c->pme_infl, es * 6 * Ks},
+                    {&c->pme_bsq, 8 * 3 * (size_t)K},
+                    {&c->pme_soff, 8 * (3 * (size_t)c->pme_nblk + 3)},
+                    {&c->pme_base, 4 * 3 * (size_t)N},
+                    {&c->pme_w, es * 3 * (size_t)N * kMaxOrder},
+                    {&c->pme_vpk, 6 * es * (size_t)N * ((nr + 1) / 2)},
+                    {&c->rl_pos, 32 * (size_t)N}});
+  if (s != BD_OK || (s = mesh_alloc(c)) != BD_OK || (s = real_alloc(c)) != BD_OK) return s;
   if (!fft_has_size(K)) {
     // one pair's three interleaved components, in place
     int n[3] = {K, K, K};
@@ -263,12 +258,23 @@ int pme_alloc(bd_ctx* c) {
 
 void pme_free(bd_ctx* c) {
   if (c->pme_plan) cufftDestroy((cufftHandle)(c->pme_plan - 1));
+  c->pme_plan = 0;
   mesh_free(c);
   real_free(c);
-  void* ptrs[] = {c->pme_vpk, c->pme_grid, c->pme_tw, c->pme_infl, c->pme_bsq, c->pme_soff,
-                  c->pme_base, c->pme_w, c->rl_pos};
-  for (void* q : ptrs)
-    if (q) cudaFree(q);
+  free_all({&c->pme_vpk, &c->pme_grid, &c->pme_tw, &c->pme_infl, &c->pme_bsq, &c->pme_soff,
+            &c->pme_base, &c->pme_w, &c->rl_pos});
+}
+
+// The mobility's buffers and plan, all or none (pme_grid tells).
+static int pme_alloc(bd_ctx* c) {
+  if (c->pme_grid) return BD_OK;
+  const size_t before = c->bytes;
+  const int s = pme_parts(c);
+  if (s != BD_OK) {
+    pme_free(c);
+    c->bytes = before;
+  }
+  return s;
 }
 
 // Preparation for the current positions, in the frame calcHI reads them
@@ -278,6 +284,7 @@ void pme_free(bd_ctx* c) {
 // configuration until the next preparation, as the dense matrix does.
 int pme_prepare(bd_ctx* c, const Lat& l) {
   int s;
+  c->pme_ready = c->hi_built = false;  // until it is complete
   if ((s = pme_alloc(c)) != BD_OK) return s;
   Cell cell = make_cell(l);
   double cr = 1.0, sr = 0.0;

@@ -230,15 +230,15 @@ static int pre_alloc(bd_ctx* c, int S) {
   size_t need = nb * n * n;
   if (c->pre_G && c->pre_cap >= need) return BD_OK;
   lanczos_graphs_reset(c);  // captured products hold the block pointers
-  if (c->pre_G) cudaFree(c->pre_G);
-  if (c->pre_Gi) cudaFree(c->pre_Gi);
-  c->pre_G = c->pre_Gi = nullptr;
-  CU(cudaMalloc(&c->pre_G, 8 * need));
-  CU(cudaMalloc(&c->pre_Gi, 8 * need));
-  if (!c->pre_bad) CU(cudaMalloc(&c->pre_bad, 16));
+  free_all({&c->pre_G, &c->pre_Gi});
+  c->pre_ready = false;
+  c->bytes -= 16 * c->pre_cap;
+  c->pre_cap = 0;
+  int s;
+  if (!c->pre_bad && (s = alloc_all(c, {{&c->pre_bad, 16}})) != BD_OK) return s;
+  if ((s = alloc_all(c, {{&c->pre_G, 8 * need}, {&c->pre_Gi, 8 * need}})) != BD_OK) return s;
   CU(cudaMemsetAsync(c->pre_bad, 0, 16, c->stream));
   c->pre_cap = need;
-  c->bytes += 16 * need;
   return BD_OK;
 }
 
@@ -271,11 +271,9 @@ int precond_build(bd_ctx* c, const Lat& l) {
     // segment blocks first, then the learned bead blocks applied on top
     int S = c->pre_S;
     if ((s = pre_alloc(c, S)) != BD_OK) return s;
-    if (!c->pre_B) {
-      CU(cudaMalloc(&c->pre_B, 72 * (size_t)c->N));
-      CU(cudaMalloc(&c->pre_Bi, 72 * (size_t)c->N));
-      c->bytes += 144 * (size_t)c->N;
-    }
+    if (!c->pre_B && (s = alloc_all(c, {{&c->pre_B, 72 * (size_t)c->N},
+                                        {&c->pre_Bi, 72 * (size_t)c->N}})) != BD_OK)
+      return s;
     size_t smem = 2 * 8 * (size_t)(3 * S) * (3 * S);
     cudaFuncSetAttribute(k_seg_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     c->launches += 3;

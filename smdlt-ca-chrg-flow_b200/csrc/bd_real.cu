@@ -580,59 +580,58 @@ int apply_t(bd_ctx* c, int np, const Finish& fin) {
 
 namespace bd {
 
-// Rows of cap entries for every group.
+// Rows of cap entries for every group; without memory for them there are none
+// (rl_rows null) and the mobility is not built.
 static int rows_alloc(bd_ctx* c, int cap) {
   size_t ng = ((size_t)c->N + kGroup - 1) / kGroup, es = c->pme_f32 ? 4 : 8;
   size_t old = (size_t)c->rl_cap, each = 4 + 4 * es * kGroup;
   if (c->rl_rows) {
     CU(cudaStreamSynchronize(c->stream));
-    cudaFree(c->rl_rows);
-    cudaFree(c->rl_w);
-    c->rl_rows = nullptr;
-    c->rl_w = nullptr;
+    free_all({&c->rl_rows, &c->rl_w});
     c->bytes -= each * ng * old;
   }
-  c->rl_cap = cap;
-  CU(cudaMalloc(&c->rl_rows, 4 * ng * cap));
-  CU(cudaMalloc(&c->rl_w, 4 * es * kGroup * ng * cap));
-  c->bytes += each * ng * cap;
-  return BD_OK;
+  c->rl_cap = 0;
+  int s = alloc_all(c, {{&c->rl_rows, 4 * ng * cap}, {&c->rl_w, 4 * es * kGroup * ng * cap}});
+  if (s == BD_OK) c->rl_cap = cap;
+  return s;
 }
 
-int real_alloc(bd_ctx* c) {
-  int N = c->N, s;
-  // row cap: an explicit cap per bead bounds a group's row by four times that;
-  // the default is 2.5 times the mean number of beads within the cutoff at the
-  // system's density, at least 512 (rows that overflow it are grown); no row
-  // is longer than N
+// Rows before any have overflowed: an explicit cap per bead bounds a group's
+// row by four times that; the default is 2.5 times the mean number of beads
+// within the cutoff at the system's density, at least 512 (rows that overflow
+// it are grown); no row is longer than N.
+static int first_cap(const bd_ctx* c) {
   long cap;
   if (c->p.pme_max_pairs > 0) {
     cap = (long)kGroup * c->p.pme_max_pairs;
   } else {
-    double mean = 4.0 / 3.0 * M_PI * c->pme_rc * c->pme_rc * c->pme_rc * N / c->boxvol;
+    double mean = 4.0 / 3.0 * M_PI * c->pme_rc * c->pme_rc * c->pme_rc * c->N / c->boxvol;
     cap = std::max(512, ((int)ceil(2.5 * mean) + 31) / 32 * 32);
   }
-  if ((s = rows_alloc(c, (int)std::min(cap, (long)std::max(N, 1)))) != BD_OK) return s;
-  CU(cudaMalloc(&c->rl_cnt, 4 * (size_t)N));
-  CU(cudaMalloc(&c->rl_need, 4));
-  CU(cudaMemsetAsync(c->rl_need, 0, 4, c->stream));
+  return (int)std::min(cap, (long)std::max(c->N, 1));
+}
+
+int real_alloc(bd_ctx* c) {
+  const size_t N = c->N;
   c->rl_ncell_cap = 4096;
-  CU(cudaMalloc(&c->rl_cell_of, 4 * (size_t)N));
-  CU(cudaMalloc(&c->rl_spos, 32 * (size_t)N));
-  CU(cudaMalloc(&c->rl_beads, 4 * (size_t)N));
-  CU(cudaMalloc(&c->rl_cell_count, 4 * (size_t)c->rl_ncell_cap));
-  CU(cudaMalloc(&c->rl_cell_start, 4 * (size_t)(c->rl_ncell_cap + 1)));
-  CU(cudaMalloc(&c->rl_cursor, 4 * (size_t)c->rl_ncell_cap));
+  int s = alloc_all(c, {{&c->rl_cnt, 4 * N},
+                        {&c->rl_need, 4},
+                        {&c->rl_cell_of, 4 * N},
+                        {&c->rl_spos, 32 * N},
+                        {&c->rl_beads, 4 * N},
+                        {&c->rl_cell_count, 4 * (size_t)c->rl_ncell_cap},
+                        {&c->rl_cell_start, 4 * (size_t)(c->rl_ncell_cap + 1)},
+                        {&c->rl_cursor, 4 * (size_t)c->rl_ncell_cap}});
+  if (s != BD_OK) return s;
+  CU(cudaMemsetAsync(c->rl_need, 0, 4, c->stream));
   CU(cudaMemsetAsync(c->rl_cell_count, 0, 4 * (size_t)c->rl_ncell_cap, c->stream));
-  c->bytes += 44 * (size_t)N + 12 * (size_t)c->rl_ncell_cap;
   return BD_OK;
 }
 
 void real_free(bd_ctx* c) {
-  void* ptrs[] = {c->rl_rows, c->rl_w, c->rl_cnt, c->rl_need, c->rl_cell_of, c->rl_spos, c->rl_beads,
-                  c->rl_cell_count, c->rl_cell_start, c->rl_cursor};
-  for (void* q : ptrs)
-    if (q) cudaFree(q);
+  free_all({&c->rl_rows, &c->rl_w, &c->rl_cnt, &c->rl_need, &c->rl_cell_of, &c->rl_spos,
+            &c->rl_beads, &c->rl_cell_count, &c->rl_cell_start, &c->rl_cursor});
+  c->rl_cap = 0;
 }
 
 // The groups' rows for the positions in rl_pos (lab frame; rx, ry, rz and the
@@ -640,6 +639,7 @@ void real_free(bd_ctx* c) {
 int real_prepare(bd_ctx* c, const Cell& cell, double cr, double sr, double alpha_ref) {
   int s, N = c->N;
   double rc = c->pme_rc, alpha = c->pme_alpha;
+  if (!c->rl_rows && (s = rows_alloc(c, first_cap(c))) != BD_OK) return s;
   // real-space cells: perpendicular widths V/|a_j x a_k|
   double w[3];
   {
@@ -687,9 +687,9 @@ int real_prepare(bd_ctx* c, const Cell& cell, double cr, double sr, double alpha
     CU(cudaMemcpyAsync(&longest, need, 4, cudaMemcpyDeviceToHost, c->stream));
     if ((s = check(c)) != BD_OK) return s;
     if (longest <= c->rl_cap) break;
+    CU(cudaMemsetAsync(c->rl_need, 0, 4, c->stream));
     if ((s = rows_alloc(c, std::min(N, ((int)ceil(1.25 * longest) + 31) / 32 * 32))) != BD_OK)
       return s;
-    CU(cudaMemsetAsync(c->rl_need, 0, 4, c->stream));
   }
   c->launches++;
   if (c->pme_f32)
