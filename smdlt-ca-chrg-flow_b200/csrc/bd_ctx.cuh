@@ -215,7 +215,8 @@ struct bd_ctx {
   void *rl_pos;      // lab-frame positions of the last preparation (double4)
   void *rl_spos;     // the same in real-space cell order, bead index in w
   void *pme_vpk;     // a product's input values, packed pairs side by side per bead and component
-  void *rl_w;        // per entry the four tensors (t1, w), FP64 or FP32
+  void *rl_w;        // per entry the four pair tensors: (t1, w), or (t1, t2 / r^2)
+  bd::Lat rl_lat;    // lattice of the last preparation
   // spreading by grid columns and interpolation (bd_mesh.cu): up to two column
   // layouts (packed pairs per warp), beads per column and base index, starts
   int mesh_ng[2];

@@ -315,7 +315,7 @@ int pme_prepare(bd_ctx* c, const Lat& l) {
         cell, K, alpha, c->pme_bsq, (double*)c->pme_infl, c->pme_soff + 3);
   k_pme_soff_fin<<<1, 256, 0, c->stream>>>(c->pme_soff + 3, c->pme_nblk, c->pme_soff);
   if ((s = launch_ok(c)) != BD_OK) return s;
-  if ((s = real_prepare(c, cell, cr, sr, alpha_ref)) != BD_OK) return s;
+  if ((s = real_prepare(c, l, cell, cr, sr, alpha_ref)) != BD_OK) return s;
   double a = alpha;
   c->pme_self = 1.0 - 6.0 / sqrt(M_PI) * a + 40.0 / (3.0 * sqrt(M_PI)) * a * a * a;
   c->Dtr[0] = c->Dtr[1] = c->Dtr[2] = c->pme_self;

@@ -3,12 +3,21 @@
 // No counterpart in the reference (see bd_pme.cu).  The beads are taken four
 // at a time (consecutive indices: neighbours along a chain, whose cutoff
 // spheres nearly coincide).  A group's row lists every bead within the cutoff
-// of one of its four, and per entry the four pair tensors T = t1 I + s w w^T,
-// w = sqrt(|t2| / r^2) d, the sign s of t2 in the lowest mantissa bit of t1
-// (zero where a pair is beyond the cutoff).  The product then reads a
-// neighbour's input values once for four pairs, and positions and minimum
-// images not at all.  The beads of a cell are in increasing index, so a row's
-// order, and with it a product's rounding, is the same in every build.
+// of one of its four, and per entry the four pair tensors (zero where a pair is
+// beyond the cutoff), so that a product reads a neighbour once for four pairs.
+// Two forms:
+//  * whole tensors, in FP32 contexts with noise blocks: T = t1 I + s w w^T, w =
+//    sqrt(|t2| / r^2) d, the sign s of t2 in the lowest mantissa bit of t1.  64
+//    bytes an entry; positions and minimum images are not needed, and up to five
+//    pairs of right-hand sides share the reading (k_real_apply, FP32 sums);
+//  * t1 and t2 / r^2 in FP64 contexts and in FP32 ones with one right-hand side:
+//    64 and 32 bytes an entry, the displacements from the frozen FP64 positions,
+//    FP64 inputs and sums (k_real_sum).  Whole FP64 tensors are twice the bytes
+//    and give up a bit of t1: a single FP64 product of 50 000 beads (cutoff 14.5)
+//    took 580 us with them, 392 so; of 8000 (12.1) 143 and 114; five pairs of 8000
+//    333 and 331.
+// The beads of a cell are in increasing index, so a row's order, and with it a
+// product's rounding, is the same in every build.
 #include <math.h>
 
 #include <algorithm>
@@ -144,25 +153,38 @@ __global__ void __launch_bounds__(256) k_rl_order(const int* __restrict__ cell_s
 }
 
 // t1 with the sign of t2 in its lowest mantissa bit.
-__device__ __forceinline__ float with_sign(float, double t1, double t2) {
+__device__ __forceinline__ float with_sign(double t1, double t2) {
   return __uint_as_float((__float_as_uint((float)t1) & ~1u) | (t2 < 0.0 ? 1u : 0u));
-}
-__device__ __forceinline__ double with_sign(double, double t1, double t2) {
-  return __longlong_as_double((__double_as_longlong(t1) & ~1ll) | (t2 < 0.0 ? 1ll : 0ll));
 }
 
 // The four tensors of an entry: 16 numbers, for beads (0, 1) and (2, 3) the
 // pairs of t1, w_x, w_y, w_z, so that the product takes two beads per
 // instruction.
-template <typename R>
-__device__ __forceinline__ void store_tensor(R* entry, int b, double t1, double t2, double sw,
+__device__ __forceinline__ void store_tensor(float* entry, int b, double t1, double t2, double sw,
                                              double dx, double dy, double dz) {
-  R* o = entry + 8 * (b >> 1) + (b & 1);
-  o[0] = with_sign((R)0, t1, t2);
-  o[2] = (R)(sw * dx);
-  o[4] = (R)(sw * dy);
-  o[6] = (R)(sw * dz);
+  float* o = entry + 8 * (b >> 1) + (b & 1);
+  o[0] = with_sign(t1, t2);
+  o[2] = (float)(sw * dx);
+  o[4] = (float)(sw * dy);
+  o[6] = (float)(sw * dz);
 }
+
+// Place of bead b's pair in entry k of a row of (t1, t2 / r^2): 32 entries of
+// each bead side by side.
+__device__ __forceinline__ size_t pair_at(int k, int b) {
+  return ((size_t)(k >> 5) * kGroup + b) * 32 + (k & 31);
+}
+
+template <typename R>
+struct Real2;
+template <>
+struct Real2<float> {
+  using T = float2;
+};
+template <>
+struct Real2<double> {
+  using T = double2;
+};
 
 // Neighbour indices of the groups' rows, cap entries a row, in no order.  One
 // warp per group.  For each of its beads the at most 27 neighbour cells form
@@ -252,42 +274,55 @@ __global__ void __launch_bounds__(128, 4)
   }
 }
 
-// The four tensors of every entry, a warp per group, and each bead's number of
-// pairs against an explicit cap.  Entry k at rw[16 (group cap + k)].  32 entries
-// at a time are formed in shared memory and written side by side (from the
-// lanes, 64 bytes apart, every sector would be written eight times).
-// Overlapping pairs (r < 2), whose terms cost three times as much, are queued
-// and formed 32 at a time.  Bound by the FP64 pipe (erfc, exp): 0.62 ms at
-// 50 000 beads, cutoff 14.5; 0.76 with each lane writing its own entry.
-template <typename R>
+// The pair tensors of every entry, a warp per group, and each bead's number of
+// pairs against an explicit cap.  WHOLE: 16 numbers an entry at rw[16 (group cap
+// + k)]; 32 entries at a time are formed in shared memory and written side by
+// side (from the lanes, 64 bytes apart, every sector would be written eight
+// times).  Else (t1, t2 / r^2) at pair_at.  Overlapping pairs (r < 2), whose
+// terms cost three times as much, are queued and formed 32 at a time.  Bound by
+// the FP64 pipe (erfc, exp): 0.62 ms at 50 000 beads, cutoff 14.5; 0.76 with each
+// lane writing its own entry.
+template <typename R, bool WHOLE>
 __global__ void __launch_bounds__(128, 4)
     k_rl_tensors(Cell cell, const double4* __restrict__ pos, int N, int ngroup,
                  const int* __restrict__ cnt, const int* __restrict__ rows, int cap, double rc2,
-                 double alpha, double alpha_ref, int bead_cap, R* rw, int* err) {
+                 double alpha, double alpha_ref, int bead_cap, void* rw, int* err) {
+  using T2 = typename Real2<R>::T;
   __shared__ int c_queue[4][160];  // 4 k + b of overlapping pairs
-  __shared__ alignas(16) R s_entry[4][32 * 20];  // entries 20 apart: fewer bank conflicts
+  // entries 20 numbers apart: fewer bank conflicts
+  __shared__ alignas(16) float s_entry[WHOLE ? 4 : 1][WHOLE ? 32 * 20 : 4];
   const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = blockIdx.x * 4 + wl;
   if (grp >= ngroup) return;
   const int i0 = kGroup * grp, nb = min(kGroup, N - i0), n = cnt[grp];
   const Image image(cell);
   const int* row = rows + (size_t)grp * cap;
-  R* out = rw + 16 * (size_t)grp * cap;
+  float* whole = (float*)rw + 16 * (size_t)grp * cap;
+  T2* out = (T2*)rw + kGroup * (size_t)grp * cap;
   int* queue = c_queue[wl];
   int nq = 0, count[kGroup] = {0, 0, 0, 0};
-  auto form = [&](auto overlap, R* entry, int b, double rr, double dx, double dy, double dz) {
+  // pair (k, b): to entry (WHOLE) or to its place
+  auto form = [&](auto overlap, float* entry, int k, int b, double rr, double dx, double dy,
+                  double dz) {
     constexpr bool OV = decltype(overlap)::value;
     const double r = sqrt(rr), ir = 1.0 / r, irr = ir * ir;
     double t1, t2;
     pair_terms<OV>(alpha, alpha_ref, rr, r, ir, irr, t1, t2);
-    store_tensor(entry, b, t1, t2, sqrt(fabs(t2)) * ir, dx, dy, dz);
+    if constexpr (WHOLE) {
+      store_tensor(entry, b, t1, t2, sqrt(fabs(t2)) * ir, dx, dy, dz);
+    } else {
+      T2 t;
+      t.x = (R)t1;
+      t.y = (R)(t2 * irr);
+      out[pair_at(k, b)] = t;
+    }
   };
   auto flush = [&](int m) {
     if (lane < m) {
       const int k = queue[nq - m + lane] >> 2, b = queue[nq - m + lane] & 3;
       double dx, dy, dz;
       const double rr = image(pos[row[k]], pos[i0 + b], dx, dy, dz);
-      form(std::integral_constant<bool, true>(), out + 16 * (size_t)k, b, rr, dx, dy, dz);
+      form(std::integral_constant<bool, true>(), whole + 16 * (size_t)k, k, b, rr, dx, dy, dz);
     }
     nq -= m;
     __syncwarp();
@@ -295,7 +330,7 @@ __global__ void __launch_bounds__(128, 4)
 #pragma unroll 1
   for (int k0 = 0; k0 < n; k0 += 32) {
     const int k = k0 + lane, m = min(32, n - k0);
-    R* entry = s_entry[wl] + 20 * lane;
+    float* entry = s_entry[WHOLE ? wl : 0] + (WHOLE ? 20 * lane : 0);
     const int j = k < n ? row[k] : 0;
     const double4 pj = pos[j];
 #pragma unroll 1
@@ -306,20 +341,25 @@ __global__ void __launch_bounds__(128, 4)
       if (k < n && b < nb && j != i0 + b && !(rr >= rc2)) {
         count[0] += b == 0, count[1] += b == 1, count[2] += b == 2, count[3] += b == 3;
         near = rr < 4.0;
-        if (!near) form(std::integral_constant<bool, false>(), entry, b, rr, dx, dy, dz);
-      } else {
+        if (!near) form(std::integral_constant<bool, false>(), entry, k, b, rr, dx, dy, dz);
+      } else if constexpr (WHOLE) {
         store_tensor(entry, b, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0);
+      } else if (k < n) {
+        T2 t;
+        t.x = t.y = (R)0;
+        out[pair_at(k, b)] = t;
       }
       const unsigned hit = __ballot_sync(0xffffffffu, near);
       if (near) queue[nq + __popc(hit & ((1u << lane) - 1u))] = 4 * k + b;
       nq += __popc(hit);
     }
     __syncwarp();
-    constexpr int WORDS = (int)sizeof(R);  // 16-byte words an entry
-    float4* to = (float4*)(out + 16 * (size_t)k0);
-    for (int e = lane; e < m * WORDS; e += 32)
-      to[e] = ((const float4*)(s_entry[wl] + 20 * (e / WORDS)))[e % WORDS];
-    __syncwarp();
+    if constexpr (WHOLE) {
+      float4* to = (float4*)(whole + 16 * (size_t)k0);
+      for (int e = lane; e < 4 * m; e += 32)
+        to[e] = ((const float4*)(s_entry[wl] + 20 * (e / 4)))[e % 4];
+      __syncwarp();
+    }
     while (nq >= 32) flush(32);
   }
   if (nq > 0) flush(nq);
@@ -336,7 +376,6 @@ __global__ void __launch_bounds__(128, 4)
 
 // Two beads at a time: the beads' numbers in the halves, one input value for both.
 __device__ __forceinline__ float2 twice(float x) { return make_float2(x, x); }
-__device__ __forceinline__ double twice(double x) { return x; }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   unsigned long long d, x = *reinterpret_cast<unsigned long long*>(&a),
                         y = *reinterpret_cast<unsigned long long*>(&b);
@@ -350,35 +389,11 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(x), "l"(y), "l"(z));
   return *reinterpret_cast<float2*>(&d);
 }
-__device__ __forceinline__ double2 mul2(double2 a, double b) {
-  return make_double2(a.x * b, a.y * b);
-}
-__device__ __forceinline__ double2 fma2(double2 a, double b, double2 c) {
-  return make_double2(fma(a.x, b, c.x), fma(a.y, b, c.y));
-}
-__device__ __forceinline__ double2 fma2(double2 a, double2 b, double2 c) {
-  return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
-}
 // negative where the bead's t1 carries a negative sign
 __device__ __forceinline__ float2 signed_by(float2 t1, float2 a) {
   return make_float2(__uint_as_float(__float_as_uint(a.x) ^ (__float_as_uint(t1.x) << 31)),
                      __uint_as_float(__float_as_uint(a.y) ^ (__float_as_uint(t1.y) << 31)));
 }
-__device__ __forceinline__ double2 signed_by(double2 t1, double2 a) {
-  return make_double2(__double_as_longlong(t1.x) & 1 ? -a.x : a.x,
-                      __double_as_longlong(t1.y) & 1 ? -a.y : a.y);
-}
-
-template <typename R>
-struct Real2;
-template <>
-struct Real2<float> {
-  using T = float2;
-};
-template <>
-struct Real2<double> {
-  using T = double2;
-};
 
 __device__ __forceinline__ void copy_async(void* to, const void* from, int bytes16) {
   unsigned d = (unsigned)__cvta_generic_to_shared(to);
@@ -406,26 +421,25 @@ __device__ __forceinline__ void copy_wait() {
 // (a warp per bead, every neighbour's values read once per bead: 435); at 8000
 // beads, cutoff 12.1, 38 us by one warp a group against 50.
 // SPLIT warps share a group's row.
-template <int NP, typename R>
+template <int NP>
 struct Stage {
   static constexpr int S = 32 / NP, ITS = 32 / S, CH = S * ITS;  // entries a piece
-  alignas(16) R w[16 * CH];
+  alignas(16) float w[16 * CH];
   int j[(CH + 3) / 4 * 4];
 };
 
-template <int NP, int SPLIT, typename R>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2)
+template <int NP, int SPLIT>
+__global__ void __launch_bounds__(128, 4)
     k_real_apply(const int* __restrict__ cnt, const int* __restrict__ rows,
-                 const R* __restrict__ rw, int cap,
-                 const typename Real2<R>::T* __restrict__ vpk, int np, int p0, int N, int ngroup,
-                 Finish fin) {
-  using V = typename Real2<R>::T;
-  using P = Stage<NP, R>;
-  constexpr int S = P::S, ITS = P::ITS, CH = P::CH, DEEP = sizeof(R) == 4 ? 3 : 2, W = 25;
-  constexpr int FOLD = 16 / ITS, PER = (int)sizeof(R);  // 16-byte words an entry
+                 const float* __restrict__ rw, int cap, const float2* __restrict__ vpk, int np,
+                 int p0, int N, int ngroup, Finish fin) {
+  using V = float2;
+  using P = Stage<NP>;
+  constexpr int S = P::S, ITS = P::ITS, CH = P::CH, DEEP = 3, W = 25;
+  constexpr int FOLD = 16 / ITS, PER = 4;  // 16-byte words an entry
   union Shared {
     P stage[4][DEEP];
-    R sum[4][32 * W];
+    float sum[4][32 * W];
   };
   __shared__ __align__(16) unsigned char raw[sizeof(Shared)];
   Shared& sh = *reinterpret_cast<Shared*>(raw);
@@ -440,7 +454,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2)
   if (grp < ngroup) {
     const int n = cnt[grp];
     const int* row = rows + (size_t)grp * cap;
-    const R* rq = rw + 16 * (size_t)grp * cap;
+    const float* rq = rw + 16 * (size_t)grp * cap;
     const V* vp = vpk + p0 + pr;
     const size_t plane = (size_t)N * np;
     P* st = sh.stage[wl];
@@ -477,16 +491,10 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2)
         if (slot < S && k < m) {
 #pragma unroll
           for (int b = 0; b < 2; b++) {
-            V t1, w0, w1, w2;
-            if constexpr (sizeof(R) == 4) {
-              const float4 u = *(const float4*)(p.w + 16 * k + 8 * b),
-                           v = *(const float4*)(p.w + 16 * k + 8 * b + 4);
-              t1 = make_float2(u.x, u.y), w0 = make_float2(u.z, u.w);
-              w1 = make_float2(v.x, v.y), w2 = make_float2(v.z, v.w);
-            } else {
-              const V* q = (const V*)(p.w + 16 * k + 8 * b);
-              t1 = q[0], w0 = q[1], w1 = q[2], w2 = q[3];
-            }
+            const float4 u = *(const float4*)(p.w + 16 * k + 8 * b),
+                         v = *(const float4*)(p.w + 16 * k + 8 * b + 4);
+            const V t1 = make_float2(u.x, u.y), w0 = make_float2(u.z, u.w),
+                    w1 = make_float2(v.x, v.y), w2 = make_float2(v.z, v.w);
 #pragma unroll
             for (int h = 0; h < 2; h++) {
               const auto y0 = twice(h ? x[t][0].y : x[t][0].x),
@@ -517,7 +525,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2)
     copy_wait<0>();
   }
   __syncthreads();  // the stages' memory holds the sums from here on
-  R* o = sh.sum[wl] + lane * W;
+  float* o = sh.sum[wl] + lane * W;
 #pragma unroll
   for (int b = 0; b < 2; b++)
 #pragma unroll
@@ -538,20 +546,212 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 2)
   }
 }
 
-template <int NP, typename R>
+// ---------------------------------------------------------------------------
+
+// The real-space sums from rows of (t1, t2 / r^2), FP64 throughout: NP packed
+// pairs (p0 on), or with ONE a single right-hand side read where it lies.  One
+// warp (SPLIT: that many) per group of four beads, 32 entries of the row at a
+// time: the lanes form an entry's four minimum-image displacements each; for a
+// single vector or pair a lane then serves its own entry, else the displacements
+// go through shared memory and a lane serves one pair and every S-th entry.  The
+// row streams through shared memory three pieces deep and the neighbours'
+// positions (and values, NP = 1) are read a piece ahead.
+template <typename R>
+struct PairStage {
+  alignas(16) typename Real2<R>::T t[kGroup][32];
+  int j[32];
+};
+
+template <int NP, bool ONE, int SPLIT, typename R>
+__global__ void __launch_bounds__(128, ONE ? 4 : 2)
+    k_real_sum(Cell cell, const double4* __restrict__ pos, const int* __restrict__ cnt,
+               const int* __restrict__ rows, const typename Real2<R>::T* __restrict__ rt, int cap,
+               VecIn v, const double2* __restrict__ vpk, int np, int p0, int N, int ngroup,
+               Finish fin) {
+  using T2 = typename Real2<R>::T;
+  using P = PairStage<R>;
+  constexpr int S = 32 / NP, ITS = (32 + S - 1) / S, DEEP = 3, NS = ONE ? 3 : 6;
+  constexpr int W = kGroup * NS + 1, WORDS = kGroup * 32 * (int)sizeof(T2) / 16;
+  struct Streams {
+    P stage[4][DEEP];
+    double d[NP > 1 ? 4 : 1][3 * kGroup][32];  // displacements of a piece
+  };
+  union Shared {
+    Streams in;
+    double sum[4][32 * W];
+  };
+  __shared__ __align__(16) unsigned char raw[sizeof(Shared)];
+  Shared& sh = *reinterpret_cast<Shared*>(raw);
+  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = blockIdx.x * (4 / SPLIT) + wl / SPLIT, piece0 = wl % SPLIT;
+  const int slot = lane / NP, pr = lane % NP;  // slot S and up: idle lanes
+  const int i0 = kGroup * grp;
+  double sum[kGroup][NS];
+#pragma unroll
+  for (int b = 0; b < kGroup; b++)
+#pragma unroll
+    for (int e = 0; e < NS; e++) sum[b][e] = 0.0;
+  if (grp < ngroup) {
+    const int n = cnt[grp];
+    const int* row = rows + (size_t)grp * cap;
+    const T2* rq = rt + kGroup * (size_t)grp * cap;
+    const size_t plane = (size_t)N * np;
+    const Image image(cell);
+    double4 pb[kGroup];
+#pragma unroll
+    for (int b = 0; b < kGroup; b++) pb[b] = pos[min(i0 + b, N - 1)];
+    P* st = sh.in.stage[wl];
+    auto issue = [&](int piece, int buf) {
+      const int m = min(32, n - 32 * piece);
+      if (m > 0) {
+        const char* from = (const char*)(rq + (size_t)kGroup * 32 * piece);
+        for (int e = lane; e < WORDS; e += 32)
+          copy_async((char*)st[buf].t + 16 * e, from + 16 * e, 1);
+        if (lane < m) copy_async(st[buf].j + lane, row + 32 * piece + lane, 0);
+      }
+      copy_commit();
+    };
+    // a piece's gathers for this lane's entry
+    struct Near {
+      double4 p;
+      double2 x[3];
+    } cur, next;
+    auto gather = [&](int piece, int buf, Near& g) {
+      const int j = 32 * piece + lane < n ? st[buf].j[lane] : i0;
+      g.p = pos[j];
+      if constexpr (ONE) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) g.x[c].x = v.p[c][(size_t)j * v.stride];
+      } else if constexpr (NP == 1) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) g.x[c] = __ldg(vpk + p0 + (size_t)j * np + c * plane);
+      }
+    };
+    auto add = [&](int b, const T2& t, double dx, double dy, double dz, const double2* x) {
+      const double t1 = t.x, t2 = t.y;
+      double* o = sum[b];
+      const double q = t2 * (dx * x[0].x + dy * x[1].x + dz * x[2].x);
+      o[0] += t1 * x[0].x + q * dx;
+      o[1] += t1 * x[1].x + q * dy;
+      o[2] += t1 * x[2].x + q * dz;
+      if constexpr (!ONE) {
+        const double u = t2 * (dx * x[0].y + dy * x[1].y + dz * x[2].y);
+        o[3] += t1 * x[0].y + u * dx;
+        o[4] += t1 * x[1].y + u * dy;
+        o[5] += t1 * x[2].y + u * dz;
+      }
+    };
+#pragma unroll
+    for (int d = 0; d < DEEP; d++) issue(piece0 + d * SPLIT, d);
+    copy_wait<DEEP - 1>();
+    __syncwarp();
+    gather(piece0, 0, cur);
+    int buf = 0;
+#pragma unroll 1
+    for (int piece = piece0; 32 * piece < n; piece += SPLIT) {
+      copy_wait<DEEP - 2>();  // this piece and the next
+      __syncwarp();
+      gather(piece + SPLIT, buf + 1 == DEEP ? 0 : buf + 1, next);
+      const int m = min(32, n - 32 * piece);
+      const P& p = st[buf];
+      if constexpr (NP == 1) {
+        if (lane < m) {
+#pragma unroll
+          for (int b = 0; b < kGroup; b++) {
+            double dx, dy, dz;
+            image(cur.p, pb[b], dx, dy, dz);
+            add(b, p.t[b][lane], dx, dy, dz, cur.x);
+          }
+        }
+      } else {
+        double(*d)[32] = sh.in.d[wl];
+#pragma unroll
+        for (int b = 0; b < kGroup; b++) {
+          double dx, dy, dz;
+          image(cur.p, pb[b], dx, dy, dz);
+          d[3 * b][lane] = dx;
+          d[3 * b + 1][lane] = dy;
+          d[3 * b + 2][lane] = dz;
+        }
+        double2 x[ITS][3];
+#pragma unroll
+        for (int t = 0; t < ITS; t++) {
+          const int k = t * S + slot;
+          const double2* vj = vpk + p0 + pr + (size_t)(slot < S && k < m ? p.j[k] : i0) * np;
+#pragma unroll
+          for (int c = 0; c < 3; c++) x[t][c] = __ldg(vj + c * plane);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int t = 0; t < ITS; t++) {
+          const int k = t * S + slot;
+          if (slot < S && k < m) {
+#pragma unroll
+            for (int b = 0; b < kGroup; b++)
+              add(b, p.t[b][k], d[3 * b][k], d[3 * b + 1][k], d[3 * b + 2][k], x[t]);
+          }
+        }
+      }
+      __syncwarp();  // the piece has been read
+      issue(piece + DEEP * SPLIT, buf);
+      buf = buf + 1 == DEEP ? 0 : buf + 1;
+      cur = next;
+    }
+    copy_wait<0>();
+  }
+  __syncthreads();  // the streams' memory holds the sums from here on
+  double* o = sh.sum[wl] + lane * W;
+#pragma unroll
+  for (int b = 0; b < kGroup; b++)
+#pragma unroll
+    for (int e = 0; e < NS; e++) o[NS * b + e] = sum[b][e];
+  __syncthreads();
+  if (grp >= ngroup) return;
+  const int w0 = wl / SPLIT * SPLIT;
+  for (int e = lane + 32 * piece0; e < NS * kGroup * NP; e += 32 * SPLIT) {
+    const int b = e / (NS * NP), p = e / NS % NP, i = i0 + b;
+    if (i >= N) break;
+    double s = 0;
+    for (int w = w0; w < w0 + SPLIT; w++)
+      for (int u = 0; u < S; u++) s += sh.sum[w][(u * NP + p) * W + NS * b + e % NS];
+    fin.write(s, p0 + p, e % NS, i);
+  }
+}
+
+// Warps a group of a row of (t1, t2 / r^2).
+int few_warps(int ng) { return ng < 148 * 12 ? 4 : ng < 148 * 40 ? 2 : 1; }
+
+template <int NP, bool ONE, typename R>
+void launch_sum(bd_ctx* c, int np, int p0, const Finish& fin) {
+  const int ng = (c->N + kGroup - 1) / kGroup;
+  const Cell cell = make_cell(c->rl_lat);
+#define SUM(SPLIT_)                                                                         \
+  k_real_sum<NP, ONE, SPLIT_, R><<<nblk(ng, 4 / SPLIT_), 128, 0, c->stream>>>(              \
+      cell, (const double4*)c->rl_pos, c->rl_cnt, c->rl_rows,                               \
+      (const typename Real2<R>::T*)c->rl_w, c->rl_cap, fin.v, (const double2*)c->pme_vpk, np, \
+      p0, c->N, ng, fin)
+  switch (few_warps(ng)) {
+    case 4: SUM(4); break;
+    case 2: SUM(2); break;
+    default: SUM(1);
+  }
+#undef SUM
+}
+
+template <int NP>
 void launch_apply(bd_ctx* c, int np, int p0, const Finish& fin) {
   const int ng = (c->N + kGroup - 1) / kGroup;
 #define REAL(SPLIT_)                                                                      \
-  k_real_apply<NP, SPLIT_, R><<<nblk(ng, 4 / SPLIT_), 128, 0, c->stream>>>(               \
-      c->rl_cnt, c->rl_rows, (const R*)c->rl_w, c->rl_cap,                                \
-      (const typename Real2<R>::T*)c->pme_vpk, np, p0, c->N, ng, fin)
+  k_real_apply<NP, SPLIT_><<<nblk(ng, 4 / SPLIT_), 128, 0, c->stream>>>(                  \
+      c->rl_cnt, c->rl_rows, (const float*)c->rl_w, c->rl_cap, (const float2*)c->pme_vpk, \
+      np, p0, c->N, ng, fin)
   // More warps a group fill the chip sooner, fewer start fewer pieces.  By four,
   // two and one, five pairs FP32: 500 beads 6.1, 8.0, 12.6 us, 8000 41.8, 46.5, 63.7,
   // 16 000 70, 74, 79; FP64 8000 85, 90, 107, 16 000 151, 147, 160; one pair FP32
   // 8000 24.0, 20.9, 24.4, 16 000 45.5, 35.2, 34.5.  At 50 000 beads of a run's
   // chains five pairs took 268 by four and 257 by one, one pair 118 by two and 114
   // by one.
-  const int four = NP < 5 ? 148 * 12 : sizeof(R) == 8 ? 148 * 20 : 148 * 40;
+  const int four = NP < 5 ? 148 * 12 : 148 * 40;
   if (ng >= 148 * 40)
     REAL(1);
   else if (ng < four)
@@ -561,20 +761,23 @@ void launch_apply(bd_ctx* c, int np, int p0, const Finish& fin) {
 #undef REAL
 }
 
-template <typename R>
-int apply_t(bd_ctx* c, int np, const Finish& fin) {
+// In passes of up to five pairs.
+template <class F>
+void by_fives(bd_ctx* c, int np, F launch) {
   for (int p0 = 0; p0 < np; p0 += 5) {
     c->launches++;
     switch (std::min(5, np - p0)) {
-      case 1: launch_apply<1, R>(c, np, p0, fin); break;
-      case 2: launch_apply<2, R>(c, np, p0, fin); break;
-      case 3: launch_apply<3, R>(c, np, p0, fin); break;
-      case 4: launch_apply<4, R>(c, np, p0, fin); break;
-      default: launch_apply<5, R>(c, np, p0, fin);
+      case 1: launch(std::integral_constant<int, 1>(), p0); break;
+      case 2: launch(std::integral_constant<int, 2>(), p0); break;
+      case 3: launch(std::integral_constant<int, 3>(), p0); break;
+      case 4: launch(std::integral_constant<int, 4>(), p0); break;
+      default: launch(std::integral_constant<int, 5>(), p0);
     }
   }
-  return launch_ok(c);
 }
+
+// Rows hold whole tensors (FP32 contexts with noise blocks) or (t1, t2 / r^2).
+bool whole_tensors(const bd_ctx* c) { return c->pme_f32 && c->nbk > 1; }
 
 }  // namespace
 
@@ -583,32 +786,28 @@ namespace bd {
 // Rows of cap entries for every group; without memory for them there are none
 // (rl_rows null) and the mobility is not built.
 static int rows_alloc(bd_ctx* c, int cap) {
-  size_t ng = ((size_t)c->N + kGroup - 1) / kGroup, es = c->pme_f32 ? 4 : 8;
-  size_t old = (size_t)c->rl_cap, each = 4 + 4 * es * kGroup;
+  size_t ng = ((size_t)c->N + kGroup - 1) / kGroup, old = (size_t)c->rl_cap;
+  size_t tensor = whole_tensors(c) ? 16 : c->pme_f32 ? 8 : 16, each = 4 + tensor * kGroup;
+  cap = (cap + 31) / 32 * 32;
   if (c->rl_rows) {
     CU(cudaStreamSynchronize(c->stream));
     free_all({&c->rl_rows, &c->rl_w});
     c->bytes -= each * ng * old;
   }
   c->rl_cap = 0;
-  int s = alloc_all(c, {{&c->rl_rows, 4 * ng * cap}, {&c->rl_w, 4 * es * kGroup * ng * cap}});
+  int s = alloc_all(c, {{&c->rl_rows, 4 * ng * cap}, {&c->rl_w, tensor * kGroup * ng * cap}});
   if (s == BD_OK) c->rl_cap = cap;
   return s;
 }
 
-// Rows before any have overflowed: an explicit cap per bead bounds a group's
-// row by four times that; the default is 2.5 times the mean number of beads
-// within the cutoff at the system's density, at least 512 (rows that overflow
-// it are grown); no row is longer than N.
+// Entries of a row before any have overflowed: an explicit cap per bead, or 2.5
+// times the mean number of beads within the cutoff at the system's density, at
+// least 512.  Rows that overflow it are grown; no row is longer than N, nor with
+// an explicit cap than four beads' pairs.
 static int first_cap(const bd_ctx* c) {
-  long cap;
-  if (c->p.pme_max_pairs > 0) {
-    cap = (long)kGroup * c->p.pme_max_pairs;
-  } else {
-    double mean = 4.0 / 3.0 * M_PI * c->pme_rc * c->pme_rc * c->pme_rc * c->N / c->boxvol;
-    cap = std::max(512, ((int)ceil(2.5 * mean) + 31) / 32 * 32);
-  }
-  return (int)std::min(cap, (long)std::max(c->N, 1));
+  const double mean = 4.0 / 3.0 * M_PI * c->pme_rc * c->pme_rc * c->pme_rc * c->N / c->boxvol;
+  const int cap = c->p.pme_max_pairs > 0 ? c->p.pme_max_pairs : std::max(512, (int)ceil(2.5 * mean));
+  return std::min(cap, std::max(c->N, 1));
 }
 
 int real_alloc(bd_ctx* c) {
@@ -636,7 +835,8 @@ void real_free(bd_ctx* c) {
 
 // The groups' rows for the positions in rl_pos (lab frame; rx, ry, rz and the
 // rotation (cr, sr) give the same); alpha_ref is calcHI's split parameter.
-int real_prepare(bd_ctx* c, const Cell& cell, double cr, double sr, double alpha_ref) {
+int real_prepare(bd_ctx* c, const Lat& l, const Cell& cell, double cr, double sr,
+                 double alpha_ref) {
   int s, N = c->N;
   double rc = c->pme_rc, alpha = c->pme_alpha;
   if (!c->rl_rows && (s = rows_alloc(c, first_cap(c))) != BD_OK) return s;
@@ -673,38 +873,56 @@ int real_prepare(bd_ctx* c, const Cell& cell, double cr, double sr, double alpha
   k_rl_order<<<ncell, 256, 0, c->stream>>>(c->rl_cell_start, c->rl_beads,
                                            (const double4*)c->rl_pos, (double4*)c->rl_spos);
   if ((s = launch_ok(c)) != BD_OK) return s;
-  // the rows; with the default cap (no pme_max_pairs), rows that
-  // overflow it are grown to 1.25 times the longest row and built again
-  int* need = c->p.pme_max_pairs > 0 ? nullptr : c->rl_need;
+  // the rows; those that overflow are grown to 1.25 times the longest one and
+  // built again, an error where they must not be longer
   const int ng = (N + kGroup - 1) / kGroup;
-  for (int pass = 0; pass < 2; pass++) {
+  const int most = c->p.pme_max_pairs > 0
+                       ? (int)std::min((long)N, (long)kGroup * c->p.pme_max_pairs)
+                       : N;
+  for (bool grow = c->rl_cap < most;; grow = false) {
     c->launches++;
     k_rl_find<<<nblk(ng, 4), 128, 0, c->stream>>>(
         cell, g, (const double4*)c->rl_pos, N, ng, c->rl_cell_start, (const double4*)c->rl_spos,
-        rc * rc, c->rl_cap, c->rl_cnt, c->rl_rows, need, c->err);
-    if (!need) break;
+        rc * rc, c->rl_cap, c->rl_cnt, c->rl_rows, grow ? c->rl_need : nullptr, c->err);
+    if (!grow) break;
     int longest = 0;
-    CU(cudaMemcpyAsync(&longest, need, 4, cudaMemcpyDeviceToHost, c->stream));
+    CU(cudaMemcpyAsync(&longest, c->rl_need, 4, cudaMemcpyDeviceToHost, c->stream));
     if ((s = check(c)) != BD_OK) return s;
     if (longest <= c->rl_cap) break;
     CU(cudaMemsetAsync(c->rl_need, 0, 4, c->stream));
-    if ((s = rows_alloc(c, std::min(N, ((int)ceil(1.25 * longest) + 31) / 32 * 32))) != BD_OK)
-      return s;
+    if ((s = rows_alloc(c, std::min(most, (int)ceil(1.25 * longest)))) != BD_OK) return s;
   }
   c->launches++;
-  if (c->pme_f32)
-    k_rl_tensors<float><<<nblk(ng, 4), 128, 0, c->stream>>>(
-        cell, (const double4*)c->rl_pos, N, ng, c->rl_cnt, c->rl_rows, c->rl_cap, rc * rc, alpha,
-        alpha_ref, c->p.pme_max_pairs, (float*)c->rl_w, c->err);
+#define TENSORS(...)                                                                          \
+  k_rl_tensors<__VA_ARGS__><<<nblk(ng, 4), 128, 0, c->stream>>>(                              \
+      cell, (const double4*)c->rl_pos, N, ng, c->rl_cnt, c->rl_rows, c->rl_cap, rc * rc, alpha, \
+      alpha_ref, c->p.pme_max_pairs, c->rl_w, c->err)
+  if (whole_tensors(c))
+    TENSORS(float, true);
+  else if (c->pme_f32)
+    TENSORS(float, false);
   else
-    k_rl_tensors<double><<<nblk(ng, 4), 128, 0, c->stream>>>(
-        cell, (const double4*)c->rl_pos, N, ng, c->rl_cnt, c->rl_rows, c->rl_cap, rc * rc, alpha,
-        alpha_ref, c->p.pme_max_pairs, (double*)c->rl_w, c->err);
+    TENSORS(double, false);
+#undef TENSORS
+  c->rl_lat = l;
   return launch_ok(c);
 }
 
 int real_apply(bd_ctx* c, int np, const Finish& fin) {
-  return c->pme_f32 ? apply_t<float>(c, np, fin) : apply_t<double>(c, np, fin);
+  if (whole_tensors(c)) {
+    by_fives(c, np, [&](auto n, int p0) { launch_apply<decltype(n)::value>(c, np, p0, fin); });
+  } else if (fin.k == 1) {
+    c->launches++;
+    if (c->pme_f32)
+      launch_sum<1, true, float>(c, np, 0, fin);
+    else
+      launch_sum<1, true, double>(c, np, 0, fin);
+  } else {  // FP64: FP32 contexts without noise blocks have one right-hand side
+    by_fives(c, np, [&](auto n, int p0) {
+      launch_sum<decltype(n)::value, false, double>(c, np, p0, fin);
+    });
+  }
+  return launch_ok(c);
 }
 
 }  // namespace bd

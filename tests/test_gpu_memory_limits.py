@@ -3,6 +3,8 @@ error status, leaves the context without a mobility (products are refused, not
 run on missing buffers), fails the same way when it is called again, and works
 once there is memory.  The memory is filled through torch; 4000 beads within a
 few radii of each other need rows of 4000 entries, 140 MB and more."""
+import gc
+
 import numpy as np
 import pytest
 import torch
@@ -38,6 +40,8 @@ class Filled:
         self.left = left
 
     def __enter__(self):
+        gc.collect()  # contexts that earlier tests left behind
+        gc.disable()
         torch.cuda.synchronize()
         self.held = []
         step = 1 << 34
@@ -54,6 +58,7 @@ class Filled:
     def __exit__(self, *a):
         self.held.clear()
         torch.cuda.empty_cache()
+        gc.enable()
 
 
 def _status(call):
