@@ -130,10 +130,10 @@ typedef struct {
    * B-spline order (even, 4..8; 0 -> 8), real-space cutoff (0 -> the smaller
    * of 10 and 0.43 L; at most 0.43 L), split parameter (0 -> 4 / cutoff) and the cap on
    * real-space pairs per bead (0 -> 2.5 times the mean number of beads within
-   * the cutoff, at least 512; four consecutive beads in cell order share a row,
-   * and rows that overflow it are grown to 1.25 times the longest one at the
-   * mobility build; an explicit cap that a bead's pairs overflow is
-   * BD_ERR_NBR_OVERFLOW). */
+   * the cutoff, at least 512; four beads share a row, consecutive ones along
+   * the chains, neighbours in space where chains are short, and rows that overflow
+   * the cap are grown to 1.25 times the longest one at the mobility build; an
+   * explicit cap that a bead's own pairs overflow is BD_ERR_NBR_OVERFLOW). */
   int pme_grid;
   int pme_order;
   double pme_rc;

@@ -212,8 +212,9 @@ struct bd_ctx {
   int rl_cap, rl_ncell_cap;
   int *rl_cnt, *rl_rows, *rl_beads, *rl_cell_of, *rl_cell_count, *rl_cell_start, *rl_cursor;
   int *rl_need;      // longest pair row of the last build that overflowed the cap (0: none)
-  void *rl_pos;      // lab-frame positions of the last preparation (double4)
-  void *rl_spos;     // the same in real-space cell order, bead index in w
+  void *rl_pos;      // lab-frame positions of the last preparation, index in w (double4)
+  void *rl_gpos;     // the same in the groups' order (null: by index)
+  void *rl_spos;     // the same in real-space cell order
   void *pme_vpk;     // a product's input values, packed pairs side by side per bead and component
   void *rl_w;        // per entry the four pair tensors: (t1, w), or (t1, t2 / r^2)
   bd::Lat rl_lat;    // lattice of the last preparation

@@ -56,7 +56,8 @@ using namespace bd;
 // direction (u = K s, s wrapped into [0,1)).  Positions held in the rotated
 // frame are taken to the lab frame with (cr, sr) = (cos, sin) of the lattice
 // angle, x = x' cr - y' sr, y = x' sr + y' cr (inverseCoords,
-// extensional/src/main14.c:1525-1535); lab-frame positions pass (1, 0).
+// extensional/src/main14.c:1525-1535); lab-frame positions pass (1, 0).  pos
+// gets the lab-frame position with the index in its fourth component.
 template <typename R>
 __global__ void k_pme_weights(Cell cell, const double* __restrict__ rx,
                               const double* __restrict__ ry, const double* __restrict__ rz,
@@ -65,7 +66,7 @@ __global__ void k_pme_weights(Cell cell, const double* __restrict__ rx,
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   double x = rx[i] * cr - ry[i] * sr, y = rx[i] * sr + ry[i] * cr, z = rz[i];
-  pos[i] = make_double4(x, y, z, 0.0);
+  pos[i] = make_double4(x, y, z, __longlong_as_double((long long)i));
   double s[3];
   frac_of(cell, x, y, z, s);
   for (int d = 0; d < 3; d++) {
@@ -285,7 +286,9 @@ static int pme_alloc(bd_ctx* c) {
 int pme_prepare(bd_ctx* c, const Lat& l) {
   int s;
   c->pme_ready = c->hi_built = false;  // until it is complete
-  if ((s = pme_alloc(c)) != BD_OK) return s;
+  // every buffer before the first launch: an allocation beside running kernels
+  // takes several times as long
+  if ((s = pme_alloc(c)) != BD_OK || (s = real_rows(c)) != BD_OK) return s;
   Cell cell = make_cell(l);
   double cr = 1.0, sr = 0.0;
   if (l.flow == BD_FLOW_EXT) {

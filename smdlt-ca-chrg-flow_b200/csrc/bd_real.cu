@@ -1,8 +1,9 @@
 // Real-space part of the particle-mesh mobility: pair lists, tensors, products.
 //
 // No counterpart in the reference (see bd_pme.cu).  The beads are taken four
-// at a time (consecutive indices: neighbours along a chain, whose cutoff
-// spheres nearly coincide).  A group's row lists every bead within the cutoff
+// at a time, neighbours whose cutoff spheres nearly coincide: consecutive indices
+// along a chain, or neighbours in space where chains are short (by_index).  A
+// group's row lists every bead within the cutoff
 // of one of its four, and per entry the four pair tensors (zero where a pair is
 // beyond the cutoff), so that a product reads a neighbour once for four pairs.
 // Two forms:
@@ -32,6 +33,21 @@ using namespace bd;
 namespace {
 
 constexpr int kGroup = 4;  // beads per row
+
+// Whether groups are consecutive indices: chains of a multiple of four beads fill
+// whole groups, of long ones few groups straddle two.  The others go by small
+// cells: products of 50 000 beads (cutoff 14.5) by index and by cells, single FP32,
+// single FP64 and ten FP32, monomers 558, 759, 1367 and 319, 452, 931 us; chains of
+// 5 333, 448, 1009 and 294, 406, 916; of 8 286, 392, 892 and 292, 404, 913; of 10
+// 308, 423, 963 and 290, 402, 918; of 25 304, 420, 958 and 300, 413, 941, for which
+// the build takes 1.90 and 2.04 ms.
+inline bool by_index(int Nb) { return Nb % kGroup == 0 || Nb >= 16; }
+
+// Bead of a place in the groups' order: gpos holds the beads' positions in that
+// order, the index in the fourth component.
+__device__ __forceinline__ int bead_of(const double4& p) {
+  return (int)__double_as_longlong(p.w);
+}
 
 // Real-space Beenakker kernel t1 I + t2 r r^T/r^2 (shear/src/main26.c:
 // 1727-1741) at split parameter alpha; with FAR the r > 2 form at any r.  irr
@@ -124,8 +140,7 @@ __global__ void k_rl_fill(const int* __restrict__ cell_of, const int* __restrict
   beads[cell_start[c] + atomicAdd(&cursor[c], 1)] = i;
 }
 
-// Positions in cell order, a cell's beads in increasing index, the index in the
-// fourth component: the row build streams a cell's beads with one contiguous
+// Positions in cell order, a cell's beads in increasing index: the row build streams a cell's beads with one contiguous
 // load each.  One block per cell, each bead placed by its rank.
 __global__ void __launch_bounds__(256) k_rl_order(const int* __restrict__ cell_start,
                                                   const int* __restrict__ beads,
@@ -144,11 +159,23 @@ __global__ void __launch_bounds__(256) k_rl_order(const int* __restrict__ cell_s
       if (e < n)
         for (int q = 0; q < m; q++) rank += s[q] < v;
     }
-    if (e < n) {
-      double4 p = pos[v];
-      p.w = __longlong_as_double((long long)v);
-      spos[lo + rank] = p;
-    }
+    if (e < n) spos[lo + rank] = pos[v];
+  }
+}
+
+// Positions in the order of the cells, a cell's beads in increasing index: the
+// groups' order of unchained beads.  One warp per cell of a bead or two.
+__global__ void __launch_bounds__(256) k_rl_group(const int* __restrict__ cell_start, int ncell,
+                                                  const int* __restrict__ beads,
+                                                  const double4* __restrict__ pos, double4* gpos) {
+  const int c = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (c >= ncell) return;
+  const int lo = cell_start[c], n = cell_start[c + 1] - lo;
+  for (int e = lane; e < n; e += 32) {
+    const int v = beads[lo + e];
+    int rank = 0;
+    for (int q = 0; q < n; q++) rank += beads[lo + q] < v;
+    gpos[lo + rank] = pos[v];
   }
 }
 
@@ -196,11 +223,12 @@ struct Real2<double> {
 // warp per bead 1.3; this and k_rl_tensors 1.5, for rows the product reads 1.7 times
 // faster).
 __global__ void __launch_bounds__(128, 4)
-    k_rl_find(Cell cell, RGeom g, const double4* __restrict__ pos, int N, int ngroup,
+    k_rl_find(Cell cell, RGeom g, const double4* __restrict__ gpos, int N, int ngroup,
               const int* __restrict__ cell_start, const double4* __restrict__ spos, double rc2,
               int cap, int* cnt, int* rows, int* need, int* err) {
   __shared__ CandList c_list[4];
   __shared__ int c_queue[4][64];
+  __shared__ double4 s_group[4][kGroup];
   const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = blockIdx.x * 4 + wl;
   if (grp >= ngroup) return;
@@ -208,6 +236,9 @@ __global__ void __launch_bounds__(128, 4)
   const Image image(cell);
   int* row = rows + (size_t)grp * cap;
   int* queue = c_queue[wl];
+  const double4* group = s_group[wl];
+  if (lane < nb) s_group[wl][lane] = gpos[i0 + lane];
+  __syncwarp();
   int n = 0, nq = 0;
   // the first m hits of bead b: those that no earlier bead lists
   auto list = [&](int b, int m) {
@@ -215,10 +246,11 @@ __global__ void __launch_bounds__(128, 4)
     int j = 0;
     if (keep) {
       const double4 pj = spos[queue[lane]];
-      j = (int)__double_as_longlong(pj.w);
+      j = bead_of(pj);
       for (int q = 0; q < b; q++) {
+        const double4 pq = group[q];
         double dx, dy, dz;
-        if (j != i0 + q && !(image(pj, pos[i0 + q], dx, dy, dz) >= rc2)) keep = false;
+        if (j != bead_of(pq) && !(image(pj, pq, dx, dy, dz) >= rc2)) keep = false;
       }
     }
     const unsigned hit = __ballot_sync(0xffffffffu, keep);
@@ -233,7 +265,8 @@ __global__ void __launch_bounds__(128, 4)
   };
 #pragma unroll 1
   for (int b = 0; b < nb; b++) {
-    const double4 pb = pos[i0 + b];
+    const double4 pb = group[b];
+    const int own = bead_of(pb);
     int cd[3], cl = 0, next_at = -1;
     cell_of_pos(cell, g.n, pb.x, pb.y, pb.z, cd);
     const int total = c_list[wl].open(g.n, cd, cell_start);
@@ -254,7 +287,7 @@ __global__ void __launch_bounds__(128, 4)
       fetch(m0 + 32 + lane);
       double dx, dy, dz;
       const double rr = image(pj, pb, dx, dy, dz);
-      const bool in = at >= 0 && !(rr >= rc2) && (int)__double_as_longlong(pj.w) != i0 + b;
+      const bool in = at >= 0 && !(rr >= rc2) && bead_of(pj) != own;
       const unsigned hit = __ballot_sync(0xffffffffu, in);
       if (in) queue[nq + __popc(hit & ((1u << lane) - 1u))] = at;
       nq += __popc(hit);
@@ -284,7 +317,8 @@ __global__ void __launch_bounds__(128, 4)
 // lane writing its own entry.
 template <typename R, bool WHOLE>
 __global__ void __launch_bounds__(128, 4)
-    k_rl_tensors(Cell cell, const double4* __restrict__ pos, int N, int ngroup,
+    k_rl_tensors(Cell cell, const double4* __restrict__ pos, const double4* __restrict__ gpos,
+                 int N, int ngroup,
                  const int* __restrict__ cnt, const int* __restrict__ rows, int cap, double rc2,
                  double alpha, double alpha_ref, int bead_cap, void* rw, int* err) {
   using T2 = typename Real2<R>::T;
@@ -321,7 +355,7 @@ __global__ void __launch_bounds__(128, 4)
     if (lane < m) {
       const int k = queue[nq - m + lane] >> 2, b = queue[nq - m + lane] & 3;
       double dx, dy, dz;
-      const double rr = image(pos[row[k]], pos[i0 + b], dx, dy, dz);
+      const double rr = image(pos[row[k]], gpos[i0 + b], dx, dy, dz);
       form(std::integral_constant<bool, true>(), whole + 16 * (size_t)k, k, b, rr, dx, dy, dz);
     }
     nq -= m;
@@ -337,8 +371,9 @@ __global__ void __launch_bounds__(128, 4)
     for (int b = 0; b < kGroup; b++) {
       bool near = false;
       double dx, dy, dz;
-      const double rr = image(pj, pos[min(i0 + b, N - 1)], dx, dy, dz);
-      if (k < n && b < nb && j != i0 + b && !(rr >= rc2)) {
+      const double4 pb = gpos[min(i0 + b, N - 1)];
+      const double rr = image(pj, pb, dx, dy, dz);
+      if (k < n && b < nb && j != bead_of(pb) && !(rr >= rc2)) {
         count[0] += b == 0, count[1] += b == 1, count[2] += b == 2, count[3] += b == 3;
         near = rr < 4.0;
         if (!near) form(std::integral_constant<bool, false>(), entry, k, b, rr, dx, dy, dz);
@@ -432,7 +467,7 @@ template <int NP, int SPLIT>
 __global__ void __launch_bounds__(128, 4)
     k_real_apply(const int* __restrict__ cnt, const int* __restrict__ rows,
                  const float* __restrict__ rw, int cap, const float2* __restrict__ vpk, int np,
-                 int p0, int N, int ngroup, Finish fin) {
+                 int p0, const double4* __restrict__ gpos, int N, int ngroup, Finish fin) {
   using V = float2;
   using P = Stage<NP>;
   constexpr int S = P::S, ITS = P::ITS, CH = P::CH, DEEP = 3, W = 25;
@@ -537,8 +572,9 @@ __global__ void __launch_bounds__(128, 4)
   if (grp >= ngroup) return;
   const int w0 = wl / SPLIT * SPLIT;
   for (int e = lane + 32 * piece0; e < 6 * kGroup * NP; e += 32 * SPLIT) {
-    const int b = e / (6 * NP), p = e / 6 % NP, i = kGroup * grp + b;
-    if (i >= N) break;
+    const int b = e / (6 * NP), p = e / 6 % NP, at = kGroup * grp + b;
+    if (at >= N) break;
+    const int i = bead_of(gpos[at]);
     double s = 0;
     for (int w = w0; w < w0 + SPLIT; w++)
       for (int u = 0; u < S; u++) s += (double)sh.sum[w][(u * NP + p) * W + 6 * b + e % 6];
@@ -564,7 +600,8 @@ struct PairStage {
 
 template <int NP, bool ONE, int SPLIT, typename R>
 __global__ void __launch_bounds__(128, ONE ? 4 : 2)
-    k_real_sum(Cell cell, const double4* __restrict__ pos, const int* __restrict__ cnt,
+    k_real_sum(Cell cell, const double4* __restrict__ pos, const double4* __restrict__ gpos,
+               const int* __restrict__ cnt,
                const int* __restrict__ rows, const typename Real2<R>::T* __restrict__ rt, int cap,
                VecIn v, const double2* __restrict__ vpk, int np, int p0, int N, int ngroup,
                Finish fin) {
@@ -599,7 +636,7 @@ __global__ void __launch_bounds__(128, ONE ? 4 : 2)
     const Image image(cell);
     double4 pb[kGroup];
 #pragma unroll
-    for (int b = 0; b < kGroup; b++) pb[b] = pos[min(i0 + b, N - 1)];
+    for (int b = 0; b < kGroup; b++) pb[b] = gpos[min(i0 + b, N - 1)];
     P* st = sh.in.stage[wl];
     auto issue = [&](int piece, int buf) {
       const int m = min(32, n - 32 * piece);
@@ -709,13 +746,19 @@ __global__ void __launch_bounds__(128, ONE ? 4 : 2)
   if (grp >= ngroup) return;
   const int w0 = wl / SPLIT * SPLIT;
   for (int e = lane + 32 * piece0; e < NS * kGroup * NP; e += 32 * SPLIT) {
-    const int b = e / (NS * NP), p = e / NS % NP, i = i0 + b;
-    if (i >= N) break;
+    const int b = e / (NS * NP), p = e / NS % NP;
+    if (i0 + b >= N) break;
+    const int i = bead_of(gpos[i0 + b]);
     double s = 0;
     for (int w = w0; w < w0 + SPLIT; w++)
       for (int u = 0; u < S; u++) s += sh.sum[w][(u * NP + p) * W + NS * b + e % NS];
     fin.write(s, p0 + p, e % NS, i);
   }
+}
+
+// The beads in the groups' order: cells' or, of chains, the index.
+const double4* group_order(const bd_ctx* c) {
+  return (const double4*)(c->rl_gpos ? c->rl_gpos : c->rl_pos);
 }
 
 // Warps a group of a row of (t1, t2 / r^2).
@@ -727,7 +770,7 @@ void launch_sum(bd_ctx* c, int np, int p0, const Finish& fin) {
   const Cell cell = make_cell(c->rl_lat);
 #define SUM(SPLIT_)                                                                         \
   k_real_sum<NP, ONE, SPLIT_, R><<<nblk(ng, 4 / SPLIT_), 128, 0, c->stream>>>(              \
-      cell, (const double4*)c->rl_pos, c->rl_cnt, c->rl_rows,                               \
+      cell, (const double4*)c->rl_pos, group_order(c), c->rl_cnt, c->rl_rows,               \
       (const typename Real2<R>::T*)c->rl_w, c->rl_cap, fin.v, (const double2*)c->pme_vpk, np, \
       p0, c->N, ng, fin)
   switch (few_warps(ng)) {
@@ -744,7 +787,7 @@ void launch_apply(bd_ctx* c, int np, int p0, const Finish& fin) {
 #define REAL(SPLIT_)                                                                      \
   k_real_apply<NP, SPLIT_><<<nblk(ng, 4 / SPLIT_), 128, 0, c->stream>>>(                  \
       c->rl_cnt, c->rl_rows, (const float*)c->rl_w, c->rl_cap, (const float2*)c->pme_vpk, \
-      np, p0, c->N, ng, fin)
+      np, p0, group_order(c), c->N, ng, fin)
   // More warps a group fill the chip sooner, fewer start fewer pieces.  By four,
   // two and one, five pairs FP32: 500 beads 6.1, 8.0, 12.6 us, 8000 41.8, 46.5, 63.7,
   // 16 000 70, 74, 79; FP64 8000 85, 90, 107, 16 000 151, 147, 160; one pair FP32
@@ -783,6 +826,8 @@ bool whole_tensors(const bd_ctx* c) { return c->pme_f32 && c->nbk > 1; }
 
 namespace bd {
 
+constexpr int kRowCells = 4096;  // most cells of the rows' search
+
 // Rows of cap entries for every group; without memory for them there are none
 // (rl_rows null) and the mobility is not built.
 static int rows_alloc(bd_ctx* c, int cap) {
@@ -810,10 +855,17 @@ static int first_cap(const bd_ctx* c) {
   return std::min(cap, std::max(c->N, 1));
 }
 
+// The rows of a first preparation, or of one after rows that could not be grown.
+int real_rows(bd_ctx* c) { return c->rl_rows ? BD_OK : rows_alloc(c, first_cap(c)); }
+
 int real_alloc(bd_ctx* c) {
   const size_t N = c->N;
-  c->rl_ncell_cap = 4096;
-  int s = alloc_all(c, {{&c->rl_cnt, 4 * N},
+  // as many cells as the groups' order has where beads are not chained
+  const bool order = !by_index(c->Nb);
+  c->rl_ncell_cap = order ? (int)std::max((size_t)kRowCells, 2 * N) : kRowCells;
+  int s;
+  if (order && (s = alloc_all(c, {{&c->rl_gpos, 32 * N}})) != BD_OK) return s;
+  s = alloc_all(c, {{&c->rl_cnt, 4 * N},
                         {&c->rl_need, 4},
                         {&c->rl_cell_of, 4 * N},
                         {&c->rl_spos, 32 * N},
@@ -828,9 +880,27 @@ int real_alloc(bd_ctx* c) {
 }
 
 void real_free(bd_ctx* c) {
-  free_all({&c->rl_rows, &c->rl_w, &c->rl_cnt, &c->rl_need, &c->rl_cell_of, &c->rl_spos,
+  free_all({&c->rl_rows, &c->rl_w, &c->rl_gpos, &c->rl_cnt, &c->rl_need, &c->rl_cell_of, &c->rl_spos,
             &c->rl_beads, &c->rl_cell_count, &c->rl_cell_start, &c->rl_cursor});
   c->rl_cap = 0;
+}
+
+// The beads by cells of geometry g (reduced to at most `most` cells) in rl_beads,
+// the cells' ranges in rl_cell_start; returns their number.
+static int bin_beads(bd_ctx* c, const Cell& cell, RGeom& g, int most, double cr, double sr) {
+  const int N = c->N;
+  while ((long)g.n[0] * g.n[1] * g.n[2] > most) {
+    int d = g.n[0] >= g.n[1] && g.n[0] >= g.n[2] ? 0 : (g.n[1] >= g.n[2] ? 1 : 2);
+    g.n[d]--;
+  }
+  const int ncell = g.n[0] * g.n[1] * g.n[2];
+  c->launches += 3;
+  k_rl_count<<<nblk(N, 256), 256, 0, c->stream>>>(cell, g, c->rx, c->ry, c->rz, cr, sr, N,
+                                                  c->rl_cell_of, c->rl_cell_count);
+  k_rl_scan<<<1, 1024, 0, c->stream>>>(ncell, c->rl_cell_count, c->rl_cell_start, c->rl_cursor);
+  k_rl_fill<<<nblk(N, 256), 256, 0, c->stream>>>(c->rl_cell_of, c->rl_cell_start, c->rl_cursor,
+                                                 c->rl_beads, N);
+  return ncell;
 }
 
 // The groups' rows for the positions in rl_pos (lab frame; rx, ry, rz and the
@@ -839,7 +909,6 @@ int real_prepare(bd_ctx* c, const Lat& l, const Cell& cell, double cr, double sr
                  double alpha_ref) {
   int s, N = c->N;
   double rc = c->pme_rc, alpha = c->pme_alpha;
-  if (!c->rl_rows && (s = rows_alloc(c, first_cap(c))) != BD_OK) return s;
   // real-space cells: perpendicular widths V/|a_j x a_k|
   double w[3];
   {
@@ -858,17 +927,18 @@ int real_prepare(bd_ctx* c, const Lat& l, const Cell& cell, double cr, double sr
   if (2 * rc > std::min(w[0], std::min(w[1], w[2]))) return BD_ERR_ARG;  // rc beyond half a width
   RGeom g;
   for (int d = 0; d < 3; d++) g.n[d] = std::max(1, (int)floor(w[d] / rc));
-  while ((long)g.n[0] * g.n[1] * g.n[2] > c->rl_ncell_cap) {
-    int d = g.n[0] >= g.n[1] && g.n[0] >= g.n[2] ? 0 : (g.n[1] >= g.n[2] ? 1 : 2);
-    g.n[d]--;
+  if (c->rl_gpos) {
+    // the groups' order: columns of four beads' mean width, cut so that a cell
+    // holds one bead
+    const double h = cbrt(4.0 * cell.V / N);
+    RGeom o;
+    for (int d = 0; d < 3; d++) o.n[d] = std::max(1, (int)(w[d] / (d < 2 ? h : 0.25 * h)));
+    const int n = bin_beads(c, cell, o, c->rl_ncell_cap, cr, sr);
+    c->launches++;
+    k_rl_group<<<nblk(n, 8), 256, 0, c->stream>>>(c->rl_cell_start, n, c->rl_beads,
+                                                  (const double4*)c->rl_pos, (double4*)c->rl_gpos);
   }
-  int ncell = g.n[0] * g.n[1] * g.n[2];
-  c->launches += 4;
-  k_rl_count<<<nblk(N, 256), 256, 0, c->stream>>>(cell, g, c->rx, c->ry, c->rz, cr, sr, N,
-                                                  c->rl_cell_of, c->rl_cell_count);
-  k_rl_scan<<<1, 1024, 0, c->stream>>>(ncell, c->rl_cell_count, c->rl_cell_start, c->rl_cursor);
-  k_rl_fill<<<nblk(N, 256), 256, 0, c->stream>>>(c->rl_cell_of, c->rl_cell_start, c->rl_cursor,
-                                                 c->rl_beads, N);
+  const int ncell = bin_beads(c, cell, g, kRowCells, cr, sr);
   c->launches++;
   k_rl_order<<<ncell, 256, 0, c->stream>>>(c->rl_cell_start, c->rl_beads,
                                            (const double4*)c->rl_pos, (double4*)c->rl_spos);
@@ -882,7 +952,7 @@ int real_prepare(bd_ctx* c, const Lat& l, const Cell& cell, double cr, double sr
   for (bool grow = c->rl_cap < most;; grow = false) {
     c->launches++;
     k_rl_find<<<nblk(ng, 4), 128, 0, c->stream>>>(
-        cell, g, (const double4*)c->rl_pos, N, ng, c->rl_cell_start, (const double4*)c->rl_spos,
+        cell, g, group_order(c), N, ng, c->rl_cell_start, (const double4*)c->rl_spos,
         rc * rc, c->rl_cap, c->rl_cnt, c->rl_rows, grow ? c->rl_need : nullptr, c->err);
     if (!grow) break;
     int longest = 0;
@@ -895,8 +965,8 @@ int real_prepare(bd_ctx* c, const Lat& l, const Cell& cell, double cr, double sr
   c->launches++;
 #define TENSORS(...)                                                                          \
   k_rl_tensors<__VA_ARGS__><<<nblk(ng, 4), 128, 0, c->stream>>>(                              \
-      cell, (const double4*)c->rl_pos, N, ng, c->rl_cnt, c->rl_rows, c->rl_cap, rc * rc, alpha, \
-      alpha_ref, c->p.pme_max_pairs, c->rl_w, c->err)
+      cell, (const double4*)c->rl_pos, group_order(c), N, ng, c->rl_cnt, c->rl_rows, c->rl_cap, \
+      rc * rc, alpha, alpha_ref, c->p.pme_max_pairs, c->rl_w, c->err)
   if (whole_tensors(c))
     TENSORS(float, true);
   else if (c->pme_f32)

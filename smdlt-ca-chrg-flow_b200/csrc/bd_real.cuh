@@ -45,6 +45,7 @@ struct Finish {
 namespace bd {
 int real_alloc(bd_ctx* c);
 void real_free(bd_ctx* c);
+int real_rows(bd_ctx* c);
 int real_prepare(bd_ctx* c, const Lat& l, const Cell& cell, double cr, double sr, double alpha_ref);
 int real_apply(bd_ctx* c, int np, const Finish& fin);
 }  // namespace bd

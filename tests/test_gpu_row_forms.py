@@ -36,11 +36,13 @@ def _system(N):
     return L, (x, y, z), v.reshape(-1), ref.reshape(-1)
 
 
-@pytest.mark.parametrize("precision,block", [("fp64", 1), ("fp64", 9), ("fp32", 1), ("fp32", 9)])
-@pytest.mark.parametrize("N", [2, 33, 7104, 7105, 23677])
-def test_forms_match_model(N, precision, block):
+FORMS = pytest.mark.parametrize("precision,block", [("fp64", 1), ("fp64", 9), ("fp32", 1),
+                                                    ("fp32", 9)])
+
+
+def _check(N, Nb, precision, block):
     L, pos, v, ref = _system(N)
-    c = B.Context(B.make_params(0, N, 1, L, 0.2, 5e-4, mobility="pme", noise="philox",
+    c = B.Context(B.make_params(0, Nb, N // Nb, L, 0.2, 5e-4, mobility="pme", noise="philox",
                                 precision=precision, pme_grid=K, pme_order=ORDER, pme_rc=RC,
                                 pme_alpha=ALPHA, noise_block=block))
     c.set_positions(*pos)
@@ -52,6 +54,40 @@ def test_forms_match_model(N, precision, block):
     for k in (2, 4, 5, 8, 9) if block > 1 else ():  # an odd last vector among them
         got = c.mobility_apply_block(FACTORS[:k, None] * v)
         assert max(rel_err(got[r], FACTORS[r] * ref) for r in range(k)) < tol, k
+
+
+@FORMS
+@pytest.mark.parametrize("N", [2, 33, 7104, 7105, 23677])
+def test_forms_match_model(N, precision, block):
+    _check(N, N, precision, block)
+
+
+@FORMS
+@pytest.mark.parametrize("N,Nb", [(2, 1), (33, 11), (33, 3), (7105, 1), (7105, 7), (7105, 5),
+                                  (7104, 2)])
+def test_beads_grouped_in_space_match_model(N, Nb, precision, block):
+    """Short chains, whose groups follow the space and not the index."""
+    _check(N, Nb, precision, block)
+
+
+@pytest.mark.parametrize("precision,block", [("fp64", 1), ("fp32", 4)])
+def test_monomers_need_no_longer_rows(precision, block):
+    """Beads in no spatial order: grouped by index, four of them would share hardly
+    a neighbour and their rows overflow the default cap."""
+    N, L = 8000, 60.0
+    r, used = np.random.default_rng(9), {}
+    chains = np.stack(B.random_chains(100, N // 100, L, 3), 1)
+    for Nb, pos in ((100, chains), (1, r.uniform(-L / 2, L / 2, (N, 3)))):
+        c = B.Context(B.make_params(0, Nb, N // Nb, L, 0.2, 5e-4, mobility="pme", noise="philox",
+                                    precision=precision, noise_block=block, pme_rc=12.1))
+        c.set_positions(*(np.ascontiguousarray(a) for a in pos.T))
+        c.set_time(0, 0)
+        c.update_lattice(0)
+        c.apply_pbc()
+        c.calc_hi()
+        used[Nb] = c.device_bytes()
+        c.close()
+    assert used[1] < 1.1 * used[100], used
 
 
 def test_single_vector_contexts_take_fp64_inputs():
