@@ -206,8 +206,12 @@ struct bd_ctx {
   int pme_nblk;      // blocks of the influence kernel
   int *pme_base;     // per bead base grid index, 3 x N
   void *pme_w;       // per bead spline weights, 3 x N x 8 (FP64 or FP32, as the grids)
-  int pme_plan;      // 1 + cuFFT plan of one pair's grid, for sizes bd_fft.cuh does not
-                     // cover (0: none)
+  // grid sizes bd_fft.cuh does not cover: components one after the other; 1 + cuFFT
+  // plan of a single right-hand side (real, forward and back), its half spectrum,
+  // and of up to four numbers of pairs (0: none)
+  bool pme_planar;
+  int pme_plan_f, pme_plan_b, pme_mplan[4], pme_mplan_np[4];
+  void *pme_spec;
   // real-space rows of groups of four beads (bd_real.cu)
   int rl_cap, rl_ncell_cap;
   int *rl_cnt, *rl_rows, *rl_beads, *rl_cell_of, *rl_cell_count, *rl_cell_start, *rl_cursor;
@@ -286,6 +290,7 @@ int pme_prepare(bd_ctx* c, const Lat& l);
 int pme_apply(bd_ctx* c, const VecIn& v, double* o0, double* o1, double* o2, int ostride);
 // Y_r = M X_r for k vectors in Lanczos layout (3 x NTp), RHS strides xs, ys
 int pme_apply_multi(bd_ctx* c, int k, const double* X, size_t xs, double* Y, size_t ys);
+int pme_pairs_plan(bd_ctx* c, int k);  // the transforms' plan for k >= 2, if one is needed
 void pme_free(bd_ctx* c);
 
 // CA-TEA sampling

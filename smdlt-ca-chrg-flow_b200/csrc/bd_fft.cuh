@@ -385,8 +385,8 @@ int run(bd_ctx* c, void* grid, int np, const void* infl, const void* tw) {
 }
 
 // The sizes with a pair of factors up to 16 that the transforms in registers
-// cover: every 2^a 3^b 5^c grid of the default rule from 20 to 160, and the
-// larger ones whose factors allow it; other sizes go through cuFFT.
+// cover: every 2^a 3^b 5^c from 20 to 160 but 125, and up to 256 those that are
+// not 162, 200, 216, 243 or 250.  Other sizes go through cuFFT (bd_pme.cu).
 #define BD_FFT_SIZES(X)                                                                       \
   X(4, 5) X(4, 6) X(5, 5) X(3, 9) X(5, 6) X(4, 8) X(6, 6) X(5, 8) X(5, 9) X(6, 8) X(5, 10)    \
   X(6, 9) X(6, 10) X(8, 8) X(8, 9) X(5, 15) X(8, 10) X(9, 9) X(9, 10) X(8, 12) X(10, 10)      \

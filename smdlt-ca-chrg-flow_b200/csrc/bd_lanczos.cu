@@ -1641,6 +1641,7 @@ static int lanczos_sqrt_block(bd_ctx* c, int k) {
   if ((s = alloc_lanczos(c)) != BD_OK) return s;
   if ((s = alloc_blocks(c)) != BD_OK) return s;
   if (k < 1 || k > c->nbk) return BD_ERR_ARG;
+  if ((s = pme_pairs_plan(c, k)) != BD_OK) return s;
   size_t n = 3 * (size_t)c->NT * 32;
   bool pre = c->pre_kind != BD_PRECOND_NONE && c->pre_ready;
   std::vector<int> mr;
@@ -1785,7 +1786,9 @@ int bd_mobility_apply_block(bd_ctx* c, int k, const double* v, double* out) {
     return BD_OK;
   }
   int s;
-  if ((s = io_alloc(c)) != BD_OK || (s = io_in(c, k, v)) != BD_OK) return s;
+  if ((s = pme_pairs_plan(c, k)) != BD_OK || (s = io_alloc(c)) != BD_OK ||
+      (s = io_in(c, k, v)) != BD_OK)
+    return s;
   const size_t n = 3 * (size_t)c->NT * 32;
   prof_begin(c, BD_PROF_BLOCK);  // the product alone, for timing (autotuner)
   s = pme_apply_multi(c, k, c->io_x, n, c->io_y, n);

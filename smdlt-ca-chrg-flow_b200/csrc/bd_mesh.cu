@@ -2,7 +2,8 @@
 //
 // No counterpart in the reference (see bd_pme.cu).  Grids hold, per packed
 // pair of right-hand sides, K^3 points of three complex components, the
-// component fastest.
+// component fastest; where cuFFT transforms them (pme_planar), the components one
+// after the other, and a single right-hand side's grid is real.
 //
 // Spreading: the grid is cut into columns of CY x CZ points in (y, z), running
 // along x.  A warp owns a column (or a segment of it) for NG packed pairs, a
@@ -256,6 +257,8 @@ struct SpreadArgs {
   const int* bin;
   int K, npz, npatch, nseg, nset, np, N;
   const void* vpk;  // packed values
+  int ps;           // grid layout: a point's, a component's stride
+  size_t cs;
 };
 
 template <int P, typename R, int NG, int CY, int CZ, bool ONE>
@@ -280,7 +283,8 @@ __global__ void __launch_bounds__(32, sizeof(R) == 4 ? 16 : 8)
   const int pr = set * NG + g;
   const bool own = lane < NG * CY * CZ && pr < m.np && y0 + ly < K && z0 + lz < K;
   const size_t K2 = (size_t)K * K;
-  T* out = (T*)grid + 3 * ((size_t)(own ? pr : 0) * K2 * K + (size_t)(y0 + ly) * K + (z0 + lz));
+  const size_t here = (size_t)(y0 + ly) * K + (z0 + lz);
+  T* out = (T*)grid + 3 * (size_t)(own ? pr : 0) * K2 * K + here * m.ps;
   // bases xs .. xe + P - 2, wrapped: entries [e0, e0 + n0), then [f0, f0 + n1)
   const int* bin = m.bin + (size_t)patch * K;
   const int top = xe + P - 1;
@@ -295,10 +299,15 @@ __global__ void __launch_bounds__(32, sizeof(R) == 4 ? 16 : 8)
   int lo = xs - (P - 1);  // grid level of acc[0]
   auto advance = [&]() {
     if (lo >= xs && own) {
-      T* o = out + 3 * K2 * (size_t)lo;
-      o[0] = as_pair(acc[0][0]);
-      o[1] = as_pair(acc[0][1]);
-      o[2] = as_pair(acc[0][2]);
+      if (ONE && m.ps == 1) {
+        R* o = grid + here + K2 * (size_t)lo;
+#pragma unroll
+        for (int c = 0; c < 3; c++) o[c * m.cs] = as_pair(acc[0][c]).x;
+      } else {
+        T* o = out + m.ps * K2 * (size_t)lo;
+#pragma unroll
+        for (int c = 0; c < 3; c++) o[c * m.cs] = as_pair(acc[0][c]);
+      }
     }
 #pragma unroll
     for (int a = 0; a + 1 < P; a++)
@@ -378,7 +387,9 @@ __global__ void __launch_bounds__(32, sizeof(R) == 4 ? 16 : 8)
 // component (2 t + lane) mod 3: one sum for each t mod 3, put in component
 // order at the end.  FP32 sums per lane (order 8: 16 terms each) and over four
 // lanes, FP64 beyond.
-template <int P, typename R>
+enum Layout { kInterleaved, kPlanar, kReal };
+
+template <int P, typename R, Layout LAY>
 __global__ void __launch_bounds__(256)
     k_mesh_gather(const int* __restrict__ base, const R* __restrict__ w,
                   const R* __restrict__ grid, int N, int K, double* __restrict__ val) {
@@ -390,11 +401,46 @@ __global__ void __launch_bounds__(256)
   const R* w2 = w1 + kMaxOrder;
   const int b0 = base[3 * i], b1 = base[3 * i + 1], b2 = base[3 * i + 2];
   const size_t K2 = (size_t)K * K;
-  const T* gp = (const T*)grid + (size_t)pr * 3 * K2 * K;
+  constexpr int ps = LAY == kInterleaved ? 3 : 1;
+  const size_t cs = LAY == kInterleaved ? 1 : K2 * K;
+  using E = std::conditional_t<LAY == kReal, R, T>;
+  const E* gp = (const E*)grid + (size_t)pr * 3 * K2 * K;
+  auto value = [](E x) {
+    if constexpr (LAY == kReal)
+      return as_pair(x);
+    else
+      return x;
+  };
   T s[3];
 #pragma unroll
   for (int j = 0; j < 3; j++) s[j].x = s[j].y = 0;
-  if constexpr (P == 8) {
+  constexpr bool own_sums = P == 8 && LAY != kInterleaved;  // component c in sum c
+  if constexpr (own_sums) {
+    // four rows of one component a load
+    unsigned off[2];
+    R wyz[2];
+    int gz = b2 - (P - 1) + lane % 8;
+    gz += gz < 0 ? K : 0;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      int gy = b1 - (4 * h + lane / 8);
+      gy += gy < 0 ? K : 0;
+      off[h] = (unsigned)(gy * K + gz);
+      wyz[h] = w1[4 * h + lane / 8] * w2[P - 1 - lane % 8];
+    }
+#pragma unroll
+    for (int a = 0; a < P; a++) {
+      int gx = b0 - a;
+      gx += gx < 0 ? K : 0;
+      const E* gl = gp + K2 * (size_t)gx;
+      const R wx = w0[a];
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+          madd(weight(wx * wyz[h]), value(gl[off[h] + (size_t)j * cs]), s[j]);
+    }
+  } else if constexpr (P == 8) {
     // four rows in three loads; rows 4 q + (0..3) of x level q / 2: the lane's
     // point and its offset within (y, z) depend on q only by its parity
     int off[3][2];
@@ -436,15 +482,15 @@ __global__ void __launch_bounds__(256)
         gy += gy < 0 ? K : 0;
         gz += gz < 0 ? K : 0;
         madd(weight(w0[a] * w1[b] * w2[P - 1 - z]),
-             gp[3 * ((size_t)gx * K2 + (size_t)gy * K + gz) + f % 3], s[j]);
+             value(gp[ps * ((size_t)gx * K2 + (size_t)gy * K + gz) + (f % 3) * cs]), s[j]);
       }
     }
   }
   // component c is in sum 2 (c - lane) mod 3
-  const int r = lane % 3;
-  T c0 = r == 0 ? s[0] : r == 1 ? s[1] : s[2];
-  T c1 = r == 0 ? s[2] : r == 1 ? s[0] : s[1];
-  T c2 = r == 0 ? s[1] : r == 1 ? s[2] : s[0];
+  const int r = own_sums ? -1 : lane % 3;
+  T c0 = r <= 0 ? s[0] : r == 1 ? s[1] : s[2];
+  T c1 = r < 0 ? s[1] : r == 0 ? s[2] : r == 1 ? s[0] : s[1];
+  T c2 = r < 0 ? s[2] : r == 0 ? s[1] : r == 1 ? s[2] : s[0];
   // real parts to the lower, imaginary parts to the upper half of the warp
   const bool up = lane & 16;
   R x[3] = {up ? c0.y : c0.x, up ? c1.y : c1.x, up ? c2.y : c2.x};
@@ -532,6 +578,8 @@ int spread_t(bd_ctx* c, int k, const VecIn& v, size_t vr, R* grid) {
   m.np = np;
   m.N = c->N;
   m.vpk = c->pme_vpk;
+  m.ps = c->pme_planar ? 1 : 3;
+  m.cs = c->pme_planar ? (size_t)K * K * K : 1;
   c->launches++;
   k_mesh_pack<<<dim3(nblk(c->N, 128), np), 128, 0, c->stream>>>(
       v, vr, k, np, c->N, (typename GridVal<R>::T*)c->pme_vpk);
@@ -545,20 +593,29 @@ int spread_t(bd_ctx* c, int k, const VecIn& v, size_t vr, R* grid) {
   return BD_OK;
 }
 
-template <typename R>
-int gather_t(bd_ctx* c, int k, const R* grid) {
+template <int P, typename R>
+void launch_gather(bd_ctx* c, int k, const R* grid) {
   const dim3 g(nblk(c->N, 8), (k + 1) / 2);
   const R* w = (const R*)c->pme_w;
+#define GATHER(LAY_)                                                                      \
+  k_mesh_gather<P, R, LAY_><<<g, 256, 0, c->stream>>>(c->pme_base, w, grid, c->N, c->pmeK, \
+                                                      c->mesh_val)
+  if (!c->pme_planar)
+    GATHER(kInterleaved);
+  else if (k > 1)
+    GATHER(kPlanar);
+  else
+    GATHER(kReal);
+#undef GATHER
+}
+
+template <typename R>
+int gather_t(bd_ctx* c, int k, const R* grid) {
   c->launches++;
   switch (c->pme_p) {
-    case 4:
-      k_mesh_gather<4, R><<<g, 256, 0, c->stream>>>(c->pme_base, w, grid, c->N, c->pmeK, c->mesh_val);
-      break;
-    case 6:
-      k_mesh_gather<6, R><<<g, 256, 0, c->stream>>>(c->pme_base, w, grid, c->N, c->pmeK, c->mesh_val);
-      break;
-    default:
-      k_mesh_gather<8, R><<<g, 256, 0, c->stream>>>(c->pme_base, w, grid, c->N, c->pmeK, c->mesh_val);
+    case 4: launch_gather<4, R>(c, k, grid); break;
+    case 6: launch_gather<6, R>(c, k, grid); break;
+    default: launch_gather<8, R>(c, k, grid);
   }
   return BD_OK;
 }

@@ -93,25 +93,30 @@ __global__ void k_pme_weights(Cell cell, const double* __restrict__ rx,
 // give both products, with no unpacking.  An odd last right-hand side, or a
 // single one, has a zero imaginary part.
 
-// The influence tensor on the full spectrum of the packed pairs, for grid sizes
-// that go through cuFFT (thread per point and pair): points with m2 > K/2 take
-// the tensor of their mirror -m, stored in the half spectrum.
-template <typename R, typename Cx>
-__global__ void k_pme_apply_influence(const R* __restrict__ infl, Cx* cgrid, int K, size_t np) {
-  size_t K3 = (size_t)K * K * K;
+// The influence tensor on spectra of cuFFT's, for grid sizes that bd_fft.cuh does
+// not cover (thread per point and pair), the components n entries apart: a single
+// right-hand side's half spectrum, or the full spectrum of packed pairs, where
+// points with m2 > K/2 take the tensor of their mirror -m.
+template <bool HALF, typename R, typename Cx>
+__global__ void k_pme_apply_influence(const R* __restrict__ infl, Cx* spec, int K, size_t n,
+                                      size_t np) {
   size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= K3 * np) return;
-  size_t m = e % K3;
-  int Kh = K / 2 + 1;
-  int m0 = (int)(m / ((size_t)K * K)), m1 = (int)((m / K) % K), m2 = (int)(m % K);
-  if (m2 > K / 2) {
-    m0 = (K - m0) % K;
-    m1 = (K - m1) % K;
-    m2 = K - m2;
+  if (e >= n * np) return;
+  const size_t m = e % n;
+  size_t at = m;
+  if constexpr (!HALF) {
+    const int Kh = K / 2 + 1;
+    int m0 = (int)(m / ((size_t)K * K)), m1 = (int)((m / K) % K), m2 = (int)(m % K);
+    if (m2 > K / 2) {
+      m0 = (K - m0) % K;
+      m1 = (K - m1) % K;
+      m2 = K - m2;
+    }
+    at = ((size_t)m0 * K + m1) * Kh + m2;
   }
-  const R* t = infl + 6 * (((size_t)m0 * K + m1) * Kh + m2);
-  Cx* b = cgrid + 3 * e;
-  Cx x = b[0], y = b[1], z = b[2];
+  const R* t = infl + 6 * at;
+  Cx* b = spec + 3 * n * (e / n) + m;
+  Cx x = b[0], y = b[n], z = b[2 * n];
   Cx u, v, ww;
   u.x = t[0] * x.x + t[1] * y.x + t[2] * z.x;
   u.y = t[0] * x.y + t[1] * y.y + t[2] * z.y;
@@ -120,8 +125,8 @@ __global__ void k_pme_apply_influence(const R* __restrict__ infl, Cx* cgrid, int
   ww.x = t[2] * x.x + t[4] * y.x + t[5] * z.x;
   ww.y = t[2] * x.y + t[4] * y.y + t[5] * z.y;
   b[0] = u;
-  b[1] = v;
-  b[2] = ww;
+  b[n] = v;
+  b[2 * n] = ww;
 }
 
 // Influence tensor on the half spectrum: (phi(k)/V)(I - k k^T/k^2) |b|^2,
@@ -211,6 +216,45 @@ __global__ void k_pme_soff_fin(const double* __restrict__ part, int nb, double* 
 
 namespace bd {
 
+// cuFFT plan of `batch` contiguous grids, distances id and od apart.
+static int make_plan(bd_ctx* c, int* slot, int id, int od, cufftType type, int batch) {
+  int n[3] = {c->pmeK, c->pmeK, c->pmeK};
+  cufftHandle f;
+  CF(cufftPlanMany(&f, 3, n, nullptr, 1, id, nullptr, 1, od, type, batch));
+  *slot = (int)f + 1;
+  CF(cufftSetStream(f, c->stream));
+  return BD_OK;
+}
+
+static void drop_plan(int* plan) {
+  if (*plan) cufftDestroy((cufftHandle)(*plan - 1));
+  *plan = 0;
+}
+
+// In-place transforms of the packed pairs of k right-hand sides, for grid sizes
+// bd_fft.cuh does not cover: one plan for all their grids, made outside any
+// capture and kept for up to four numbers of pairs (replacing one drops the
+// captured iterations that use it).
+int pme_pairs_plan(bd_ctx* c, int k) {
+  if (!c->pme_planar || k < 2) return BD_OK;
+  const int np = (k + 1) / 2;
+  int slot = -1;
+  for (int q = 3; q >= 0; q--) {
+    if (c->pme_mplan[q] && c->pme_mplan_np[q] == np) return BD_OK;
+    if (!c->pme_mplan[q]) slot = q;
+  }
+  if (slot < 0) {
+    slot = 3;
+    lanczos_graphs_reset(c);
+    drop_plan(&c->pme_mplan[slot]);
+  }
+  const int K3 = c->pmeK * c->pmeK * c->pmeK;
+  c->pme_mplan_np[slot] = np;
+  const int s = make_plan(c, &c->pme_mplan[slot], K3, K3, c->pme_f32 ? CUFFT_C2C : CUFFT_Z2Z, 3 * np);
+  if (s != BD_OK) drop_plan(&c->pme_mplan[slot]);
+  return s;
+}
+
 static int pme_parts(bd_ctx* c) {
   int s, K = c->pmeK, N = c->N;
   size_t K3 = (size_t)K * K * K, Ks = (size_t)K * K * (K / 2 + 1);
@@ -230,13 +274,16 @@ static int pme_parts(bd_ctx* c) {
                     {&c->pme_vpk, 6 * es * (size_t)N * ((nr + 1) / 2)},
                     {&c->rl_pos, 32 * (size_t)N}});
   if (s != BD_OK || (s = mesh_alloc(c)) != BD_OK || (s = real_alloc(c)) != BD_OK) return s;
-  if (!fft_has_size(K)) {
-    // one pair's three interleaved components, in place
-    int n[3] = {K, K, K};
-    cufftHandle f;
-    CF(cufftPlanMany(&f, 3, n, n, 3, 1, n, 3, 1, c->pme_f32 ? CUFFT_C2C : CUFFT_Z2Z, 3));
-    CF(cufftSetStream(f, c->stream));
-    c->pme_plan = (int)f + 1;
+  c->pme_planar = !fft_has_size(K);
+  if (c->pme_planar) {
+    // a single right-hand side's three real grids, and a full block's pairs
+    if ((s = alloc_all(c, {{&c->pme_spec, 2 * es * 3 * Ks}})) != BD_OK) return s;
+    const bool f32 = c->pme_f32;
+    const int nk = (int)K3, nh = (int)Ks;
+    if ((s = make_plan(c, &c->pme_plan_f, nk, nh, f32 ? CUFFT_R2C : CUFFT_D2Z, 3)) != BD_OK ||
+        (s = make_plan(c, &c->pme_plan_b, nh, nk, f32 ? CUFFT_C2R : CUFFT_Z2D, 3)) != BD_OK ||
+        (nr > 1 && (s = pme_pairs_plan(c, (int)nr)) != BD_OK))
+      return s;
   }
   std::vector<double> tw(2 * (size_t)K);
   std::vector<float> tw32(2 * (size_t)K);
@@ -258,11 +305,12 @@ static int pme_parts(bd_ctx* c) {
 }
 
 void pme_free(bd_ctx* c) {
-  if (c->pme_plan) cufftDestroy((cufftHandle)(c->pme_plan - 1));
-  c->pme_plan = 0;
+  for (int* plan : {&c->pme_plan_f, &c->pme_plan_b, &c->pme_mplan[0], &c->pme_mplan[1],
+                    &c->pme_mplan[2], &c->pme_mplan[3]})
+    drop_plan(plan);
   mesh_free(c);
   real_free(c);
-  free_all({&c->pme_vpk, &c->pme_grid, &c->pme_tw, &c->pme_infl, &c->pme_bsq, &c->pme_soff,
+  free_all({&c->pme_vpk, &c->pme_grid, &c->pme_spec, &c->pme_tw, &c->pme_infl, &c->pme_bsq, &c->pme_soff,
             &c->pme_base, &c->pme_w, &c->rl_pos});
 }
 
@@ -286,8 +334,6 @@ static int pme_alloc(bd_ctx* c) {
 int pme_prepare(bd_ctx* c, const Lat& l) {
   int s;
   c->pme_ready = c->hi_built = false;  // until it is complete
-  // every buffer before the first launch: an allocation beside running kernels
-  // takes several times as long
   if ((s = pme_alloc(c)) != BD_OK || (s = real_rows(c)) != BD_OK) return s;
   Cell cell = make_cell(l);
   double cr = 1.0, sr = 0.0;
@@ -327,38 +373,66 @@ int pme_prepare(bd_ctx* c, const Lat& l) {
   return launch_ok(c);
 }
 
+// The transforms through cuFFT, for grid sizes bd_fft.cuh does not cover: single
+// right-hand sides by real transforms, packed pairs all at once in place.
+// The grids hold their components one after the other: interleaved ones (element
+// stride 3) cost cuFFT more than the transforms themselves.  30 000 beads on 125^3,
+// ten vectors FP32, one FP32, one FP64: 1351, 231, 306 us; interleaved, a pair at a
+// time and complex throughout 1767, 376, 603.  150 000 on 216^3: 6790, 936, 1369;
+// 10400, 2100, 4080.
+template <typename R, typename Cx>
+static int cufft_influence(bd_ctx* c, int k) {
+  const int K = c->pmeK, np = (k + 1) / 2;
+  const size_t K3 = (size_t)K * K * K, Ks = (size_t)K * K * (K / 2 + 1);
+  constexpr bool F = sizeof(R) == 4;
+  c->launches++;
+  if (k == 1) {
+    const cufftHandle f = (cufftHandle)(c->pme_plan_f - 1), b = (cufftHandle)(c->pme_plan_b - 1);
+    if constexpr (F)
+      CF(cufftExecR2C(f, (cufftReal*)c->pme_grid, (cufftComplex*)c->pme_spec));
+    else
+      CF(cufftExecD2Z(f, (cufftDoubleReal*)c->pme_grid, (cufftDoubleComplex*)c->pme_spec));
+    k_pme_apply_influence<true, R, Cx><<<nblk((long long)Ks, 256), 256, 0, c->stream>>>(
+        (const R*)c->pme_infl, (Cx*)c->pme_spec, K, Ks, 1);
+    if constexpr (F)
+      CF(cufftExecC2R(b, (cufftComplex*)c->pme_spec, (cufftReal*)c->pme_grid));
+    else
+      CF(cufftExecZ2D(b, (cufftDoubleComplex*)c->pme_spec, (cufftDoubleReal*)c->pme_grid));
+    return BD_OK;
+  }
+  int q = 0;
+  while (q < 4 && !(c->pme_mplan[q] && c->pme_mplan_np[q] == np)) q++;
+  if (q == 4) return BD_ERR_STATE;  // pme_pairs_plan(c, k) first
+  for (int dir : {CUFFT_FORWARD, CUFFT_INVERSE}) {
+    const cufftHandle f = (cufftHandle)(c->pme_mplan[q] - 1);
+    Cx* g = (Cx*)c->pme_grid;
+    if constexpr (F)
+      CF(cufftExecC2C(f, (cufftComplex*)g, (cufftComplex*)g, dir));
+    else
+      CF(cufftExecZ2Z(f, (cufftDoubleComplex*)g, (cufftDoubleComplex*)g, dir));
+    if (dir == CUFFT_FORWARD)
+      k_pme_apply_influence<false, R, Cx><<<nblk((long long)K3 * np, 256), 256, 0, c->stream>>>(
+          (const R*)c->pme_infl, g, K, K3, (size_t)np);
+  }
+  return BD_OK;
+}
+
 // out_r = M v_r by PME for k right-hand sides given by component pointers
 // (VecIn) and RHS strides vr (input) and orr (output).
 template <typename R, typename Cx>
 static int pme_apply_t(bd_ctx* c, int k, const VecIn& v, size_t vr, double* o0, double* o1,
                        double* o2, int ostride, size_t orr) {
   int K = c->pmeK, N = c->N, s;
-  size_t K3 = (size_t)K * K * K;
   if (k < 1 || k > std::max(1, c->nbk)) return BD_ERR_ARG;
   int np = (k + 1) / 2;
   Cx* g = (Cx*)c->pme_grid;
   if ((s = mesh_spread(c, k, v, vr, g)) != BD_OK) return s;
-  if (!c->pme_plan) {
+  if (c->pme_planar)
+    s = cufft_influence<R, Cx>(c, k);
+  else
     s = sizeof(R) == 4 ? fft_influence_f32(c, K, g, np, c->pme_infl, c->pme_tw)
                        : fft_influence_f64(c, K, g, np, c->pme_infl, c->pme_tw);
-    if (s != BD_OK) return s;
-  } else {
-    for (int dir : {CUFFT_FORWARD, CUFFT_INVERSE}) {
-      for (int p = 0; p < np; p++) {
-        Cx* gp = g + 3 * K3 * p;
-        if constexpr (sizeof(R) == 4)
-          CF(cufftExecC2C((cufftHandle)(c->pme_plan - 1), (cufftComplex*)gp, (cufftComplex*)gp, dir));
-        else
-          CF(cufftExecZ2Z((cufftHandle)(c->pme_plan - 1), (cufftDoubleComplex*)gp,
-                          (cufftDoubleComplex*)gp, dir));
-      }
-      if (dir == CUFFT_FORWARD) {
-        c->launches++;
-        k_pme_apply_influence<R, Cx><<<nblk((long long)K3 * np, 256), 256, 0, c->stream>>>(
-            (const R*)c->pme_infl, g, K, (size_t)np);
-      }
-    }
-  }
+  if (s != BD_OK) return s;
   if ((s = mesh_gather(c, k, g)) != BD_OK) return s;
   Finish fin;
   fin.val = c->mesh_val;
