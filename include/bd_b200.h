@@ -436,8 +436,8 @@ int bd_batch_step_lanczos(bd_batch *batch, unsigned long t0, int nsteps, int wit
 int bd_batch_destroy(bd_batch *batch);
 /* Particle-mesh grid for a box of edge L: of the 2^a 3^b 5^c sizes between
  * 1.29 L (the accuracy bound of the default discretisation) and 25 % above,
- * the one with the fastest three-component FFT round trip on the current
- * device (bd_precision for the storage); results are cached per process. */
+ * the one on which the transforms of two right-hand sides are fastest on the
+ * current device (bd_precision for the storage); results are cached per process. */
 int bd_autotune_pme_grid(double L, int precision, int *K_out);
 /* The default particle-mesh grid bd_create picks for a box of edge L and a
  * real-space cutoff rc (rc <= 0: the default cutoff, the smaller of 10 and

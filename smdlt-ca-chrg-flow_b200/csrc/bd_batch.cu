@@ -11,10 +11,8 @@
 //
 // bd_autotune_pme_grid picks the particle-mesh grid for a box: among the
 // FFT-friendly sizes (2^a 3^b 5^c) from the accuracy bound 1.29 L up to 25 %
-// above it, the one whose batched three-component R2C + C2R round trip is
-// fastest on this GPU (timed with CUDA events, cached per size and
-// precision).
-#include <cufft.h>
+// above it, the one on which a packed pair's transforms, those a product runs, are
+// fastest on this GPU (timed with CUDA events, cached per size and precision).
 #include <math.h>
 
 #include <algorithm>
@@ -141,50 +139,8 @@ int bd_autotune_pme_grid(double L, int precision, int* K_out) {
     if (it != cache.end()) {
       ms = it->second;
     } else {
-      size_t K3 = (size_t)K * K * K, Ks = (size_t)K * K * (K / 2 + 1);
-      size_t es = precision ? 4 : 8;
-      void *grid = nullptr, *spec = nullptr;
-      if (cudaMalloc(&grid, es * 3 * K3) != cudaSuccess) return BD_ERR_OOM;
-      if (cudaMalloc(&spec, 2 * es * 3 * Ks) != cudaSuccess) {
-        cudaFree(grid);
-        return BD_ERR_OOM;
-      }
-      cudaMemset(grid, 0, es * 3 * K3);
-      int dims[3] = {K, K, K};
-      cufftHandle f = 0, bk = 0;
-      bool okf = cufftPlanMany(&f, 3, dims, nullptr, 1, (int)K3, nullptr, 1, (int)Ks,
-                               precision ? CUFFT_R2C : CUFFT_D2Z, 3) == CUFFT_SUCCESS;
-      bool okb = okf && cufftPlanMany(&bk, 3, dims, nullptr, 1, (int)Ks, nullptr, 1, (int)K3,
-                                      precision ? CUFFT_C2R : CUFFT_Z2D, 3) == CUFFT_SUCCESS;
-      if (okf && !okb) cufftDestroy(f);
-      bool ok = okf && okb;
-      cudaEvent_t e0, e1;
-      cudaEventCreate(&e0);
-      cudaEventCreate(&e1);
-      ms = 1e30f;
-      if (ok) {
-        for (int rep = 0; rep < 8; rep++) {
-          if (rep == 3) cudaEventRecord(e0, 0);
-          if (precision) {
-            cufftExecR2C(f, (cufftReal*)grid, (cufftComplex*)spec);
-            cufftExecC2R(bk, (cufftComplex*)spec, (cufftReal*)grid);
-          } else {
-            cufftExecD2Z(f, (cufftDoubleReal*)grid, (cufftDoubleComplex*)spec);
-            cufftExecZ2D(bk, (cufftDoubleComplex*)spec, (cufftDoubleReal*)grid);
-          }
-        }
-        cudaEventRecord(e1, 0);
-        cudaEventSynchronize(e1);
-        cudaEventElapsedTime(&ms, e0, e1);
-        ms /= 5;
-        cufftDestroy(f);
-        cufftDestroy(bk);
-      }
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
-      cudaFree(grid);
-      cudaFree(spec);
-      if (cudaGetLastError() != cudaSuccess) return BD_ERR_CUDA;
+      int st = bd::pme_time_transforms(K, precision == 1, &ms);
+      if (st != BD_OK) return st;
       cache[key] = ms;
     }
     if (ms < best_ms) {

@@ -292,6 +292,7 @@ int pme_apply(bd_ctx* c, const VecIn& v, double* o0, double* o1, double* o2, int
 int pme_apply_multi(bd_ctx* c, int k, const double* X, size_t xs, double* Y, size_t ys);
 int pme_pairs_plan(bd_ctx* c, int k);  // the transforms' plan for k >= 2, if one is needed
 void pme_free(bd_ctx* c);
+int pme_time_transforms(int K, bool f32, float* ms);
 
 // CA-TEA sampling
 int ewald_bin(bd_ctx* c, double* eps, std::vector<double>& rowsum);

@@ -450,6 +450,51 @@ static int pme_apply_t(bd_ctx* c, int k, const VecIn& v, size_t vr, double* o0, 
   return real_apply(c, np, fin);
 }
 
+// Forward transform, tensor and inverse transform of one packed pair's grid, as a
+// product runs them.
+static int transform_pair(bd_ctx* c) {
+  if (c->pme_planar)
+    return c->pme_f32 ? cufft_influence<float, cufftComplex>(c, 2)
+                      : cufft_influence<double, cufftDoubleComplex>(c, 2);
+  return (c->pme_f32 ? fft_influence_f32 : fft_influence_f64)(c, c->pmeK, c->pme_grid, 1,
+                                                              c->pme_infl, c->pme_tw);
+}
+
+// Time of one packed pair's transforms on K^3 points, on the default stream.
+int pme_time_transforms(int K, bool f32, float* ms) {
+  bd_ctx* c = new bd_ctx();  // a workspace without beads
+  c->pmeK = K;
+  c->pme_p = 8;
+  c->p.precision = f32 ? BD_PREC_FP32 : BD_PREC_FP64;
+  c->nbk = 2;
+  c->boxvol = 1.0;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  auto run = [&]() -> int {
+    int s = pme_alloc(c);
+    if (s != BD_OK) return s;
+    const size_t es = f32 ? 4 : 8, K3 = (size_t)K * K * K, Ks = (size_t)K * K * (K / 2 + 1);
+    CU(cudaMemsetAsync(c->pme_grid, 0, 6 * es * K3, c->stream));
+    CU(cudaMemsetAsync(c->pme_infl, 0, 6 * es * Ks, c->stream));
+    CU(cudaEventCreate(&e0));
+    CU(cudaEventCreate(&e1));
+    for (int rep = 0; rep < 8; rep++) {
+      if (rep == 3) CU(cudaEventRecord(e0, c->stream));
+      if ((s = transform_pair(c)) != BD_OK) return s;
+    }
+    CU(cudaEventRecord(e1, c->stream));
+    CU(cudaEventSynchronize(e1));
+    CU(cudaEventElapsedTime(ms, e0, e1));
+    *ms /= 5;
+    return launch_ok(c);
+  };
+  const int s = run();
+  if (e0) cudaEventDestroy(e0);
+  if (e1) cudaEventDestroy(e1);
+  pme_free(c);
+  delete c;
+  return s;
+}
+
 static int pme_apply_k(bd_ctx* c, int k, const VecIn& v, size_t vr, double* o0, double* o1,
                        double* o2, int ostride, size_t orr) {
   if (!c->pme_ready) return BD_ERR_STATE;
