@@ -210,6 +210,7 @@ struct bd_ctx {
   // plan of a single right-hand side (real, forward and back), its half spectrum,
   // and of up to four numbers of pairs (0: none)
   bool pme_planar;
+  bool pme_real1;    // single right-hand sides take real grids and cuFFT's transforms
   int pme_plan_f, pme_plan_b, pme_mplan[4], pme_mplan_np[4];
   void *pme_spec;
   // real-space rows of groups of four beads (bd_real.cu)

@@ -578,8 +578,9 @@ int spread_t(bd_ctx* c, int k, const VecIn& v, size_t vr, R* grid) {
   m.np = np;
   m.N = c->N;
   m.vpk = c->pme_vpk;
-  m.ps = c->pme_planar ? 1 : 3;
-  m.cs = c->pme_planar ? (size_t)K * K * K : 1;
+  const bool planar = k == 1 ? c->pme_real1 : c->pme_planar;
+  m.ps = planar ? 1 : 3;
+  m.cs = planar ? (size_t)K * K * K : 1;
   c->launches++;
   k_mesh_pack<<<dim3(nblk(c->N, 128), np), 128, 0, c->stream>>>(
       v, vr, k, np, c->N, (typename GridVal<R>::T*)c->pme_vpk);
@@ -600,12 +601,12 @@ void launch_gather(bd_ctx* c, int k, const R* grid) {
 #define GATHER(LAY_)                                                                      \
   k_mesh_gather<P, R, LAY_><<<g, 256, 0, c->stream>>>(c->pme_base, w, grid, c->N, c->pmeK, \
                                                       c->mesh_val)
-  if (!c->pme_planar)
-    GATHER(kInterleaved);
-  else if (k > 1)
+  if (k == 1 && c->pme_real1)
+    GATHER(kReal);
+  else if (c->pme_planar)
     GATHER(kPlanar);
   else
-    GATHER(kReal);
+    GATHER(kInterleaved);
 #undef GATHER
 }
 

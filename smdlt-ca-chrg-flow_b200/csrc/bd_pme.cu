@@ -255,14 +255,30 @@ int pme_pairs_plan(bd_ctx* c, int k) {
   return s;
 }
 
+// Whether a single right-hand side on a grid that bd_fft.cuh covers goes through
+// cuFFT's real transforms: half the data, but a pass more and planar grids.
+// Products by them and by the five complex passes, us, FP64: 80^3 140 and 130, 96^3
+// 214 and 193, 100^3 179 and 212, 128^3 324 and 452, 135^3 514 and 495, 144^3 425
+// and 591, 225^3 2052 and 2384, 256^3 2263 and 3532.  FP32: 120^3 218 and 206, 128^3
+// 235 and 236 (a thousand beads 127 and 149), 144^3 302 and 321, 150^3 425 and 381,
+// 160^3 444 and 468, 192^3 698 and 781, 240^3 1550 and 1486, 256^3 1502 and 1730.
+static bool real_single(int K, bool f32) {
+  return f32 ? K >= 128 && K % 16 == 0 && K % 15 != 0 : K >= 100 && (K % 2 == 0 || K > 200);
+}
+
 static int pme_parts(bd_ctx* c) {
   int s, K = c->pmeK, N = c->N;
   size_t K3 = (size_t)K * K * K, Ks = (size_t)K * K * (K / 2 + 1);
   c->pme_f32 = c->p.precision == BD_PREC_FP32;
   size_t es = c->pme_f32 ? 4 : 8;  // grid, spectrum, influence and pair tensors
-  // the packed pairs' grids for the largest number of right-hand sides
+  c->pme_planar = !fft_has_size(K);
+  c->pme_real1 = c->pme_planar || real_single(K, c->pme_f32);
+  // the packed pairs' grids for the largest number of right-hand sides; with
+  // pme_real1 a single one's real grids and behind them its half spectra
   size_t nr = (size_t)std::max(1, c->nbk);
-  size_t grid_bytes = 2 * es * 3 * K3 * ((nr + 1) / 2);
+  size_t real_bytes = (es * 3 * K3 + 255) / 256 * 256;
+  size_t grid_bytes = c->pme_real1 && nr == 1 ? 0 : 2 * es * 3 * K3 * ((nr + 1) / 2);
+  if (c->pme_real1) grid_bytes = std::max(grid_bytes, real_bytes + 2 * es * 3 * Ks);
   c->pme_nblk = (int)((Ks + 255) / 256);
   s = alloc_all(c, {{&c->pme_grid, grid_bytes},
                     {&c->pme_tw, 2 * es * K},
@@ -274,17 +290,15 @@ static int pme_parts(bd_ctx* c) {
                     {&c->pme_vpk, 6 * es * (size_t)N * ((nr + 1) / 2)},
                     {&c->rl_pos, 32 * (size_t)N}});
   if (s != BD_OK || (s = mesh_alloc(c)) != BD_OK || (s = real_alloc(c)) != BD_OK) return s;
-  c->pme_planar = !fft_has_size(K);
-  if (c->pme_planar) {
-    // a single right-hand side's three real grids, and a full block's pairs
-    if ((s = alloc_all(c, {{&c->pme_spec, 2 * es * 3 * Ks}})) != BD_OK) return s;
+  if (c->pme_real1) {
+    c->pme_spec = (char*)c->pme_grid + real_bytes;
     const bool f32 = c->pme_f32;
     const int nk = (int)K3, nh = (int)Ks;
     if ((s = make_plan(c, &c->pme_plan_f, nk, nh, f32 ? CUFFT_R2C : CUFFT_D2Z, 3)) != BD_OK ||
-        (s = make_plan(c, &c->pme_plan_b, nh, nk, f32 ? CUFFT_C2R : CUFFT_Z2D, 3)) != BD_OK ||
-        (nr > 1 && (s = pme_pairs_plan(c, (int)nr)) != BD_OK))
+        (s = make_plan(c, &c->pme_plan_b, nh, nk, f32 ? CUFFT_C2R : CUFFT_Z2D, 3)) != BD_OK)
       return s;
   }
+  if (c->pme_planar && nr > 1 && (s = pme_pairs_plan(c, (int)nr)) != BD_OK) return s;
   std::vector<double> tw(2 * (size_t)K);
   std::vector<float> tw32(2 * (size_t)K);
   for (int m = 0; m < K; m++) {
@@ -310,7 +324,7 @@ void pme_free(bd_ctx* c) {
     drop_plan(plan);
   mesh_free(c);
   real_free(c);
-  free_all({&c->pme_vpk, &c->pme_grid, &c->pme_spec, &c->pme_tw, &c->pme_infl, &c->pme_bsq, &c->pme_soff,
+  free_all({&c->pme_vpk, &c->pme_grid, &c->pme_tw, &c->pme_infl, &c->pme_bsq, &c->pme_soff,
             &c->pme_base, &c->pme_w, &c->rl_pos});
 }
 
@@ -427,7 +441,7 @@ static int pme_apply_t(bd_ctx* c, int k, const VecIn& v, size_t vr, double* o0, 
   int np = (k + 1) / 2;
   Cx* g = (Cx*)c->pme_grid;
   if ((s = mesh_spread(c, k, v, vr, g)) != BD_OK) return s;
-  if (c->pme_planar)
+  if (k == 1 ? c->pme_real1 : c->pme_planar)
     s = cufft_influence<R, Cx>(c, k);
   else
     s = sizeof(R) == 4 ? fft_influence_f32(c, K, g, np, c->pme_infl, c->pme_tw)
