@@ -519,6 +519,17 @@ double layout_cost(int np, int ng, int P) {
   return (P - 1 + cy) * (P - 1 + cz) / (cy * cz) * ((np + ng - 1) / ng);
 }
 
+// Few beads for the grid's points: writing the points is most of the work, and the
+// layout of one pair a warp writes the longest runs.  Ten vectors by it and by five
+// pairs a warp, us, FP32: 144^3 1000 beads 965 and 1080, 32 000 1217 and 1333, 50 000
+// 1425 and 1464; 100^3 8000 beads 408 and 420, 16 000 502 and 485, 50 000 1010 and 937.
+// FP64: 144^3 8000 beads 1720 and 1873, 32 000 2252 and 2276, 50 000 2705 and 2618;
+// 100^3 8000 beads 752 and 742.
+bool sparse(const bd_ctx* c) {
+  const size_t K = c->pmeK;
+  return (size_t)c->N * (c->pme_f32 ? 64 : 128) < K * K * K;
+}
+
 // Segments of a column: about 14 warps on every SM (16 fit), none shorter than
 // half a stencil (a segment repeats P - 1 levels of its beads).  Segments
 // measured, us: 1700 columns of 100 levels 1: 154, 2: 159, 3: 155, 6: 163; 704
@@ -563,7 +574,9 @@ int spread_t(bd_ctx* c, int k, const VecIn& v, size_t vr, R* grid) {
   const int np = (k + 1) / 2, K = c->pmeK, P = c->pme_p;
   // of the context's layouts the one with the least work for np pairs
   int l = 0;
-  if (c->mesh_ng[1] && layout_cost(np, c->mesh_ng[1], P) < layout_cost(np, c->mesh_ng[0], P)) l = 1;
+  if (c->mesh_ng[1] && !sparse(c) &&
+      layout_cost(np, c->mesh_ng[1], P) < layout_cost(np, c->mesh_ng[0], P))
+    l = 1;
   const int ng = c->mesh_ng[l];
   SpreadArgs m;
   m.base = c->pme_base;
