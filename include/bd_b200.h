@@ -73,8 +73,15 @@ typedef enum {
 #define BD_PRECOND_MAX_SEGMENT 25
 /* Largest noise block of bd_step_lanczos (bd_params.noise_block). */
 #define BD_MAX_NOISE_BLOCK 64
-/* Storage of the packed mobility tiles used by the products: FP64, or FP32
- * with FP64 accumulation. */
+/* Storage of the mobility used by the products: FP64, or FP32.  Packed tiles
+ * in FP32 are accumulated in FP64.  Particle-mesh products in FP32 hold grids,
+ * transforms, influence and pair tensors in FP32; spline weights are FP64,
+ * rounded to FP32 where they multiply grid values (along x, and once for the
+ * product of those along y and z in spreading); interpolation sums the at most
+ * eight levels along x of order 8 in FP32 and everything else in FP64; the
+ * real-space part has FP64 inputs, displacements and sums in contexts without
+ * noise blocks, FP32 inputs and partial sums, added in FP64, in those with them.
+ * Vectors, recurrences and results are FP64 throughout. */
 typedef enum { BD_PREC_FP64 = 0, BD_PREC_FP32 = 1 } bd_precision;
 typedef enum { BD_SPRING_HOOKEAN = 0, BD_SPRING_FENE = 1 } bd_spring;
 /* Electrostatics: the reference's Debye-Hueckel pair force over all charged

@@ -205,7 +205,7 @@ struct bd_ctx {
   double *pme_soff;  // self-block off-diagonal (xy, xz, yz), then per-block partials
   int pme_nblk;      // blocks of the influence kernel
   int *pme_base;     // per bead base grid index, 3 x N
-  void *pme_w;       // per bead spline weights, 3 x N x 8 (FP64 or FP32, as the grids)
+  double *pme_w;     // per bead spline weights, 3 x N x 8
   // grid sizes bd_fft.cuh does not cover: components one after the other; 1 + cuFFT
   // plan of a single right-hand side (real, forward and back), its half spectrum,
   // and of up to four numbers of pairs (0: none)

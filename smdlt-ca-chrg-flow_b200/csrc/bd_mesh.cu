@@ -21,17 +21,17 @@
 // Bound by the FP32 (FP64) pipe and the issue of its instructions: 48 (P = 8)
 // multiply-adds per lane and bead, two at a time (fma.rn.f32x2) in FP32, next
 // to about 20 others.
-// Five pairs, order 8: 150 us at 50 000 beads on 100^3 (one complex L2 atomic
-// per stencil point, component and pair took about 400), 42 us at 8000 beads on
+// Five pairs, order 8: 163 us at 50 000 beads on 100^3 (one complex L2 atomic
+// per stencil point, component and pair took about 400), 43 us at 8000 beads on
 // 64^3 (74); FP64 66 us there (385).
 //
 // Interpolation: a warp per bead and pair reads the stencil's 64 rows of 24
 // complex values (192 contiguous bytes, FP32), a lane the same third of a row
 // position throughout, so its y and z weights and addresses stay in registers.
 // Bound by L1 throughput.
-// Five pairs, order 8: 238 us at 50 000 beads on 100^3 (separate component
-// grids, 64 bytes a row, FP64 sums per lane: about 300), 40 us at 8000 beads on
-// 64^3 (54); FP64 72 us there.
+// Five pairs, order 8: 253 us at 50 000 beads on 100^3 (separate component
+// grids, 64 bytes a row: about 300), 42 us at 8000 beads on 64^3 (54); FP64 70 us
+// there.
 //
 // The columns' lists are built once per mobility build (the positions are
 // frozen until the next): per column and base index the beads in increasing
@@ -207,6 +207,11 @@ __device__ __forceinline__ void madd(double w, double2 x, double2& a) {
 }
 __device__ __forceinline__ void madd(float w, float x, float& a) { a = fmaf(w, x, a); }
 __device__ __forceinline__ void madd(double w, double x, double& a) { a = fma(w, x, a); }
+// grid values into FP64 sums
+__device__ __forceinline__ void madd(double w, float2 x, double2& a) {
+  a.x = fma(w, (double)x.x, a.x);
+  a.y = fma(w, (double)x.y, a.y);
+}
 __device__ __forceinline__ float2 weight(float x) { return make_float2(x, x); }
 __device__ __forceinline__ double weight(double x) { return x; }
 __device__ __forceinline__ void put(float2& w, float x) { w = make_float2(x, x); }
@@ -234,14 +239,14 @@ __device__ __forceinline__ void set_pair(float& f, float x, float) { f = x; }
 __device__ __forceinline__ void set_pair(double& f, double x, double) { f = x; }
 
 // One bead of a column's walk in shared memory: x-weights from the lowest
-// level up, the weights of the column's rows and points, the pairs' values,
-// the base index along x.  Padded to an odd number of 16-byte words, so that
+// level up, the (y, z) weights of the column's points (products of FP64 weights,
+// rounded once), the pairs' values, the base index along x.  Padded to an odd number of 16-byte words, so that
 // the lanes of a warp store their records without bank conflicts.
 template <int P, typename R, int NG, int CY, int CZ, bool ONE>
 struct RecData {
   std::conditional_t<ONE, R, typename GridVal<R>::W> wx[P];
   std::conditional_t<ONE, R, typename GridVal<R>::T> f[NG][3];
-  R wy[CY], wz[CZ];
+  R wyz[CY * CZ];
   int at;
 };
 template <typename S>
@@ -252,7 +257,7 @@ struct alignas(16) Rec : S {
 
 struct SpreadArgs {
   const int* base;
-  const void* w;  // 8 weights per bead and direction, R
+  const double* w;  // 8 weights per bead and direction
   const int* ent;
   const int* bin;
   int K, npz, npatch, nseg, nset, np, N;
@@ -324,22 +329,25 @@ __global__ void __launch_bounds__(32, sizeof(R) == 4 ? 16 : 8)
   auto stage = [&](int t, int i) {
     if (t >= n) return;
     S& r = s_rec[lane];
-    const R* w = (const R*)m.w + (size_t)i * 3 * kMaxOrder;
+    const double* w = m.w + (size_t)i * 3 * kMaxOrder;
     const int b1 = m.base[3 * i + 1], b2 = m.base[3 * i + 2];
     r.at = m.base[3 * i] + (t < n0 ? 0 : K);
 #pragma unroll
-    for (int a = 0; a < P; a++) put(r.wx[a], w[P - 1 - a]);
-#pragma unroll
-    for (int q = 0; q < CY; q++) {
-      int d = b1 - (y0 + q);
-      d += d < 0 ? K : 0;
-      r.wy[q] = d < P && y0 + q < K ? w[kMaxOrder + d] : (R)0;
-    }
+    for (int a = 0; a < P; a++) put(r.wx[a], (R)w[P - 1 - a]);
+    double wz[CZ];
 #pragma unroll
     for (int q = 0; q < CZ; q++) {
       int d = b2 - (z0 + q);
       d += d < 0 ? K : 0;
-      r.wz[q] = d < P && z0 + q < K ? w[2 * kMaxOrder + d] : (R)0;
+      wz[q] = d < P && z0 + q < K ? w[2 * kMaxOrder + d] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < CY; q++) {
+      int d = b1 - (y0 + q);
+      d += d < 0 ? K : 0;
+      const double wy = d < P && y0 + q < K ? w[kMaxOrder + d] : 0.0;
+#pragma unroll
+      for (int e = 0; e < CZ; e++) r.wyz[q * CZ + e] = (R)(wy * wz[e]);
     }
 #pragma unroll
     for (int u = 0; u < NG; u++) {
@@ -361,7 +369,7 @@ __global__ void __launch_bounds__(32, sizeof(R) == 4 ? 16 : 8)
 #pragma unroll 1
     for (int u = 0; u < nb; u++) {
       const S& q = s_rec[u];
-      const R wyz = q.wy[ly] * q.wz[lz];
+      const R wyz = q.wyz[ly * CZ + lz];
       V t[3];
 #pragma unroll
       for (int c = 0; c < 3; c++) t[c] = scaled(wyz, q.f[g][c]);
@@ -385,20 +393,25 @@ __global__ void __launch_bounds__(32, sizeof(R) == 4 ? 16 : 8)
 // a time in memory order (rows of P points along z, three components each);
 // 96 values are a whole number of points, so load t of a lane always holds
 // component (2 t + lane) mod 3: one sum for each t mod 3, put in component
-// order at the end.  FP32 sums per lane (order 8: 16 terms each) and over four
-// lanes, FP64 beyond.
+// order at the end.  Order 8 takes a lane's sums along x (8 levels) in the grid's
+// type and the rest in FP64: 253 us for the five pairs above, 404 with every FP32
+// value converted (four a clock and quarter of an SM), 448 with FP32 sums that keep
+// what they round away.  The product's error against FP64, geometric mean of 12
+// systems of 900 to 32 000 beads, ten vectors: 1.34e-7, 1.33e-7 by those last two
+// (1.89e-7 by atomics, cuFFT and FP64 sums of every term, 1.40e-7 with FP32 weights
+// and lanes).
 enum Layout { kInterleaved, kPlanar, kReal };
 
 template <int P, typename R, Layout LAY>
 __global__ void __launch_bounds__(256)
-    k_mesh_gather(const int* __restrict__ base, const R* __restrict__ w,
+    k_mesh_gather(const int* __restrict__ base, const double* __restrict__ w,
                   const R* __restrict__ grid, int N, int K, double* __restrict__ val) {
   using T = typename GridVal<R>::T;
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, pr = blockIdx.y;
   if (i >= N) return;
-  const R* w0 = w + (size_t)i * 3 * kMaxOrder;
-  const R* w1 = w0 + kMaxOrder;
-  const R* w2 = w1 + kMaxOrder;
+  const double* w0 = w + (size_t)i * 3 * kMaxOrder;
+  const double* w1 = w0 + kMaxOrder;
+  const double* w2 = w1 + kMaxOrder;
   const int b0 = base[3 * i], b1 = base[3 * i + 1], b2 = base[3 * i + 2];
   const size_t K2 = (size_t)K * K;
   constexpr int ps = LAY == kInterleaved ? 3 : 1;
@@ -411,14 +424,15 @@ __global__ void __launch_bounds__(256)
     else
       return x;
   };
-  T s[3];
+  double2 s[3];
 #pragma unroll
-  for (int j = 0; j < 3; j++) s[j].x = s[j].y = 0;
+  for (int j = 0; j < 3; j++) zero(s[j]);
   constexpr bool own_sums = P == 8 && LAY != kInterleaved;  // component c in sum c
   if constexpr (own_sums) {
     // four rows of one component a load
     unsigned off[2];
-    R wyz[2];
+    double wyz[2];
+    T u[2][3];
     int gz = b2 - (P - 1) + lane % 8;
     gz += gz < 0 ? K : 0;
 #pragma unroll
@@ -427,24 +441,30 @@ __global__ void __launch_bounds__(256)
       gy += gy < 0 ? K : 0;
       off[h] = (unsigned)(gy * K + gz);
       wyz[h] = w1[4 * h + lane / 8] * w2[P - 1 - lane % 8];
+#pragma unroll
+      for (int j = 0; j < 3; j++) zero(u[h][j]);
     }
 #pragma unroll
     for (int a = 0; a < P; a++) {
       int gx = b0 - a;
       gx += gx < 0 ? K : 0;
       const E* gl = gp + K2 * (size_t)gx;
-      const R wx = w0[a];
+      const auto wx = weight((R)w0[a]);
 #pragma unroll
       for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int j = 0; j < 3; j++)
-          madd(weight(wx * wyz[h]), value(gl[off[h] + (size_t)j * cs]), s[j]);
+        for (int j = 0; j < 3; j++) madd(wx, value(gl[off[h] + (size_t)j * cs]), u[h][j]);
     }
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int j = 0; j < 3; j++) madd(wyz[h], u[h][j], s[j]);
   } else if constexpr (P == 8) {
     // four rows in three loads; rows 4 q + (0..3) of x level q / 2: the lane's
     // point and its offset within (y, z) depend on q only by its parity
     int off[3][2];
-    R wyz[3][2];
+    double wyz[3][2];
+    T u[3][2];
 #pragma unroll
     for (int j = 0; j < 3; j++) {
       const int f = 32 * j + lane, ro = f / 24, z = f % 24 / 3;
@@ -456,6 +476,7 @@ __global__ void __launch_bounds__(256)
         gy += gy < 0 ? K : 0;
         off[j][h] = (gy * K + gz) * 3 + f % 3;
         wyz[j][h] = w1[4 * h + ro] * w2[P - 1 - z];
+        zero(u[j][h]);
       }
     }
 #pragma unroll
@@ -463,12 +484,16 @@ __global__ void __launch_bounds__(256)
       int gx = b0 - a;
       gx += gx < 0 ? K : 0;
       const T* gl = gp + 3 * K2 * (size_t)gx;
-      const R wx = w0[a];
+      const auto wx = weight((R)w0[a]);
 #pragma unroll
       for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int j = 0; j < 3; j++) madd(weight(wx * wyz[j][h]), gl[off[j][h]], s[j]);
+        for (int j = 0; j < 3; j++) madd(wx, gl[off[j][h]], u[j][h]);
     }
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int j = 0; j < 3; j++) madd(wyz[j][h], u[j][h], s[j]);
   } else {
 #pragma unroll 1
     for (int t0 = 0; 32 * t0 < 3 * P * P * P; t0 += 3) {
@@ -481,31 +506,28 @@ __global__ void __launch_bounds__(256)
         gx += gx < 0 ? K : 0;
         gy += gy < 0 ? K : 0;
         gz += gz < 0 ? K : 0;
-        madd(weight(w0[a] * w1[b] * w2[P - 1 - z]),
+        madd(w0[a] * w1[b] * w2[P - 1 - z],
              value(gp[ps * ((size_t)gx * K2 + (size_t)gy * K + gz) + (f % 3) * cs]), s[j]);
       }
     }
   }
   // component c is in sum 2 (c - lane) mod 3
   const int r = own_sums ? -1 : lane % 3;
-  T c0 = r <= 0 ? s[0] : r == 1 ? s[1] : s[2];
-  T c1 = r < 0 ? s[1] : r == 0 ? s[2] : r == 1 ? s[0] : s[1];
-  T c2 = r < 0 ? s[2] : r == 0 ? s[1] : r == 1 ? s[2] : s[0];
+  const double2 c0 = r <= 0 ? s[0] : r == 1 ? s[1] : s[2];
+  const double2 c1 = r < 0 ? s[1] : r == 0 ? s[2] : r == 1 ? s[0] : s[1];
+  const double2 c2 = r < 0 ? s[2] : r == 0 ? s[1] : r == 1 ? s[2] : s[0];
   // real parts to the lower, imaginary parts to the upper half of the warp
   const bool up = lane & 16;
-  R x[3] = {up ? c0.y : c0.x, up ? c1.y : c1.x, up ? c2.y : c2.x};
-  R y[3] = {up ? c0.x : c0.y, up ? c1.x : c1.y, up ? c2.x : c2.y};
-  double d[3];
+  double x[3] = {up ? c0.y : c0.x, up ? c1.y : c1.x, up ? c2.y : c2.x};
+  const double y[3] = {up ? c0.x : c0.y, up ? c1.x : c1.y, up ? c2.x : c2.y};
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     x[c] += __shfl_xor_sync(0xffffffffu, y[c], 16);
-    x[c] += __shfl_xor_sync(0xffffffffu, x[c], 8);
-    d[c] = (double)x[c];
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) d[c] += __shfl_xor_sync(0xffffffffu, d[c], o);
+    for (int o = 8; o > 0; o >>= 1) x[c] += __shfl_xor_sync(0xffffffffu, x[c], o);
   }
   const int e = lane & 15;
-  if (e < 3) val[((size_t)pr * N + i) * 6 + (up ? 3 : 0) + e] = e == 0 ? d[0] : e == 1 ? d[1] : d[2];
+  if (e < 3) val[((size_t)pr * N + i) * 6 + (up ? 3 : 0) + e] = e == 0 ? x[0] : e == 1 ? x[1] : x[2];
 }
 
 // ---------------------------------------------------------------------------
@@ -610,9 +632,8 @@ int spread_t(bd_ctx* c, int k, const VecIn& v, size_t vr, R* grid) {
 template <int P, typename R>
 void launch_gather(bd_ctx* c, int k, const R* grid) {
   const dim3 g(nblk(c->N, 8), (k + 1) / 2);
-  const R* w = (const R*)c->pme_w;
 #define GATHER(LAY_)                                                                      \
-  k_mesh_gather<P, R, LAY_><<<g, 256, 0, c->stream>>>(c->pme_base, w, grid, c->N, c->pmeK, \
+  k_mesh_gather<P, R, LAY_><<<g, 256, 0, c->stream>>>(c->pme_base, c->pme_w, grid, c->N, c->pmeK, \
                                                       c->mesh_val)
   if (k == 1 && c->pme_real1)
     GATHER(kReal);

@@ -58,10 +58,9 @@ using namespace bd;
 // angle, x = x' cr - y' sr, y = x' sr + y' cr (inverseCoords,
 // extensional/src/main14.c:1525-1535); lab-frame positions pass (1, 0).  pos
 // gets the lab-frame position with the index in its fourth component.
-template <typename R>
 __global__ void k_pme_weights(Cell cell, const double* __restrict__ rx,
                               const double* __restrict__ ry, const double* __restrict__ rz,
-                              double cr, double sr, int N, int K, int p, int* base, R* w,
+                              double cr, double sr, int N, int K, int p, int* base, double* w,
                               double4* pos, int* err) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -80,9 +79,7 @@ __global__ void k_pme_weights(Cell cell, const double* __restrict__ rx,
     double f = u - fl;
     if (fl >= K) fl -= K;
     base[3 * i + d] = fl;
-    double wd[kMaxOrder];
-    bspline(f, p, wd);
-    for (int k = 0; k < p; k++) w[((size_t)3 * i + d) * kMaxOrder + k] = (R)wd[k];
+    bspline(f, p, w + ((size_t)3 * i + d) * kMaxOrder);
   }
 }
 
@@ -286,7 +283,7 @@ static int pme_parts(bd_ctx* c) {
                     {&c->pme_bsq, 8 * 3 * (size_t)K},
                     {&c->pme_soff, 8 * (3 * (size_t)c->pme_nblk + 3)},
                     {&c->pme_base, 4 * 3 * (size_t)N},
-                    {&c->pme_w, es * 3 * (size_t)N * kMaxOrder},
+                    {&c->pme_w, 8 * 3 * (size_t)N * kMaxOrder},
                     {&c->pme_vpk, 6 * es * (size_t)N * ((nr + 1) / 2)},
                     {&c->rl_pos, 32 * (size_t)N}});
   if (s != BD_OK || (s = mesh_alloc(c)) != BD_OK || (s = real_alloc(c)) != BD_OK) return s;
@@ -361,14 +358,9 @@ int pme_prepare(bd_ctx* c, const Lat& l) {
   double rce = l.treal <= c->tp / 2 ? l.L2yp : 2.0 * l.L2yp;
   double alpha_ref = 4.0 / rce;
   c->launches += 3;
-  if (c->pme_f32)
-    k_pme_weights<float><<<nblk(N, 128), 128, 0, c->stream>>>(
-        cell, c->rx, c->ry, c->rz, cr, sr, N, K, c->pme_p, c->pme_base, (float*)c->pme_w,
-        (double4*)c->rl_pos, c->err);
-  else
-    k_pme_weights<double><<<nblk(N, 128), 128, 0, c->stream>>>(
-        cell, c->rx, c->ry, c->rz, cr, sr, N, K, c->pme_p, c->pme_base, (double*)c->pme_w,
-        (double4*)c->rl_pos, c->err);
+  k_pme_weights<<<nblk(N, 128), 128, 0, c->stream>>>(cell, c->rx, c->ry, c->rz, cr, sr, N, K,
+                                                     c->pme_p, c->pme_base, c->pme_w,
+                                                     (double4*)c->rl_pos, c->err);
   if ((s = mesh_prepare(c)) != BD_OK) return s;
   if (c->pme_f32)
     k_pme_influence<float><<<c->pme_nblk, 256, 0, c->stream>>>(
