@@ -601,7 +601,9 @@ __global__ void __launch_bounds__(32) k_gasdev_seq(Ran1* gs, double* R, int n) {
   __shared__ unsigned s_y[64];
   const int lane = threadIdx.x;
   int at = 0;
-  if (gs->idum <= 0) {  // the first call initialises the generator
+  const bool first = gs->idum <= 0;
+  __syncwarp();  // every lane has read it
+  if (first) {  // the first call initialises the generator
     if (lane == 0) {
       Ran1 g = *gs;
       for (; at < min(n, 2); at++) R[at] = (double)gasdev_dev(g);
