@@ -127,7 +127,7 @@ def test_single_vector_contexts_take_fp64_inputs():
 def test_memory_of_an_explicit_pair_cap(precision, block, most):
     """An entry of the cap costs a bead at most an index and its own pair's
     numbers (FP64 4 + 16 bytes; FP32 4 + 8, with blocks 4 + 8 + 16)."""
-    N, L = 4000, 60.0
+    N, L = 10000, 82.0  # four beads' caps stay below N
     pos = np.random.default_rng(5).uniform(-L / 2, L / 2, (3, N))
     used = []
     for cap in (1024, 2048):
@@ -159,3 +159,52 @@ def test_explicit_cap_grows_rows_of_four_beads():
         c.calc_hi()
         out.append(c.mobility_apply(v))
     assert np.array_equal(out[0], out[1])
+
+
+def _compact(Nb, Nc, spacing):
+    """Chains folded on a cubic lattice, consecutive beads on neighbouring sites."""
+    N = Nb * Nc
+    m = int(np.ceil(N ** (1 / 3)))
+    i = np.arange(N)
+    z, y, x = i // (m * m), i // m % m, i % m
+    y = np.where(z % 2, m - 1 - y, y)
+    x = np.where((i // m) % 2, m - 1 - x, x)
+    return [(a - (m - 1) / 2) * spacing for a in (x, y, z)]
+
+
+@pytest.mark.parametrize("precision,block", [("fp64", 1), ("fp32", 1), ("fp32", 4)])
+def test_rows_grow_between_the_steps_of_a_run(precision, block):
+    """A run whose chains have collapsed by the next mobility build: the rows grow,
+    and the captured iterations of the earlier steps are not used on them.  The
+    steps equal those of a run that starts there, but for where the Krylov runs
+    stop (tolerance 1e-6)."""
+    Nb, Nc, L = 50, 80, 60.0
+
+    def run():
+        c = B.Context(B.make_params(0, Nb, Nc, L, 0.01, 5e-4, mobility="pme", noise="philox",
+                                    precision=precision, noise_block=block, pme_rc=12.0,
+                                    philox_seed=3))
+        c.set_time(0, 0)
+        c.update_lattice(0)
+        return c
+
+    compact = _compact(Nb, Nc, 2.05)
+    moved = []
+    for collapsed in (False, True):
+        c = run()
+        if not collapsed:
+            c.set_positions(*B.random_chains(Nb, Nc, L, 4, bond=2.0, min_sep=1.9))
+            c.step_lanczos(0, 4, with_hop=False)
+            small = c.device_bytes()
+        else:
+            for _ in range(4):  # the draws of the other run's first steps
+                c.get_noise()
+        c.noise_block_release()
+        c.set_positions(*compact)
+        c.build_neighbors()  # positions set from outside: the lists are not told
+        c.step_lanczos(100, 4, with_hop=False)
+        moved.append(np.stack(c.positions()) - np.stack(compact))
+        if not collapsed:
+            assert c.device_bytes() > small  # the rows did grow
+        c.close()
+    assert rel_err(moved[0], moved[1]) < 1e-5
