@@ -452,10 +452,9 @@ __device__ __forceinline__ void copy_wait() {
 // way: with loads to registers, an entry ahead, too few bytes were in flight
 // to cover the latency of L2 and HBM (430 us at 50 000 beads, cutoff 14.5,
 // five pairs).  FP32: partial sums of about 16 entries folded into a second
-// set; lanes added in FP64.  Five pairs: 257 us at 50 000 beads, cutoff 14.5
-// (a warp per bead, every neighbour's values read once per bead: 435); at 8000
-// beads, cutoff 12.1, 38 us by one warp a group against 50.
-// SPLIT warps share a group's row.
+// set; lanes added in FP64.  Five pairs: 261 us at 50 000 beads, cutoff 14.5
+// (a warp per bead, every neighbour's values read once per bead: 435), 37 us at 8000
+// beads, cutoff 12.1 (50).  SPLIT warps share a group's row.
 template <int NP>
 struct Stage {
   static constexpr int S = 32 / NP, ITS = 32 / S, CH = S * ITS;  // entries a piece
@@ -761,8 +760,20 @@ const double4* group_order(const bd_ctx* c) {
   return (const double4*)(c->rl_gpos ? c->rl_gpos : c->rl_pos);
 }
 
-// Warps a group of a row of (t1, t2 / r^2).
-int few_warps(int ng) { return ng < 148 * 12 ? 4 : ng < 148 * 40 ? 2 : 1; }
+// Warps a group of four beads.  More of them fill the chip sooner, fewer start fewer
+// pieces.  Whole products by one, two and four, us.  FP32, whole tensors: ten
+// vectors, 500 beads 69, 63, 60, 8000 207, 201, 198, 12 000 312, 301, 301, 24 000 559,
+// 553, 557, 50 000 (chains of 100) 935, 935, 953; four vectors, 4000 96, 95, 95, 8000
+// 128, 126, 128, 50 000 468, 472, 493; one vector, 2000 61, 59, 59, 4000 75, 75, 77, 8000
+// 95, 93, 99, 16 000 142, 144, 154, 50 000 293, 302, 345.  FP64 sums: ten vectors, 8000
+// 352, 337, 335, 12 000 606, 584, 584, 50 000 1825, 1829, 1875; two vectors, 2000 81, 76,
+// 78, 24 000 273, 281, 304; one vector, 8000 120, 118, 120, 24 000 239, 239, 249, 50 000
+// 345, 349, 376.
+template <int NP, bool ONE>
+int warps_of(int ng) {
+  constexpr int four = 148 * (NP < 4 ? 4 : 4 * NP - 4), one = 148 * (NP == 1 && !ONE ? 24 : 40);
+  return ng < four ? 4 : ng < one ? 2 : 1;
+}
 
 template <int NP, bool ONE, typename R>
 void launch_sum(bd_ctx* c, int np, int p0, const Finish& fin) {
@@ -773,7 +784,7 @@ void launch_sum(bd_ctx* c, int np, int p0, const Finish& fin) {
       cell, (const double4*)c->rl_pos, group_order(c), c->rl_cnt, c->rl_rows,               \
       (const typename Real2<R>::T*)c->rl_w, c->rl_cap, fin.v, (const double2*)c->pme_vpk, np, \
       p0, c->N, ng, fin)
-  switch (few_warps(ng)) {
+  switch (warps_of<NP, ONE>(ng)) {
     case 4: SUM(4); break;
     case 2: SUM(2); break;
     default: SUM(1);
@@ -788,19 +799,11 @@ void launch_apply(bd_ctx* c, int np, int p0, const Finish& fin) {
   k_real_apply<NP, SPLIT_><<<nblk(ng, 4 / SPLIT_), 128, 0, c->stream>>>(                  \
       c->rl_cnt, c->rl_rows, (const float*)c->rl_w, c->rl_cap, (const float2*)c->pme_vpk, \
       np, p0, group_order(c), c->N, ng, fin)
-  // More warps a group fill the chip sooner, fewer start fewer pieces.  By four,
-  // two and one, five pairs FP32: 500 beads 6.1, 8.0, 12.6 us, 8000 41.8, 46.5, 63.7,
-  // 16 000 70, 74, 79; FP64 8000 85, 90, 107, 16 000 151, 147, 160; one pair FP32
-  // 8000 24.0, 20.9, 24.4, 16 000 45.5, 35.2, 34.5.  At 50 000 beads of a run's
-  // chains five pairs took 268 by four and 257 by one, one pair 118 by two and 114
-  // by one.
-  const int four = NP < 5 ? 148 * 12 : 148 * 40;
-  if (ng >= 148 * 40)
-    REAL(1);
-  else if (ng < four)
-    REAL(4);
-  else
-    REAL(2);
+  switch (warps_of<NP, false>(ng)) {
+    case 4: REAL(4); break;
+    case 2: REAL(2); break;
+    default: REAL(1);
+  }
 #undef REAL
 }
 

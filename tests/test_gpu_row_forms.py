@@ -57,7 +57,7 @@ def _check(N, Nb, precision, block):
 
 
 @FORMS
-@pytest.mark.parametrize("N", [2, 33, 7104, 7105, 23677])
+@pytest.mark.parametrize("N", [2, 33, 2364, 2365, 7104, 7105, 9469, 14205, 23677])
 def test_forms_match_model(N, precision, block):
     _check(N, N, precision, block)
 
