@@ -41,12 +41,15 @@ static const int kDotBlocks = 148;  // one CTA per SM for the vector reductions
 static const int kOrthShort = 6144;
 
 // CTAs per vector of the orthogonalisation: at most `most`, none with fewer
-// than 256 entries down to 8 CTAs.  Every CTA sums all CTAs' partials, one set
-// per basis vector, so more of them only add reads: with 148 CTAs instead of 12
-// the square root of 1024 beads by these kernels took 3.48 ms, not 3.43; from
-// 38 000 entries on the rule changes nothing.
-static int orth_chunks(size_t n, int most) {
-  return std::min(most, std::max(8, (int)(n / 256)));
+// than `least` entries down to 8 CTAs.  Every CTA sums all CTAs' partials, one set
+// per basis vector, so more of them only add reads; fewer leave multiprocessors
+// idle.  Single solves of 2500, 4000, 8000 and 12 000 beads FP32 (60 to 88 vectors)
+// with at least 64, 128, 192 and 256 entries: 5.08, 5.10, 5.07, 5.25 ms; 6.67, 6.79,
+// 6.74, 7.01; 9.92, 9.91, 9.78, 10.37; 14.2, 14.2, 14.2, 14.5.  Blocks of ten, whose
+// vectors fill the chip together, 2500 beads: 8.94, 8.94, 8.91, 8.85 ms for ten
+// steps, the same from 4000 on.
+static int orth_chunks(size_t n, int most, int least) {
+  return std::min(most, std::max(8, (int)(n / least)));
 }
 
 // Fixed-order sum of n partials by one warp: lane-strided sums, then a
@@ -986,7 +989,7 @@ static int lanczos_iteration(bd_ctx* c, bool pre, bool force) {
   q.kst = 1;
   q.jd = c->Ljd;
   q.n = n;
-  orth_step(c, q, orth_chunks(n, blk), 1, c->Ljd);
+  orth_step(c, q, orth_chunks(n, blk, 192), 1, c->Ljd);
   return launch_ok(c);
 }
 
@@ -1213,7 +1216,7 @@ void noise_blocks_release(bd_ctx* c) {
 
 // Chunks per right-hand side of the block orthogonalisation kernels.
 static int block_chunks(size_t n, int k) {
-  return orth_chunks(n, std::min(kDotBlocks, std::max(8, 4 * kDotBlocks / k)));
+  return orth_chunks(n, std::min(kDotBlocks, std::max(8, 4 * kDotBlocks / k)), 256);
 }
 
 // Layout of a block of k right-hand sides: basis vector j of r at
