@@ -212,8 +212,15 @@ __device__ __forceinline__ void madd(double w, float2 x, double2& a) {
   a.x = fma(w, (double)x.x, a.x);
   a.y = fma(w, (double)x.y, a.y);
 }
-__device__ __forceinline__ float2 weight(float x) { return make_float2(x, x); }
-__device__ __forceinline__ double weight(double x) { return x; }
+__device__ __forceinline__ void madd(double w, float x, double& a) { a = fma(w, (double)x, a); }
+// a weight as the sums of V take it
+template <typename V, typename R>
+__device__ __forceinline__ auto weight(R x) {
+  if constexpr (std::is_same_v<V, float2>)
+    return make_float2(x, x);
+  else
+    return x;
+}
 __device__ __forceinline__ void put(float2& w, float x) { w = make_float2(x, x); }
 __device__ __forceinline__ void put(float& w, float x) { w = x; }
 __device__ __forceinline__ void put(double& w, double x) { w = x; }
@@ -246,7 +253,8 @@ template <int P, typename R, int NG, int CY, int CZ, bool ONE>
 struct RecData {
   std::conditional_t<ONE, R, typename GridVal<R>::W> wx[P];
   std::conditional_t<ONE, R, typename GridVal<R>::T> f[NG][3];
-  R wyz[CY * CZ];
+  double wy[NG == 1 ? CY : 1], wz[NG == 1 ? CZ : 1];
+  R wyz[NG == 1 ? 1 : CY * CZ];
   int at;
 };
 template <typename S>
@@ -346,8 +354,16 @@ __global__ void __launch_bounds__(32, sizeof(R) == 4 ? 16 : 8)
       int d = b1 - (y0 + q);
       d += d < 0 ? K : 0;
       const double wy = d < P && y0 + q < K ? w[kMaxOrder + d] : 0.0;
+      if constexpr (NG == 1) {
+        r.wy[q] = wy;
+      } else {
 #pragma unroll
-      for (int e = 0; e < CZ; e++) r.wyz[q * CZ + e] = (R)(wy * wz[e]);
+        for (int e = 0; e < CZ; e++) r.wyz[q * CZ + e] = (R)(wy * wz[e]);
+      }
+    }
+    if constexpr (NG == 1) {
+#pragma unroll
+      for (int e = 0; e < CZ; e++) r.wz[e] = wz[e];
     }
 #pragma unroll
     for (int u = 0; u < NG; u++) {
@@ -369,7 +385,11 @@ __global__ void __launch_bounds__(32, sizeof(R) == 4 ? 16 : 8)
 #pragma unroll 1
     for (int u = 0; u < nb; u++) {
       const S& q = s_rec[u];
-      const R wyz = q.wyz[ly * CZ + lz];
+      R wyz;
+      if constexpr (NG == 1)
+        wyz = (R)(q.wy[ly] * q.wz[lz]);
+      else
+        wyz = q.wyz[ly * CZ + lz];
       V t[3];
 #pragma unroll
       for (int c = 0; c < 3; c++) t[c] = scaled(wyz, q.f[g][c]);
@@ -400,7 +420,10 @@ __global__ void __launch_bounds__(32, sizeof(R) == 4 ? 16 : 8)
 // systems of 900 to 32 000 beads, ten vectors: 1.34e-7, 1.33e-7 by those last two
 // (1.89e-7 by atomics, cuFFT and FP64 sums of every term, 1.40e-7 with FP32 weights
 // and lanes).
-enum Layout { kInterleaved, kPlanar, kReal };
+// A single right-hand side's values are real: they fill planar real grids (kReal) or
+// are the real parts of an interleaved one (kSingle; with the zero imaginary parts an
+// iteration of a 4000-bead solve on 64^3 FP64 took 120.7 us, 114.0 without).
+enum Layout { kInterleaved, kSingle, kPlanar, kReal };
 
 template <int P, typename R, Layout LAY>
 __global__ void __launch_bounds__(256)
@@ -414,25 +437,21 @@ __global__ void __launch_bounds__(256)
   const double* w2 = w1 + kMaxOrder;
   const int b0 = base[3 * i], b1 = base[3 * i + 1], b2 = base[3 * i + 2];
   const size_t K2 = (size_t)K * K;
-  constexpr int ps = LAY == kInterleaved ? 3 : 1;
-  const size_t cs = LAY == kInterleaved ? 1 : K2 * K;
-  using E = std::conditional_t<LAY == kReal, R, T>;
-  const E* gp = (const E*)grid + (size_t)pr * 3 * K2 * K;
-  auto value = [](E x) {
-    if constexpr (LAY == kReal)
-      return as_pair(x);
-    else
-      return x;
-  };
-  double2 s[3];
+  constexpr bool RE = LAY == kSingle || LAY == kReal, INTER = LAY == kInterleaved || LAY == kSingle;
+  constexpr int ps = INTER ? 3 : 1, es = LAY == kSingle ? 2 : 1;
+  const size_t cs = INTER ? 1 : K2 * K;
+  using V = std::conditional_t<RE, R, T>;
+  using S = std::conditional_t<RE, double, double2>;
+  const V* gp = (const V*)grid + (size_t)pr * 3 * K2 * K;  // pair 0 where RE
+  S s[3];
 #pragma unroll
   for (int j = 0; j < 3; j++) zero(s[j]);
-  constexpr bool own_sums = P == 8 && LAY != kInterleaved;  // component c in sum c
+  constexpr bool own_sums = P == 8 && !INTER;  // component c in sum c
   if constexpr (own_sums) {
     // four rows of one component a load
     unsigned off[2];
     double wyz[2];
-    T u[2][3];
+    V u[2][3];
     int gz = b2 - (P - 1) + lane % 8;
     gz += gz < 0 ? K : 0;
 #pragma unroll
@@ -448,12 +467,12 @@ __global__ void __launch_bounds__(256)
     for (int a = 0; a < P; a++) {
       int gx = b0 - a;
       gx += gx < 0 ? K : 0;
-      const E* gl = gp + K2 * (size_t)gx;
-      const auto wx = weight((R)w0[a]);
+      const V* gl = gp + K2 * (size_t)gx;
+      const auto wx = weight<V>((R)w0[a]);
 #pragma unroll
       for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int j = 0; j < 3; j++) madd(wx, value(gl[off[h] + (size_t)j * cs]), u[h][j]);
+        for (int j = 0; j < 3; j++) madd(wx, gl[off[h] + (size_t)j * cs], u[h][j]);
     }
 #pragma unroll
     for (int h = 0; h < 2; h++)
@@ -464,7 +483,7 @@ __global__ void __launch_bounds__(256)
     // point and its offset within (y, z) depend on q only by its parity
     int off[3][2];
     double wyz[3][2];
-    T u[3][2];
+    V u[3][2];
 #pragma unroll
     for (int j = 0; j < 3; j++) {
       const int f = 32 * j + lane, ro = f / 24, z = f % 24 / 3;
@@ -483,12 +502,12 @@ __global__ void __launch_bounds__(256)
     for (int a = 0; a < P; a++) {
       int gx = b0 - a;
       gx += gx < 0 ? K : 0;
-      const T* gl = gp + 3 * K2 * (size_t)gx;
-      const auto wx = weight((R)w0[a]);
+      const V* gl = gp + es * 3 * K2 * (size_t)gx;
+      const auto wx = weight<V>((R)w0[a]);
 #pragma unroll
       for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int j = 0; j < 3; j++) madd(wx, gl[off[j][h]], u[j][h]);
+        for (int j = 0; j < 3; j++) madd(wx, gl[es * off[j][h]], u[j][h]);
     }
 #pragma unroll
     for (int h = 0; h < 2; h++)
@@ -507,27 +526,36 @@ __global__ void __launch_bounds__(256)
         gy += gy < 0 ? K : 0;
         gz += gz < 0 ? K : 0;
         madd(w0[a] * w1[b] * w2[P - 1 - z],
-             value(gp[ps * ((size_t)gx * K2 + (size_t)gy * K + gz) + (f % 3) * cs]), s[j]);
+             gp[es * (ps * ((size_t)gx * K2 + (size_t)gy * K + gz) + (f % 3) * cs)], s[j]);
       }
     }
   }
   // component c is in sum 2 (c - lane) mod 3
   const int r = own_sums ? -1 : lane % 3;
-  const double2 c0 = r <= 0 ? s[0] : r == 1 ? s[1] : s[2];
-  const double2 c1 = r < 0 ? s[1] : r == 0 ? s[2] : r == 1 ? s[0] : s[1];
-  const double2 c2 = r < 0 ? s[2] : r == 0 ? s[1] : r == 1 ? s[2] : s[0];
-  // real parts to the lower, imaginary parts to the upper half of the warp
-  const bool up = lane & 16;
-  double x[3] = {up ? c0.y : c0.x, up ? c1.y : c1.x, up ? c2.y : c2.x};
-  const double y[3] = {up ? c0.x : c0.y, up ? c1.x : c1.y, up ? c2.x : c2.y};
+  const S c0 = r <= 0 ? s[0] : r == 1 ? s[1] : s[2];
+  const S c1 = r < 0 ? s[1] : r == 0 ? s[2] : r == 1 ? s[0] : s[1];
+  const S c2 = r < 0 ? s[2] : r == 0 ? s[1] : r == 1 ? s[2] : s[0];
+  if constexpr (RE) {
+    double x[3] = {c0, c1, c2};
 #pragma unroll
-  for (int c = 0; c < 3; c++) {
-    x[c] += __shfl_xor_sync(0xffffffffu, y[c], 16);
+    for (int c = 0; c < 3; c++)
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) x[c] += __shfl_xor_sync(0xffffffffu, x[c], o);
+      for (int o = 16; o > 0; o >>= 1) x[c] += __shfl_xor_sync(0xffffffffu, x[c], o);
+    if (lane < 3) val[(size_t)i * 6 + lane] = lane == 0 ? x[0] : lane == 1 ? x[1] : x[2];
+  } else {
+    // real parts to the lower, imaginary parts to the upper half of the warp
+    const bool up = lane & 16;
+    double x[3] = {up ? c0.y : c0.x, up ? c1.y : c1.x, up ? c2.y : c2.x};
+    const double y[3] = {up ? c0.x : c0.y, up ? c1.x : c1.y, up ? c2.x : c2.y};
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      x[c] += __shfl_xor_sync(0xffffffffu, y[c], 16);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) x[c] += __shfl_xor_sync(0xffffffffu, x[c], o);
+    }
+    const int e = lane & 15;
+    if (e < 3) val[((size_t)pr * N + i) * 6 + (up ? 3 : 0) + e] = e == 0 ? x[0] : e == 1 ? x[1] : x[2];
   }
-  const int e = lane & 15;
-  if (e < 3) val[((size_t)pr * N + i) * 6 + (up ? 3 : 0) + e] = e == 0 ? x[0] : e == 1 ? x[1] : x[2];
 }
 
 // ---------------------------------------------------------------------------
@@ -639,6 +667,8 @@ void launch_gather(bd_ctx* c, int k, const R* grid) {
     GATHER(kReal);
   else if (c->pme_planar)
     GATHER(kPlanar);
+  else if (k == 1)
+    GATHER(kSingle);
   else
     GATHER(kInterleaved);
 #undef GATHER
