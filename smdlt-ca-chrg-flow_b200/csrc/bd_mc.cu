@@ -469,8 +469,9 @@ int charge_hop(bd_ctx* c) {
 // wide (R = hop_radius, default 3 Debye lengths), with an even number of
 // cells per direction; the parity of the three cell indices gives eight
 // colours, and cells of one colour are at least R apart.  A sweep runs the
-// eight colours in turn; within a colour every cell is one CTA that visits its
-// charges in index order, each exactly once.  A trial follows the reference's
+// eight colours in turn; within a colour the trials' energies against the charges at
+// the colour's start are formed at once, and a warp per cell then visits its charges
+// in index order, each exactly once.  A trial follows the reference's
 // proposal rules (partner search, chain ends, occupancy, the two barriers) and
 // accepts with min(1, exp(-barrier - dE/2)) (the reference's factor, without
 // its stale starting energy), dE the energy change of the move against every

@@ -575,9 +575,11 @@ double layout_cost(int np, int ng, int P) {
 // 1425 and 1464; 100^3 8000 beads 408 and 420, 16 000 502 and 485, 50 000 1010 and 937.
 // FP64: 144^3 8000 beads 1720 and 1873, 32 000 2252 and 2276, 50 000 2705 and 2618;
 // 100^3 8000 beads 752 and 742.
+// On 64^3 and below, 500 FP32 beads on 32^3 for one, five pairs a warp are faster at
+// any density (10.7 us and 14.7).
 bool sparse(const bd_ctx* c) {
   const size_t K = c->pmeK;
-  return (size_t)c->N * (c->pme_f32 ? 64 : 128) < K * K * K;
+  return K >= 90 && (size_t)c->N * (c->pme_f32 ? 64 : 128) < K * K * K;
 }
 
 // Segments of a column: about 14 warps on every SM (16 fit), none shorter than

@@ -14,9 +14,10 @@
 //    (the coefficient of shear/src/main26.c:1622), evaluated by smooth PME
 //    (Essmann et al., J. Chem. Phys. 103, 8577 (1995)) on the deforming
 //    cell: fractional coordinates s = H^-1 r, cardinal B-splines of even
-//    order p on a K^3 grid, three-component R2C FFT, multiplication by
-//    (phi/V)(I - k k^T/k^2) |b1 b2 b3|^2 with k = 2 pi H^-T m, C2R FFT and
-//    interpolation with the same weights.
+//    order p on a K^3 grid, three-component transforms (complex ones of two
+//    right-hand sides at a time, or real ones of a single one), between them
+//    multiplication by (phi/V)(I - k k^T/k^2) |b1 b2 b3|^2 with k = 2 pi H^-T m,
+//    and interpolation with the same weights.
 // The periodic lattice is described by its Gauss-reduced basis (shortest
 // vectors of the lattice spanned by L1, L2 and L e_z): the lattice sums do
 // not depend on the basis, and the reduced one keeps the grid spacing and the
