@@ -206,6 +206,7 @@ struct bd_ctx {
   int pme_nblk;      // blocks of the influence kernel
   int *pme_base;     // per bead base grid index, 3 x N
   double *pme_w;     // per bead spline weights, 3 x N x 8
+  float *pme_wx;     // FP32 grids: the first direction's rounded, N x 8
   // grid sizes bd_fft.cuh does not cover: components one after the other; 1 + cuFFT
   // plan of a single right-hand side (real, forward and back), its half spectrum,
   // and of up to four numbers of pairs (0: none)

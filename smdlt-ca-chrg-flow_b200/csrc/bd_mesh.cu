@@ -21,16 +21,16 @@
 // Bound by the FP32 (FP64) pipe and the issue of its instructions: 48 (P = 8)
 // multiply-adds per lane and bead, two at a time (fma.rn.f32x2) in FP32, next
 // to about 20 others.
-// Five pairs, order 8: 163 us at 50 000 beads on 100^3 (one complex L2 atomic
-// per stencil point, component and pair took about 400), 43 us at 8000 beads on
+// Five pairs, order 8: 153 us at 50 000 beads on 100^3 (one complex L2 atomic
+// per stencil point, component and pair took about 400), 41 us at 8000 beads on
 // 64^3 (74); FP64 66 us there (385).
 //
 // Interpolation: a warp per bead and pair reads the stencil's 64 rows of 24
 // complex values (192 contiguous bytes, FP32), a lane the same third of a row
 // position throughout, so its y and z weights and addresses stay in registers.
 // Bound by L1 throughput.
-// Five pairs, order 8: 253 us at 50 000 beads on 100^3 (separate component
-// grids, 64 bytes a row: about 300), 42 us at 8000 beads on 64^3 (54); FP64 70 us
+// Five pairs, order 8: 245 us at 50 000 beads on 100^3 (separate component
+// grids, 64 bytes a row: about 300), 39 us at 8000 beads on 64^3 (54); FP64 70 us
 // there.
 //
 // The columns' lists are built once per mobility build (the positions are
@@ -263,9 +263,20 @@ struct alignas(16) Rec : S {
   char fill[16 * (words + (words % 2 == 0 ? 1 : 0)) - sizeof(S)];
 };
 
+// The weights along x in the grid's type: FP32 ones are kept beside the FP64 ones
+// (converted by every warp that meets the bead, spreading and interpolation of the five
+// pairs above took 163 and 253 us).
+__device__ __forceinline__ const float* level_weights(const float* wx, const double*, int i) {
+  return wx + (size_t)i * kMaxOrder;
+}
+__device__ __forceinline__ const double* level_weights(const double*, const double* w, int i) {
+  return w + (size_t)i * 3 * kMaxOrder;
+}
+
 struct SpreadArgs {
   const int* base;
   const double* w;  // 8 weights per bead and direction
+  const void* wx;   // the first direction's in the grid's type
   const int* ent;
   const int* bin;
   int K, npz, npatch, nseg, nset, np, N;
@@ -338,10 +349,11 @@ __global__ void __launch_bounds__(32, sizeof(R) == 4 ? 16 : 8)
     if (t >= n) return;
     S& r = s_rec[lane];
     const double* w = m.w + (size_t)i * 3 * kMaxOrder;
+    const R* wx = level_weights((const R*)m.wx, m.w, i);
     const int b1 = m.base[3 * i + 1], b2 = m.base[3 * i + 2];
     r.at = m.base[3 * i] + (t < n0 ? 0 : K);
 #pragma unroll
-    for (int a = 0; a < P; a++) put(r.wx[a], (R)w[P - 1 - a]);
+    for (int a = 0; a < P; a++) put(r.wx[a], wx[P - 1 - a]);
     double wz[CZ];
 #pragma unroll
     for (int q = 0; q < CZ; q++) {
@@ -414,7 +426,7 @@ __global__ void __launch_bounds__(32, sizeof(R) == 4 ? 16 : 8)
 // 96 values are a whole number of points, so load t of a lane always holds
 // component (2 t + lane) mod 3: one sum for each t mod 3, put in component
 // order at the end.  Order 8 takes a lane's sums along x (8 levels) in the grid's
-// type and the rest in FP64: 253 us for the five pairs above, 404 with every FP32
+// type and the rest in FP64: 245 us for the five pairs above, 404 with every FP32
 // value converted (four a clock and quarter of an SM), 448 with FP32 sums that keep
 // what they round away.  The product's error against FP64, geometric mean of 12
 // systems of 900 to 32 000 beads, ten vectors: 1.34e-7, 1.33e-7 by those last two
@@ -428,6 +440,7 @@ enum Layout { kInterleaved, kSingle, kPlanar, kReal };
 template <int P, typename R, Layout LAY>
 __global__ void __launch_bounds__(256)
     k_mesh_gather(const int* __restrict__ base, const double* __restrict__ w,
+                  const R* __restrict__ wxs,
                   const R* __restrict__ grid, int N, int K, double* __restrict__ val) {
   using T = typename GridVal<R>::T;
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, pr = blockIdx.y;
@@ -435,6 +448,7 @@ __global__ void __launch_bounds__(256)
   const double* w0 = w + (size_t)i * 3 * kMaxOrder;
   const double* w1 = w0 + kMaxOrder;
   const double* w2 = w1 + kMaxOrder;
+  const R* wl = level_weights(wxs, w, i);
   const int b0 = base[3 * i], b1 = base[3 * i + 1], b2 = base[3 * i + 2];
   const size_t K2 = (size_t)K * K;
   constexpr bool RE = LAY == kSingle || LAY == kReal, INTER = LAY == kInterleaved || LAY == kSingle;
@@ -468,7 +482,7 @@ __global__ void __launch_bounds__(256)
       int gx = b0 - a;
       gx += gx < 0 ? K : 0;
       const V* gl = gp + K2 * (size_t)gx;
-      const auto wx = weight<V>((R)w0[a]);
+      const auto wx = weight<V>(wl[a]);
 #pragma unroll
       for (int h = 0; h < 2; h++)
 #pragma unroll
@@ -503,16 +517,23 @@ __global__ void __launch_bounds__(256)
       int gx = b0 - a;
       gx += gx < 0 ? K : 0;
       const V* gl = gp + es * 3 * K2 * (size_t)gx;
-      const auto wx = weight<V>((R)w0[a]);
+      const auto wx = weight<V>(wl[a]);
 #pragma unroll
       for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int j = 0; j < 3; j++) madd(wx, gl[es * off[j][h]], u[j][h]);
+        for (int j = 0; j < 3; j++) {
+          if constexpr (sizeof(R) == 4)
+            madd(wx, gl[es * off[j][h]], u[j][h]);
+          else  // fewer sums to hold: 4000 beads 10.6 us a pair, not 14.2
+            madd(wx * wyz[j][h], gl[es * off[j][h]], s[j]);
+        }
     }
+    if constexpr (sizeof(R) == 4) {
 #pragma unroll
-    for (int h = 0; h < 2; h++)
+      for (int h = 0; h < 2; h++)
 #pragma unroll
-      for (int j = 0; j < 3; j++) madd(wyz[j][h], u[j][h], s[j]);
+        for (int j = 0; j < 3; j++) madd(wyz[j][h], u[j][h], s[j]);
+    }
   } else {
 #pragma unroll 1
     for (int t0 = 0; 32 * t0 < 3 * P * P * P; t0 += 3) {
@@ -633,6 +654,7 @@ int spread_t(bd_ctx* c, int k, const VecIn& v, size_t vr, R* grid) {
   SpreadArgs m;
   m.base = c->pme_base;
   m.w = c->pme_w;
+  m.wx = c->pme_wx;
   m.ent = c->mesh_ent[l];
   m.bin = c->mesh_bin[l];
   m.K = K;
@@ -663,7 +685,7 @@ template <int P, typename R>
 void launch_gather(bd_ctx* c, int k, const R* grid) {
   const dim3 g(nblk(c->N, 8), (k + 1) / 2);
 #define GATHER(LAY_)                                                                      \
-  k_mesh_gather<P, R, LAY_><<<g, 256, 0, c->stream>>>(c->pme_base, c->pme_w, grid, c->N, c->pmeK, \
+  k_mesh_gather<P, R, LAY_><<<g, 256, 0, c->stream>>>(c->pme_base, c->pme_w, (const R*)c->pme_wx, grid, c->N, c->pmeK, \
                                                       c->mesh_val)
   if (k == 1 && c->pme_real1)
     GATHER(kReal);

@@ -57,11 +57,13 @@ using namespace bd;
 // direction (u = K s, s wrapped into [0,1)).  Positions held in the rotated
 // frame are taken to the lab frame with (cr, sr) = (cos, sin) of the lattice
 // angle, x = x' cr - y' sr, y = x' sr + y' cr (inverseCoords,
-// extensional/src/main14.c:1525-1535); lab-frame positions pass (1, 0).  pos
-// gets the lab-frame position with the index in its fourth component.
+// extensional/src/main14.c:1525-1535); lab-frame positions pass (1, 0).  wx (FP32
+// grids) gets the weights along the first direction rounded, pos the lab-frame
+// position with the index in its fourth component.
 __global__ void k_pme_weights(Cell cell, const double* __restrict__ rx,
                               const double* __restrict__ ry, const double* __restrict__ rz,
                               double cr, double sr, int N, int K, int p, int* base, double* w,
+                              float* wx,
                               double4* pos, int* err) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -80,7 +82,10 @@ __global__ void k_pme_weights(Cell cell, const double* __restrict__ rx,
     double f = u - fl;
     if (fl >= K) fl -= K;
     base[3 * i + d] = fl;
-    bspline(f, p, w + ((size_t)3 * i + d) * kMaxOrder);
+    double* wd = w + ((size_t)3 * i + d) * kMaxOrder;
+    bspline(f, p, wd);
+    if (wx && d == 0)
+      for (int k = 0; k < p; k++) wx[(size_t)i * kMaxOrder + k] = (float)wd[k];
   }
 }
 
@@ -287,6 +292,7 @@ static int pme_parts(bd_ctx* c) {
                     {&c->pme_w, 8 * 3 * (size_t)N * kMaxOrder},
                     {&c->pme_vpk, 6 * es * (size_t)N * ((nr + 1) / 2)},
                     {&c->rl_pos, 32 * (size_t)N}});
+  if (s == BD_OK && c->pme_f32) s = alloc_all(c, {{&c->pme_wx, 4 * (size_t)N * kMaxOrder}});
   if (s != BD_OK || (s = mesh_alloc(c)) != BD_OK || (s = real_alloc(c)) != BD_OK) return s;
   if (c->pme_real1) {
     c->pme_spec = (char*)c->pme_grid + real_bytes;
@@ -323,7 +329,7 @@ void pme_free(bd_ctx* c) {
   mesh_free(c);
   real_free(c);
   free_all({&c->pme_vpk, &c->pme_grid, &c->pme_tw, &c->pme_infl, &c->pme_bsq, &c->pme_soff,
-            &c->pme_base, &c->pme_w, &c->rl_pos});
+            &c->pme_base, &c->pme_w, &c->pme_wx, &c->rl_pos});
 }
 
 // The mobility's buffers and plan, all or none (pme_grid tells).
@@ -360,7 +366,7 @@ int pme_prepare(bd_ctx* c, const Lat& l) {
   double alpha_ref = 4.0 / rce;
   c->launches += 3;
   k_pme_weights<<<nblk(N, 128), 128, 0, c->stream>>>(cell, c->rx, c->ry, c->rz, cr, sr, N, K,
-                                                     c->pme_p, c->pme_base, c->pme_w,
+                                                     c->pme_p, c->pme_base, c->pme_w, c->pme_wx,
                                                      (double4*)c->rl_pos, c->err);
   if ((s = mesh_prepare(c)) != BD_OK) return s;
   if (c->pme_f32)
