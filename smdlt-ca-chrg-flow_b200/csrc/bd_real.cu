@@ -480,6 +480,8 @@ __global__ void __launch_bounds__(128, 4)
   const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = blockIdx.x * (4 / SPLIT) + wl / SPLIT, piece0 = wl % SPLIT;
   const int slot = lane / NP, pr = lane % NP;  // slot S and up: idle lanes
+  __shared__ int s_bead[4][kGroup];  // the group's beads, for the results
+  if (lane < kGroup) s_bead[wl][lane] = bead_of(gpos[min(kGroup * grp + lane, N - 1)]);
   V sum[2][6], part[2][6];  // beads (0, 1), (2, 3); values 3 h + c
 #pragma unroll
   for (int b = 0; b < 2; b++)
@@ -573,7 +575,7 @@ __global__ void __launch_bounds__(128, 4)
   for (int e = lane + 32 * piece0; e < 6 * kGroup * NP; e += 32 * SPLIT) {
     const int b = e / (6 * NP), p = e / 6 % NP, at = kGroup * grp + b;
     if (at >= N) break;
-    const int i = bead_of(gpos[at]);
+    const int i = s_bead[wl][b];
     double s = 0;
     for (int w = w0; w < w0 + SPLIT; w++)
       for (int u = 0; u < S; u++) s += (double)sh.sum[w][(u * NP + p) * W + 6 * b + e % 6];
@@ -622,6 +624,8 @@ __global__ void __launch_bounds__(128, ONE ? 4 : 2)
   const int grp = blockIdx.x * (4 / SPLIT) + wl / SPLIT, piece0 = wl % SPLIT;
   const int slot = lane / NP, pr = lane % NP;  // slot S and up: idle lanes
   const int i0 = kGroup * grp;
+  __shared__ int s_bead[4][kGroup];  // the group's beads, for the results
+  if (lane < kGroup) s_bead[wl][lane] = bead_of(gpos[min(i0 + lane, N - 1)]);
   double sum[kGroup][NS];
 #pragma unroll
   for (int b = 0; b < kGroup; b++)
@@ -747,7 +751,7 @@ __global__ void __launch_bounds__(128, ONE ? 4 : 2)
   for (int e = lane + 32 * piece0; e < NS * kGroup * NP; e += 32 * SPLIT) {
     const int b = e / (NS * NP), p = e / NS % NP;
     if (i0 + b >= N) break;
-    const int i = bead_of(gpos[i0 + b]);
+    const int i = s_bead[wl][b];
     double s = 0;
     for (int w = w0; w < w0 + SPLIT; w++)
       for (int u = 0; u < S; u++) s += sh.sum[w][(u * NP + p) * W + NS * b + e % NS];
