@@ -416,10 +416,10 @@ def build_context(w, seed, path="lanczos32", device_noise="philox", noise_seed=N
     return c
 
 
-# DRAM bytes (read + write, cold cache) of one block product, summed over its
-# kernels; keyed by (beads, grid, cutoff, right-hand sides per product).  None
-# measured for the kernels that run now
-PRODUCT_TRAFFIC = {}
+# DRAM bytes (read + write) of one block product, summed over its kernels as they
+# follow one another (profiles/product_50k.md); keyed by (beads, grid, cutoff,
+# right-hand sides per product)
+PRODUCT_TRAFFIC = {(50000, 100, 14.5, 10): 2.031e9}
 
 
 def ranks_max(values, dist):
