@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 import bd_b200 as B
+import oracle as O
 import pme_oracle as P
 from conftest import rel_err
 
@@ -53,3 +54,38 @@ def test_layouts_at_the_density_rule(N, precision):
     c, tol = _context(pos, 30, 8, precision, 5)
     got = c.mobility_apply_block(V)
     assert max(rel_err(got[r], ref[r]) for r in range(5)) < tol
+
+
+@functools.lru_cache(maxsize=None)
+def _sheared(N, K, t):
+    """Positions in a sheared cell, a vector and its product."""
+    edge = (N / 0.02) ** (1 / 3)
+    r = np.random.default_rng(N)
+    x, y, z = (np.ascontiguousarray(v) for v in r.uniform(-edge / 2, edge / 2, (3, N)))
+    o = O.Oracle(0, 20, N // 20, edge, 0.2, 5e-4)
+    o.lattice(t)
+    o.apply_pbc(x, y, z)
+    v = r.normal(size=(N, 3))
+    ref = P.pme_apply(P.reduced_cell(list(o.s.L1), list(o.s.L2), edge), np.stack([x, y, z], 1), v,
+                      K, 8, 0.3, 6.0, alpha_ref=P.ref_alpha(t, o.s.tp, o.s.L2yp))
+    return edge, (x, y, z), v.reshape(-1), ref.reshape(-1)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("N,K", [(14000, 96), (60, 100)])
+def test_columns_in_one_segment(N, K, precision):
+    """Enough columns to fill the chip: each is walked whole, from the wrapped bases
+    below its first level to the last; five pairs a warp (14 000 beads) and one."""
+    t = 2000
+    edge, pos, v, ref = _sheared(N, K, t)
+    c = B.Context(B.make_params(0, 20, N // 20, edge, 0.2, 5e-4, mobility="pme", noise="philox",
+                                precision=precision, pme_grid=K, pme_rc=6.0, pme_alpha=0.3,
+                                noise_block=10))
+    c.set_positions(*pos)
+    c.set_time(t, t)
+    c.update_lattice(t)
+    c.calc_hi()
+    factors = np.array([1.0, -2.0, 3.0, 0.5, -1.25, 0.75, 2.5, -0.375, 1.5, -0.6])
+    got = c.mobility_apply_block(factors[:, None] * v)
+    tol = 1e-11 if precision == "fp64" else 2e-6
+    assert max(rel_err(got[r], f * ref) for r, f in enumerate(factors)) < tol
