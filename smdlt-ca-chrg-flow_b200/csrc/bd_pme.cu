@@ -390,8 +390,8 @@ int pme_prepare(bd_ctx* c, const Lat& l) {
 // right-hand sides by real transforms, packed pairs all at once in place.
 // The grids hold their components one after the other: interleaved ones (element
 // stride 3) cost cuFFT more than the transforms themselves.  30 000 beads on 125^3,
-// ten vectors FP32, one FP32, one FP64: 1351, 231, 306 us; interleaved, a pair at a
-// time and complex throughout 1767, 376, 603.  150 000 on 216^3: 6790, 936, 1369;
+// ten vectors FP32, one FP32, one FP64: 1263, 226, 304 us; interleaved, a pair at a
+// time and complex throughout 1767, 376, 603.  150 000 on 216^3: 5637, 951, 1377;
 // 10400, 2100, 4080.
 template <typename R, typename Cx>
 static int cufft_influence(bd_ctx* c, int k) {
